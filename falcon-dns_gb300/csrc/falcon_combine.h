@@ -1,9 +1,7 @@
-// Recombination of exact integer-slice sums into one FP64 value, and the
-// fixed-point conversions of the tensor-core DFT stages, with integer
-// instructions only (GB300's FP64 pipe issues ~2 instructions per clock
-// per SM, so one FP64 add per output of a tensor-core contraction or DFT
-// stage costs as much as the rest of its epilogue).  Host and device: the
-// CPU tests compile this header with g++ and check it bit for bit.
+// Recombination of exact integer-slice sums into one FP64 value and
+// fixed-point conversions, with integer instructions only (GB300's FP64 pipe
+// issues ~2 instructions per clock per SM).  Host and device: the CPU tests
+// compile this header with g++ and check it bit for bit.
 #pragma once
 #include <math.h>
 #include <stdint.h>
@@ -99,8 +97,8 @@ FALCON_HD long long bits_of_double(double a) {
 
 // a 2^(FB - e) truncated toward zero, as a signed integer, for |a| < 2^e
 // (so below 2^FB in magnitude; FB <= 62); zero and subnormal a give 0.
-// The fixed-point form of the DFT stages: every value of a butterfly at
-// the scale of its largest, so sums and differences are exact integer adds.
+// With every value at the scale of the largest, sums and differences are
+// exact integer adds.
 template <int FB>
 FALCON_HD long long fix_of(double a, int e) {
   const long long bits = bits_of_double(a);

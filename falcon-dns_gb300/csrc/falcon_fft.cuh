@@ -1,21 +1,16 @@
 // The azimuthal transforms and the nonlinear pass (Nr_maxLOOP,
-// src/nonlin.F90:35-91): complex helpers, the odd-prime DFT coefficient
-// tables, the FMA and tensor-core butterfly stages, the warp-per-line and
-// block-per-line kernels and their launchers.  Included by one translation
-// unit per largest radix class (falcon_fft7.cu, falcon_fft17.cu,
-// falcon_fft31.cu), which compile in parallel; everything here has internal
-// linkage, so each unit holds its own coefficient tables in constant memory
-// (filled by init_dft_tables, falcon_kernels.cu, through each unit's
-// init_dft_tables_<MAXP>).
+// src/nonlin.F90:35-91) in 64-bit fixed point (falcon_fixed.h): the
+// butterfly stages on integer instructions and, for radices 11 to 31 of
+// prime-factor plans, on the fp16 tensor cores; the kernel and its launcher.
+// Included by one translation unit per class of plans (falcon_fft8.cu,
+// falcon_fft17.cu, falcon_fft31.cu), which compile in parallel; everything
+// here has internal linkage.
 #pragma once
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
-#include <stdio.h>
 
-#include <algorithm>
-#include <atomic>
-#include <vector>
-
+#include "falcon_fixed.h"
 #include "falcon_internal.h"
 #include "falcon_slices.cuh"
 
@@ -23,982 +18,675 @@ namespace falcon {
 namespace {
 
 // ---------------------------------------------------------------------------
-// complex helpers
+// Tensor-core butterflies.  The symmetric butterfly (fx_dft) of an odd prime
+// p, h = (p - 1)/2:  A_j - v_0 = sum_q a_q cos(2 pi jq/p) and B_j = sum_q b_q
+// sin(2 pi jq/p) as integer matrix products.  Coefficients (Q62) and values
+// (|a|, |b| < 2^61) are cut into kFxS = 7 signed 9-bit digits, balanced in
+// [-256, 255] (the top one by its sign), which fp16 holds exactly; the 28
+// digit pairs s + t <= 6 are summed per diagonal d = s + t in FP32.  Every
+// accumulator starts at 1.5 2^23: with balanced digits a diagonal's partial
+// sums stay below 0.9 2^22 (p = 31: sum over pairs and products of |digit
+// of c| 256), so the sums are exact and the accumulator's bits are
+// 0x4b400000 + sum, an integer with no conversion instruction.  The dropped
+// pairs weigh below 2^-16 of a unit per product.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cmul(double2 a, double2 w) {
-  return make_double2(fma(a.x, w.x, -a.y * w.y), fma(a.x, w.y, a.y * w.x));
-}
+constexpr int kFxS = 7;
+constexpr int kFxMagic = 0x4b400000;  // bits of 1.5 2^23
+constexpr unsigned long long kFxBias = 256ull * ((1ull << 63) / 511ull);  // 256 (512^7 - 1)/511
 
-// ---------------------------------------------------------------------------
-// Odd-prime DFT coefficient tables: kC<p>[i] = cos(2 pi i/p), kS<p>[i] =
-// sin(2 pi i/p), filled from the host once per process.
-// ---------------------------------------------------------------------------
-template <int p> struct DftTab;
-#define FALCON_DEF_TAB(p)                                                    \
-  __constant__ double kC##p[p];                                              \
-  __constant__ double kS##p[p];                                              \
-  template <> struct DftTab<p> {                                             \
-    __device__ static __forceinline__ double c(int i) { return kC##p[i]; }   \
-    __device__ static __forceinline__ double s(int i) { return kS##p[i]; }   \
-  };
-FALCON_DEF_TAB(3)
-FALCON_DEF_TAB(5)
-FALCON_DEF_TAB(7)
-FALCON_DEF_TAB(11)
-FALCON_DEF_TAB(13)
-FALCON_DEF_TAB(17)
-FALCON_DEF_TAB(19)
-FALCON_DEF_TAB(23)
-FALCON_DEF_TAB(29)
-FALCON_DEF_TAB(31)
-
-template <int p>
-static cudaError_t set_tab(const void* csym, const void* ssym) {
-  double c[p], s[p];
-  const double two_pi = 8.0 * atan(1.0);
-  for (int i = 0; i < p; ++i) {
-    c[i] = cos(two_pi * i / p);
-    s[i] = sin(two_pi * i / p);
+constexpr int fx_digit(long long c, int s) {  // digit s (0 = leading) of a Q62 constant
+  int d = 0;
+  for (int i = kFxS - 1; i >= s; --i) {
+    d = i ? (int)(((c + 256) % 512 + 512) % 512) - 256 : (int)c;
+    c = (c - d) / 512;
   }
-  cudaError_t e = cudaMemcpyToSymbol(csym, c, sizeof(c));
-  if (e != cudaSuccess) return e;
-  return cudaMemcpyToSymbol(ssym, s, sizeof(s));
+  return d;
 }
-
-cudaError_t init_tables_here() {
-  static std::atomic<bool> done[64];  // tables uploaded, per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && done[dev].load()) return cudaSuccess;
-  cudaError_t e = cudaSuccess;
-#define FALCON_SET(p) if (e == cudaSuccess) e = set_tab<p>(kC##p, kS##p);
-  FALCON_SET(3) FALCON_SET(5) FALCON_SET(7) FALCON_SET(11) FALCON_SET(13)
-  FALCON_SET(17) FALCON_SET(19) FALCON_SET(23) FALCON_SET(29) FALCON_SET(31)
-#undef FALCON_SET
-  // the copies may return before they land; the kernels reading the tables
-  // run on non-blocking streams
-  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev].store(true);
-  return e;
+constexpr uint32_t fx_half_bits(int q) {  // fp16 bits of an integer |q| <= 2048
+  if (q == 0) return 0u;
+  const uint32_t a = (uint32_t)(q < 0 ? -q : q);
+  int e = 0;
+  while ((2u << e) <= a) ++e;
+  return (q < 0 ? 0x8000u : 0u) | (uint32_t)((15 + e) << 10) | ((a << (10 - e)) & 0x3ffu);
 }
-
-// Forward DFT of length p in registers: v_j <- sum_q v_q exp(-2 pi i j q/p)
-// (radix 2, 4 and 6; odd primes go through dft_odd_store below).  Radix 6
-// is the 6-point axis of a prime-factor plan, computed as a Good-Thomas
-// 2 x 3: inputs n = (3 n1 + 2 n2) mod 6, two 3-point DFTs over n2 in the
-// symmetric form of dft_odd_store (cos(2 pi/3) = -1/2 exactly), then
-// y_k = W_0[k mod 3] +- W_1[k mod 3] with the sign (-1)^(k mod 2).
 template <int p>
-__device__ __forceinline__ void dft_small(double2 (&v)[p]) {
-  if constexpr (p == 6) {
-    const double c = -0.5, sn = DftTab<3>::s(1);
-    double2 w0[3], w1[3];
-    {
-      const double2 v0 = v[0], a = cadd(v[2], v[4]), b = csub(v[2], v[4]);
-      const double2 A = make_double2(fma(a.x, c, v0.x), fma(a.y, c, v0.y)), B = make_double2(b.x * sn, b.y * sn);
-      w0[0] = cadd(v0, a); w0[1] = make_double2(A.x + B.y, A.y - B.x); w0[2] = make_double2(A.x - B.y, A.y + B.x);
-    }
-    {
-      const double2 v0 = v[3], a = cadd(v[5], v[1]), b = csub(v[5], v[1]);
-      const double2 A = make_double2(fma(a.x, c, v0.x), fma(a.y, c, v0.y)), B = make_double2(b.x * sn, b.y * sn);
-      w1[0] = cadd(v0, a); w1[1] = make_double2(A.x + B.y, A.y - B.x); w1[2] = make_double2(A.x - B.y, A.y + B.x);
-    }
-    v[0] = cadd(w0[0], w1[0]); v[3] = csub(w0[0], w1[0]);
-    v[4] = cadd(w0[1], w1[1]); v[1] = csub(w0[1], w1[1]);
-    v[2] = cadd(w0[2], w1[2]); v[5] = csub(w0[2], w1[2]);
-  } else if constexpr (p == 2) {
-    double2 a = v[0], b = v[1];
-    v[0] = cadd(a, b); v[1] = csub(a, b);
-  } else {
-    double2 t0 = cadd(v[0], v[2]), t1 = csub(v[0], v[2]);
-    double2 t2 = cadd(v[1], v[3]), t3 = csub(v[1], v[3]);
-    v[0] = cadd(t0, t2); v[2] = csub(t0, t2);
-    v[1] = make_double2(t1.x + t3.y, t1.y - t3.x);
-    v[3] = make_double2(t1.x - t3.y, t1.y + t3.x);
-  }
-}
-
-// Odd-prime forward DFT in the symmetric form
-//   y_0 = v_0 + sum a_q,  y_j = A_j - i B_j,  y_{p-j} = A_j + i B_j,
-//   a_q = v_q + v_{p-q}, b_q = v_q - v_{p-q}, A_j = v_0 + sum a_q cos(2 pi jq/p),
-//   B_j = sum b_q sin(2 pi jq/p),
-// with each output pair multiplied by its twiddle (DIF) and stored as soon
-// as it is formed, so only a, b stay live.
-template <int p>
-__device__ __forceinline__ void dft_odd_store(double2 (&v)[p], double2* __restrict__ dst, int base, int m,
-                                              const double2* __restrict__ tw, int ks, bool post_tw) {
+constexpr uint32_t fx_coef_pair(bool sine, int j, int q, int s) {  // digits of (j, q), (j, q + 1) as an fp16 pair
   constexpr int h = (p - 1) / 2;
-  double2 a[h], b[h];
-#pragma unroll
-  for (int q = 1; q <= h; ++q) { a[q - 1] = cadd(v[q], v[p - q]); b[q - 1] = csub(v[q], v[p - q]); }
-  const double2 v0 = v[0];
-  double2 y0 = v0;
-#pragma unroll
-  for (int q = 0; q < h; ++q) y0 = cadd(y0, a[q]);
-  dst[base] = y0;
-#pragma unroll
-  for (int j = 1; j <= h; ++j) {
-    double2 A = v0;
-    double2 Bv = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int q = 1; q <= h; ++q) {
-      const int idx = (j * q) % p;
-      const double c = DftTab<p>::c(idx), s = DftTab<p>::s(idx);
-      A.x = fma(a[q - 1].x, c, A.x); A.y = fma(a[q - 1].y, c, A.y);
-      Bv.x = fma(b[q - 1].x, s, Bv.x); Bv.y = fma(b[q - 1].y, s, Bv.y);
-    }
-    double2 yj = make_double2(A.x + Bv.y, A.y - Bv.x);
-    double2 yk = make_double2(A.x - Bv.y, A.y + Bv.x);
-    if (post_tw) {
-      yj = cmul(yj, tw[j * ks]);
-      yk = cmul(yk, tw[(p - j) * ks]);
-    }
-    dst[base + j * m] = yj;
-    dst[base + (p - j) * m] = yk;
-  }
+  uint32_t r = 0;
+  for (int i = 0; i < 2; ++i)
+    if (j <= h && q + i <= h)
+      r |= fx_half_bits(fx_digit(sine ? FxDft<p>::s[(j * (q + i)) % p] : FxDft<p>::c[(j * (q + i)) % p], s)) << (16 * i);
+  return r;
 }
 
-// One in-place stage of radix p and span m on NB (1 or 2) buffers, its
-// butterflies shared by nl cooperating lanes (lane < nl).
-// DIT (dif = false): twiddles exp(-2 pi i q k / (m p)) on the inputs; DIF:
-// on the outputs; none for the prime-factor plan (twid = false).
-// tw[k] = exp(-2 pi i k / P); stride = P / (m p).
-template <int p, int NB>
-__device__ __forceinline__ void fft_stage(double2* __restrict__ A, double2* __restrict__ Bf, int P, int m,
-                                          int stride, const double2* __restrict__ tw, int lane, int nl, bool dif,
-                                          bool twid) {
-  const int mp = m * p, nb = P / p;
-  const float inv_m = 1.0f / (float)m;
-  for (int t = lane; t < nb; t += nl) {
-    const int g = (int)(((float)t + 0.5f) * inv_m);
-    const int k = t - g * m;
-    const int base = g * mp + k;
-    const bool tk = twid && k > 0;
-    const int ks = k * stride;
-    double2 va[p], vb[p];
-#pragma unroll
-    for (int q = 0; q < p; ++q) {
-      va[q] = A[base + q * m];
-      if (NB == 2) vb[q] = Bf[base + q * m];
-    }
-    if (tk && !dif) {
-#pragma unroll
-      for (int q = 1; q < p; ++q) {
-        const double2 w = tw[q * ks];
-        va[q] = cmul(va[q], w);
-        if (NB == 2) vb[q] = cmul(vb[q], w);
-      }
-    }
-    if constexpr (p == 2 || p == 4 || p == 6) {
-      dft_small<p>(va);
-      if (NB == 2) dft_small<p>(vb);
-      if (tk && dif) {
-#pragma unroll
-        for (int q = 1; q < p; ++q) {
-          const double2 w = tw[q * ks];
-          va[q] = cmul(va[q], w);
-          if (NB == 2) vb[q] = cmul(vb[q], w);
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < p; ++q) {
-        A[base + q * m] = va[q];
-        if (NB == 2) Bf[base + q * m] = vb[q];
-      }
-    } else {
-      dft_odd_store<p>(va, A, base, m, tw, ks, tk && dif);
-      if (NB == 2) dft_odd_store<p>(vb, Bf, base, m, tw, ks, tk && dif);
-    }
-  }
-}
-
-// Generic prime radix (p <= 64) with coefficients read from the P-point
-// twiddle table: exp(-2 pi i j/p) = tw[j * P/p].  Bf may be null (one buffer).
-__device__ void generic_stage(double2* A, double2* Bf, int P, int p, int m, int stride,
-                              const double2* tw, int lane, int nl, bool dif, bool twid) {
-  const int mp = m * p, nb = P / p, tp = P / p;
-  double2* B2 = Bf ? Bf : A;  // with one buffer the second transform is a repeat, not stored
-  for (int t = lane; t < nb; t += nl) {
-    const int g = t / m, k = t - g * m, base = g * mp + k;
-    double2 va[64], vb[64], ya[64], yb[64];
-    for (int q = 0; q < p; ++q) { va[q] = A[base + q * m]; vb[q] = B2[base + q * m]; }
-    if (twid && !dif && k > 0)
-      for (int q = 1; q < p; ++q) { double2 w = tw[q * k * stride]; va[q] = cmul(va[q], w); vb[q] = cmul(vb[q], w); }
-    for (int j = 0; j < p; ++j) {
-      double2 sa = make_double2(0, 0), sb = make_double2(0, 0);
-      for (int q = 0; q < p; ++q) {
-        double2 w = tw[((j * q) % p) * tp];
-        sa = cadd(sa, cmul(va[q], w)); sb = cadd(sb, cmul(vb[q], w));
-      }
-      ya[j] = sa; yb[j] = sb;
-    }
-    if (twid && dif && k > 0)
-      for (int q = 1; q < p; ++q) { double2 w = tw[q * k * stride]; ya[q] = cmul(ya[q], w); yb[q] = cmul(yb[q], w); }
-    for (int q = 0; q < p; ++q) {
-      A[base + q * m] = ya[q];
-      if (Bf) Bf[base + q * m] = yb[q];
-    }
-  }
-}
-
+// The A fragments of mma.m16n8k16, [digit][lane][words].  h <= 8: the
+// block-diagonal [C 0; 0 S] (rows j; K = the h values a_q, then b_q), words
+// (a0, a3).  h <= 15: C and S as two 16 x 16 tiles, words (a0, a1, a2, a3)
+// of C, then of S.
 template <int p>
-__device__ void dft_mma_stage(double2* A, double2* Bf, int P, int m, int lane, int warp, int nw);
+struct FxFrag {
+  static constexpr int kWords = p <= 17 ? 2 : 8;
+  static constexpr int kInts = kFxS * 32 * kWords;
+  uint32_t v[kInts];
+};
 template <int p>
-__device__ void dft_mma_stage_wide(double2* A, double2* Bf, int P, int m, int lane, int warp, int nw);
-
-// MAXP bounds the radices compiled into one kernel instance, so a plan
-// with small radices is not held to the register budget of radix 31.
-template <int MAXP>
-__device__ __forceinline__ void run_stage(int p, bool dif, bool twid, double2* A, double2* Bf, int P, int m,
-                                          int stride, const double2* tw, int lane) {
-  // two buffers interleaved up to radix 7; one at a time above, to bound
-  // the live registers of the butterfly
-#define FALCON_CASE2(q) case q: fft_stage<q, 2>(A, Bf, P, m, stride, tw, lane, 32, dif, twid); return;
-#define FALCON_CASE1(q)                                                      \
-  case q:                                                                    \
-    if constexpr (q <= MAXP) {                                               \
-      fft_stage<q, 1>(A, nullptr, P, m, stride, tw, lane, 32, dif, twid);    \
-      fft_stage<q, 1>(Bf, nullptr, P, m, stride, tw, lane, 32, dif, twid);   \
-      return;                                                                \
-    }                                                                        \
-    break;
-  if constexpr (MAXP == 31) {  // the wide primes of prime-factor plans on the tensor cores
-    if (!twid && (p == 19 || p == 23 || p == 29 || p == 31)) {
-      if (p == 19) dft_mma_stage_wide<19>(A, Bf, P, m, lane, 0, 1);
-      else if (p == 23) dft_mma_stage_wide<23>(A, Bf, P, m, lane, 0, 1);
-      else if (p == 29) dft_mma_stage_wide<29>(A, Bf, P, m, lane, 0, 1);
-      else dft_mma_stage_wide<31>(A, Bf, P, m, lane, 0, 1);
-      return;
-    }
-  }
-  if constexpr (MAXP == 17) {  // plans with a prime above 17 keep the FMA butterflies
-    if (!twid && (p == 11 || p == 13 || p == 17)) {
-      if (p == 11) dft_mma_stage<11>(A, Bf, P, m, lane, 0, 1);
-      else if (p == 13) dft_mma_stage<13>(A, Bf, P, m, lane, 0, 1);
-      else dft_mma_stage<17>(A, Bf, P, m, lane, 0, 1);
-      return;
-    }
-  }
-  switch (p) {
-    FALCON_CASE2(2) FALCON_CASE2(3) FALCON_CASE2(4) FALCON_CASE2(5) FALCON_CASE2(6) FALCON_CASE2(7)
-    FALCON_CASE1(11) FALCON_CASE1(13) FALCON_CASE1(17)
-    FALCON_CASE1(19) FALCON_CASE1(23) FALCON_CASE1(29) FALCON_CASE1(31)
-    default: break;
-  }
-#undef FALCON_CASE1
-#undef FALCON_CASE2
-  generic_stage(A, Bf, P, p, m, stride, tw, lane, 32, dif, twid);
-}
-
-// One buffer, its butterflies shared by nl lanes (the block-per-line form).
-template <int MAXP>
-__device__ __forceinline__ void run_stage1(int p, bool dif, bool twid, double2* A, int P, int m, int stride,
-                                           const double2* tw, int lane, int nl) {
-#define FALCON_CASE(q)                                                   \
-  case q:                                                                \
-    if constexpr (q <= MAXP) {                                           \
-      fft_stage<q, 1>(A, nullptr, P, m, stride, tw, lane, nl, dif, twid); \
-      return;                                                            \
-    }                                                                    \
-    break;
-  switch (p) {
-    FALCON_CASE(2) FALCON_CASE(3) FALCON_CASE(4) FALCON_CASE(5) FALCON_CASE(6) FALCON_CASE(7)
-    FALCON_CASE(11) FALCON_CASE(13) FALCON_CASE(17) FALCON_CASE(19) FALCON_CASE(23)
-    FALCON_CASE(29) FALCON_CASE(31)
-    default: break;
-  }
-#undef FALCON_CASE
-  generic_stage(A, nullptr, P, p, m, stride, tw, lane, nl, dif, twid);
-}
-
-// Odd prime p >= 17 of a prime-factor plan (no twiddles) on both buffers
-// of a block at once, the output pairs of each butterfly shared by G lanes:
-// with one thread per butterfly the stage would run a few dozen long
-// butterflies on a few warps.  Work items are ordered lane group first, so
-// a warp's lanes share their lane group (uniform coefficient loads).  Each
-// output is formed with exactly the operations of dft_odd_store, so the
-// results are bit for bit those of the one-thread form.  In place: every
-// item loads its inputs before any item of the round stores.
-template <int p, int G>
-__device__ void fft_stage_split(double2* A, double2* Bf, int P, int m, int tid, int nt) {
-  constexpr int h = (p - 1) / 2;
-  const int nb = P / p, mp = m * p, items = 2 * nb * G;
-  const int rounds = (items + nt - 1) / nt;
-  const float inv_m = 1.0f / (float)m;
-  for (int rd = 0; rd < rounds; ++rd) {
-    const int it = rd * nt + tid;
-    const bool act = it < items;
-    int jg = 0, base = 0;
-    double2* buf = A;
-    double2 v[p];
-    if (act) {
-      jg = it / (2 * nb);
-      const int rem = it - jg * 2 * nb;
-      const int bsel = rem >= nb;
-      const int t = rem - bsel * nb;
-      buf = bsel ? Bf : A;
-      const int g = (int)(((float)t + 0.5f) * inv_m);
-      base = g * mp + (t - g * m);
-#pragma unroll
-      for (int q = 0; q < p; ++q) v[q] = buf[base + q * m];
-    }
-    __syncthreads();
-    if (act) {
-      double2 a[h], b[h];
-#pragma unroll
-      for (int q = 1; q <= h; ++q) { a[q - 1] = cadd(v[q], v[p - q]); b[q - 1] = csub(v[q], v[p - q]); }
-      const double2 v0 = v[0];
-      if (jg == 0) {
-        double2 y0 = v0;
-#pragma unroll
-        for (int q = 0; q < h; ++q) y0 = cadd(y0, a[q]);
-        buf[base] = y0;
-      }
-      for (int j = 1 + jg; j <= h; j += G) {
-        double2 Av = v0;
-        double2 Bv = make_double2(0.0, 0.0);
-#pragma unroll
-        for (int q = 1; q <= h; ++q) {
-          const int idx = (j * q) % p;
-          const double c = DftTab<p>::c(idx), sn = DftTab<p>::s(idx);
-          Av.x = fma(a[q - 1].x, c, Av.x); Av.y = fma(a[q - 1].y, c, Av.y);
-          Bv.x = fma(b[q - 1].x, sn, Bv.x); Bv.y = fma(b[q - 1].y, sn, Bv.y);
-        }
-        buf[base + j * m] = make_double2(Av.x + Bv.y, Av.y - Bv.x);
-        buf[base + (p - j) * m] = make_double2(Av.x - Bv.y, Av.y + Bv.x);
+constexpr FxFrag<p> fx_frag() {
+  FxFrag<p> f{};
+  constexpr int W = FxFrag<p>::kWords;
+  for (int s = 0; s < kFxS; ++s)
+    for (int lane = 0; lane < 32; ++lane) {
+      const int j = (lane >> 2) + 1, q = 2 * (lane & 3) + 1;
+      for (int w = 0; w < W; ++w) {
+        uint32_t r = 0;
+        if constexpr (W == 2) r = fx_coef_pair<p>(w == 1, j, q, s);
+        else r = fx_coef_pair<p>(w >= 4, j + 8 * (w & 1), q + 8 * ((w >> 1) & 1), s);
+        f.v[(s * 32 + lane) * W + w] = r;
       }
     }
-    __syncthreads();
-  }
+  return f;
+}
+template <int p>
+__device__ const FxFrag<p> kFxFrag = fx_frag<p>();
+
+// 32-bit words of fragments a plan's block holds in shared memory.
+__host__ __device__ constexpr int fx_frag_ints(int p) { return p <= 7 ? 0 : p <= 17 ? FxFrag<17>::kInts : FxFrag<31>::kInts; }
+
+__device__ __forceinline__ void fx_mma(float (&d)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3, unsigned b0,
+                                       unsigned b1, float c0, float c1, float c2, float c3) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%11,%12,%13};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c0), "f"(c1), "f"(c2), "f"(c3));
 }
 
-// Odd-prime stage (p = 11, 13, 17, so h = (p - 1)/2 <= 8) of a prime-factor
-// plan on the fp16 tensor cores, in fixed point: no FP64 arithmetic.  The
-// symmetric butterfly of dft_odd_store,
-//   y_0 = v_0 + sum a_q,  y_j = A_j - i B_j,  y_{p-j} = A_j + i B_j,
-//   A_j = v_0 + sum_q a_q cos(2 pi jq/p),  B_j = sum_q b_q sin(2 pi jq/p),
-//   a_q = v_q + v_{p-q},  b_q = v_q - v_{p-q},
-// with every value of a butterfly (both components) as an integer at the
-// scale of its largest, 2^e: V = trunc(v 2^(kDftFB - e)), |V| < 2^58.  The
-// pre-adds and the y_0 sum are then exact 64-bit integer adds (|y_0| <
-// 2^63), and A_j, B_j come from one product of the block-diagonal [C 0; 0 S]
-// (rows j; K = the h values a_q, then the h values b_q) with a column per
-// component: one m16n8k16 MMA per slice pair takes 8 columns, 4
-// butterflies x (re, im).  The coefficients (|cos|, |sin| < 1) and the
-// integers 2^4 a, 2^4 b (< 2^63) are cut into kDftS = 7 signed 9-bit slices
-// (fp16 holds them exactly), and the 28 pairs s + t <= 6 are summed in
-// FP32: at most 8 products per output keep every sum exact (7 pairs x 8
-// products x 511^2 < 2^24).  The diagonal sums give A_j - v_0 and B_j as
-// exact integers H 2^36 + L in units of 2^(e - 71); v_0 and the output
-// pairs A_j +- i B_j are added in those integers and each output is
-// rounded once to FP64 (combine_rn).  Errors: the inputs' truncation
-// (2^(e - 58) each), the dropped pairs (below 2^(e - 56) per output) and the
-// final rounding; a butterfly with an Inf or NaN gives NaN.  A butterfly's
-// outputs depend only on its inputs, so any tiling (warp or block form)
-// gives the same bits.  Lane (g, t) of a tile holds v_q, v_{p-q} for q =
-// 2t + 1, 2t + 2 and v_0 of column g, and receives A_{g+1}, B_{g+1} of
-// butterfly t, re and im, from which it stores y_j and y_{p-j}.  Tiles over
-// both buffers go to warps warp, warp + nw, ...; the caller synchronises
-// before (inputs complete) and after (outputs stored).
-constexpr int kDftFB = 58;
+// Digit s of two biased values (u = v + kFxBias) as an fp16 pair: fp16(1536 +
+// d) has the bits 0x6600 + d for 0 <= d < 512, so one packed subtraction of
+// 1792 gives the balanced digits d - 256.
+__device__ __forceinline__ uint32_t fx_digits(unsigned long long u0, unsigned long long u1, int s) {
+  const int sh = 9 * (kFxS - 1 - s);
+  const uint32_t both = __byte_perm((uint32_t)(u0 >> sh), (uint32_t)(u1 >> sh), 0x5410);
+  const uint32_t biased = (both & 0x01ff01ffu) | 0x66006600u;
+  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&biased), __floats2half2_rn(1792.f, 1792.f));
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
 
+// The product sum_d q_d 512^(12 - d) 2^-62 from the accumulator bits of its
+// diagonals (modulo 2^64 every term may wrap; the result is below 2^62):
+// weights 2^(46 - 9 d), the last diagonal shifted down.
+__device__ __forceinline__ long long fx_undigit(const float (&acc)[kFxS][4], int i) {
+  constexpr unsigned long long B = (unsigned long long)kFxMagic;
+  constexpr unsigned long long off = 0ull - ((B << 46) + (B << 37) + (B << 28) + (B << 19) + (B << 10) + (B << 1) + (B >> 8));
+  const int b0 = __float_as_int(acc[0][i]), b1 = __float_as_int(acc[1][i]), b2 = __float_as_int(acc[2][i]),
+            b3 = __float_as_int(acc[3][i]), b4 = __float_as_int(acc[4][i]), b5 = __float_as_int(acc[5][i]),
+            b6 = __float_as_int(acc[6][i]);
+  long long w = fx_madw(b2, 1 << 28, (long long)off);
+  w = fx_madw(b3, 1 << 19, w);
+  w = fx_madw(b4, 1 << 10, w);
+  w = fx_madw(b5, 2, w);
+  w = fx_madw(b6 >> 8, 1, w);
+  const unsigned hi = (unsigned)b0 * (1u << 14) + (unsigned)b1 * (1u << 5);
+  return (long long)((unsigned long long)w + ((unsigned long long)hi << 32));
+}
+
+// One stage (p = 11, 13, 17; no twiddles) of one buffer, inputs scaled by
+// 2^-d: tiles of 4 butterflies x (re, im) = 8 columns to warps warp, warp +
+// nw, ...  Lane (g, t) holds v_q, v_{p-q} for q = 2t + 1, 2t + 2 and v_0 of
+// column g, and receives A_{g+1}, B_{g+1} of butterfly t, re and im, from
+// which it stores y_j and y_{p-j}.  y_0 = v_0 + sum a_q by shuffles.  The
+// caller synchronises before (inputs complete) and after (outputs stored).
+// Results do not depend on the tiling.
 template <int p>
-__device__ void dft_mma_stage(double2* A, double2* Bf, int P, int m, int lane, int warp, int nw) {
+__device__ void fx_mma_stage(longlong2* buf, int P, int m, int d, const uint32_t* frag, int lane, int warp, int nw,
+                             FxMax& o) {
   constexpr int h = (p - 1) / 2;
   static_assert(h <= 8, "the block-diagonal form holds h <= 8");
   constexpr unsigned FULL = 0xffffffffu;
-  constexpr int UP = 63 - (kDftFB + 1);  // |a|, |b| < 2^(kDftFB + 1): 2^UP |a| < 2^63
+  const float magic = __int_as_float(kFxMagic);
   const int gid = lane >> 2, tig = lane & 3;
-  const int nb = P / p, mp = m * p, nbt = 2 * nb, ntile = (nbt + 3) / 4;
+  const int nb = P / p, mp = m * p, ntile = (nb + 3) / 4;
   const float inv_m = 1.0f / (float)m;
-  const int q1 = 2 * tig + 1, q2 = 2 * tig + 2;  // K rows 2t, 2t + 1 (a) and 2t + 8, 2t + 9 (b)
+  const int q1 = 2 * tig + 1, q2 = 2 * tig + 2;
   const bool has1 = q1 <= h, has2 = q2 <= h;
-  // coefficient fragments: a0 = C(row g; q1, q2), a3 = S(row g; q1, q2), j = g + 1,
-  // as 63-bit fractions (every |cos|, |sin| here is below 1)
-  uint32_t fc[kDftS], fs[kDftS];
-  {
-    const int j = gid + 1;
-    double c1 = 0.0, c2 = 0.0, s1 = 0.0, s2 = 0.0;
-    if (j <= h) {
-      if (has1) { c1 = DftTab<p>::c((j * q1) % p); s1 = DftTab<p>::s((j * q1) % p); }
-      if (has2) { c2 = DftTab<p>::c((j * q2) % p); s2 = DftTab<p>::s((j * q2) % p); }
-    }
-    const unsigned long long tc1 = dft_mag(c1, 0), tc2 = dft_mag(c2, 0), ts1 = dft_mag(s1, 0), ts2 = dft_mag(s2, 0);
-    const uint32_t sc = sign2(c1, c2), ss = sign2(s1, s2);
-#pragma unroll
-    for (int sl = 0; sl < kDftS; ++sl) {
-      fc[sl] = dft_slice2(tc1, tc2, sc, sl);
-      fs[sl] = dft_slice2(ts1, ts2, ss, sl);
-    }
-  }
+  const uint2* fr = reinterpret_cast<const uint2*>(frag) + lane;
   for (int tile = warp; tile < ntile; tile += nw) {
-    // column g: butterfly bi (over both buffers), component g & 1
     const int bi = tile * 4 + (gid >> 1), comp = gid & 1;
-    double x1 = 0.0, y1 = 0.0, x2 = 0.0, y2 = 0.0, v0 = 0.0;
-    double* pi = nullptr;
-    if (bi < nbt) {
-      const int sel = bi >= nb, t = bi - sel * nb;
-      const int g = (int)(((float)t + 0.5f) * inv_m);
-      pi = reinterpret_cast<double*>((sel ? Bf : A) + g * mp + (t - g * m)) + comp;
+    long long x1 = 0, y1 = 0, x2 = 0, y2 = 0, v0 = 0;
+    long long* pi = nullptr;
+    if (bi < nb) {
+      const int g = (int)(((float)bi + 0.5f) * inv_m);
+      pi = reinterpret_cast<long long*>(buf + g * mp + (bi - g * m)) + comp;
       if (has1) { x1 = pi[2 * q1 * m]; y1 = pi[2 * (p - q1) * m]; }
       if (has2) { x2 = pi[2 * q2 * m]; y2 = pi[2 * (p - q2) * m]; }
       v0 = pi[0];
     }
-    // the butterfly's exponent: |v| < 2^e over its 2p values (8 lanes)
-    int fb = max(max(max(biased_exp(x1), biased_exp(y1)), max(biased_exp(x2), biased_exp(y2))), biased_exp(v0));
-    fb = max(fb, __shfl_xor_sync(FULL, fb, 1));
-    fb = max(fb, __shfl_xor_sync(FULL, fb, 2));
-    fb = max(fb, __shfl_xor_sync(FULL, fb, 4));
-    const int e = fb - 1022;
-    const long long X1 = fix_of<kDftFB>(x1, e), Y1 = fix_of<kDftFB>(y1, e), X2 = fix_of<kDftFB>(x2, e),
-                    Y2 = fix_of<kDftFB>(y2, e), V0 = fix_of<kDftFB>(v0, e);
-    const long long a1 = X1 + Y1, b1 = X1 - Y1, a2 = X2 + Y2, b2 = X2 - Y2;
-    // y_0 = v_0 + sum_q a_q per component (the same sum on the four lanes)
+    if (d > 0) { x1 >>= d; y1 >>= d; x2 >>= d; y2 >>= d; v0 >>= d; }
+    else if (d < 0) {
+      x1 = fx_scale(x1, d); y1 = fx_scale(y1, d); x2 = fx_scale(x2, d); y2 = fx_scale(y2, d); v0 = fx_scale(v0, d);
+    }
+    const long long a1 = x1 + y1, a2 = x2 + y2;
+    const unsigned long long ua1 = (unsigned long long)a1 + kFxBias, ua2 = (unsigned long long)a2 + kFxBias,
+                             ub1 = (unsigned long long)(x1 - y1) + kFxBias,
+                             ub2 = (unsigned long long)(x2 - y2) + kFxBias;
     long long ys = a1 + a2;
     ys += __shfl_xor_sync(FULL, ys, 1);
     ys += __shfl_xor_sync(FULL, ys, 2);
-    uint32_t fa[kDftS], fbq[kDftS];
-    {
-      const unsigned long long ta1 = (unsigned long long)(a1 < 0 ? -a1 : a1) << UP,
-                               ta2 = (unsigned long long)(a2 < 0 ? -a2 : a2) << UP,
-                               tb1 = (unsigned long long)(b1 < 0 ? -b1 : b1) << UP,
-                               tb2 = (unsigned long long)(b2 < 0 ? -b2 : b2) << UP;
-      const uint32_t sa = (a1 < 0 ? 0x8000u : 0u) | (a2 < 0 ? 0x80000000u : 0u);
-      const uint32_t sb = (b1 < 0 ? 0x8000u : 0u) | (b2 < 0 ? 0x80000000u : 0u);
+    __syncwarp();  // every load of the tile precedes its stores
+    if (tig == 0 && pi) {
+      pi[0] = v0 + ys;
+      if (comp) fx_cover(o, fx_make(0, v0 + ys));
+      else fx_cover(o, fx_make(v0 + ys, 0));
+    }
+    float acc[kFxS][4];
+    uint32_t fa[kFxS], fb[kFxS];
 #pragma unroll
-      for (int sl = 0; sl < kDftS; ++sl) {
-        fa[sl] = dft_slice2(ta1, ta2, sa, sl);
-        fbq[sl] = dft_slice2(tb1, tb2, sb, sl);
+    for (int t = 0; t < kFxS; ++t) {
+      fa[t] = fx_digits(ua1, ua2, t);
+      fb[t] = fx_digits(ub1, ub2, t);
+    }
+#pragma unroll
+    for (int s = 0; s < kFxS; ++s) {
+      const uint2 c = fr[s * 32];
+#pragma unroll
+      for (int t = 0; s + t < kFxS; ++t) {
+        float(&ac)[4] = acc[s + t];
+        if (s == 0) fx_mma(ac, c.x, 0u, 0u, c.y, fa[t], fb[t], magic, magic, magic, magic);
+        else fx_mma(ac, c.x, 0u, 0u, c.y, fa[t], fb[t], ac[0], ac[1], ac[2], ac[3]);
       }
     }
-    __syncwarp();  // every load of the tile precedes its stores
-    if (tig == 0 && pi)
-      pi[0] = fb == 2047 ? __longlong_as_double(0x7ff8000000000000LL) : dbl_of_fix(V0 + ys, e - kDftFB);
-    float acc[kDftD + 1][4];
-#pragma unroll
-    for (int d = 0; d <= kDftD; ++d)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[d][i] = 0.f;
-#pragma unroll
-    for (int sl = 0; sl < kDftS; ++sl)
-#pragma unroll
-      for (int t = 0; t < kDftS && sl + t <= kDftD; ++t) mma_f16(acc[sl + t], fc[sl], 0u, 0u, fs[sl], fa[t], fbq[t]);
-    // this lane's butterfly bo: its exponent and v_0 (lanes 8t, 8t + 4 loaded them)
+    // this lane's butterfly bo; lanes 8t, 8t + 4 loaded its v_0
     const int bo = tile * 4 + tig;
-    const int eo = __shfl_sync(FULL, e, 8 * tig);
-    const long long w_re = __shfl_sync(FULL, V0, 8 * tig), w_im = __shfl_sync(FULL, V0, 8 * tig + 4);
-    if (gid < h && bo < nbt) {
-      const int sel = bo >= nb, t = bo - sel * nb;
-      const int g = (int)(((float)t + 0.5f) * inv_m);
-      double2* po = (sel ? Bf : A) + g * mp + (t - g * m);
-      // (A_j - v_0).re, .im, B_j.re, .im = 2^(e - 71) (H 2^36 + L),
-      // H = sum_{d<=2} Q_d 512^(2-d), L = sum_{d=3..6} Q_d 512^(6-d)
-      long long H[4], L[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        H[i] = ((long long)__float2int_rn(acc[0][i]) << 18) + ((long long)__float2int_rn(acc[1][i]) << 9) +
-               __float2int_rn(acc[2][i]);
-        L[i] = ((long long)__float2int_rn(acc[3][i]) << 27) + ((long long)__float2int_rn(acc[4][i]) << 18) +
-               ((long long)__float2int_rn(acc[5][i]) << 9) + __float2int_rn(acc[6][i]);
-      }
-      // v_0 (units 2^(e - 58)) in the same integers: 2^13 V = (V >> 23) 2^36 + (V mod 2^23) 2^13
-      const long long hr = H[0] + (w_re >> 23), lr = L[0] + ((w_re & ((1LL << 23) - 1)) << 13);
-      const long long hi = H[1] + (w_im >> 23), li = L[1] + ((w_im & ((1LL << 23) - 1)) << 13);
-      const int k = eo - 71;
-      double2 yj = make_double2(combine_rn(hr + H[3], lr + L[3], k, 36), combine_rn(hi - H[2], li - L[2], k, 36));
-      double2 yk = make_double2(combine_rn(hr - H[3], lr - L[3], k, 36), combine_rn(hi + H[2], li + L[2], k, 36));
-      if (eo == 2047 - 1022) {  // Inf or NaN in the butterfly
-        yj = make_double2(__longlong_as_double(0x7ff8000000000000LL), __longlong_as_double(0x7ff8000000000000LL));
-        yk = yj;
-      }
+    const long long w_re = __shfl_sync(FULL, v0, 8 * tig), w_im = __shfl_sync(FULL, v0, 8 * tig + 4);
+    if (gid < h && bo < nb) {
+      const int g = (int)(((float)bo + 0.5f) * inv_m);
+      longlong2* po = buf + g * mp + (bo - g * m);
+      const longlong2 A = fx_make(w_re + fx_undigit(acc, 0), w_im + fx_undigit(acc, 1));
+      const longlong2 B = fx_make(fx_undigit(acc, 2), fx_undigit(acc, 3));
+      longlong2 yj, yk;
+      fx_pair(A, B, yj, yk);
       const int j = gid + 1;
       po[j * m] = yj;
       po[(p - j) * m] = yk;
+      fx_cover(o, yj);
+      fx_cover(o, yk);
     }
   }
 }
 
-// Wide odd-prime stage (p = 19, 23, 29, 31: h = 9..15) of a prime-factor
-// plan on the fp16 tensor cores: the fixed-point butterfly of
-// dft_mma_stage (integers |V| < 2^57, |y_0| < 2^63 for h <= 15) with the
-// cos and sin products as two 16 x 16 tiles (rows j, K = q, padded), 8
-// signed 8-bit slices of the coefficients and of 2^6 a, 2^6 b (64 bits)
-// and the 36 pairs s + t <= 7 per tile; at most 15 products per output keep
-// every FP32 sum exact (8 pairs x 15 x 255^2 < 2^24).  Lane (g, t) holds
-// v_q, v_{p-q} for q = 2t + 1, 2t + 2, 2t + 9, 2t + 10 of column g and
-// receives A_j, B_j for j = g + 1 and g + 9 of butterfly t.
-constexpr int kDwFB = 57;
-
+// The same for p = 19, 23, 29, 31 (h = 9..15): C and S as two 16 x 16 tiles.
+// Lane (g, t) holds v_q, v_{p-q} for q = 2t + 1, 2t + 2, 2t + 9, 2t + 10 of
+// column g and receives A_j, B_j for j = g + 1 and g + 9 of butterfly t.
 template <int p>
-__device__ void dft_mma_stage_wide(double2* A, double2* Bf, int P, int m, int lane, int warp, int nw) {
+__device__ void fx_mma_stage_wide(longlong2* buf, int P, int m, int d, const uint32_t* frag, int lane, int warp,
+                                  int nw, FxMax& o) {
   constexpr int h = (p - 1) / 2;
   static_assert(h > 8 && h <= 15, "two 16 x 16 tiles");
   constexpr unsigned FULL = 0xffffffffu;
-  constexpr int UP = 64 - (kDwFB + 1);  // 2^UP |a| < 2^64
+  const float magic = __int_as_float(kFxMagic);
   const int gid = lane >> 2, tig = lane & 3;
-  const int nb = P / p, mp = m * p, nbt = 2 * nb, ntile = (nbt + 3) / 4;
+  const int nb = P / p, mp = m * p, ntile = (nb + 3) / 4;
   const float inv_m = 1.0f / (float)m;
-  const int qa = 2 * tig + 1;  // K rows 2t, 2t + 1 -> q = qa, qa + 1; rows 2t + 8, 2t + 9 -> q = qa + 8, qa + 9
-  // coefficient fragments of the cos (C) and sin (S) tiles as 64-bit
-  // fractions: per slice [0] = (j0; qa, qa+1), [1] = (j1; qa, qa+1),
-  // [2] = (j0; qa+8, qa+9), [3] = (j1; qa+8, qa+9), j0 = g + 1, j1 = g + 9
-  uint32_t fc[kDwS][4], fs[kDwS][4];
-  {
-    double c[2][4], sn[2][4];  // [row j0 / j1][q slot]
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int j = gid + 1 + 8 * r;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int q = qa + (i & 1) + 8 * (i >> 1);
-        const bool ok = j <= h && q <= h;
-        c[r][i] = ok ? DftTab<p>::c((j * q) % p) : 0.0;
-        sn[r][i] = ok ? DftTab<p>::s((j * q) % p) : 0.0;
-      }
-    }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const int r = f & 1, i0 = 2 * (f >> 1);
-      const unsigned long long c0 = dft_mag64(c[r][i0], 0), c1 = dft_mag64(c[r][i0 + 1], 0);
-      const unsigned long long s0 = dft_mag64(sn[r][i0], 0), s1 = dft_mag64(sn[r][i0 + 1], 0);
-      const uint32_t sgc = sign2(c[r][i0], c[r][i0 + 1]), sgs = sign2(sn[r][i0], sn[r][i0 + 1]);
-#pragma unroll
-      for (int sl = 0; sl < kDwS; ++sl) {
-        fc[sl][f] = dft_slice2w(c0, c1, sgc, sl);
-        fs[sl][f] = dft_slice2w(s0, s1, sgs, sl);
-      }
-    }
-  }
+  const int qa = 2 * tig + 1;
+  const uint4* fr = reinterpret_cast<const uint4*>(frag) + 2 * lane;
   for (int tile = warp; tile < ntile; tile += nw) {
     const int bi = tile * 4 + (gid >> 1), comp = gid & 1;
-    double x[4] = {0.0, 0.0, 0.0, 0.0}, y[4] = {0.0, 0.0, 0.0, 0.0}, v0 = 0.0;
-    double* pi = nullptr;
-    if (bi < nbt) {
-      const int sel = bi >= nb, t = bi - sel * nb;
-      const int g = (int)(((float)t + 0.5f) * inv_m);
-      pi = reinterpret_cast<double*>((sel ? Bf : A) + g * mp + (t - g * m)) + comp;
+    long long av[4] = {0, 0, 0, 0}, bv[4] = {0, 0, 0, 0}, v0 = 0;
+    long long* pi = nullptr;
+    if (bi < nb) {
+      const int g = (int)(((float)bi + 0.5f) * inv_m);
+      pi = reinterpret_cast<long long*>(buf + g * mp + (bi - g * m)) + comp;
+      v0 = fx_scale(pi[0], d);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const int q = qa + (i & 1) + 8 * (i >> 1);
-        if (q <= h) { x[i] = pi[2 * q * m]; y[i] = pi[2 * (p - q) * m]; }
+        if (q <= h) {
+          const long long x = fx_scale(pi[2 * q * m], d), y = fx_scale(pi[2 * (p - q) * m], d);
+          av[i] = x + y;
+          bv[i] = x - y;
+        }
       }
-      v0 = pi[0];
     }
-    int fb = biased_exp(v0);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) fb = max(fb, max(biased_exp(x[i]), biased_exp(y[i])));
-    fb = max(fb, __shfl_xor_sync(FULL, fb, 1));
-    fb = max(fb, __shfl_xor_sync(FULL, fb, 2));
-    fb = max(fb, __shfl_xor_sync(FULL, fb, 4));
-    const int e = fb - 1022;
-    long long av[4], bv[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const long long X = fix_of<kDwFB>(x[i], e), Y = fix_of<kDwFB>(y[i], e);
-      av[i] = X + Y;
-      bv[i] = X - Y;
-    }
-    const long long V0 = fix_of<kDwFB>(v0, e);
     long long ys = (av[0] + av[1]) + (av[2] + av[3]);
     ys += __shfl_xor_sync(FULL, ys, 1);
     ys += __shfl_xor_sync(FULL, ys, 2);
     __syncwarp();  // every load of the tile precedes its stores
-    if (tig == 0 && pi)
-      pi[0] = fb == 2047 ? __longlong_as_double(0x7ff8000000000000LL) : dbl_of_fix(V0 + ys, e - kDwFB);
-    long long H[2][4], L[2][4];  // [C / S][(j0 re, j0 im, j1 re, j1 im)]: 2^(e - 71) (H 2^32 + L)
+    if (tig == 0 && pi) {
+      pi[0] = v0 + ys;
+      if (comp) fx_cover(o, fx_make(0, v0 + ys));
+      else fx_cover(o, fx_make(v0 + ys, 0));
+    }
+    long long r[2][4];  // [A - v_0 / B][(j0 re, j0 im, j1 re, j1 im)]
 #pragma unroll
     for (int part = 0; part < 2; ++part) {
       const long long* v = part ? bv : av;
-      uint32_t fx[kDwS][2];
-      {
-        unsigned long long t[4];
+      uint32_t fx[kFxS][2];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) t[i] = (unsigned long long)(v[i] < 0 ? -v[i] : v[i]) << UP;
-        const uint32_t s01 = (v[0] < 0 ? 0x8000u : 0u) | (v[1] < 0 ? 0x80000000u : 0u);
-        const uint32_t s23 = (v[2] < 0 ? 0x8000u : 0u) | (v[3] < 0 ? 0x80000000u : 0u);
+      for (int t = 0; t < kFxS; ++t) {
+        fx[t][0] = fx_digits((unsigned long long)v[0] + kFxBias, (unsigned long long)v[1] + kFxBias, t);
+        fx[t][1] = fx_digits((unsigned long long)v[2] + kFxBias, (unsigned long long)v[3] + kFxBias, t);
+      }
+      float acc[kFxS][4];
 #pragma unroll
-        for (int sl = 0; sl < kDwS; ++sl) {
-          fx[sl][0] = dft_slice2w(t[0], t[1], s01, sl);
-          fx[sl][1] = dft_slice2w(t[2], t[3], s23, sl);
+      for (int s = 0; s < kFxS; ++s) {
+        const uint4 c = fr[s * 64 + part];
+#pragma unroll
+        for (int t = 0; s + t < kFxS; ++t) {
+          float(&ac)[4] = acc[s + t];
+          if (s == 0) fx_mma(ac, c.x, c.y, c.z, c.w, fx[t][0], fx[t][1], magic, magic, magic, magic);
+          else fx_mma(ac, c.x, c.y, c.z, c.w, fx[t][0], fx[t][1], ac[0], ac[1], ac[2], ac[3]);
         }
       }
-      float acc[kDwD + 1][4];
 #pragma unroll
-      for (int d = 0; d <= kDwD; ++d)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[d][i] = 0.f;
-#pragma unroll
-      for (int sl = 0; sl < kDwS; ++sl) {
-        const uint32_t* f = part ? fs[sl] : fc[sl];
-#pragma unroll
-        for (int t = 0; t < kDwS && sl + t <= kDwD; ++t) mma_f16(acc[sl + t], f[0], f[1], f[2], f[3], fx[t][0], fx[t][1]);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        long long hh = 0, ll = 0;
-#pragma unroll
-        for (int d = 0; d <= 3; ++d) hh = hh * 256 + __float2int_rn(acc[d][i]);
-#pragma unroll
-        for (int d = 4; d <= kDwD; ++d) ll = ll * 256 + __float2int_rn(acc[d][i]);
-        H[part][i] = hh;
-        L[part][i] = ll;
-      }
+      for (int i = 0; i < 4; ++i) r[part][i] = fx_undigit(acc, i);
     }
     const int bo = tile * 4 + tig;
-    const int eo = __shfl_sync(FULL, e, 8 * tig);
-    const long long w_re = __shfl_sync(FULL, V0, 8 * tig), w_im = __shfl_sync(FULL, V0, 8 * tig + 4);
-    if (bo < nbt) {
-      const int sel = bo >= nb, t = bo - sel * nb;
-      const int g = (int)(((float)t + 0.5f) * inv_m);
-      double2* po = (sel ? Bf : A) + g * mp + (t - g * m);
-      // v_0 (units 2^(e - 57)) as 2^14 V = (V >> 18) 2^32 + (V mod 2^18) 2^14
-      const long long vhr = w_re >> 18, vlr = (w_re & ((1LL << 18) - 1)) << 14;
-      const long long vhi = w_im >> 18, vli = (w_im & ((1LL << 18) - 1)) << 14;
-      const int k = eo - 71;
-      const double nan = __longlong_as_double(0x7ff8000000000000LL);
+    const long long w_re = __shfl_sync(FULL, v0, 8 * tig), w_im = __shfl_sync(FULL, v0, 8 * tig + 4);
+    if (bo < nb) {
+      const int g = (int)(((float)bo + 0.5f) * inv_m);
+      longlong2* po = buf + g * mp + (bo - g * m);
 #pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        const int j = gid + 1 + 8 * r;
+      for (int i = 0; i < 2; ++i) {
+        const int j = gid + 1 + 8 * i;
         if (j <= h) {
-          const long long hr = H[0][2 * r] + vhr, lr = L[0][2 * r] + vlr;
-          const long long hi = H[0][2 * r + 1] + vhi, li = L[0][2 * r + 1] + vli;
-          double2 yj = make_double2(combine_rn(hr + H[1][2 * r + 1], lr + L[1][2 * r + 1], k, 32),
-                                    combine_rn(hi - H[1][2 * r], li - L[1][2 * r], k, 32));
-          double2 yk = make_double2(combine_rn(hr - H[1][2 * r + 1], lr - L[1][2 * r + 1], k, 32),
-                                    combine_rn(hi + H[1][2 * r], li + L[1][2 * r], k, 32));
-          if (eo == 2047 - 1022) yj = yk = make_double2(nan, nan);
+          longlong2 yj, yk;
+          fx_pair(fx_make(w_re + r[0][2 * i], w_im + r[0][2 * i + 1]), fx_make(r[1][2 * i], r[1][2 * i + 1]), yj, yk);
           po[j * m] = yj;
           po[(p - j) * m] = yk;
+          fx_cover(o, yj);
+          fx_cover(o, yk);
         }
       }
     }
   }
 }
 
-// One stage of the block-per-line form: large odd primes of a prime-factor
-// plan through fft_stage_split over the whole block, the rest per buffer
-// half (run_stage1).  Called by every thread of the block.
-template <int MAXP>
-__device__ __forceinline__ void run_stage_block(int p, bool dif, bool twid, double2* A, double2* Bf, double2* mine,
-                                                int P, int m, int stride, const double2* tw, int tid, int nt, int hl,
-                                                int nl) {
-  if constexpr (MAXP == 31) {
-    if (!twid && (p == 19 || p == 23 || p == 29 || p == 31)) {
-      if (p == 19) dft_mma_stage_wide<19>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      else if (p == 23) dft_mma_stage_wide<23>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      else if (p == 29) dft_mma_stage_wide<29>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      else dft_mma_stage_wide<31>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      __syncthreads();
-      return;
-    }
+// Radices of one kernel instance: MAXP = 8 all register butterflies, 17 and
+// 31 the tensor-core ones of prime-factor plans too (TWID = false), and
+// TWID with MAXP = 31 every twiddled plan with a prime above 7.
+template <int MAXP, bool TWID>
+__device__ __forceinline__ void fx_run_stage(int p, longlong2* buf, const uint16_t* tab, int sp, int P, int m,
+                                             const int4* tw, const int4* root, const uint32_t* frag, int lane, int nl, bool dif,
+                                             int d, FxMax& o) {
+  switch (p) {
+    case 2: fx_stage<2, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return;
+    case 3: fx_stage<3, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return;
+    case 4: fx_stage<4, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return;
+    case 5: fx_stage<5, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return;
+    case 6: fx_stage<6, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return;
+    case 7: fx_stage<7, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return;
+    default: break;
   }
-  if constexpr (MAXP == 17) {  // plans with a prime above 17 keep the FMA butterflies
-    if (!twid && (p == 11 || p == 13 || p == 17)) {
-      if (p == 11) dft_mma_stage<11>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      else if (p == 13) dft_mma_stage<13>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      else dft_mma_stage<17>(A, Bf, P, m, tid & 31, tid >> 5, nt >> 5);
-      __syncthreads();
-      return;
-    }
+  if constexpr (TWID) {
+    if (p == 8) { fx_stage<8, TWID>(buf, tab, sp, P, m, tw, lane, nl, dif, d, o); return; }
   }
-  if (!twid) {
+  if constexpr (!TWID && MAXP >= 17) {
+    const int ln = lane & 31, wp = lane >> 5, nw = nl >> 5;
     switch (p) {
-#define FALCON_SPLIT(q, g)                                  \
-  case q:                                                   \
-    if constexpr (q <= MAXP) {                              \
-      fft_stage_split<q, g>(A, Bf, P, m, tid, nt);          \
-      return;                                               \
-    }                                                       \
-    break;
-      FALCON_SPLIT(17, 2) FALCON_SPLIT(19, 2) FALCON_SPLIT(23, 3) FALCON_SPLIT(29, 3) FALCON_SPLIT(31, 3)
-#undef FALCON_SPLIT
+      case 11: fx_mma_stage<11>(buf, P, m, d, frag, ln, wp, nw, o); return;
+      case 13: fx_mma_stage<13>(buf, P, m, d, frag, ln, wp, nw, o); return;
+      case 17: fx_mma_stage<17>(buf, P, m, d, frag, ln, wp, nw, o); return;
       default: break;
     }
+    if constexpr (MAXP == 31) {
+      switch (p) {
+        case 19: fx_mma_stage_wide<19>(buf, P, m, d, frag, ln, wp, nw, o); return;
+        case 23: fx_mma_stage_wide<23>(buf, P, m, d, frag, ln, wp, nw, o); return;
+        case 29: fx_mma_stage_wide<29>(buf, P, m, d, frag, ln, wp, nw, o); return;
+        case 31: fx_mma_stage_wide<31>(buf, P, m, d, frag, ln, wp, nw, o); return;
+        default: break;
+      }
+    }
   }
-  run_stage1<MAXP>(p, dif, twid, mine, P, m, stride, tw, hl, nl);
-  __syncthreads();
+  if constexpr (TWID && MAXP == 31) fx_stage_any(buf, P, p, m, tw, root, lane, nl, dif, d, o);
 }
 
-// ---------------------------------------------------------------------------
-// Nonlinear pass (Nr_maxLOOP, src/nonlin.F90:55-86): one warp per radial
-// line (r, b).  invfft of T, omega, u_phi, u_r (two complex inverse FFTs of
-// length P, each carrying two real fields), the four grid products, and the
-// two forward FFTs that return u_phi*T, u_r*T, u_phi*omega, u_r*omega
-// truncated to modes 0..Nm and divided by P.
-// ---------------------------------------------------------------------------
-// A prime-factor plan of radices <= 17 reads no twiddles (its butterflies
-// take their coefficients from constant memory), so its blocks carry only
-// the index table and the line buffers: 3 blocks of 4 lines fit an SM.
-template <int MAXP>
-constexpr int nonlin_min_blocks() { return MAXP == 17 ? 3 : 1; }
+// The left shift that brings values covered by the high-word bits o (below
+// 2^30) to just below 2^62.
+__device__ __forceinline__ int fx_headroom(unsigned o) { return o ? __clz((int)o) - 2 : 30; }
 
-template <int MAXP>
-__global__ void __launch_bounds__(128, nonlin_min_blocks<MAXP>()) nonlin_kernel(NonlinArgs a) {
-  extern __shared__ double2 smem[];
-  const int P = a.plan.P;
-  const bool no_tw = MAXP == 17 && a.plan.pfa;
-  const int tw_len = no_tw ? 0 : P;
-  double2* tw = smem;
-  int* pos = reinterpret_cast<int*>(smem + tw_len);
-  const int pos_pad = (P + 3) / 4;  // ints rounded up to double2 units (16 B)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nwarp = blockDim.x >> 5;
-  double2* bufA = smem + tw_len + pos_pad + (size_t)warp * 2 * P;
-  double2* bufB = bufA + P;
+// Barrier number first + i (i < COUNT <= 6) for N threads, with immediate
+// ids: a block then holds only the hardware barriers it names.
+template <int ID, int N>
+__device__ __forceinline__ void fx_bar() {
+  asm volatile("bar.sync %0, %1;" ::"n"(ID), "n"(N) : "memory");
+}
+template <int N, int COUNT, int FIRST>
+__device__ __forceinline__ void fx_bar_of(int i) {
+  static_assert(COUNT <= 6, "six barriers at most");
+  if (COUNT > 5 && i == 5) fx_bar<FIRST + 5, N>();
+  else if (COUNT > 4 && i == 4) fx_bar<FIRST + 4, N>();
+  else if (COUNT > 3 && i == 3) fx_bar<FIRST + 3, N>();
+  else if (COUNT > 2 && i == 2) fx_bar<FIRST + 2, N>();
+  else if (COUNT > 1 && i == 1) fx_bar<FIRST + 1, N>();
+  else fx_bar<FIRST, N>();
+}
+
+// Per-line scratch of the kernel: reduction slots of the two halves (the
+// magnitudes' in two sets, used by turns), what the halves exchange, and the
+// velocity maxima.
+template <int S>
+struct alignas(16) FxLine {
+  unsigned eb[2][S][2];
+  unsigned mx[2][2][S][2];
+  unsigned prod[2 * S][2];
+  int head[2][2], exp[2][2], bad[2];
+  unsigned long long umax[2];
+};
+
+// ---------------------------------------------------------------------------
+// Nonlinear pass (Nr_maxLOOP, src/nonlin.F90:55-86).  A radial line (r, b)
+// takes 2 S warps: one half transforms T + i omega, the other u_phi + i u_r
+// (two complex FFTs of length P, each carrying two real fields), the halves
+// meet for the four grid products, and each half transforms two of them
+// back: u_phi T + i u_r T, and u_phi omega + i u_r omega, truncated to modes
+// 0..Nm and divided by P.
+//
+// Values are integers, |V| < 2^61, each of the two packed fields at its own
+// power of two (59 bits from the largest exponent of its line, so neither
+// loses digits to the other's magnitude) and both shifted together before a
+// stage by what its growth can take, from the largest value of the stage
+// before.  The grid values are shifted up to 62 bits (by the largest of each
+// field) before they are multiplied.  Every sum is exact; errors are those
+// of the products with constants (half a unit rms each).  All the maxima behind
+// the scales are integers, so results do not depend on S.  A line with an
+// Inf or NaN input gives NaN.
+//
+// Bound: issue of integer instructions (about half of the cycles) and their
+// latency at the 16 warps an SM that registers and shared memory allow.
+// Against FP64 butterflies on grids of 3 Nm points (radix 11 to 31 on the
+// tensor cores), us for Nr = 65, Nm = 170, 128 instances: 950 -> 200; Nr =
+// 129, Nm = 512, 8: 500 -> 125; one instance of Nr = 97, Nm = 341: 80 -> 30.
+// The error against 64 bits fell from 7e-16 to 4e-16 (products with omega)
+// and from 7e-14 to 4e-16 (with T, which FP64 packed with a larger omega).
+// ---------------------------------------------------------------------------
+template <int MAXP, bool TWID, int S, int LPB, int MINB>
+__global__ void __launch_bounds__(64 * S * LPB, MINB) nonlin_kernel(NonlinArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int NH = 32 * S;  // threads of a half
+  const int P = a.plan.P, M = a.M, B = a.B, Nm = a.Nm;
+  const int PP = a.plan.rad[0] * a.plan.span[0], inner = a.plan.rad[a.plan.nrad - 1];
+  int4* tw = reinterpret_cast<int4*>(smem_raw);
+  longlong2* bufs = reinterpret_cast<longlong2*>(tw + (TWID ? P - inner : 0));
+  FxLine<S>* lines = reinterpret_cast<FxLine<S>*>(bufs + (size_t)LPB * 2 * PP);
+  uint32_t* frag = reinterpret_cast<uint32_t*>(lines + LPB);
+  int nfrag = 0;
+  if constexpr (!TWID && MAXP >= 17) {
+    for (int i = 0; i < a.plan.nrad; ++i) {
+      const uint32_t* src = nullptr;
+      switch (a.plan.rad[i]) {
+        case 11: src = kFxFrag<11>.v; break;
+        case 13: src = kFxFrag<13>.v; break;
+        case 17: src = kFxFrag<17>.v; break;
+        default: break;
+      }
+      if constexpr (MAXP == 31) {
+        switch (a.plan.rad[i]) {
+          case 19: src = kFxFrag<19>.v; break;
+          case 23: src = kFxFrag<23>.v; break;
+          case 29: src = kFxFrag<29>.v; break;
+          case 31: src = kFxFrag<31>.v; break;
+          default: break;
+        }
+      }
+      const int n = fx_frag_ints(a.plan.rad[i]);
+      for (int k = threadIdx.x; k < n; k += blockDim.x) frag[nfrag + k] = src[k];
+      nfrag += n;
+    }
+  }
+  uint16_t* pos = reinterpret_cast<uint16_t*>(frag + nfrag);  // places of the spectrum and of the line's points
+  uint16_t* tab = pos + P;
   for (int i = threadIdx.x; i < P; i += blockDim.x) {
-    if (!no_tw) tw[i] = a.tw[i];
-    pos[i] = a.pos[i];
+    if (TWID && i < P - inner) tw[i] = a.tw[i];
+    const unsigned both = a.pos[i];
+    pos[i] = (uint16_t)both;
+    tab[i] = (uint16_t)(both >> 16);
   }
   __syncthreads();
-  const int nlines = a.R * a.B;
-  const int line = blockIdx.x * nwarp + warp;
-  if (line >= nlines) return;
-  const int r = line / a.B, b = line - r * a.B;
-  const int M = a.M, B = a.B, Nm = a.Nm;
-  for (int j = lane; j < P; j += 32) { bufA[j] = make_double2(0, 0); bufB[j] = make_double2(0, 0); }
-  __syncwarp();
-  // Scatter conj(Z) at digit-reversed positions, Z_k = X_k + i Y_k for the
-  // Hermitian spectra X, Y of two real lines (only Re of mode 0 counts, as
-  // in a c2r transform).  IFFT(Z) = conj(FFT(conj(Z))).
-  const size_t row = (size_t)r * M * B + b;
-  for (int k = lane; k <= Nm; k += 32) {
-    const size_t e = row + (size_t)k * B;
-    const double2 T = a.t[e], W = a.w[e], U = a.up[e], V = a.ur[e];
-    if (k == 0) {
-      bufA[pos[0]] = make_double2(T.x, -W.x);
-      bufB[pos[0]] = make_double2(U.x, -V.x);
+  const int lw = threadIdx.x / (2 * NH), lt = threadIdx.x - lw * 2 * NH;  // line of the block, thread of the line
+  const int half = lt / NH, hl = lt - half * NH, lane = threadIdx.x & 31, hw = hl >> 5;
+  const int line = blockIdx.x * LPB + lw;
+  if (line >= a.R * B) return;
+  // barriers of a half and of a line (immediate ids: a block then holds
+  // only the hardware barriers it names)
+  auto half_sync = [&]() {
+    if constexpr (S == 1) {
+      __syncwarp();
     } else {
-      // conj(Z_k) = (T.x - W.y, -(T.y + W.x)); conj(Z_{P-k}) = (T.x + W.y, T.y - W.x)
-      bufA[pos[k]] = make_double2(T.x - W.y, -(T.y + W.x));
-      bufA[pos[P - k]] = make_double2(T.x + W.y, T.y - W.x);
-      bufB[pos[k]] = make_double2(U.x - V.y, -(U.y + V.x));
-      bufB[pos[P - k]] = make_double2(U.x + V.y, U.y - V.x);
+      fx_bar_of<NH, (S > 1 ? 2 * LPB : 1), 1>(2 * lw + half);
+    }
+  };
+  auto line_sync = [&]() { fx_bar_of<2 * NH, LPB, (S > 1 ? 2 * LPB : 0) + 1>(lw); };
+  FxLine<S>& L = lines[lw];
+  longlong2* bufA = bufs + (size_t)lw * 2 * PP;
+  longlong2* bufB = bufA + PP;
+  longlong2* buf = half ? bufB : bufA;
+  const size_t row = (size_t)(line / B) * M * B + line % B;
+  const double2* X = (half ? a.up : a.t) + row;
+  const double2* Y = (half ? a.ur : a.w) + row;
+
+  // The half's two fields: the first kHeld modes of a thread are read once
+  // and held, longer spectra are read again for the conversion.
+  constexpr int kHeld = 6;
+  double2 xs[kHeld], ys[kHeld];
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    const int k = hl + i * NH;
+    xs[i] = ys[i] = make_double2(0.0, 0.0);
+    if (k <= Nm) {
+      xs[i] = __ldg(X + (size_t)k * B);
+      ys[i] = __ldg(Y + (size_t)k * B);
     }
   }
-  __syncwarp();
-  {  // DIT: radices processed innermost first
-    int m = 1;
-    for (int s = a.plan.nrad - 1; s >= 0; --s) {
-      const int p = a.plan.rad[s];
-      run_stage<MAXP>(p, false, !a.plan.pfa, bufA, bufB, P, m, P / (m * p), tw, lane);
-      m *= p;
+  if (hl == 0) xs[0].y = ys[0].y = 0.0;  // only Re of mode 0 counts, as in a c2r transform
+  // The grid of 3 Nm points folds mode 2 Nm of a product, f_Nm g_Nm, onto
+  // mode -Nm: its conjugate onto mode Nm.  Lane i < 4 of the half adds
+  // component i of the two products' (re, im).
+  const bool alias = P != 3 * Nm;
+  double fold = 0.0;
+  if (alias && hl < 4) {
+    const size_t e = row + (size_t)Nm * B;
+    const double2 F = __ldg((half ? a.w : a.t) + e), G = __ldg((hl < 2 ? a.up : a.ur) + e);
+    fold = (hl & 1) ? -(F.x * G.y + F.y * G.x) : F.x * G.x - F.y * G.y;
+  }
+  // the largest high word of each field's magnitudes: its biased exponent, 0
+  // for a field of zeros
+  unsigned ex = 0, ey = 0;
+  auto high = [](double2 v) {
+    return max((unsigned)__double2hiint(v.x) & 0x7fffffffu, (unsigned)__double2hiint(v.y) & 0x7fffffffu);
+  };
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i) {
+    ex = max(ex, high(xs[i]));
+    ey = max(ey, high(ys[i]));
+  }
+  for (int k = hl + kHeld * NH; k <= Nm; k += NH) {
+    ex = max(ex, high(__ldg(X + (size_t)k * B)));
+    ey = max(ey, high(__ldg(Y + (size_t)k * B)));
+  }
+  ex = __reduce_max_sync(FULL, ex);
+  ey = __reduce_max_sync(FULL, ey);
+  if constexpr (S > 1) {
+    if (lane == 0) { L.eb[half][hw][0] = ex; L.eb[half][hw][1] = ey; }
+    half_sync();
+#pragma unroll
+    for (int i = 0; i < S; ++i) { ex = max(ex, L.eb[half][i][0]); ey = max(ey, L.eb[half][i][1]); }
+  }
+  const bool bad = ex >= 0x7ff00000u || ey >= 0x7ff00000u;
+  // products with a field of zeros are zeros: whatever the other field packed
+  // with it leaves there, an exponent below all numbers
+  const int zx = ex ? 0 : 1 << 20, zy = ey ? 0 : 1 << 20;
+  ex = bad ? 4095u : max(ex >> 20, 1u);  // (4095: every value shifts to zero)
+  ey = bad ? 4095u : max(ey >> 20, 1u);
+  // Scatter conj(Z) at digit-reversed positions, Z_k = X_k + i Y_k for the
+  // Hermitian spectra X, Y of two real lines.  IFFT(Z) = conj(FFT(conj(Z))).
+  auto scatter = [&](int k, double2 x, double2 y) {
+    auto fix = [&](double v, unsigned eb) -> long long {
+      const unsigned long long bits = (unsigned long long)__double_as_longlong(v);
+      const unsigned long long t = fx_mag_of(bits, (int)eb);
+      return (long long)bits < 0 ? -(long long)t : (long long)t;
+    };
+    const long long xr = fix(x.x, ex), yr = fix(y.x, ey), xi = fix(x.y, ex), yi = fix(y.y, ey);
+    buf[pos[k]] = fx_make(xr - yi, -(xi + yr));
+    if (k) buf[pos[P - k]] = fx_make(xr + yi, xi - yr);
+  };
+#pragma unroll
+  for (int i = 0; i < kHeld; ++i)
+    if (hl + i * NH <= Nm) scatter(hl + i * NH, xs[i], ys[i]);
+  for (int k = hl + kHeld * NH; k <= Nm; k += NH) scatter(k, __ldg(X + (size_t)k * B), __ldg(Y + (size_t)k * B));
+  for (int k = Nm + 1 + hl; k < P - Nm; k += NH) buf[pos[k]] = fx_make(0, 0);
+  half_sync();
+  // values are V 2^(E + e), e = ex - 1022 - 59 for the first field, ey - ...
+  // for the second; every component is below 2^60
+  int E = 0, bits = 60, turn = 0;
+  FxMax o{0, 0};
+  auto stage = [&](int s, int m, const uint32_t* fr, const int4* root, bool dif) {
+    const int p = a.plan.rad[s];
+    const int d = bits + fx_growth(p) - 61;
+    E += d;
+    o = FxMax{0, 0};
+    fx_run_stage<MAXP, TWID>(p, buf, tab, a.plan.span[s], P, m, tw + (m - inner), root, fr, hl, NH, dif, d, o);
+    o.x = __reduce_or_sync(FULL, o.x);
+    o.y = __reduce_or_sync(FULL, o.y);
+    if constexpr (S > 1) {
+      if (lane == 0) { L.mx[turn][half][hw][0] = o.x; L.mx[turn][half][hw][1] = o.y; }
+      half_sync();
+#pragma unroll
+      for (int i = 0; i < S; ++i) { o.x |= L.mx[turn][half][i][0]; o.y |= L.mx[turn][half][i][1]; }
+      turn ^= 1;
+    } else {
       __syncwarp();
     }
-  }
-  // Grid values: bufA = conj(t + i omg) -> t = A.x, omg = -A.y; likewise for
-  // (u_phi, u_r) in bufB.  Products, in natural order for the DIF.
-  double urmax = 0.0, upmax = 0.0;
-  const bool want_max = a.umax != nullptr;
-  for (int j = lane; j < P; j += 32) {
-    const double2 za = bufA[j], zb = bufB[j];
-    const double tt = za.x, om = -za.y, up = zb.x, ur = -zb.y;
-    bufA[j] = make_double2(up * tt, ur * tt);
-    bufB[j] = make_double2(up * om, ur * om);
-    if (want_max) {  // FP64 max instructions only when the CFL inputs are read
-      urmax = fmax(urmax, fabs(ur));
-      upmax = fmax(upmax, fabs(up));
+    bits = fx_bits(o.x | o.y);
+  };
+  {  // DIT: radices processed innermost first
+    int m = 1, f = nfrag;
+    const int4* root = a.tw + fx_table_size(a.plan);
+    for (int s = a.plan.nrad - 1; s >= 0; --s) {
+      const int p = a.plan.rad[s];
+      f -= fx_frag_ints(p);
+      root -= fx_root_size(a.plan, p);
+      stage(s, m, frag + f, root, false);
+      m *= p;
     }
   }
-  __syncwarp();
+  if (hl == 0) {
+    L.head[half][0] = fx_headroom(o.x);
+    L.head[half][1] = fx_headroom(o.y);
+    L.exp[half][0] = E + (int)ex - 1081 - zx;
+    L.exp[half][1] = E + (int)ey - 1081 - zy;
+    L.bad[half] = bad;
+    L.umax[half] = 0;
+  }
+  line_sync();
+  // Grid values: bufA = conj(t + i omg) -> t = A.x, omg = -A.y; likewise for
+  // (u_phi, u_r) in bufB.  Products, in natural order for the DIF.
+  const int ht = L.head[0][0], ho = L.head[0][1], hp = L.head[1][0], hr = L.head[1][1];
+  const int e_half = L.exp[0][half] - (half ? ho : ht) + 64;  // of T, omega (in the products of this half)
+  const int e1 = e_half + L.exp[1][0] - hp, e2 = e_half + L.exp[1][1] - hr;
+  const bool any_bad = L.bad[0] || L.bad[1];
+  unsigned long long urmax = 0, upmax = 0;
+  FxMax oA{0, 0}, oB{0, 0};
+  for (int j = lt; j < P; j += 2 * NH) {
+    const int at = tab[j];
+    const longlong2 za = bufA[at], zb = bufB[at];
+    const long long tt = za.x << ht, om = -(za.y << ho), up = zb.x << hp, ur = -(zb.y << hr);
+    const longlong2 pa = fx_make(fx_mulhi(up, tt), fx_mulhi(ur, tt)), pb = fx_make(fx_mulhi(up, om), fx_mulhi(ur, om));
+    bufA[at] = pa;
+    bufB[at] = pb;
+    fx_cover(oA, pa);
+    fx_cover(oB, pb);
+    if (a.umax) {  // only when the CFL inputs are read
+      urmax = max(urmax, (unsigned long long)(zb.y < 0 ? -zb.y : zb.y));
+      upmax = max(upmax, (unsigned long long)(zb.x < 0 ? -zb.x : zb.x));
+    }
+  }
+  const unsigned ma = __reduce_or_sync(FULL, oA.x | oA.y), mb = __reduce_or_sync(FULL, oB.x | oB.y);
+  if (lane == 0) { L.prod[lt >> 5][0] = ma; L.prod[lt >> 5][1] = mb; }
+  if (a.umax) {
+#pragma unroll
+    for (int w = 16; w > 0; w >>= 1) {
+      urmax = max(urmax, __shfl_xor_sync(FULL, urmax, w));
+      upmax = max(upmax, __shfl_xor_sync(FULL, upmax, w));
+    }
+    if (lane == 0) {
+      atomicMax(&L.umax[0], urmax);
+      atomicMax(&L.umax[1], upmax);
+    }
+  }
+  line_sync();
+  if (a.umax && lt == 0) {
+    a.umax[2 * (size_t)line] = L.bad[1] ? 0.0 : ldexp((double)L.umax[0], L.exp[1][1]);
+    a.umax[2 * (size_t)line + 1] = L.bad[1] ? 0.0 : ldexp((double)L.umax[1], L.exp[1][0]);
+  }
+  {
+    unsigned w = 0;
+#pragma unroll
+    for (int i = 0; i < 2 * S; ++i) w |= L.prod[i][half];
+    bits = fx_bits(w);
+  }
+  E = 0;
   {  // DIF: outermost radix first
-    int m = P;
+    int m = P, f = 0;
+    const int4* root = a.tw + P;
     for (int s = 0; s < a.plan.nrad; ++s) {
       const int p = a.plan.rad[s];
       m /= p;
-      run_stage<MAXP>(p, true, !a.plan.pfa, bufA, bufB, P, m, P / (m * p), tw, lane);
-      __syncwarp();
+      stage(s, m, frag + f, root, true);
+      f += fx_frag_ints(p);
+      root += fx_root_size(a.plan, p);
     }
   }
   // Split the two-for-one spectra: X_k = (Z_k + conj Z_{P-k})/2,
-  // Y_k = (Z_k - conj Z_{P-k})/(2i), then divide by P.
-  const double s = 0.5 / (double)P;
-  for (int k = lane; k <= Nm; k += 32) {
-    const size_t e = row + (size_t)k * B;
-    const double2 za = bufA[pos[k]], ca = bufA[pos[k == 0 ? 0 : P - k]];
-    const double2 zb = bufB[pos[k]], cb = bufB[pos[k == 0 ? 0 : P - k]];
-    a.ntp[e] = make_double2((za.x + ca.x) * s, (za.y - ca.y) * s);
-    a.ntr[e] = make_double2((za.y + ca.y) * s, (ca.x - za.x) * s);
-    a.nwp[e] = make_double2((zb.x + cb.x) * s, (zb.y - cb.y) * s);
-    a.nwr[e] = make_double2((zb.y + cb.y) * s, (cb.x - zb.x) * s);
-  }
-  if (a.umax) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      urmax = fmax(urmax, __shfl_xor_sync(0xffffffffu, urmax, o));
-      upmax = fmax(upmax, __shfl_xor_sync(0xffffffffu, upmax, o));
+  // Y_k = (Z_k - conj Z_{P-k})/(2i), then divide by P: an odd P's factor in
+  // fixed point, the power of two in the exponent
+  const int sh = 31 - __clz(P), odd = P & (P - 1);  // P = 2^sh (1 + ...)
+  const FxC over = a.over_p;                          // 2^sh / P
+  const int x1 = e1 + E - sh - 1, x2 = e2 + E - sh - 1;
+  double* o1 = reinterpret_cast<double*>((half ? a.nwp : a.ntp) + row);
+  double* o2 = reinterpret_cast<double*>((half ? a.nwr : a.ntr) + row);
+  auto part = [&](int k, int i) {  // component i of mode k's (u, v) as an integer
+    const longlong2 z = buf[pos[k]], c = buf[pos[k == 0 ? 0 : P - k]];
+    const long long v = i == 0 ? z.x + c.x : i == 1 ? z.y - c.y : i == 2 ? z.y + c.y : c.x - z.x;
+    return odd ? fx_mul(fx_prep(v >> 1), over) * 2 : v;
+  };
+  const int last = alias ? Nm - 1 : Nm;
+  if (!any_bad && min(x1, x2) > -960 && max(x1, x2) < 960) {  // every result is a normal number or zero
+    auto to_double = [&](long long v, int x) {
+      const double r = (double)v;
+      return v ? __hiloint2double(__double2hiint(r) + (x << 20), __double2loint(r)) : 0.0;
+    };
+    for (int k = hl; k <= last; k += NH) {
+      const size_t e = (size_t)k * B;
+      reinterpret_cast<double2*>(o1)[e] = make_double2(to_double(part(k, 0), x1), to_double(part(k, 1), x1));
+      reinterpret_cast<double2*>(o2)[e] = make_double2(to_double(part(k, 2), x2), to_double(part(k, 3), x2));
     }
-    if (lane == 0) {
-      a.umax[2 * ((size_t)r * B + b)] = urmax;
-      a.umax[2 * ((size_t)r * B + b) + 1] = upmax;
-    }
+    if (alias && hl < 4)
+      (hl < 2 ? o1 : o2)[2 * (size_t)Nm * B + (hl & 1)] = to_double(part(Nm, hl), hl < 2 ? x1 : x2) + fold;
+  } else {
+    for (int k = hl; k <= Nm; k += NH)
+      for (int i = 0; i < 4; ++i)
+        (i < 2 ? o1 : o2)[2 * (size_t)k * B + (i & 1)] =
+            any_bad ? __longlong_as_double(0x7ff8000000000000LL) : ldexp((double)part(k, i), i < 2 ? x1 : x2);
+    half_sync();
+    if (alias && hl < 4) (hl < 2 ? o1 : o2)[2 * (size_t)Nm * B + (hl & 1)] += fold;
   }
 }
 
-// Block-per-line form of the same pass, for launches with too few radial
-// lines to fill the GPU at one warp per line (one instance, or a small
-// group): the (T, omega) and (u_phi, u_r) transforms run on the two halves of
-// the block, each spread over S warps, with block barriers between stages.
-// Same arithmetic per element as nonlin_kernel (bit-identical results).
-template <int MAXP, int S>
-__global__ void __launch_bounds__(64 * S) nonlin_line_kernel(NonlinArgs a) {
-  extern __shared__ double2 smem[];
-  __shared__ double red[2][2 * S];
+template <int MAXP, bool TWID, int S, int LPB, int MINB>
+static cudaError_t launch_nonlin_s(const NonlinArgs& a, cudaStream_t s) {
   const int P = a.plan.P;
-  double2* tw = smem;
-  int* pos = reinterpret_cast<int*>(smem + P);
-  const int pos_pad = (P + 3) / 4;
-  double2* bufA = smem + P + pos_pad;
-  double2* bufB = bufA + P;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int nl = 32 * S, half = tid / nl, hl = tid - half * nl;
-  double2* mine = half ? bufB : bufA;
-  for (int i = tid; i < P; i += nt) {
-    tw[i] = a.tw[i];
-    pos[i] = a.pos[i];
-    bufA[i] = make_double2(0, 0);
-    bufB[i] = make_double2(0, 0);
-  }
-  __syncthreads();
-  const int line = blockIdx.x;
-  const int r = line / a.B, b = line - r * a.B;
-  const int M = a.M, B = a.B, Nm = a.Nm;
-  const size_t row = (size_t)r * M * B + b;
-  for (int k = tid; k <= Nm; k += nt) {
-    const size_t e = row + (size_t)k * B;
-    const double2 T = a.t[e], W = a.w[e], U = a.up[e], V = a.ur[e];
-    if (k == 0) {
-      bufA[pos[0]] = make_double2(T.x, -W.x);
-      bufB[pos[0]] = make_double2(U.x, -V.x);
-    } else {
-      bufA[pos[k]] = make_double2(T.x - W.y, -(T.y + W.x));
-      bufA[pos[P - k]] = make_double2(T.x + W.y, T.y - W.x);
-      bufB[pos[k]] = make_double2(U.x - V.y, -(U.y + V.x));
-      bufB[pos[P - k]] = make_double2(U.x + V.y, U.y - V.x);
-    }
-  }
-  __syncthreads();
-  {
-    int m = 1;
-    for (int s = a.plan.nrad - 1; s >= 0; --s) {
-      const int p = a.plan.rad[s];
-      run_stage_block<MAXP>(p, false, !a.plan.pfa, bufA, bufB, mine, P, m, P / (m * p), tw, tid, nt, hl, nl);
-      m *= p;
-    }
-  }
-  double urmax = 0.0, upmax = 0.0;
-  const bool want_max = a.umax != nullptr;
-  for (int j = tid; j < P; j += nt) {
-    const double2 za = bufA[j], zb = bufB[j];
-    const double tt = za.x, om = -za.y, up = zb.x, ur = -zb.y;
-    bufA[j] = make_double2(up * tt, ur * tt);
-    bufB[j] = make_double2(up * om, ur * om);
-    if (want_max) {  // FP64 max instructions only when the CFL inputs are read
-      urmax = fmax(urmax, fabs(ur));
-      upmax = fmax(upmax, fabs(up));
-    }
-  }
-  __syncthreads();
-  {
-    int m = P;
-    for (int s = 0; s < a.plan.nrad; ++s) {
-      const int p = a.plan.rad[s];
-      m /= p;
-      run_stage_block<MAXP>(p, true, !a.plan.pfa, bufA, bufB, mine, P, m, P / (m * p), tw, tid, nt, hl, nl);
-    }
-  }
-  const double sc = 0.5 / (double)P;
-  for (int k = tid; k <= Nm; k += nt) {
-    const size_t e = row + (size_t)k * B;
-    const double2 za = bufA[pos[k]], ca = bufA[pos[k == 0 ? 0 : P - k]];
-    const double2 zb = bufB[pos[k]], cb = bufB[pos[k == 0 ? 0 : P - k]];
-    a.ntp[e] = make_double2((za.x + ca.x) * sc, (za.y - ca.y) * sc);
-    a.ntr[e] = make_double2((za.y + ca.y) * sc, (ca.x - za.x) * sc);
-    a.nwp[e] = make_double2((zb.x + cb.x) * sc, (zb.y - cb.y) * sc);
-    a.nwr[e] = make_double2((zb.y + cb.y) * sc, (cb.x - zb.x) * sc);
-  }
-  if (a.umax) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      urmax = fmax(urmax, __shfl_xor_sync(0xffffffffu, urmax, o));
-      upmax = fmax(upmax, __shfl_xor_sync(0xffffffffu, upmax, o));
-    }
-    const int w = tid >> 5;
-    if ((tid & 31) == 0) { red[0][w] = urmax; red[1][w] = upmax; }
-    __syncthreads();
-    if (tid == 0) {
-      for (int i = 1; i < 2 * S; ++i) { urmax = fmax(urmax, red[0][i]); upmax = fmax(upmax, red[1][i]); }
-      a.umax[2 * ((size_t)r * B + b)] = urmax;
-      a.umax[2 * ((size_t)r * B + b) + 1] = upmax;
-    }
-  }
-}
-
-static int nonlin_warps(int P, bool no_tw, int* smem_bytes) {
-  int dev = 0, maxsm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  const int fixed = ((no_tw ? 0 : P) + (P + 3) / 4) * 16;
-  int w = 4;
-  while (w > 1 && fixed + w * 2 * P * 16 > maxsm) --w;
-  *smem_bytes = fixed + w * 2 * P * 16;
-  return w;
-}
-
-template <int MAXP, int S>
-static cudaError_t launch_nonlin_line(const NonlinArgs& a, cudaStream_t s) {
-  const int P = a.plan.P;
-  const int smem = (P + (P + 3) / 4 + 2 * P) * 16;
-  cudaError_t e = cudaFuncSetAttribute(nonlin_line_kernel<MAXP, S>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  if (P > kMaxLine) return cudaErrorInvalidValue;
+  int frag = 0;
+  if (!TWID)
+    for (int i = 0; i < a.plan.nrad; ++i) frag += fx_frag_ints(a.plan.rad[i]);
+  const int PP = a.plan.rad[0] * a.plan.span[0];
+  const int smem = (TWID ? P - a.plan.rad[a.plan.nrad - 1] : 0) * 16 + LPB * (2 * PP * 16 + (int)sizeof(FxLine<S>)) +
+                   4 * (frag + (P + 3) / 4 * 4);
+  const cudaError_t e = cudaFuncSetAttribute(nonlin_kernel<MAXP, TWID, S, LPB, MINB>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  nonlin_line_kernel<MAXP, S><<<a.R * a.B, 64 * S, smem, s>>>(a);
-  return cudaGetLastError();
-}
-
-// Resident warps per SM of the warp-per-line form (w warps a block, smem
-// bytes) and of the block-per-line form with 8 warps a line, from the
-// occupancy calculator; memoised per (form, P).
-template <int MAXP>
-static bool line_form_holds_more_warps(int P, int w, int smem) {
-  struct Memo { int P, w, smem; bool line; };
-  thread_local std::vector<Memo> memo;
-  for (const Memo& m : memo)
-    if (m.P == P && m.w == w && m.smem == smem) return m.line;
-  const int smem_line = (P + (P + 3) / 4 + 2 * P) * 16;
-  int nb_warp = 0, nb_line = 0;
-  bool line = false;
-  if (cudaFuncSetAttribute(nonlin_kernel<MAXP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-      cudaFuncSetAttribute(nonlin_line_kernel<MAXP, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_line) ==
-          cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb_warp, nonlin_kernel<MAXP>, 32 * w, smem) == cudaSuccess &&
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb_line, nonlin_line_kernel<MAXP, 4>, 256, smem_line) ==
-          cudaSuccess)
-    line = nb_line * 8 > nb_warp * w;
-  memo.push_back(Memo{P, w, smem, line});
-  return line;
-}
-
-// Lines that one warp each cannot spread over the GPU (fewer than two per
-// SM) go to the block-per-line form: 8 warps per line up to one line per
-// SM, 4 up to two.  So do long lines whose warp-per-line blocks (a whole
-// line per warp in shared memory) would leave fewer warps on an SM than the
-// block-per-line form (Np = 1023, 1536: 3-4 against 16 warps per SM).
-template <int MAXP>
-static cudaError_t launch_nonlin_t(const NonlinArgs& a, cudaStream_t s) {
-  int dev = 0, nsm = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const int nlines = a.R * a.B;
-  if (nlines <= nsm) return launch_nonlin_line<MAXP, 4>(a, s);
-  if (nlines <= 2 * nsm) return launch_nonlin_line<MAXP, 2>(a, s);
-  int smem = 0;
-  const int w = nonlin_warps(a.plan.P, MAXP == 17 && a.plan.pfa, &smem);
-  if (line_form_holds_more_warps<MAXP>(a.plan.P, w, smem)) return launch_nonlin_line<MAXP, 4>(a, s);
-  cudaError_t e = cudaFuncSetAttribute(nonlin_kernel<MAXP>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
-  const int grid = (nlines + w - 1) / w;
-  nonlin_kernel<MAXP><<<grid, 32 * w, smem, s>>>(a);
+  nonlin_kernel<MAXP, TWID, S, LPB, MINB><<<(a.R * a.B + LPB - 1) / LPB, 64 * S * LPB, smem, s>>>(a);
   return cudaGetLastError();
 }
 

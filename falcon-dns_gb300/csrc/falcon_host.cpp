@@ -807,13 +807,51 @@ int scheme_weights(int type, int imp, int exp, Scheme* s) {
 // ---------------------------------------------------------------------------
 }  // namespace
 
-void falcon::fft_tables_host(const FftPlan& plan, double2* tw, int* pos) {
+void falcon::fft_tables_host(const FftPlan& plan, int4* tw, unsigned* pos) {
   const int P = plan.P;
-  const double two_pi = 8.0 * std::atan(1.0);
+  std::vector<unsigned> place(P);  // of element i in the buffer
   for (int i = 0; i < P; ++i) {
-    pos[i] = fft_position(plan, i);
-    const double a = two_pi * (double)i / (double)P;
-    tw[i] = make_double2(std::cos(a), -std::sin(a));
+    unsigned at = 0;
+    for (int s = plan.nrad - 1, x = i; s >= 0; x /= plan.rad[s--]) at += (unsigned)(x % plan.rad[s] * plan.span[s]);
+    place[i] = at;
+  }
+  for (int i = 0; i < P; ++i) pos[i] = place[fft_position(plan, i)] | place[i] << 16;
+  if (plan.pfa) return;
+  // exp(-2 pi i n/P): the angle (pi/2) a/P, a in [0, 4P), reduced to the
+  // first octant in integers, where cos and sin are rounded to Q61 (the
+  // products take an even Q62 constant) once per angle
+  const double half_pi = 2.0 * std::atan(1.0);
+  std::vector<long long> oct(2 * (size_t)(P / 2 + 1), -1);
+  std::vector<int4> all(P);
+  for (int i = 0; i < P; ++i) {
+    int a = 4 * i;
+    const bool neg_s = a > 2 * P;
+    if (neg_s) a = 4 * P - a;
+    const bool neg_c = a > P;
+    if (neg_c) a = 2 * P - a;
+    const bool swap = 2 * a > P;
+    if (swap) a = P - a;
+    long long* q = &oct[2 * (size_t)a];
+    if (q[0] < 0) {
+      const double t = half_pi * (double)a / (double)P;
+      q[0] = 2 * std::llrint(std::cos(t) * 0x1p61);
+      q[1] = 2 * std::llrint(std::sin(t) * 0x1p61);
+    }
+    const long long c = swap ? q[1] : q[0], s = swap ? q[0] : q[1];
+    all[i] = fx_twiddle(neg_c ? -c : c, neg_s ? s : -s);
+  }
+  const int inner = plan.rad[plan.nrad - 1];
+  for (int s = plan.nrad - 2, m = inner; s >= 0; --s) {
+    const int p = plan.rad[s], stride = P / (m * p);
+    for (int q = 1; q < p; ++q)
+      for (int k = 0; k < m; ++k) tw[m - inner + (q - 1) * m + k] = all[q * k * stride];
+    m *= p;
+  }
+  int at = P;
+  for (int s = 0; s < plan.nrad; ++s) {
+    const int n = fx_root_size(plan, plan.rad[s]);
+    for (int j = 0; j < n; ++j) tw[at + j] = all[j * (P / n)];
+    at += n;
   }
 }
 
@@ -821,17 +859,22 @@ namespace {
 
 struct FftTables {
   FftPlan plan{};
-  double2* tw = nullptr;
-  int* pos = nullptr;
+  int4* tw = nullptr;
+  unsigned* pos = nullptr;
   ~FftTables() { cudaFree(tw); cudaFree(pos); }
 };
 
-int make_fft(int P, std::unique_ptr<FftTables>* out) {
+// The transform for 3 Nm azimuthal points: with `grid` on exactly these
+// points (the velocity maxima of a variable time step are taken on them),
+// else of the cheapest length (make_line_plan).
+int make_fft(int Nm, bool grid, std::unique_ptr<FftTables>* out) {
   auto f = std::make_unique<FftTables>();
-  if (make_fft_plan(P, &f->plan) != 0)
+  if (make_fft_plan(3 * Nm, &f->plan) != 0)
     return fail(FALCON_EINVAL, "azimuthal length 3*Nm has a prime factor above 64 or too many factors");
-  std::vector<int> pos(P);
-  std::vector<double2> tw(P);
+  if (!grid) make_line_plan(Nm, kMaxPadded, &f->plan);
+  const int P = f->plan.P;
+  std::vector<unsigned> pos(P);
+  std::vector<int4> tw(fx_table_size(f->plan));
   fft_tables_host(f->plan, tw.data(), pos.data());
   int rc;
   if ((rc = upload(&f->tw, tw, nullptr))) return rc;
@@ -1124,7 +1167,7 @@ int group_init(Group* g, const std::vector<falcon_params>& ps, const std::vector
   for (size_t k = 1; k < g->subs.size(); ++k)
     if ((rc = build_opset(key_of(ps[members[g->subs[k].b0]], g->sch), &g->subs[k].ops))) return rc;
   if ((rc = build_stage_ops(g, g->p.dt))) return rc;
-  if ((rc = make_fft(g->P, &g->fft))) return rc;
+  if ((rc = make_fft(g->Nm, g->p.l_vartimestep != 0, &g->fft))) return rc;
   if ((rc = oz_scratch_init(g))) return rc;
   const size_t n = g->nel();
   const int R = g->R, B = g->B;
@@ -1731,7 +1774,7 @@ int elementwise(Group* g, double flops_per_el, std::function<cudaError_t()> f) {
 int run_nonlin(Group* g) {
   NonlinArgs a{};
   a.R = g->R; a.M = g->M; a.B = g->B; a.Nm = g->Nm;
-  a.plan = g->fft->plan; a.tw = g->fft->tw; a.pos = g->fft->pos;
+  a.plan = g->fft->plan; a.tw = g->fft->tw; a.pos = g->fft->pos; a.over_p = fx_over(a.plan.P);
   a.t = g->T(); a.w = g->W(); a.up = g->up; a.ur = g->ur;
   a.ntp = g->ntp; a.ntr = g->ntr; a.nwp = g->nwp; a.nwr = g->nwr;
   a.umax = g->vardt ? g->umax : nullptr;
@@ -3254,7 +3297,6 @@ static int batch_create(const falcon_params* ps, int n, falcon_batch** out) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
     return fail(FALCON_ECUDA, "no CUDA device: the GB300 library has no CPU fallback");
-  CK(init_dft_tables());
   std::unique_ptr<falcon_batch> b(new falcon_batch());
   b->params.assign(ps, ps + n);
   CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
@@ -3857,13 +3899,12 @@ int falcon_nonlin_dev(int nr, int nm, int nb, const double* t_dev, const double*
                       const double* ur_dev, double* uphi_t_dev, double* ur_t_dev, double* uphi_omg_dev,
                       double* ur_omg_dev, void* stream) {
   if (nr < 1 || nm < 1 || nb < 1) return fail(FALCON_EINVAL, "invalid sizes");
-  CK(init_dft_tables());
   std::unique_ptr<FftTables> f;
-  int rc = make_fft(3 * nm, &f);
+  int rc = make_fft(nm, false, &f);
   if (rc) return rc;
   NonlinArgs a{};
   a.R = nr; a.M = nm + 1; a.B = nb; a.Nm = nm;
-  a.plan = f->plan; a.tw = f->tw; a.pos = f->pos;
+  a.plan = f->plan; a.tw = f->tw; a.pos = f->pos; a.over_p = fx_over(a.plan.P);
   a.t = reinterpret_cast<const double2*>(t_dev); a.w = reinterpret_cast<const double2*>(omg_dev);
   a.up = reinterpret_cast<const double2*>(up_dev); a.ur = reinterpret_cast<const double2*>(ur_dev);
   a.ntp = reinterpret_cast<double2*>(uphi_t_dev); a.ntr = reinterpret_cast<double2*>(ur_t_dev);
@@ -4152,7 +4193,6 @@ int falcon_server_create(size_t hbm_budget_bytes, int max_active, falcon_server*
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
     return fail(FALCON_ECUDA, "no CUDA device: the GB300 library has no CPU fallback");
-  CK(init_dft_tables());
   auto* s = new falcon_server();
   s->budget = hbm_budget_bytes;
   s->max_active = max_active > 0 ? max_active : (1 << 30);

@@ -12,9 +12,13 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "falcon_fixed.h"
+
 namespace falcon {
 
 constexpr int kMaxRadix = 16;     // stages of a mixed-radix FFT plan
+constexpr int kMaxLine = 4464;    // longest azimuthal transform (a line and its tables in shared memory)
+constexpr int kMaxPadded = 4096;  // the same with padding
 constexpr int kMaxStages = 8;     // IMEXRK stages supported (KC885 has 8)
 
 // Plan of the azimuthal transform of length P = 3*Nm.  Two forms:
@@ -31,6 +35,7 @@ struct FftPlan {
   int pfa;
   int rad[kMaxRadix];   // radices / axis sizes, outermost first
   int cinv[kMaxRadix];
+  int span[kMaxRadix];  // distance of an axis' elements in the line's buffer (padded: make_line_plan)
 };
 
 // Builds the plan for length P (host).  Returns 0, or -1 when P has a prime
@@ -71,10 +76,16 @@ inline int make_fft_plan(int P, FftPlan* plan) {
       f.cinv[i] = (Nd == 1) ? 0 : c;
     }
   } else {
-    int k = 0;
-    n = P;
-    while (n % 4 == 0 && k < kMaxRadix) { f.rad[k++] = 4; n /= 4; }
-    while (n % 2 == 0 && k < kMaxRadix) { f.rad[k++] = 2; n /= 2; }
+    // powers of two as 8s, with 4s or a 2 for the rest (6 takes an odd 2 and
+    // a 3): the fewest passes over the line
+    int k = 0, twos = 0;
+    for (n = P; n % 2 == 0; n /= 2) ++twos;
+    if (twos % 3 == 1 && n % 3 == 0) { f.rad[k++] = 6; n /= 3; twos -= 1; }
+    for (; twos > 0 && k < kMaxRadix; ++k) {
+      const int e = twos == 1 ? 1 : twos == 2 || twos == 4 ? 2 : 3;
+      f.rad[k] = 1 << e;
+      twos -= e;
+    }
     for (int q = 3; q * q <= n && k < kMaxRadix; q += 2)
       while (n % q == 0 && k < kMaxRadix) { f.rad[k++] = q; n /= q; }
     if (n > 1) {
@@ -84,7 +95,48 @@ inline int make_fft_plan(int P, FftPlan* plan) {
     if (n > 1 && n > 64) return -1;
     f.nrad = k;
   }
+  for (int i = f.nrad - 1, m = 1; i >= 0; m *= f.rad[i--]) f.span[i] = m;
   *plan = f;
+  return 0;
+}
+
+// The transform of the nonlinear pass for modes 0..Nm of a line.  Every
+// length P' > 3 Nm gives the products' modes 0..Nm free of aliasing; the
+// reference's grid P = 3 Nm adds to mode Nm the aliased mode 2 Nm, conj(f_Nm
+// g_Nm), which the kernel does by itself when P' /= P.  So the length is
+// free: the cheapest with radices up to 8 on the FFT's instruction counts
+// per point (measured: 30, 44, 27, 59, 43, 87, 32 for radices 2 to 8, ~20 for
+// a stage's twiddles), at most `most` points.  Nm = 170: 512 = 8 x 8 x 8, 134
+// instructions per point, against 302 for 510 = 6 x 5 x 17.  Returns -1 when
+// there is none.
+inline int make_line_plan(int Nm, int most, FftPlan* plan) {
+  const int P = 3 * Nm;
+  static const int cost[9] = {0, 0, 30, 44, 27, 59, 43, 87, 32};
+  long best = 0;
+  for (int odd = 1; odd <= 63; odd += 2) {
+    int n = odd;
+    for (int q : {3, 5, 7})
+      while (n % q == 0) n /= q;
+    if (n != 1) continue;
+    long q = odd;
+    while (q < P) q *= 2;
+    for (; q <= 2L * P + 2 && q <= most; q *= 2) {
+      FftPlan f;
+      if (make_fft_plan((int)q, &f) != 0 || f.pfa) continue;
+      long c = 20L * (f.nrad - 1);
+      for (int i = 0; i < f.nrad; ++i) c += cost[f.rad[i]];
+      c *= q;
+      if (best == 0 || c < best) {
+        best = c;
+        *plan = f;
+      }
+    }
+  }
+  if (!best) return -1;
+  // Odd distances: lanes that differ in one axis (the butterflies of a stage,
+  // the digit-reversed spectrum) read different shared-memory banks.
+  plan->span[plan->nrad - 1] = 1;
+  for (int i = plan->nrad - 2; i >= 0; --i) plan->span[i] = (plan->rad[i + 1] * plan->span[i + 1]) | 1;
   return 0;
 }
 
@@ -111,21 +163,40 @@ inline int fft_position(const FftPlan& f, int k) {
   return pp;
 }
 
-// Tables of the transform of length plan.P, built on the host (falcon_host.cpp):
-// tw[k] = exp(-2 pi i k/P) from the host's cos/sin and pos[k] =
-// fft_position(plan, k).  Every entry point that runs the nonlinear pass
-// takes its tables from here, so they all use the same bits.
-void fft_tables_host(const FftPlan& plan, double2* tw, int* pos);
+// Tables of the transform of length plan.P, built on the host (falcon_host.cpp)
+// from the host's cos/sin of the first octant, in Q62:
+//  - tw, twiddled plans only (fx_twiddle, falcon_fixed.h): per stage of span m
+//    (innermost first, without m = 1) exp(-2 pi i q k/(m p)) at
+//    m - rad[nrad - 1] + (q - 1) m + k, and from entry P on the roots
+//    exp(-2 pi i j/p) of each radix above 8;
+//  - pos[i]: the place in the line's buffer of spectral index i (low half) and
+//    of element i (high half).
+// Every entry point that runs the nonlinear pass takes its tables from here,
+// so they all use the same bits.
+void fft_tables_host(const FftPlan& plan, int4* tw, unsigned* pos);
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int fx_root_size(const FftPlan& f, int p) { return !f.pfa && p > 8 ? p : 0; }
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int fx_table_size(const FftPlan& f) {
+  int n = f.P;
+  for (int i = 0; i < f.nrad; ++i) n += fx_root_size(f, f.rad[i]);
+  return n;
+}
 
 // Arguments of the nonlinear-pass kernel (Nr_maxLOOP, src/nonlin.F90:35-91).
 struct NonlinArgs {
   int R, M, B, Nm;
   FftPlan plan;
-  const double2* tw;    // exp(-2 pi i k/P), k < P
-  const int* pos;       // digit-reversal positions, P entries
+  const int4* tw;       // twiddles and places (fft_tables_host)
+  const unsigned* pos;
+  FxC over_p;           // 2^floor(log2 P) / P, for P no power of two
   const double2 *t, *w, *up, *ur;        // inputs  [r][m][b]
   double2 *ntp, *ntr, *nwp, *nwr;        // outputs [r][m][b]
-  double* umax;                          // optional [r][b][2]: max|ur|, max|uphi|
+  double* umax;                          // optional [r][b][2]: max|ur|, max|uphi| on the grid of plan.P points
 };
 
 // Y[row][n] = alpha * sum_k A[k*lda + row] * X[k*ldx + n] for
@@ -361,7 +432,5 @@ cudaError_t launch_getrs_rows(int n, int nb, const double* lu, size_t mstride, c
 double measure_fp64_peak();
 // Same for the FP64 tensor-core MMA (mma.sync m8n8k4 f64).
 double measure_fp64_mma_peak();
-// Set the odd-prime DFT coefficient tables (constant memory); idempotent.
-cudaError_t init_dft_tables();
 
 }  // namespace falcon

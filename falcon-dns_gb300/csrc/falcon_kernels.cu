@@ -1,11 +1,10 @@
 // sm_103a kernels of the FAlCon-DNS time step (FP64 throughout).
 //
 // On GB300 the FP64 FMA pipe (~1.2 TFLOP/s measured) is ~30x slower than
-// HBM relative to the bytes these kernels move, so every kernel here is
+// HBM relative to the bytes these kernels move, so the FP64 kernels here are
 // bound by FP64 issue, not memory: the code minimises FP64 instructions
-// (two-for-one real transforms, symmetric odd-prime butterflies with
-// constant-bank coefficients, register-tiled DFMA GEMMs) and keeps the
-// non-FP64 instruction count per FMA below one.
+// (register-tiled DFMA GEMMs) and keeps the non-FP64 instruction count per
+// FMA below one.  The nonlinear pass is in fixed point (falcon_fft.cuh).
 #include <math.h>
 #include <stdio.h>
 
@@ -21,28 +20,18 @@
 namespace falcon {
 
 // ---------------------------------------------------------------------------
-// The nonlinear pass and its tables live in falcon_fft.cuh, compiled once
-// per largest radix class (7, 17, 31) in its own translation unit.
+// The nonlinear pass lives in falcon_fft.cuh, compiled once per class of
+// FFT plans in its own translation unit.
 // ---------------------------------------------------------------------------
-cudaError_t init_dft_tables_7();
-cudaError_t init_dft_tables_17();
-cudaError_t init_dft_tables_31();
-cudaError_t launch_nonlin_7(const NonlinArgs& a, cudaStream_t s);
+cudaError_t launch_nonlin_8(const NonlinArgs& a, cudaStream_t s);
 cudaError_t launch_nonlin_17(const NonlinArgs& a, cudaStream_t s);
 cudaError_t launch_nonlin_31(const NonlinArgs& a, cudaStream_t s);
-
-cudaError_t init_dft_tables() {
-  cudaError_t e = init_dft_tables_7();
-  if (e == cudaSuccess) e = init_dft_tables_17();
-  if (e == cudaSuccess) e = init_dft_tables_31();
-  return e;
-}
 
 cudaError_t launch_nonlin(const NonlinArgs& a, cudaStream_t s) {
   int maxp = 0;
   for (int i = 0; i < a.plan.nrad; ++i) maxp = a.plan.rad[i] > maxp ? a.plan.rad[i] : maxp;
-  if (maxp <= 7) return launch_nonlin_7(a, s);
-  if (maxp <= 17) return launch_nonlin_17(a, s);
+  if (maxp <= 8) return launch_nonlin_8(a, s);
+  if (maxp <= 17 && a.plan.pfa) return launch_nonlin_17(a, s);
   return launch_nonlin_31(a, s);
 }
 
@@ -924,9 +913,9 @@ double measure_fp64_mma_peak() {
 namespace falcon {
 
 constexpr int kNoAllocMaxP = 4096;
-// twiddles (kNoAllocMaxP double2) followed by positions (kNoAllocMaxP int):
+// twiddles (kNoAllocMaxP int4) followed by positions (kNoAllocMaxP int):
 // 80 KiB, held by every GPU that loads the library until the process exits.
-constexpr size_t kNoAllocScratchBytes = (size_t)kNoAllocMaxP * (sizeof(double2) + sizeof(int));
+constexpr size_t kNoAllocScratchBytes = (size_t)kNoAllocMaxP * (sizeof(int4) + sizeof(int));
 static __device__ __align__(256) unsigned char g_nonlin_scratch[kNoAllocScratchBytes];
 
 // Per-device address of g_nonlin_scratch (host code may not use the symbol
@@ -940,8 +929,8 @@ static void* g_scratch_addr[64] = {nullptr};
 // pageable host memory has consumed its source when cudaMemcpyAsync returns,
 // so the buffer is free again once the copies are issued.
 static std::mutex g_noalloc_host_mu;
-static double2 g_noalloc_tw_h[kNoAllocMaxP];
-static int g_noalloc_pos_h[kNoAllocMaxP];
+static int4 g_noalloc_tw_h[kNoAllocMaxP];
+static unsigned g_noalloc_pos_h[kNoAllocMaxP];
 
 }  // namespace falcon
 
@@ -982,6 +971,7 @@ extern "C" int falcon_nonlin_noalloc_dev(int nr, int nm, int nb, const double* t
     set_error_message("falcon_nonlin_noalloc_dev: 3*Nm_max has a prime factor above 64");
     return -1;
   }
+  make_line_plan(nm, kNoAllocMaxP, &plan);  // always finds one: 4096 itself
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= 64) { set_error_message("falcon_nonlin_noalloc_dev: no current device"); return -2; }
@@ -993,23 +983,21 @@ extern "C" int falcon_nonlin_noalloc_dev(int nr, int nm, int nb, const double* t
     set_error_message("falcon_nonlin_noalloc_dev: cudaGetSymbolAddress failed on this device");
     return -2;
   }
-  e = init_dft_tables();
-  if (e != cudaSuccess) { set_error_message(cudaGetErrorString(e)); return -2; }
-  double2* tw = reinterpret_cast<double2*>(g_scratch_addr[dev]);
-  int* pos = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(g_scratch_addr[dev]) +
-                                    (size_t)kNoAllocMaxP * sizeof(double2));
+  int4* tw = reinterpret_cast<int4*>(g_scratch_addr[dev]);
+  unsigned* pos = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(g_scratch_addr[dev]) +
+                                    (size_t)kNoAllocMaxP * sizeof(int4));
   cudaStream_t s = (cudaStream_t)stream;
   {
     std::lock_guard<std::mutex> lk(g_noalloc_host_mu);
     fft_tables_host(plan, g_noalloc_tw_h, g_noalloc_pos_h);
-    e = cudaMemcpyAsync(tw, g_noalloc_tw_h, sizeof(double2) * (size_t)P, cudaMemcpyHostToDevice, s);
+    e = cudaMemcpyAsync(tw, g_noalloc_tw_h, sizeof(int4) * (size_t)plan.P, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess)
-      e = cudaMemcpyAsync(pos, g_noalloc_pos_h, sizeof(int) * (size_t)P, cudaMemcpyHostToDevice, s);
+      e = cudaMemcpyAsync(pos, g_noalloc_pos_h, sizeof(unsigned) * (size_t)plan.P, cudaMemcpyHostToDevice, s);
   }
   if (e != cudaSuccess) { set_error_message(cudaGetErrorString(e)); return -2; }
   NonlinArgs a{};
   a.R = nr; a.M = nm + 1; a.B = nb; a.Nm = nm;
-  a.plan = plan; a.tw = tw; a.pos = pos;
+  a.plan = plan; a.tw = tw; a.pos = pos; a.over_p = fx_over(plan.P);
   a.t = reinterpret_cast<const double2*>(t_dev); a.w = reinterpret_cast<const double2*>(omg_dev);
   a.up = reinterpret_cast<const double2*>(up_dev); a.ur = reinterpret_cast<const double2*>(ur_dev);
   a.ntp = reinterpret_cast<double2*>(uphi_t_dev); a.ntr = reinterpret_cast<double2*>(ur_t_dev);

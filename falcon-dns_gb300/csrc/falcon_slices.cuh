@@ -1,11 +1,9 @@
-// Device helpers shared by the integer-slice products (operator GEMMs in
-// falcon_ozaki.cu, odd-prime DFT stages in falcon_fft.cuh): an FP64
-// value cut into signed integers of a few bits relative to a power of two
-// that bounds its row or column, their bf16 / fp16 encodings, the exact
-// recombination, and the mma.sync used on them.
+// Device helpers of the integer-slice products (operator GEMMs in
+// falcon_ozaki.cu and falcon_tc.cu): an FP64 value cut into signed integers of
+// a few bits relative to a power of two that bounds its row or column, their
+// bf16 encodings, the exact recombination, and the mma.sync used on them.
 #pragma once
 #include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <stdint.h>
 
 #include "falcon_combine.h"
@@ -82,10 +80,9 @@ __device__ __forceinline__ uint32_t oz_slice_pair(uint32_t lo0, uint32_t hi0, ui
 
 // The recombination of a slice product's two partial sums, H of the
 // leading diagonals and L of the rest: RN(H 2^(k + sh) + L 2^k), each sum
-// exact, one rounding: by integer instructions (combine_rn,
-// falcon_combine.h) where the FP64 pipe bounds the kernel (the DFT stages),
-// as two exact scalings and one FP64 add where it is idle (the
-// contraction epilogues, which are bound by integer work).  The same bits.
+// exact, one rounding, as two exact scalings and one FP64 add (the FP64 pipe
+// is idle there; combine_rn, falcon_combine.h, gives the same bits by integer
+// instructions).
 __device__ __forceinline__ double oz_recombine_2t(long long H, long long L, int k, int sh) {
   return i64_scaled(H, k + sh) + i64_scaled(L, k);
 }
@@ -94,74 +91,6 @@ __device__ __forceinline__ double oz_recombine_2t(long long H, long long L, int 
 template <int W, int A, int B, class Q>
 __device__ __forceinline__ long long oz_diag_sum(Q q) {
   return diag_sum<W, A, B>(q);
-}
-
-// fp16 slices of 9 bits for short sums (the DFT butterflies: at most 8
-// products per output): kDftS slices of kDftW bits hold 63 bits of each
-// operand, and the pairs s + t <= kDftD keep every FP32 sum exact
-// (7 pairs x 8 products x 511^2 < 2^24) while the dropped pairs weigh less
-// than 2^-59 of the largest product.
-constexpr int kDftS = 7, kDftW = 9, kDftD = 6;
-
-// |a| * 2^(63 - e) truncated (< 2^63 when |a| < 2^e); zero and subnormal
-// inputs give 0.
-__device__ __forceinline__ unsigned long long dft_mag(double a, int e) {
-  const long long bits = __double_as_longlong(a);
-  const int eb = (int)((bits >> 52) & 0x7ff);
-  if (eb == 0) return 0ull;
-  const unsigned long long m = (unsigned long long)(bits & 0xfffffffffffffLL) | (1ull << 52);
-  const int sh = eb - 1012 - e;  // a = m 2^(eb-1075): T = m 2^(eb - 1075 + 63 - e), sh <= 10
-  if (sh >= 0) return m << sh;
-  if (sh <= -64) return 0ull;
-  return m >> (-sh);
-}
-
-// Slice s (0 = most significant) of two values as an fp16 pair: fp16(1536 +
-// q) has the bits 0x6600 + q for 0 <= q < 512, so q = fp16(0x6600 + q) -
-// 1536 exactly; the signs (bits 15 and 31 of sgn) are applied to the result.
-__device__ __forceinline__ uint32_t dft_slice2(unsigned long long tlo, unsigned long long thi, uint32_t sgn, int s) {
-  const int sh = kDftW * (kDftS - 1 - s);
-  const uint32_t biased = (((uint32_t)(tlo >> sh) & 511u) | (((uint32_t)(thi >> sh) & 511u) << 16)) + 0x66006600u;
-  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&biased), __floats2half2_rn(1536.f, 1536.f));
-  return *reinterpret_cast<const uint32_t*>(&v) ^ sgn;
-}
-
-// The wider odd primes (h = (p-1)/2 up to 15 products per output): 8 slices
-// of 8 bits (64 bits), pairs s + t <= 7 (8 pairs x 15 x 255^2 < 2^24).
-constexpr int kDwS = 8, kDwW = 8, kDwD = 7;
-
-// |a| * 2^(64 - e) truncated (< 2^64 when |a| < 2^e).
-__device__ __forceinline__ unsigned long long dft_mag64(double a, int e) {
-  const long long bits = __double_as_longlong(a);
-  const int eb = (int)((bits >> 52) & 0x7ff);
-  if (eb == 0) return 0ull;
-  const unsigned long long m = (unsigned long long)(bits & 0xfffffffffffffLL) | (1ull << 52);
-  const int sh = eb - 1011 - e;  // <= 11
-  if (sh >= 0) return m << sh;
-  if (sh <= -64) return 0ull;
-  return m >> (-sh);
-}
-
-// Slice s of two 64-bit magnitudes in the 8-bit format as an fp16 pair
-// (same construction as dft_slice2).
-__device__ __forceinline__ uint32_t dft_slice2w(unsigned long long tlo, unsigned long long thi, uint32_t sgn, int s) {
-  const int sh = kDwW * (kDwS - 1 - s);
-  const uint32_t biased = (((uint32_t)(tlo >> sh) & 255u) | (((uint32_t)(thi >> sh) & 255u) << 16)) + 0x66006600u;
-  const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&biased), __floats2half2_rn(1536.f, 1536.f));
-  return *reinterpret_cast<const uint32_t*>(&v) ^ sgn;
-}
-
-__device__ __forceinline__ uint32_t sign2(double lo, double hi) {
-  return (__double_as_longlong(lo) < 0 ? 0x8000u : 0u) | (__double_as_longlong(hi) < 0 ? 0x80000000u : 0u);
-}
-
-__device__ __forceinline__ void mma_f16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
-                                        unsigned b0, unsigned b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};\n"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
 __device__ __forceinline__ void mma_bf16(float (&c)[4], unsigned a0, unsigned a1, unsigned a2, unsigned a3,
