@@ -1,0 +1,441 @@
+// Operator contractions Y = alpha A X in 59-bit fixed point on integer
+// multiply-adds.
+//
+// GB300's FP64 pipe takes 64 cycles per warp instruction and sub-partition,
+// its 32 x 32 + 64-bit multiply-add 5, so a product of two such numbers in
+// three of those (and one of 32 bits) is 4 times cheaper than an FMA.  An
+// operator row and an X column are taken as integers at the scale of their
+// largest element (|a| < 2^e: trunc(a 2^(bits - e)), 58 bits for A, 59 for X,
+// exact for elements within 2^5 of it), split as h 2^32 + l with l signed.
+// Per product
+//   ha hx 2^64 + (ha lx + la hx) 2^32 + (la >> 20)(lx >> 20) 2^40
+// is summed in three integers (64, 64 and 32 bits; |ha| <= 2^26, |hx| <= 2^27
+// and K <= 257 keep them exact: the middle one is carried into the first every
+// 16 k).  The low x low term's bits below 2^40 are left out: 2^-64 of the
+// largest product.  The sum is rounded once to FP64.  Sums of integers do not
+// depend on their order, so results depend neither on the tile nor on the
+// launch: the tile and the narrow kernel give the same bits.  A column (or
+// row) with an Inf or NaN gives NaN.
+//
+// The solve operators weigh a right-hand side's rows very differently (near
+// the walls by the square of the grid spacing), and the right-hand sides are
+// large where the weights are small: their columns are divided by powers of
+// two 2^w_k (the largest element's exponent), X's rows multiplied, so that
+// neither operand's large elements push the other's out of the 58 bits.
+//
+// Bound: latency for the narrow forms (the radial and per-mode products of a
+// few instances), the integer pipes for the tiles (13 to 15 instructions per
+// product, issue 55 %).  Against FP64 FMA, us with L2 cold: 97 x 97, 342 modes,
+// 2 columns 44 -> 22; 33 x 33, 43 modes, 2 columns 14 -> 8; 65 x 65, 688
+// columns 22 -> 12.5; 65 x 65, 43776 columns 316 -> 131 (85 on tcgen05, which
+// the autotuner takes there).
+//
+// The operators' integers are made once per operator set
+// (launch_fx_operator); X is converted by each block for its own columns.
+#include <math.h>
+#include <stdint.h>
+
+#include <algorithm>
+#include <atomic>
+#include <unordered_map>
+
+#include "falcon_fixed.h"
+#include "falcon_internal.h"
+
+namespace falcon {
+namespace {
+
+constexpr int kBitsA = 58, kBitsX = 59;  // of a row's and a column's integers
+constexpr int kFxKC = 16;                // k per staged operator chunk
+constexpr int kBad = INT32_MIN;          // exponent of a row or column with an Inf or NaN
+constexpr int kNone = -100000;           // exponent of a zero
+
+// e with |a 2^w| < 2^e (kNone for a zero, INT32_MAX for Inf and NaN)
+__device__ __forceinline__ int exponent_of(double a, int w) {
+  const unsigned high = (unsigned)__double2hiint(a) & 0x7fffffffu;
+  if (high >= 0x7ff00000u) return INT32_MAX;
+  if (high == 0u && __double2loint(a) == 0) return kNone;
+  return (int)max(high >> 20, 1u) - 1022 + w;
+}
+// trunc(a 2^w 2^(bits - e)) split into (h, l signed)
+template <int BITS>
+__device__ __forceinline__ int2 split_of(double a, int w, int e) {
+  const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
+  unsigned long long t = fx_mag_of(bits, e - w + 1022) >> (59 - BITS);
+  if ((long long)bits < 0) t = 0ull - t;
+  return make_int2((int)((unsigned)(t >> 32) + ((unsigned)t >> 31)), (int)t);
+}
+// The scale of a row or column whose largest exponent is m, and its exponent.
+__device__ __forceinline__ int scale_of(int m) { return m == INT32_MAX ? 100000 : m == kNone ? 0 : m; }
+__device__ __forceinline__ int mark_of(int m) { return m == INT32_MAX ? kBad : scale_of(m); }
+
+struct Sum {
+  long long hh, mid;
+  int ll;
+};
+__device__ __forceinline__ void add_product(Sum& s, int2 a, int2 x, int a12, int x12) {
+  s.hh = fx_madw(a.x, x.x, s.hh);
+  s.mid = fx_madw(a.x, x.y, s.mid);
+  s.mid = fx_madw(a.y, x.x, s.mid);
+  s.ll += a12 * x12;
+}
+__device__ __forceinline__ void carry(Sum& s) {
+  s.hh += s.mid >> 32;
+  s.mid = (long long)(unsigned)s.mid;
+}
+// RN of the sum times 2^(ea + ex): (hh 2^32 + mid + ll 2^8) 2^32 in units of
+// 2^(ea + ex - kBitsA - kBitsX)
+__device__ __forceinline__ double value_of(Sum s, int ea, int ex, double alpha) {
+  if (ea == kBad || ex == kBad) return __longlong_as_double(0x7ff8000000000000LL);
+  s.mid += (long long)s.ll * 256;
+  carry(s);
+  // the leading 64 bits
+  const int sh = min(__clzll(s.hh ^ (s.hh >> 63)) - 1, 32);
+  const long long v = (s.hh << sh) + (long long)(((unsigned long long)s.mid << sh) >> 32);
+  const int e = ea + ex - kBitsA - kBitsX + 64 - sh;
+  double y = (double)v;
+  if (v) {
+    const int top = ((__double2hiint(y) >> 20) & 0x7ff) + e;
+    y = top > 0 && top < 2047 ? __hiloint2double(__double2hiint(y) + (e << 20), __double2loint(y)) : ldexp(y, e);
+  }
+  return alpha == 1.0 ? y : alpha * y;
+}
+
+__device__ __forceinline__ double* output_row(const GemmArgs& g, int z, int row) {
+  if (g.nout == 0) return g.Y + (size_t)z * g.sY + (size_t)row * g.ldy;
+  int o = 0;
+  while (o + 1 < g.nout && row >= g.rend[o]) ++o;
+  return g.Yo[o] + (size_t)z * g.sY + (size_t)(row - (o ? g.rend[o - 1] : 0)) * g.ldy;
+}
+
+__device__ __forceinline__ void copy8(void* dst, const void* src, bool valid) {
+  const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 8 : 0) : "memory");
+}
+
+// One thread per (entry, column k): the exponent of its largest element.
+__global__ void fx_weight_kernel(const double* A, long lda, long sA, int rows, int K, int nb, int* wk) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (t >= (long)nb * K) return;
+  const int z = (int)(t / K), k = (int)(t - (long)z * K);
+  const double* a = A + (size_t)z * sA + (size_t)k * lda;
+  int m = kNone;
+  for (int r = 0; r < rows; ++r) {
+    const int e = exponent_of(a[r], 0);
+    if (e != INT32_MAX) m = max(m, e);
+  }
+  wk[t] = m == kNone ? 0 : m;
+}
+
+// One thread per (entry, row): the row's exponent, then its integers, in the
+// operator's own layout.
+__global__ void fx_operator_kernel(const double* A, long lda, long sA, int rows, int K, int nb, const int* wk,
+                                   int2* out, int* ex) {
+  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  if (t >= (long)nb * rows) return;
+  const int z = (int)(t / rows), r = (int)(t - (long)z * rows);
+  const double* a = A + (size_t)z * sA + r;
+  const int* w = wk ? wk + (size_t)z * K : nullptr;
+  int m = kNone;
+  for (int k = 0; k < K; ++k) m = max(m, exponent_of(a[(size_t)k * lda], w ? -w[k] : 0));
+  ex[(size_t)z * lda + r] = mark_of(m);
+  int2* o = out + (size_t)z * sA + r;
+  for (int k = 0; k < K; ++k) o[(size_t)k * lda] = split_of<kBitsA>(a[(size_t)k * lda], w ? -w[k] : 0, scale_of(m));
+}
+
+// X panel of a block in shared memory, xs[k * ncol + c] (staged as doubles,
+// complete when this is called): column exponents in cex, integers in place.
+// w: the operator's weights (or null); part: blockDim.x words.
+__device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const int* w, int* cex, int* part) {
+  const int tid = threadIdx.x, J = blockDim.x / ncol, c = tid % ncol, j = tid / ncol;
+  const bool act = j < J;
+  int m = kNone;
+  if (act) {
+    for (int k = j; k < K; k += J) m = max(m, exponent_of(xs[k * ncol + c], w ? __ldg(w + k) : 0));
+    part[tid] = m;
+  }
+  __syncthreads();
+  if (act) {
+    for (int i = 0; i < J; ++i) m = max(m, part[i * ncol + c]);
+    if (j == 0) cex[c] = mark_of(m);
+    for (int k = j; k < K; k += J) {
+      const int2 v = split_of<kBitsX>(xs[k * ncol + c], w ? __ldg(w + k) : 0, scale_of(m));
+      reinterpret_cast<int2*>(xs)[k * ncol + c] = v;
+    }
+  }
+  __syncthreads();
+}
+
+// Tile: a block covers NCOL columns and nw * RG * RPT rows, RG = 64 / NCOL;
+// lane = (row group rg, column pair cp).  The X panel (all of K) stays in
+// shared memory, the operator is staged in double-buffered chunks of 16 k.
+template <int RPT, int NCOL>
+__global__ void __launch_bounds__(512) fx_tile_kernel(GemmArgs g) {
+  constexpr int RG = 64 / NCOL, CP = NCOL / 2;
+  extern __shared__ __align__(16) double fsm[];
+  const int nthr = blockDim.x, nw = nthr >> 5;
+  const int rows_blk = nw * RG * RPT;
+  double* xs = fsm;                                                   // [K][NCOL]
+  int2* as = reinterpret_cast<int2*>(fsm + (size_t)g.K * NCOL);       // [2][kFxKC][rows_blk]
+  int* cex = reinterpret_cast<int*>(as + 2 * kFxKC * rows_blk);       // [NCOL]
+  int* part = cex + NCOL;           // [nthr]
+  const int z = blockIdx.z;
+  const int2* A = g.fx + (size_t)z * g.sA;
+  const double* X = g.X + (size_t)z * g.sX;
+  const int n0 = blockIdx.x * NCOL, row0 = blockIdx.y * rows_blk;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rg = lane / CP, cp = lane - rg * CP;
+  const int rw = (warp * RG + rg) * RPT;
+  for (int i = threadIdx.x; i < g.K * NCOL; i += nthr) {
+    const int k = i / NCOL, c = i - k * NCOL;
+    const bool ok = n0 + c < g.N;
+    copy8(xs + i, ok ? X + (size_t)k * g.ldx + n0 + c : X, ok);
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  auto issue = [&](int k0, int2* buf) {
+    const int n = min(kFxKC, g.K - k0) * rows_blk;
+    for (int i = threadIdx.x; i < n; i += nthr) {
+      const int kk = i / rows_blk, rr = i - kk * rows_blk;
+      const bool ok = row0 + rr < g.rows;
+      copy8(buf + i, ok ? A + (size_t)(k0 + kk) * g.lda + row0 + rr : A, ok);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  issue(0, as);
+  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  __syncthreads();
+  const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
+  convert_panel(xs, g.K, NCOL, w, cex, part);
+  Sum acc[RPT][2];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = Sum{0, 0, 0};
+  int cur = 0;
+  for (int k0 = 0; k0 < g.K; k0 += kFxKC) {
+    const int kc = min(kFxKC, g.K - k0);
+    if (k0 + kFxKC < g.K) {
+      issue(k0 + kFxKC, as + (cur ^ 1) * kFxKC * rows_blk);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const int2* Aw = as + cur * kFxKC * rows_blk + rw;
+    const int4* Xw = reinterpret_cast<const int4*>(xs + (size_t)k0 * NCOL) + cp;
+#pragma unroll 2
+    for (int kk = 0; kk < kc; ++kk) {
+      const int4 xv = Xw[kk * (NCOL / 2)];
+      const int2 x0 = make_int2(xv.x, xv.y), x1 = make_int2(xv.z, xv.w);
+      const int x012 = x0.y >> 20, x112 = x1.y >> 20;
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const int2 av = Aw[kk * rows_blk + i];
+        const int a12 = av.y >> 20;
+        add_product(acc[i][0], av, x0, a12, x012);
+        add_product(acc[i][1], av, x1, a12, x112);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) { carry(acc[i][0]); carry(acc[i][1]); }
+    __syncthreads();  // every thread is done with this buffer before it is refilled
+    cur ^= 1;
+  }
+  const int n = n0 + 2 * cp, e0 = cex[2 * cp], e1 = cex[2 * cp + 1];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int row = row0 + rw + i;
+    if (row < g.rows && n < g.N) {
+      const int ea = g.fx_ex[(size_t)z * g.lda + row];
+      double* yp = output_row(g, z, row) + n;
+      const double y0 = value_of(acc[i][0], ea, e0, g.alpha);
+      if (n + 1 < g.N) {
+        const double y1 = value_of(acc[i][1], ea, e1, g.alpha);
+        if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
+          *reinterpret_cast<double2*>(yp) = make_double2(y0, y1);
+        } else {  // odd leading dimension or offset
+          yp[0] = y0;
+          yp[1] = y1;
+        }
+      } else {
+        yp[0] = y0;
+      }
+    }
+  }
+}
+
+// Narrow form (N <= 8 columns per batch entry): 32 rows per block, k shared
+// by its eight warps, each of which reads its share of the operator before
+// the X panel is converted (one memory latency, not two) and adds up the
+// columns' partial sums.  Bound by latency, then by the operator's bytes.
+struct alignas(16) Part {
+  long long hh;
+  unsigned mid;
+  int ll;
+};
+template <int NC>
+__global__ void __launch_bounds__(256) fx_narrow_kernel(GemmArgs g) {
+  extern __shared__ __align__(16) double fsm[];
+  Part* parts = reinterpret_cast<Part*>(fsm);                    // [8][NC][32]
+  double* xd = reinterpret_cast<double*>(parts + 8 * NC * 32);   // [K][NC]
+  __shared__ int cex[NC];
+  __shared__ int part[256];
+  constexpr int U = 16;
+  const int z = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int row = blockIdx.x * 32 + lane, kq = (g.K + 7) / 8, kb = min(warp * kq, g.K), ke = min(kb + kq, g.K);
+  const int2* A = g.fx + (size_t)z * g.sA + min(row, g.rows - 1);
+  int2 av[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u) av[u] = kb + u < ke ? __ldg(A + (size_t)(kb + u) * g.lda) : make_int2(0, 0);
+  const double* X = g.X + (size_t)z * g.sX;
+  for (int i = tid; i < g.K * NC; i += 256) {
+    const int k = i / NC, c = i - k * NC;
+    xd[i] = c < g.N ? X[(size_t)k * g.ldx + c] : 0.0;
+  }
+  __syncthreads();
+  convert_panel(xd, g.K, NC, g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr, cex, part);
+  const int2* xs = reinterpret_cast<const int2*>(xd);
+  Sum acc[NC];
+#pragma unroll
+  for (int c = 0; c < NC; ++c) acc[c] = Sum{0, 0, 0};
+  for (int k0 = kb; k0 < ke; k0 += U) {
+    if (k0 > kb) {
+#pragma unroll
+      for (int u = 0; u < U; ++u) av[u] = k0 + u < ke ? __ldg(A + (size_t)(k0 + u) * g.lda) : make_int2(0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (k0 + u >= ke) break;
+      const int a12 = av[u].y >> 20;
+#pragma unroll
+      for (int c = 0; c < NC; ++c) {
+        const int2 x = xs[(k0 + u) * NC + c];
+        add_product(acc[c], av[u], x, a12, x.y >> 20);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < NC; ++c) carry(acc[c]);
+  }
+#pragma unroll
+  for (int c = 0; c < NC; ++c) parts[(warp * NC + c) * 32 + lane] = Part{acc[c].hh, (unsigned)acc[c].mid, acc[c].ll};
+  __syncthreads();
+  if (warp >= min(NC, g.N) || row >= g.rows) return;
+  Sum s{0, 0, 0};  // column `warp`
+#pragma unroll
+  for (int w = 0; w < 8; ++w) {
+    const Part p = parts[(w * NC + warp) * 32 + lane];
+    s.hh += p.hh;
+    s.mid += p.mid;
+    s.ll += p.ll;
+  }
+  output_row(g, z, row)[warp] = value_of(s, g.fx_ex[(size_t)z * g.lda + row], cex[warp], g.alpha);
+}
+
+template <int RPT, int NCOL>
+cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream_t s) {
+  static std::atomic<bool> opted[64];  // opted in to large shared memory, per device
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!(dev >= 0 && dev < 64 && opted[dev].load())) {
+    const cudaError_t e = cudaFuncSetAttribute(fx_tile_kernel<RPT, NCOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               227 * 1024);
+    if (e != cudaSuccess) return e;
+    if (dev >= 0 && dev < 64) opted[dev].store(true);
+  }
+  const int rows_blk = nw * (64 / NCOL) * RPT;
+  const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw) * 4;
+  const dim3 grid((g.N + NCOL - 1) / NCOL, row_blocks, g.batch);
+  fx_tile_kernel<RPT, NCOL><<<grid, 32 * nw, smem, s>>>(g);
+  return cudaGetLastError();
+}
+
+// Launch shape from a cost model of the integer pipe: a block's work is
+// rows_blk x NCOL per k and a share of 6 rows' worth for converting its X
+// panel; blocks spread evenly over the SMs; an SM with fewer than 8 warps
+// cannot fill the pipe.  The cheapest (columns, row blocks, warps, rows per
+// thread) wins, ties going to deeper register tiles.
+struct TileShape { int ncol, rb, nw, rpt; };
+TileShape pick_shape(const GemmArgs& g, int nsm) {
+  TileShape best{64, 1, 8, 1};
+  double bcost = 1e300;
+  for (int ncol = 16; ncol <= 64; ncol *= 2) {
+    if (g.fma_ncol && ncol != g.fma_ncol) continue;
+    const int rg = 64 / ncol;
+    const long cb = (long)((g.N + ncol - 1) / ncol) * g.batch;
+    for (int rb = 1; rb <= 16; ++rb)
+      for (int nw = 4; nw <= 16; ++nw)
+        for (int rpt = 1; rpt <= 8; ++rpt) {
+          const int rows_blk = nw * rg * rpt;
+          if ((long)rb * rows_blk < g.rows || (long)(rb - 1) * rows_blk >= g.rows || rows_blk > 256) continue;
+          const long smem = ((long)g.K * ncol + 2 * kFxKC * rows_blk) * 8 + (ncol + 32 * nw) * 4;
+          if (smem > 227 * 1024) continue;
+          const long blocks = cb * rb;
+          const long fit = std::max(1L, std::min({220L * 1024 / smem, 64L / nw, 65536L / (32L * nw * (40 + 12 * rpt))}));
+          const long waves = (blocks + nsm - 1) / nsm;
+          const double warps = (double)nw * (double)std::min(waves, fit);
+          const double eff = std::min(1.0, warps / 8.0);
+          const double cost = (double)waves * ncol * (rows_blk * (rpt == 1 ? 1.3 : rpt == 2 ? 1.1 : 1.0) + 6.0) / eff;
+          if (cost < bcost * (1.0 - 1e-12) || (cost <= bcost * (1.0 + 1e-12) && rpt > best.rpt)) {
+            bcost = cost;
+            best = {ncol, rb, nw, rpt};
+          }
+        }
+  }
+  return best;
+}
+
+template <int NCOL>
+cudaError_t launch_ncol(const GemmArgs& g, const TileShape& t, cudaStream_t s) {
+  switch (t.rpt) {
+    case 1: return launch_fx_tile<1, NCOL>(g, t.nw, t.rb, s);
+    case 2: return launch_fx_tile<2, NCOL>(g, t.nw, t.rb, s);
+    case 3: return launch_fx_tile<3, NCOL>(g, t.nw, t.rb, s);
+    case 4: return launch_fx_tile<4, NCOL>(g, t.nw, t.rb, s);
+    case 5: return launch_fx_tile<5, NCOL>(g, t.nw, t.rb, s);
+    case 6: return launch_fx_tile<6, NCOL>(g, t.nw, t.rb, s);
+    case 7: return launch_fx_tile<7, NCOL>(g, t.nw, t.rb, s);
+    default: return launch_fx_tile<8, NCOL>(g, t.nw, t.rb, s);
+  }
+}
+
+}  // namespace
+
+cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int K, int nb, int* wk, int2* out,
+                               int* ex, cudaStream_t s) {
+  const long n = (long)nb * rows, m = (long)nb * K;
+  if (n <= 0) return cudaSuccess;
+  if (wk) fx_weight_kernel<<<(unsigned)((m + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk);
+  fx_operator_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk, out, ex);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
+  if (g.rows <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
+  if (g.K > 257 || !g.fx) return cudaErrorInvalidValue;
+  if (g.N <= 8) {
+    const dim3 grid((g.rows + 31) / 32, g.batch);
+    auto smem = [&](int nc) { return (size_t)nc * (8 * 32 * sizeof(Part) + g.K * sizeof(double)); };
+    if (g.N > 4 && g.K > 170) {  // over 48 KB with the static part
+      const cudaError_t e = cudaFuncSetAttribute(fx_narrow_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+      if (e != cudaSuccess) return e;
+    }
+    if (g.N <= 2) fx_narrow_kernel<2><<<grid, 256, smem(2), s>>>(g);
+    else if (g.N <= 4) fx_narrow_kernel<4><<<grid, 256, smem(4), s>>>(g);
+    else fx_narrow_kernel<8><<<grid, 256, smem(8), s>>>(g);
+    return cudaGetLastError();
+  }
+  int dev = 0, nsm = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // shapes are memoised per problem size: the search runs on the host once
+  struct Memo { int rows, K, N, batch, nsm, ncol; TileShape t; };
+  thread_local std::unordered_map<unsigned long long, Memo> memo;
+  unsigned long long key = 1469598103934665603ull;
+  for (int v : {g.rows, g.K, g.N, g.batch, nsm, g.fma_ncol}) key = (key ^ (unsigned)v) * 1099511628211ull;
+  Memo& m = memo[key];
+  if (m.rows != g.rows || m.K != g.K || m.N != g.N || m.batch != g.batch || m.nsm != nsm || m.ncol != g.fma_ncol)
+    m = Memo{g.rows, g.K, g.N, g.batch, nsm, g.fma_ncol, pick_shape(g, nsm)};
+  if (m.t.ncol == 16) return launch_ncol<16>(g, m.t, s);
+  if (m.t.ncol == 32) return launch_ncol<32>(g, m.t, s);
+  return launch_ncol<64>(g, m.t, s);
+}
+
+}  // namespace falcon

@@ -218,6 +218,9 @@ struct OpSet {
     int rows = 0, K = 0, nb = 0, rowsP = 0, KP = 0, w = 6;
     uint16_t* s = nullptr;
     int* ex = nullptr;
+    int2* fx = nullptr;       // fixed-point integers and row exponents (launch_fx_operator)
+    int* fx_ex = nullptr;
+    int* fx_w = nullptr;      // column weights of solve operators
     CUtensorMap tmap{};     // the slices for the tcgen05 kernel's copies
     bool tmap_ok = false;
   };
@@ -230,20 +233,20 @@ struct OpSet {
     cudaFree(D1p); cudaFree(Lp); cudaFree(ST); cudaFree(G); cudaFree(U); cudaFree(LAP);
     cudaFree(inv_r); cudaFree(inv_r2); cudaFree(wq); cudaFree(d1_0); cudaFree(d1_R);
     cudaFree(D1c); cudaFree(Lc);
-    for (auto& o : oz) { cudaFree(o.s); cudaFree(o.ex); }
+    for (auto& o : oz) { cudaFree(o.s); cudaFree(o.ex); cudaFree(o.fx); cudaFree(o.fx_ex); cudaFree(o.fx_w); }
   }
 };
 
 // Contraction paths (the modes of gemm() below): 4 (default) measured per
 // shape by the autotuner; 3 tcgen05 wherever possible; 2 tcgen05 where a
-// contraction fills the GPU, mma.sync otherwise; 1 mma.sync only; 0 FP64
-// FMA tiles.  The two sliced kernels give the same bits; all paths are
-// FP64-accurate.
+// contraction fills the GPU, mma.sync otherwise; 1 mma.sync only; 0 tiles.
+// The two sliced kernels give the same bits; all paths are FP64-accurate.
 std::atomic<int> g_gemm_mode{4};
 
-// Slices of one column-major operator array (rows x K, lda = rows, nb
-// entries of stride sA) for the tensor-core GEMM.
-int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA) {
+// Slices and fixed-point integers of one column-major operator array (rows x
+// K, lda = rows, nb entries of stride sA) for the contraction kernels; the
+// integers of a solve operator with weighted columns.
+int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA, bool solve = false) {
   if (!base || K > 257) return 0;
   OpSet::Oz o;
   o.base = base; o.lda = rows; o.sA = sA; o.rows = rows; o.K = K; o.nb = nb;
@@ -258,7 +261,13 @@ int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA) {
   CK(launch_oz_slice_rows(base, rows, sA, rows, K, nb, o.s, o.ex, o.rowsP, o.KP, o.w, 0));
   o.tmap_ok = tc_stage_layout_check(o.w, o.KP) == 0 &&
               tc_make_operator_map(&o.tmap, o.s, nb, oz_slices(o.w), o.KP, o.rowsP) == 0;
-  ops->bytes += ns * sizeof(uint16_t) + ne * sizeof(int);
+  const size_t nf = (size_t)(nb - 1) * sA + (size_t)rows * K;
+  CK(cudaMalloc(&o.fx, nf * sizeof(int2)));
+  CK(cudaMalloc(&o.fx_ex, (size_t)nb * rows * sizeof(int)));
+  if (solve) CK(cudaMalloc(&o.fx_w, (size_t)nb * K * sizeof(int)));
+  CK(launch_fx_operator(base, rows, sA, rows, K, nb, o.fx_w, o.fx, o.fx_ex, 0));
+  ops->bytes += ns * sizeof(uint16_t) + ne * sizeof(int) + nf * sizeof(int2) + (size_t)nb * rows * sizeof(int) +
+                (solve ? (size_t)nb * K * sizeof(int) : 0);
   ops->oz.push_back(o);
   return 0;
 }
@@ -661,9 +670,9 @@ int build_opset(const OpKey& k, std::shared_ptr<OpSet>* out, const HostFactors* 
   {
     const long RR = (long)R * R;
     if ((rc = add_oz(ops.get(), ops->D1p, R, R, 1, RR)) || (rc = add_oz(ops.get(), ops->Lp, R, R, 1, RR)) ||
-        (rc = add_oz(ops.get(), ops->ST, R, R, M, RR)) || (rc = add_oz(ops.get(), ops->G, 3 * R, R, M, 3 * RR)) ||
-        (rc = add_oz(ops.get(), ops->U, 2 * R, R, 1, 2 * RR)) ||
-        (rc = add_oz(ops.get(), ops->LAP, 2 * R + 2, R, M, (long)(2 * R + 2) * R)) ||
+        (rc = add_oz(ops.get(), ops->ST, R, R, M, RR, true)) || (rc = add_oz(ops.get(), ops->G, 3 * R, R, M, 3 * RR, true)) ||
+        (rc = add_oz(ops.get(), ops->U, 2 * R, R, 1, 2 * RR, true)) ||
+        (rc = add_oz(ops.get(), ops->LAP, 2 * R + 2, R, M, (long)(2 * R + 2) * R, true)) ||
         (rc = add_oz(ops.get(), ops->D1c, R, R, 1, RR)) || (rc = add_oz(ops.get(), ops->Lc, R, R, 1, RR)))
       return rc;
     CK(cudaDeviceSynchronize());
@@ -1296,6 +1305,9 @@ bool attach_oz(const OpSet* o, GemmArgs* q) {
     q->oz_row0 = (int)row0;
     q->oz_tmap = z.tmap_ok ? &z.tmap : nullptr;
     q->oz_z0 = (int)z0;
+    q->fx = z.fx + delta;
+    q->fx_ex = z.fx_ex + z0 * z.rows + row0;
+    q->fx_w = z.fx_w ? z.fx_w + z0 * z.K : nullptr;
     return true;
   }
   return false;
@@ -1346,12 +1358,13 @@ TcArgs tc_args(const GemmArgs& q) {
 
 // ---------------------------------------------------------------------------
 // Contraction paths and their autotuner.  A contraction with an attached
-// slice view can run as FP64 FMA tiles (PATH_FMA), on the mma.sync slice
-// kernel (PATH_MMA; X sliced in the kernel, or into slice planes first) or on
-// the tcgen05 kernel (PATH_TC).  PATH_MMA and PATH_TC give the same bits;
-// PATH_FMA differs from them by rounding (all are FP64-accurate).
+// view can run as tiles of 58-bit integers (PATH_FMA, falcon_fxgemm.cu; FP64
+// FMA tiles without a view), on the mma.sync slice kernel (PATH_MMA; X sliced
+// in the kernel, or into slice planes first) or on the tcgen05 kernel
+// (PATH_TC).  PATH_MMA and PATH_TC give the same bits; PATH_FMA differs from
+// them by rounding (all are FP64-accurate).
 // ---------------------------------------------------------------------------
-// PATH_FMA16/32/64: the FMA tiles with the best tile shape of that column
+// PATH_FMA16/32/64: the tiles with the best tile shape of that column
 // width (the same bits as PATH_FMA, whose shape a cost model picks).
 enum { PATH_FMA = 0, PATH_MMA = 1, PATH_TC = 2, PATH_FMA16 = 3, PATH_FMA32 = 4, PATH_FMA64 = 5, PATH_COUNT = 6 };
 inline bool is_fma_path(int p) { return p == PATH_FMA || p >= PATH_FMA16; }
@@ -1412,6 +1425,7 @@ int run_path_once(Group* g, int cls, GemmArgs q, int path, bool reuse) {
     q.oz_s = nullptr;
     q.oz_xs = nullptr;
     q.fma_ncol = path == PATH_FMA16 ? 16 : path == PATH_FMA32 ? 32 : path == PATH_FMA64 ? 64 : 0;
+    if (q.fx) return launch(g, cls, gemm_flops(q), [&]() { return launch_fx_gemm(q, g->stream); });
   }
   return launch(g, cls, gemm_flops(q), [&]() { return launch_gemm(q, g->stream); });
 }
@@ -1425,8 +1439,8 @@ int run_path_once(Group* g, int cls, GemmArgs q, int path, bool reuse) {
 // device = the CUDA device name with blanks as '_' and "_sm<SM count>";
 // per_mode = 1 when the batch entries have their own X (sX != 0); reuse = 1
 // when X's slice planes were made by the contraction before; w = the slice
-// format (6 or 7); path 0 FMA (cost-model tile shape), 1 mma.sync, 2
-// tcgen05, 3/4/5 FMA with tiles of 16/32/64 columns; us_p = the measured
+// format (6 or 7); path 0 tiles (cost-model shape), 1 mma.sync, 2 tcgen05,
+// 3/4/5 tiles of 16/32/64 columns; us_p = the measured
 // microseconds per contraction on path p (-1: not measured).
 struct TuneKey {
   std::string dev;
@@ -1589,7 +1603,7 @@ int tuned_path(Group* g, int cls, const GemmArgs& q, bool reuse, bool tc_ok, int
   for (int p = 0; p < PATH_COUNT && !rc; ++p) {
     e.us[p] = -1.f;
     if (p == PATH_TC && !tc_ok) continue;
-    if (p >= PATH_FMA16 && q.N <= 8) continue;  // one-warp GEMV, no tile shapes
+    if (p >= PATH_FMA16 && q.N <= 8) continue;  // the narrow kernel has no tile shapes
     if ((rc = time_fastest(g, flush, a, b, [&]() { return run_path(g, cls, q, p, reuse); }, &e.us[p]))) break;
     if (p == PATH_FMA || e.us[p] < best) {
       best = e.us[p];
@@ -1615,40 +1629,76 @@ int tuned_path(Group* g, int cls, const GemmArgs& q, bool reuse, bool tc_ok, int
 // since (the blocks of one operator applied to one right-hand side); its
 // slice planes are reused when they match.
 //
-// Modes: 0 FP64 FMA tiles; 1 mma.sync for every contraction with a slice
-// view; 2 fixed rules: tcgen05 for contractions that fill the GPU (at least
-// two 128 x 24 tiles per SM), mma.sync for the other ones of at least 16
-// columns per batch entry, FMA for narrower ones (the per-mode solves of
-// groups of up to 7 instances); 3 tcgen05 for every contraction with a
-// slice view (the same bits as 1); 4 (default) the measured fastest of FMA,
-// mma.sync and tcgen05 per shape.
-int gemm(Group* g, int cls, const GemmArgs& q0, bool reuse = false) {
-  GemmArgs q = q0;
-  q.oz_s = nullptr;
-  q.oz_xs = nullptr;
+// Modes: 0 tiles; 1 mma.sync for every contraction with a slice view; 2
+// fixed rules: tcgen05 for contractions that fill the GPU (at least two 128 x
+// 24 tiles per SM), mma.sync for the other ones of at least 16 columns per
+// batch entry, tiles for narrower ones (the per-mode solves of groups of up
+// to 7 instances); 3 tcgen05 for every contraction with a slice view (the
+// same bits as 1); 4 (default) the measured fastest of tiles, mma.sync and
+// tcgen05 per shape.
+// The path of q (which receives its operator's views).
+int choose_path(Group* g, int cls, GemmArgs* q, bool reuse, int* path) {
+  q->oz_s = nullptr;
+  q->oz_xs = nullptr;
   // X may have changed since the planes were made: only a call that follows
   // one on the same, unchanged X may reuse them (the paths of two such
   // calls can differ under the autotuner, so the first one need not have
   // made them)
   if (!reuse) g->oz_key.valid = false;
   const int mode = g_gemm_mode.load();
-  bool ok = false;
-  if (mode && g->oz_xs && (q.N >= 16 || mode != 2)) ok = attach_group(g, &q);
-  if (!ok) return run_path(g, cls, q, PATH_FMA, reuse);
-  const bool tc_ok = mode >= 2 && q.oz_tmap != nullptr;
-  int path = PATH_MMA;
-  if (mode == 3 && tc_ok) path = PATH_TC;
-  if ((mode == 2 || mode == 4) && tc_ok && tc_worth_it(q)) path = PATH_TC;
+  const bool view = attach_group(g, q);
+  *path = PATH_FMA;
+  if (!(view && mode && g->oz_xs && (q->N >= 16 || mode != 2))) return 0;
+  const bool tc_ok = mode >= 2 && q->oz_tmap != nullptr;
+  *path = PATH_MMA;
+  if (mode == 3 && tc_ok) *path = PATH_TC;
+  if ((mode == 2 || mode == 4) && tc_ok && tc_worth_it(*q)) *path = PATH_TC;
   if (mode == 4) {
     // the tuner weighs tcgen05 only for contractions that fill the GPU (at
     // least two tiles per SM): below that one 448-thread CTA per SM idles
     // most of its warps, and the narrow shapes stay on the kernels whose
     // launch cost is lower
-    const int fixed = q.N >= 16 ? path : PATH_FMA;
-    int rc = tuned_path(g, cls, q, reuse, tc_ok && tc_worth_it(q), fixed, &path);
+    const int fixed = q->N >= 16 ? *path : PATH_FMA;
+    return tuned_path(g, cls, *q, reuse, tc_ok && tc_worth_it(*q), fixed, path);
+  }
+  return 0;
+}
+
+int gemm(Group* g, int cls, const GemmArgs& q0, bool reuse = false) {
+  GemmArgs q = q0;
+  int path = PATH_FMA;
+  const int rc = choose_path(g, cls, &q, reuse, &path);
+  return rc ? rc : run_path(g, cls, q, path, reuse);
+}
+
+// The row blocks v one after another, or, where their path is the
+// fixed-point tiles, as one launch over the merged view `all` (X converted
+// once, one launch instead of up to four).
+int run_blocks(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArgs* all) {
+  size_t first = 0;
+  if (all && all->fx) {
+    GemmArgs q = v[0];
+    int path = PATH_FMA;
+    int rc = choose_path(g, cls, &q, false, &path);
+    if (rc) return rc;
+    if (is_fma_path(path)) {
+      GemmArgs m = *all;
+      m.nout = (int)v.size();
+      int r = 0;
+      for (size_t o = 0; o < v.size(); ++o) {
+        m.rend[o] = r += v[o].rows;
+        m.Yo[o] = v[o].Y;
+      }
+      return run_path(g, cls, m, path, false);
+    }
+    if ((rc = run_path(g, cls, q, path, false))) return rc;
+    first = 1;
+  }
+  for (size_t o = first; o < v.size(); ++o) {
+    const int rc = gemm(g, cls, v[o], o > 0);
     if (rc) return rc;
   }
-  return run_path(g, cls, q, path, reuse);
+  return 0;
 }
 
 // The merged tcgen05 launch of the row blocks v (one X, outputs after one
@@ -1666,17 +1716,16 @@ int run_merged_tc(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmA
   return launch(g, cls, gemm_flops(all), [&]() { return launch_tc_gemm(t, *map, g->stream); });
 }
 
-// Mode 4, row blocks narrower than 16 columns per batch entry: one merged
-// tcgen05 launch, or the blocks one after another on their own (autotuned)
-// paths, whichever measures faster (the blocks unless the merged launch is
-// 25 % faster: in a step graph the merged launch's 215 KB shared-memory
-// configuration costs more than its isolated timing shows) with the
-// autotuner's method; cached under per_mode = 2 + the
-// number of blocks (path 2: merged, 0: the blocks).  The blocks run once
-// untimed first, so that their own paths are measured before they are
+// Mode 4: the row blocks as one merged tcgen05 launch, or on their own
+// (autotuned) path, whichever measures faster with the autotuner's method
+// (for blocks narrower than 16 columns the blocks unless the merged launch is
+// 25 % faster: in a step graph its 215 KB shared-memory configuration costs
+// more than its isolated timing shows); cached under per_mode = 2 + the
+// number of blocks (path 2: merged tcgen05, 0: the blocks).  The blocks run
+// once untimed first, so that their own paths are measured before they are
 // timed together.
 int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArgs& all, bool* merged) {
-  *merged = false;
+  *merged = all.N >= 16;
   TuneKey k{device_tag(), all.rows, all.K, all.N, all.batch, all.oz_w, 2 + (int)v.size(), 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1691,13 +1740,7 @@ int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArg
   if (cs != cudaStreamCaptureStatusNone || g->prof) return 0;
   void* flush = tune_flush_buffer();
   if (!flush) return fail(FALCON_ENOMEM, "contraction tuning: no device memory for the L2 flush buffer");
-  auto blocks = [&]() {
-    for (size_t o = 0; o < v.size(); ++o) {
-      const int rc = gemm(g, cls, v[o], o > 0);
-      if (rc) return rc;
-    }
-    return 0;
-  };
+  auto blocks = [&]() { return run_blocks(g, cls, v, &all); };
   int rc0 = blocks();  // the blocks' own paths, measured where new
   if (rc0) return rc0;
   auto one = [&]() { return run_merged_tc(g, cls, v, all); };
@@ -1712,7 +1755,7 @@ int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArg
   cudaEventDestroy(a);
   cudaEventDestroy(b);
   if (rc) return rc;
-  e.path = e.us[PATH_TC] * 1.25f < e.us[PATH_FMA] ? PATH_TC : PATH_FMA;
+  e.path = e.us[PATH_TC] * (all.N < 16 ? 1.25f : 1.0f) < e.us[PATH_FMA] ? PATH_TC : PATH_FMA;
   g_tune_measured++;
   std::lock_guard<std::mutex> lk(g_tune_mu);
   g_tune[k] = e;
@@ -1723,48 +1766,40 @@ int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArg
 
 // Consecutive row blocks of one operator applied to one X, each written to
 // its own output (G: omega, psi, u_phi; LAP: psi, u_phi and the two wall
-// vorticity rows).  With the tcgen05 contractions they run as one launch
-// over all the rows (fewer, fuller 128-row tiles, X sliced once), unless an
-// output overlaps X (then a later block reads what an earlier one wrote,
-// and the blocks run one after another as before).  Blocks narrower than
-// 16 columns merge under mode 3, and under mode 4 where measured faster.
+// vorticity rows), as one launch over all the rows where the path allows it
+// (fixed-point tiles, tcgen05: fewer, fuller tiles, X converted once), unless
+// an output overlaps X (then a later block reads what an earlier one wrote,
+// and the blocks run one after another).
 int gemm_blocks(Group* g, int cls, std::initializer_list<GemmArgs> blocks) {
   const std::vector<GemmArgs> v(blocks);
   const int mode = g_gemm_mode.load();
-  if (mode >= 2 && g->oz_xs && !v.empty() && v.size() <= 4 && (v[0].N >= 16 || mode >= 3)) {
-    const GemmArgs& f = v[0];
-    const char* x0 = reinterpret_cast<const char*>(f.X);
-    const char* x1 = reinterpret_cast<const char*>(f.X + (size_t)(f.batch - 1) * f.sX + (size_t)f.K * f.ldx);
-    bool merge = true;
-    int rows = 0;
-    for (const GemmArgs& q : v) {
-      const char* y = reinterpret_cast<const char*>(q.Y);
-      if (q.A != f.A + rows || q.lda != f.lda || q.sA != f.sA || q.X != f.X || q.ldx != f.ldx || q.sX != f.sX ||
-          q.K != f.K || q.N != f.N || q.batch != f.batch || q.ldy != f.ldy || q.sY != f.sY || q.alpha != f.alpha ||
-          (y >= x0 && y < x1))
-        merge = false;
-      rows += q.rows;
-    }
-    if (merge) {
-      GemmArgs all = f;
-      all.rows = rows;
-      all.oz_s = nullptr;
-      all.oz_xs = nullptr;
-      const bool ok = attach_group(g, &all);
-      bool use = ok && all.oz_tmap && (mode == 3 || tc_worth_it(all));
-      if (use && mode == 4 && f.N < 16) {
-        g->oz_key.valid = false;  // the blocks' own X slicing starts afresh
-        const int rc = tuned_merge(g, cls, v, all, &use);
-        if (rc) return rc;
-      }
-      if (use) return run_merged_tc(g, cls, v, all);
-    }
+  const GemmArgs& f = v[0];
+  const char* x0 = reinterpret_cast<const char*>(f.X);
+  const char* x1 = reinterpret_cast<const char*>(f.X + (size_t)(f.batch - 1) * f.sX + (size_t)f.K * f.ldx);
+  bool merge = v.size() <= 4;
+  GemmArgs all = f;
+  all.rows = 0;
+  for (const GemmArgs& q : v) {
+    const char* y = reinterpret_cast<const char*>(q.Y);
+    if (q.A != f.A + all.rows || q.lda != f.lda || q.sA != f.sA || q.X != f.X || q.ldx != f.ldx || q.sX != f.sX ||
+        q.K != f.K || q.N != f.N || q.batch != f.batch || q.ldy != f.ldy || q.sY != f.sY || q.alpha != f.alpha ||
+        (y >= x0 && y < x1))
+      merge = false;
+    all.rows += q.rows;
   }
-  for (size_t o = 0; o < v.size(); ++o) {
-    const int rc = gemm(g, cls, v[o], o > 0);
-    if (rc) return rc;
+  all.oz_s = nullptr;
+  all.oz_xs = nullptr;
+  if (!merge || !attach_group(g, &all)) return run_blocks(g, cls, v, nullptr);
+  if (mode >= 2 && g->oz_xs && (f.N >= 16 || mode >= 3) && all.oz_tmap && (mode == 3 || tc_worth_it(all))) {
+    bool use = true;
+    if (mode == 4) {
+      g->oz_key.valid = false;  // the blocks' own X slicing starts afresh
+      const int rc = tuned_merge(g, cls, v, all, &use);
+      if (rc) return rc;
+    }
+    if (use) return run_merged_tc(g, cls, v, all);
   }
-  return 0;
+  return run_blocks(g, cls, v, &all);
 }
 
 int elementwise(Group* g, double flops_per_el, std::function<cudaError_t()> f) {

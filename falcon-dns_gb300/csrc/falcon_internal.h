@@ -226,9 +226,18 @@ struct GemmArgs {
   // this GEMM's first batch entry in it, for the tcgen05 kernel
   const void* oz_tmap;
   int oz_z0;
-  // FP64 FMA tiles (no slice view): 0 = the tile shape of the cost model,
-  // 16 / 32 / 64 = the cost model's best shape of that column width (every
-  // shape sums each output over k in the same order: the same bits)
+  // fixed-point integers of A (falcon_fxgemm.cu; the layout of A) and row
+  // exponents (batch entry z, row r: fx_ex[z lda + r]) and column weights
+  // (fx_w[z K + k], or null): launch_fx_gemm
+  const int2* fx;
+  const int* fx_ex;
+  const int* fx_w;
+  // fixed-point path: rows [rend[o-1], rend[o]) go to Yo[o] (nout = 0: all to Y)
+  int nout;
+  int rend[4];
+  double* Yo[4];
+  // fixed-point tiles: 0 = the tile shape of the cost model, 16 / 32 / 64 = the
+  // cost model's best shape of that column width (the same bits)
   int fma_ncol;
 };
 
@@ -345,6 +354,11 @@ struct AsmArgs {
 // ---- launchers (falcon_kernels.cu; the nonlinear pass dispatches to falcon_fft*.cu) ----
 cudaError_t launch_nonlin(const NonlinArgs& a, cudaStream_t s);
 cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s);
+// Y = alpha A X in fixed point (g.fx set, K <= 257), and the operator's column
+// weights (wk null: none), integers and row exponents.
+cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s);
+cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int K, int nb, int* wk, int2* out,
+                               int* ex, cudaStream_t s);
 cudaError_t launch_imex_rhs(const RhsArgs& a, cudaStream_t s);
 // rhs_w(m>=1) += coef_b * (i m / r) * t_new, coef_b = scale * ra_pr[b]
 cudaError_t launch_add_buoyancy(int R, int M, int B, const double* inv_r, const double* ra_pr,

@@ -365,14 +365,13 @@ long long falcon_launch_count(void);
  * No reference counterpart (launch mechanics of the GPU step). */
 int falcon_set_step_graphs(int enable);
 /* Operator contractions (the radial derivative / Laplacian and per-mode
- * solve products) run on one of three paths: FP64 FMA tiles; the bf16
- * tensor cores by exact integer slicing of the FP64 operands on warp-level
- * mma.sync; the same slices on the 5th-generation tcgen05 MMA with
- * accumulators in tensor memory.  The two sliced paths give the same bits;
- * all give FP64-accurate results (the slices: error of the order of
- * K 2^-56 max|A_row| max|X_col|), and the sliced ones are several times
- * faster on GB300, whose FP64 pipe is ~500x slower than its bf16 tensor
- * cores.  Modes:
+ * solve products) run on one of three paths: tiles of 58-bit fixed-point
+ * integers (FP64 FMA tiles for Nr > 257); the bf16 tensor cores by exact
+ * integer slicing of the FP64 operands on warp-level mma.sync; the same
+ * slices on the 5th-generation tcgen05 MMA with accumulators in tensor
+ * memory.  The two sliced paths give the same bits; all give FP64-accurate
+ * results (error of the order of K 2^-56 max|A_row| max|X_col|), several
+ * times faster than GB300's FP64 pipe.  Modes:
  *   4 (default) autotuned: the first time a contraction shape runs outside
  *     graph capture, every available path is timed on it (the device
  *     otherwise idle, L2 flushed before each timed run, as a step's
@@ -384,9 +383,9 @@ int falcon_set_step_graphs(int enable);
  *     (mma.sync where that view has no tensor map): the same bits as 1;
  *   2 fixed rules: tcgen05 for contractions of at least two 128 x 24 tiles
  *     per SM, mma.sync for the other ones of at least 16 columns per batch
- *     entry, FMA for narrower ones;
+ *     entry, tiles for narrower ones;
  *   1 mma.sync for every contraction with a slice view;
- *   0 FMA only.
+ *   0 tiles only.
  * Applies to launches after the call (step graphs already captured keep
  * their paths).  Returns the previous mode; an unknown mode selects 4.
  * No counterpart in the reference, which uses LAPACK dgetrs
@@ -401,11 +400,11 @@ int falcon_set_gemm_mode(int mode);
  * (falcon_device_tag); rows, K, N, batch = the contraction's shape (rows x K
  * operator, N columns per batch entry); w = slice format in bits (6 or 7);
  * per_mode = 1 when every batch entry has its own columns (2 + n: n row
- * blocks of one operator narrower than 16 columns, merged into one tcgen05
- * launch, path 2, or run one after another, path 0); reuse = 1 when
- * the X slice planes were made by the contraction before; path 0 FMA
- * tiles of the cost model's shape, 1 mma.sync, 2 tcgen05, 3 / 4 / 5 FMA
- * tiles of the best shape 16 / 32 / 64 columns wide (the same bits as 0);
+ * blocks of one operator, merged into one tcgen05 launch, path 2, or run on
+ * the blocks' own path, path 0); reuse = 1 when
+ * the X slice planes were made by the contraction before; path 0 tiles
+ * of the cost model's shape, 1 mma.sync, 2 tcgen05, 3 / 4 / 5 tiles of the
+ * best shape 16 / 32 / 64 columns wide (the same bits as 0);
  * us_p = measured microseconds per contraction on path p (-1: not
  * measured).  NULL or "" detaches the file (decisions stay in
  * memory).  The environment variable FALCON_TUNE_CACHE names a file when

@@ -1,0 +1,73 @@
+"""The fixed-point integer contractions (falcon-dns_gb300/csrc/falcon_fxgemm.cu,
+falcon_set_gemm_mode(0)): every radial and per-mode product of a step, at
+radial sizes around the kernels' row blocks, K chunks and k shares and at
+batch sizes around their column tiles.
+
+- an instance's bits do not depend on the batch it steps in (the narrow
+  kernel alone, tiles of every width in batches: sums of integers);
+- against the exact bf16 slices on mma.sync (mode 1).  Both keep 58 or more
+  bits of an operand relative to the largest of its row or column, so a
+  contraction's outputs differ by at most sqrt(2 K) 2^-57 max|A| max|X|, the
+  rounding of an FP64 product sum (K = 131: 2^-53); steps amplify a rounding
+  by the operators' condition, 1e-12 over 20 steps at Nr = 65 for FP64 tiles,
+  so 4e-12 over 3 steps at Nr <= 131."""
+import numpy as np
+import pytest
+
+from conftest import rel
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("T", "omg", "up", "ur")
+
+
+def states(fg, mode, R, Nm, scheme, B, nsteps=3):
+    prev = fg.set_gemm_mode(mode)
+    try:
+        b = fg.Batch([fg.make_params(R, Nm, scheme, ra=1e5 * (1 + k), dt=1e-6) for k in range(B)])
+        b.init_noise([70 + k for k in range(B)])
+        b.step(nsteps)
+        out = [b.get_state(i) for i in range(B)]
+        b.close()
+        return out
+    finally:
+        fg.set_gemm_mode(prev)
+
+
+@pytest.mark.parametrize("R,Nm,scheme,B", [
+    (17, 5, "CNAB2", 1), (16, 6, "SBDF2", 2), (31, 9, "SBDF3", 3), (32, 20, "CNAB2", 4), (33, 7, "ARS343", 5),
+    (64, 12, "BPR353", 8), (65, 21, "SBDF3", 9), (66, 5, "CNAB2", 17), (97, 8, "ARS443", 33), (129, 10, "SBDF3", 1),
+    (131, 5, "CNAB2", 16), (130, 4, "SBDF2", 40)])
+def test_fixed_point_contractions(fg, R, Nm, scheme, B):
+    got, ref = states(fg, 0, R, Nm, scheme, B), states(fg, 1, R, Nm, scheme, B)
+    for g, r in zip(got, ref):
+        assert max(rel(g[f], r[f]) for f in FIELDS) < 4e-12
+    prev = fg.set_gemm_mode(0)
+    try:
+        a = fg.Instance(fg.make_params(R, Nm, scheme, ra=1e5 * B, dt=1e-6))
+        a.init_noise(70 + B - 1)
+        a.step(3)
+        alone = a.get_state()
+        a.close()
+    finally:
+        fg.set_gemm_mode(prev)
+    for f in FIELDS:
+        assert np.array_equal(alone[f], got[B - 1][f]), f
+
+
+def test_longest_contraction(fg, orc):
+    """K = 257, the most the fixed-point sums hold."""
+    prev = fg.set_gemm_mode(0)
+    try:
+        g = fg.Instance(fg.make_params(257, 4, "CNAB2", ra=1e5, dt=1e-7))
+        o = orc.Sim(orc.make_params(257, 4, "CNAB2", ra=1e5, dt=1e-7))
+        g.init_noise(1)
+        o.init_noise(1)
+        g.step(3)
+        o.step(3)
+        a, b = g.get_state(), o.get_state()
+        for f in FIELDS:
+            assert rel(a[f], b[f]) < 1e-8, f
+        g.close()
+    finally:
+        fg.set_gemm_mode(prev)
