@@ -635,6 +635,21 @@ __global__ void gather_instance_kernel(int R, int M, int B, int b, const double2
     dst[i] = src[((size_t)r * M + m) * B + b];
   }
 }
+// Several fields of instance b at once (one per grid row), each to its own
+// destination, which may be page-locked host memory: the stores then cross
+// to the host as they are made, with no copy after the kernel.
+__global__ void gather_fields_kernel(int R, int M, int B, int b, GatherFields f) {
+  const int n = R * M;
+  const double2* src = f.src[blockIdx.y];
+  double2* dst = f.dst[blockIdx.y];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    dst[i] = src[(size_t)i * B + b];
+}
+cudaError_t launch_gather_fields(int R, int M, int B, int b, int nf, const GatherFields& f, cudaStream_t s) {
+  if (nf <= 0) return cudaSuccess;
+  gather_fields_kernel<<<dim3(std::min((R * M + 255) / 256, 64), nf), 256, 0, s>>>(R, M, B, b, f);
+  return cudaGetLastError();
+}
 cudaError_t launch_scatter_instance(int R, int M, int B, int b, const double2* src, double2* dst,
                                     cudaStream_t s) {
   scatter_instance_kernel<<<ew_grid((size_t)R * M), 256, 0, s>>>(R, M, B, b, src, dst);

@@ -35,7 +35,7 @@
 //   12    tensor-memory allocation and the operator's TMA copies (lane 0);
 //   13    MMA issue (lane 0).
 // Every wait on an mbarrier is bounded: after ~1 s a wait sets an error
-// word in global memory and the CTA's abort flag, and every role leaves
+// word in mapped host memory and the CTA's abort flag, and every role leaves
 // its loop; the MMA warp waits (bounded) for its own products and the TMA
 // warp for its own copies before the tensor memory is freed.  Waiting
 // threads sleep in hardware (try_wait with a suspend-time hint).
@@ -116,7 +116,7 @@ __device__ __noinline__ bool mbar_wait(uint64_t* b, uint32_t parity, volatile in
     if (*abort_flag) return false;
     if (clock64() - t0 > kSpinCycles) {
       *abort_flag = 1;
-      atomicCAS(err, 0, code);
+      *reinterpret_cast<volatile int*>(err) = code;
       return false;
     }
   }
@@ -492,14 +492,18 @@ __global__ void __launch_bounds__(448, 1) tc_gemm_kernel(const __grid_constant__
   }
 }
 
-static __device__ int g_tc_err;
+// The error word, in page-locked host memory that the kernels write directly:
+// the host reads it after a synchronisation without a copy.
 std::once_flag g_tc_err_once[64];
 int* g_tc_err_addr[64];
 
 int* tc_err_ptr(int dev) {
   std::call_once(g_tc_err_once[dev], [dev] {
     void* p = nullptr;
-    if (cudaGetSymbolAddress(&p, g_tc_err) == cudaSuccess) g_tc_err_addr[dev] = static_cast<int*>(p);
+    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
+      *static_cast<int*>(p) = 0;
+      g_tc_err_addr[dev] = static_cast<int*>(p);
+    }
   });
   return g_tc_err_addr[dev];
 }
@@ -520,8 +524,12 @@ cudaError_t launch_tc_w(const TcArgs& a, const CUtensorMap& map, cudaStream_t s)
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   TcArgs q = a;
-  q.err = tc_err_ptr(dev);
-  if (!q.err) return cudaErrorInvalidSymbol;
+  int* err = tc_err_ptr(dev);
+  if (!err) return cudaErrorMemoryAllocation;
+  void* err_dev = nullptr;
+  e = cudaHostGetDevicePointer(&err_dev, err, 0);
+  if (e != cudaSuccess) return e;
+  q.err = static_cast<int*>(err_dev);
   const long T = (long)q.batch * ((q.rows + C::BM - 1) / C::BM) * ((q.N + C::BN - 1) / C::BN);
   const int grid = (int)(T < nsm ? T : nsm);
   tc_gemm_kernel<W><<<grid, kTcThreads, C::SMEM, s>>>(map, q);
@@ -599,12 +607,12 @@ cudaError_t launch_tc_gemm(const TcArgs& a, const CUtensorMap& map, cudaStream_t
 }
 
 int tc_error_read_and_clear() {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, g_tc_err, sizeof(int)) != cudaSuccess) return -1;
-  if (v) {
-    const int z = 0;
-    cudaMemcpyToSymbol(g_tc_err, &z, sizeof(int));
-  }
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
+  volatile int* p = tc_err_ptr(dev);
+  if (!p) return 0;  // no such kernel has run
+  const int v = *p;
+  if (v) *p = 0;
   return v;
 }
 
