@@ -24,10 +24,10 @@
 // neither operand's large elements push the other's out of the 58 bits.
 //
 // Bound: latency for the narrow forms (the radial and per-mode products of a
-// few instances), the integer pipes for the tiles (13 to 15 instructions per
+// few instances), the integer pipes for the tiles (13 or so instructions per
 // product, issue 55 %).  Against FP64 FMA, us with L2 cold: 97 x 97, 342 modes,
 // 2 columns 44 -> 22; 33 x 33, 43 modes, 2 columns 14 -> 8; 65 x 65, 688
-// columns 22 -> 12.5; 65 x 65, 43776 columns 316 -> 131 (85 on tcgen05, which
+// columns 22 -> 11; 65 x 65, 43776 columns 316 -> 119 (85 on tcgen05, which
 // the autotuner takes there).
 //
 // The operators' integers are made once per operator set
@@ -73,10 +73,21 @@ struct Sum {
   long long hh, mid;
   int ll;
 };
+// a b + c as one instruction (a product and a 64-bit add on two pipes, as the
+// compiler makes of mad.wide, takes 10 % longer here: 131 against 119 us for
+// 65 x 65 x 43776)
+__device__ __forceinline__ long long madw1(int a, int b, long long c) {
+  long long r;
+  asm("{\n\t.reg .u32 lo, hi;\n\tmov.b64 {lo, hi}, %3;\n\tmad.lo.cc.s32 lo, %1, %2, lo;\n\t"
+      "madc.hi.s32 hi, %1, %2, hi;\n\tmov.b64 %0, {lo, hi};\n\t}"
+      : "=l"(r)
+      : "r"(a), "r"(b), "l"(c));
+  return r;
+}
 __device__ __forceinline__ void add_product(Sum& s, int2 a, int2 x, int a12, int x12) {
-  s.hh = fx_madw(a.x, x.x, s.hh);
-  s.mid = fx_madw(a.x, x.y, s.mid);
-  s.mid = fx_madw(a.y, x.x, s.mid);
+  s.hh = madw1(a.x, x.x, s.hh);
+  s.mid = madw1(a.x, x.y, s.mid);
+  s.mid = madw1(a.y, x.x, s.mid);
   s.ll += a12 * x12;
 }
 __device__ __forceinline__ void carry(Sum& s) {
@@ -169,8 +180,10 @@ __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const
 // Tile: a block covers NCOL columns and nw * RG * RPT rows, RG = 64 / NCOL;
 // lane = (row group rg, column pair cp).  The X panel (all of K) stays in
 // shared memory, the operator is staged in double-buffered chunks of 16 k.
+// With g.njobs, several products of one shape (rows, K) in one launch: the
+// grid's column blocks run through the jobs.
 template <int RPT, int NCOL>
-__global__ void __launch_bounds__(512) fx_tile_kernel(GemmArgs g) {
+__global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ GemmArgs g) {
   constexpr int RG = 64 / NCOL, CP = NCOL / 2;
   extern __shared__ __align__(16) double fsm[];
   const int nthr = blockDim.x, nw = nthr >> 5;
@@ -178,33 +191,55 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(GemmArgs g) {
   double* xs = fsm;                                                   // [K][NCOL]
   int2* as = reinterpret_cast<int2*>(fsm + (size_t)g.K * NCOL);       // [2][kFxKC][rows_blk]
   int* cex = reinterpret_cast<int*>(as + 2 * kFxKC * rows_blk);       // [NCOL]
-  int* part = cex + NCOL;           // [nthr]
+  int* part = cex + NCOL;                                             // [nthr]
   const int z = blockIdx.z;
+  int N = g.N, nblk = blockIdx.x;
+  long ldx = g.ldx, ldy = g.ldy;
   const int2* A = g.fx + (size_t)z * g.sA;
+  const int* aex = g.fx_ex + (size_t)z * g.lda;
+  const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
   const double* X = g.X + (size_t)z * g.sX;
-  const int n0 = blockIdx.x * NCOL, row0 = blockIdx.y * rows_blk;
+  double* Y = nullptr;
+  if (g.njobs) {
+    int j = 0;
+    for (int nb; nblk >= (nb = (g.job[j].N + NCOL - 1) / NCOL); ++j) nblk -= nb;
+    const FxJob& q = g.job[j];
+    N = q.N;
+    ldx = q.ldx;
+    ldy = q.ldy;
+    A = q.fx;
+    aex = q.fx_ex;
+    w = q.fx_w;
+    X = q.X;
+    Y = q.Y;
+  }
+  const int n0 = nblk * NCOL, row0 = blockIdx.y * rows_blk;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rg = lane / CP, cp = lane - rg * CP;
   const int rw = (warp * RG + rg) * RPT;
-  for (int i = threadIdx.x; i < g.K * NCOL; i += nthr) {
-    const int k = i / NCOL, c = i - k * NCOL;
-    const bool ok = n0 + c < g.N;
-    copy8(xs + i, ok ? X + (size_t)k * g.ldx + n0 + c : X, ok);
+  {
+    constexpr int KW = NCOL >= 32 ? 1 : 32 / NCOL, HW = NCOL >= 32 ? NCOL / 32 : 1;  // k, column halves per warp
+    for (int i = warp; i < (g.K + KW - 1) / KW * HW; i += nw) {
+      const int k = (i / HW) * KW + (NCOL >= 32 ? 0 : lane / NCOL), c = (i % HW) * 32 + (NCOL >= 32 ? lane : lane % NCOL);
+      if (k < g.K) {
+        const bool ok = n0 + c < N;
+        copy8(xs + k * NCOL + c, ok ? X + (size_t)k * ldx + n0 + c : X, ok);
+      }
+    }
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   auto issue = [&](int k0, int2* buf) {
-    const int n = min(kFxKC, g.K - k0) * rows_blk;
-    for (int i = threadIdx.x; i < n; i += nthr) {
-      const int kk = i / rows_blk, rr = i - kk * rows_blk;
-      const bool ok = row0 + rr < g.rows;
-      copy8(buf + i, ok ? A + (size_t)(k0 + kk) * g.lda + row0 + rr : A, ok);
-    }
+    const int kc = min(kFxKC, g.K - k0);
+    for (int kk = warp; kk < kc; kk += nw)
+      for (int rr = lane; rr < rows_blk; rr += 32) {
+        const bool ok = row0 + rr < g.rows;
+        copy8(buf + kk * rows_blk + rr, ok ? A + (size_t)(k0 + kk) * g.lda + row0 + rr : A, ok);
+      }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   issue(0, as);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
   convert_panel(xs, g.K, NCOL, w, cex, part);
   Sum acc[RPT][2];
 #pragma unroll
@@ -221,8 +256,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(GemmArgs g) {
     __syncthreads();
     const int2* Aw = as + cur * kFxKC * rows_blk + rw;
     const int4* Xw = reinterpret_cast<const int4*>(xs + (size_t)k0 * NCOL) + cp;
-#pragma unroll 2
-    for (int kk = 0; kk < kc; ++kk) {
+    auto one = [&](int kk) {
       const int4 xv = Xw[kk * (NCOL / 2)];
       const int2 x0 = make_int2(xv.x, xv.y), x1 = make_int2(xv.z, xv.w);
       const int x012 = x0.y >> 20, x112 = x1.y >> 20;
@@ -233,6 +267,12 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(GemmArgs g) {
         add_product(acc[i][0], av, x0, a12, x012);
         add_product(acc[i][1], av, x1, a12, x112);
       }
+    };
+    if (kc == kFxKC) {
+#pragma unroll 4
+      for (int kk = 0; kk < kFxKC; ++kk) one(kk);
+    } else {
+      for (int kk = 0; kk < kc; ++kk) one(kk);
     }
 #pragma unroll
     for (int i = 0; i < RPT; ++i) { carry(acc[i][0]); carry(acc[i][1]); }
@@ -243,11 +283,11 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(GemmArgs g) {
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
     const int row = row0 + rw + i;
-    if (row < g.rows && n < g.N) {
-      const int ea = g.fx_ex[(size_t)z * g.lda + row];
-      double* yp = output_row(g, z, row) + n;
+    if (row < g.rows && n < N) {
+      const int ea = aex[row];
+      double* yp = (Y ? Y + (size_t)row * ldy : output_row(g, z, row)) + n;
       const double y0 = value_of(acc[i][0], ea, e0, g.alpha);
-      if (n + 1 < g.N) {
+      if (n + 1 < N) {
         const double y1 = value_of(acc[i][1], ea, e1, g.alpha);
         if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
           *reinterpret_cast<double2*>(yp) = make_double2(y0, y1);
@@ -329,6 +369,13 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(GemmArgs g) {
   output_row(g, z, row)[warp] = value_of(s, g.fx_ex[(size_t)z * g.lda + row], cex[warp], g.alpha);
 }
 
+long column_blocks(const GemmArgs& g, int ncol) {
+  if (!g.njobs) return ((long)g.N + ncol - 1) / ncol;
+  long n = 0;
+  for (int j = 0; j < g.njobs; ++j) n += ((long)g.job[j].N + ncol - 1) / ncol;
+  return n;
+}
+
 template <int RPT, int NCOL>
 cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream_t s) {
   static std::atomic<bool> opted[64];  // opted in to large shared memory, per device
@@ -342,7 +389,7 @@ cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream
   }
   const int rows_blk = nw * (64 / NCOL) * RPT;
   const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw) * 4;
-  const dim3 grid((g.N + NCOL - 1) / NCOL, row_blocks, g.batch);
+  const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, g.batch);
   fx_tile_kernel<RPT, NCOL><<<grid, 32 * nw, smem, s>>>(g);
   return cudaGetLastError();
 }
@@ -359,7 +406,7 @@ TileShape pick_shape(const GemmArgs& g, int nsm) {
   for (int ncol = 16; ncol <= 64; ncol *= 2) {
     if (g.fma_ncol && ncol != g.fma_ncol) continue;
     const int rg = 64 / ncol;
-    const long cb = (long)((g.N + ncol - 1) / ncol) * g.batch;
+    const long cb = column_blocks(g, ncol) * g.batch;
     for (int rb = 1; rb <= 16; ++rb)
       for (int nw = 4; nw <= 16; ++nw)
         for (int rpt = 1; rpt <= 8; ++rpt) {
@@ -410,7 +457,7 @@ cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int
 cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.rows <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
   if (g.K > 257 || !g.fx) return cudaErrorInvalidValue;
-  if (g.N <= 8) {
+  if (g.N <= 8 && !g.njobs) {
     const dim3 grid((g.rows + 31) / 32, g.batch);
     auto smem = [&](int nc) { return (size_t)nc * (8 * 32 * sizeof(Part) + g.K * sizeof(double)); };
     if (g.N > 4 && g.K > 170) {  // over 48 KB with the static part
@@ -426,13 +473,15 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   // shapes are memoised per problem size: the search runs on the host once
-  struct Memo { int rows, K, N, batch, nsm, ncol; TileShape t; };
+  struct Memo { int rows, K, N, total, batch, nsm, ncol; TileShape t; };
   thread_local std::unordered_map<unsigned long long, Memo> memo;
   unsigned long long key = 1469598103934665603ull;
-  for (int v : {g.rows, g.K, g.N, g.batch, nsm, g.fma_ncol}) key = (key ^ (unsigned)v) * 1099511628211ull;
+  const int total = (int)column_blocks(g, 1);  // columns of all jobs
+  for (int v : {g.rows, g.K, g.N, total, g.batch, nsm, g.fma_ncol}) key = (key ^ (unsigned)v) * 1099511628211ull;
   Memo& m = memo[key];
-  if (m.rows != g.rows || m.K != g.K || m.N != g.N || m.batch != g.batch || m.nsm != nsm || m.ncol != g.fma_ncol)
-    m = Memo{g.rows, g.K, g.N, g.batch, nsm, g.fma_ncol, pick_shape(g, nsm)};
+  if (m.rows != g.rows || m.K != g.K || m.N != g.N || m.total != total || m.batch != g.batch || m.nsm != nsm ||
+      m.ncol != g.fma_ncol)
+    m = Memo{g.rows, g.K, g.N, total, g.batch, nsm, g.fma_ncol, pick_shape(g, nsm)};
   if (m.t.ncol == 16) return launch_ncol<16>(g, m.t, s);
   if (m.t.ncol == 32) return launch_ncol<32>(g, m.t, s);
   return launch_ncol<64>(g, m.t, s);

@@ -1440,7 +1440,8 @@ int run_path_once(Group* g, int cls, GemmArgs q, int path, bool reuse) {
 // line:
 //   <device> <rows> <K> <N> <batch> <w> <per_mode> <reuse> <path> <us_0> ... <us_5>
 // device = the CUDA device name with blanks as '_' and "_sm<SM count>";
-// per_mode = 1 when the batch entries have their own X (sX != 0); reuse = 1
+// per_mode = 1 when the batch entries have their own X (sX != 0), 2 + n for n
+// merged row blocks, 16 + n for n products of one launch; reuse = 1
 // when X's slice planes were made by the contraction before; w = the slice
 // format (6 or 7); path 0 tiles (cost-model shape), 1 mma.sync, 2 tcgen05,
 // 3/4/5 tiles of 16/32/64 columns; us_p = the measured
@@ -1719,6 +1720,83 @@ int run_merged_tc(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmA
   return launch(g, cls, gemm_flops(all), [&]() { return launch_tc_gemm(t, *map, g->stream); });
 }
 
+// Several radial products of one shape (the derivatives and Laplacians of a
+// stage), independent of each other.  As one launch of tiles, so that the small
+// ones share their launch and the others fill the SMs together, when every
+// one's own path is the tiles (the five of a CNAB2 step at 33 x 33 x 130: one
+// launch 10.0 us, five 29); under mode 4 where that measures faster than one
+// after another on their own paths (at 65 x 65 x 43776 tcgen05 does, 85 against
+// 119 us a product).  Cached under per_mode = 16 + the number of products with
+// the columns of all: path 0 one launch, 2 one after another; like every
+// decision kept from the first run outside capture.
+int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
+  std::vector<GemmArgs> v(products);
+  const int mode = g_gemm_mode.load();
+  GemmArgs all{};
+  bool tiles = (mode == 0 || mode == 4) && v.size() > 1 && v.size() <= (size_t)kFxJobs;
+  long cols = 0;
+  for (size_t i = 0; i < v.size() && tiles; ++i) {
+    GemmArgs q = v[i];
+    tiles = attach_group(g, &q) && q.batch == 1 && q.rows == v[0].rows && q.K == v[0].K && q.lda == v[0].lda &&
+            q.alpha == v[0].alpha;
+    if (!tiles) break;
+    if (i == 0) {
+      all = q;
+      all.oz_s = nullptr;
+      all.oz_xs = nullptr;
+    }
+    all.job[i] = FxJob{q.fx, q.fx_ex, q.fx_w, q.X, q.Y, q.ldx, q.ldy, q.N};
+    cols += q.N;
+  }
+  all.njobs = tiles ? (int)v.size() : 0;
+  auto apart = [&]() {
+    for (const GemmArgs& q : v) {
+      const int rc = gemm(g, cls, q);
+      if (rc) return rc;
+    }
+    return 0;
+  };
+  double flops = 0.0;
+  for (const GemmArgs& q : v) flops += gemm_flops(q);
+  auto together = [&]() { return launch(g, cls, flops, [&]() { return launch_fx_gemm(all, g->stream); }); };
+  if (!tiles) return apart();
+  if (mode == 0) return together();
+  TuneKey k{device_tag(), v[0].rows, v[0].K, (int)cols, 1, all.oz_w, 16 + (int)v.size(), 0};
+  int known = -1;
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    auto it = g_tune.find(k);
+    if (it != g_tune.end()) known = it->second.path;
+  }
+  if (known >= 0) return known == PATH_FMA ? together() : apart();
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  CK(cudaStreamIsCapturing(g->stream, &cs));
+  int rc = 0;
+  if (cs != cudaStreamCaptureStatusNone || g->prof) return apart();
+  void* flush = tune_flush_buffer();
+  if (!flush) return fail(FALCON_ENOMEM, "contraction tuning: no device memory for the L2 flush buffer");
+  if ((rc = apart())) return rc;  // their own paths, measured where new
+  CK(cudaDeviceSynchronize());
+  TuneEntry e{};
+  for (float& t : e.us) t = -1.f;
+  cudaEvent_t a = nullptr, b = nullptr;
+  CK(cudaEventCreate(&a));
+  CK(cudaEventCreate(&b));
+  rc = time_fastest(g, flush, a, b, apart, &e.us[PATH_TC]);
+  if (!rc) rc = time_fastest(g, flush, a, b, together, &e.us[PATH_FMA]);
+  cudaEventDestroy(a);
+  cudaEventDestroy(b);
+  if (rc) return rc;
+  e.path = e.us[PATH_FMA] <= e.us[PATH_TC] ? PATH_FMA : PATH_TC;
+  g_tune_measured++;
+  {
+    std::lock_guard<std::mutex> lk(g_tune_mu);
+    g_tune[k] = e;
+    tune_store_locked(k, e);
+  }
+  return e.path == PATH_FMA ? together() : apart();
+}
+
 // Mode 4: the row blocks as one merged tcgen05 launch, or on their own
 // (autotuned) path, whichever measures faster with the autotuner's method
 // (for blocks narrower than 16 columns the blocks unless the merged launch is
@@ -1967,18 +2045,17 @@ int step_imex(Group* g) {
   }
   const Scheme& sc = vs;
   OpSet* o = g->ops.get();
-  if ((rc = gemm(g, KC_GEMM_RADIAL, radial(o->D1p, g->ntr, g->dntr, R, M, B))) ||
-      (rc = gemm(g, KC_GEMM_RADIAL, radial(o->D1p, g->nwr, g->dnwr, R, M, B))))
-    return rc;
   const bool cn = (sc.imp == FALCON_IMP_CN);
+  const GemmArgs dt = radial(o->D1p, g->ntr, g->dntr, R, M, B), dw = radial(o->D1p, g->nwr, g->dnwr, R, M, B);
   if (cn) {
     GemmArgs gl = radial(o->Lp, g->up, g->lu0, R, M, B);
     gl.N = 2 * B; gl.ldy = 2L * B;
-    if ((rc = gemm(g, KC_GEMM_RADIAL, radial(o->Lp, g->T(), g->lt, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->Lp, g->W(), g->lw, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, gl)))
-      return rc;
+    rc = gemm_set(g, KC_GEMM_RADIAL, {dt, dw, radial(o->Lp, g->T(), g->lt, R, M, B),
+                                      radial(o->Lp, g->W(), g->lw, R, M, B), gl});
+  } else {
+    rc = gemm_set(g, KC_GEMM_RADIAL, {dt, dw});
   }
+  if (rc) return rc;
   const int ni = sc.n_imp, ne = sc.n_exp;
   const int he_new = (g->head_e + ne - 1) % ne;
   const int h_new = (g->head + ni - 1) % ni;
@@ -2082,11 +2159,10 @@ int step_imexrk(Group* g) {
     if (sa && st == ns - 1) break;  // last-stage derivatives are unused by the SA assembly
     GemmArgs gl = radial(o->Lp, g->up, g->lu0, R, M, B);
     gl.N = 2 * B; gl.ldy = 2L * B;
-    if ((rc = gemm(g, KC_GEMM_RADIAL, radial(o->D1p, g->ntr, g->dntr, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->D1p, g->nwr, g->dnwr, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->Lp, g->T(), g->lt, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->Lp, g->W(), g->lw, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, gl)))
+    if ((rc = gemm_set(g, KC_GEMM_RADIAL, {radial(o->D1p, g->ntr, g->dntr, R, M, B),
+                                           radial(o->D1p, g->nwr, g->dnwr, R, M, B),
+                                           radial(o->Lp, g->T(), g->lt, R, M, B),
+                                           radial(o->Lp, g->W(), g->lw, R, M, B), gl})))
       return rc;
     a.fat_out = g->fat[st]; a.fdt_out = g->fdt[st]; a.faw_out = g->faw[st]; a.fdw_out = g->fdw[st];
     a.buo_out = (st == 0) ? g->buo[0] : nullptr;
@@ -2208,12 +2284,11 @@ int step_rk(Group* g) {
     const bool coef = (nstep == 1 && st == 0);
     GemmArgs gl = radial(coef ? o->Lc : o->Lp, g->up, g->lu0, R, M, B);
     gl.N = 2 * B; gl.ldy = 2L * B;
-    if ((rc = gemm(g, KC_GEMM_RADIAL, radial(o->D1p, g->ntr, g->dntr, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->D1p, g->nwr, g->dnwr, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->Lp, g->T(), g->lt, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(o->Lp, g->W(), g->lw, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, radial(coef ? o->D1c : o->D1p, g->up, dup, R, M, B))) ||
-        (rc = gemm(g, KC_GEMM_RADIAL, gl)))
+    if ((rc = gemm_set(g, KC_GEMM_RADIAL, {radial(o->D1p, g->ntr, g->dntr, R, M, B),
+                                           radial(o->D1p, g->nwr, g->dnwr, R, M, B),
+                                           radial(o->Lp, g->T(), g->lt, R, M, B),
+                                           radial(o->Lp, g->W(), g->lw, R, M, B),
+                                           radial(coef ? o->D1c : o->D1p, g->up, dup, R, M, B), gl})))
       return rc;
     RkRhsArgs a{};
     a.R = R; a.M = M; a.B = B; a.inv_pr = g->inv_pr;

@@ -199,6 +199,18 @@ struct NonlinArgs {
   double* umax;                          // optional [r][b][2]: max|ur|, max|uphi| on the grid of plan.P points
 };
 
+// One product of a launch of several (launch_fx_gemm): as the fields of
+// GemmArgs, with its rows, K, lda and alpha.
+struct FxJob {
+  const int2* fx;
+  const int *fx_ex, *fx_w;
+  const double* X;
+  double* Y;
+  long ldx, ldy;
+  int N;
+};
+constexpr int kFxJobs = 6;
+
 // Y[row][n] = alpha * sum_k A[k*lda + row] * X[k*ldx + n] for
 // row < rows, n < N, with a batch index z applying the strides sA, sX, sY.
 struct GemmArgs {
@@ -236,6 +248,9 @@ struct GemmArgs {
   int nout;
   int rend[4];
   double* Yo[4];
+  // fixed-point path: several products of one shape (batch 1) in one launch
+  int njobs;
+  FxJob job[kFxJobs];
   // fixed-point tiles: 0 = the tile shape of the cost model, 16 / 32 / 64 = the
   // cost model's best shape of that column width (the same bits)
   int fma_ncol;

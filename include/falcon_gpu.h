@@ -401,7 +401,8 @@ int falcon_set_gemm_mode(int mode);
  * operator, N columns per batch entry); w = slice format in bits (6 or 7);
  * per_mode = 1 when every batch entry has its own columns (2 + n: n row
  * blocks of one operator, merged into one tcgen05 launch, path 2, or run on
- * the blocks' own path, path 0); reuse = 1 when
+ * the blocks' own path, path 0; 16 + n: n products of one launch of tiles,
+ * path 0, or one after another on their own paths, path 2); reuse = 1 when
  * the X slice planes were made by the contraction before; path 0 tiles
  * of the cost model's shape, 1 mma.sync, 2 tcgen05, 3 / 4 / 5 tiles of the
  * best shape 16 / 32 / 64 columns wide (the same bits as 0);

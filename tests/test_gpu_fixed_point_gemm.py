@@ -55,6 +55,22 @@ def test_fixed_point_contractions(fg, R, Nm, scheme, B):
         assert np.array_equal(alone[f], got[B - 1][f]), f
 
 
+@pytest.mark.parametrize("R,Nm,scheme,B", [(17, 5, "RK2", 1), (33, 16, "RK4", 1), (33, 15, "RK4", 4), (65, 21, "RK2", 9),
+                                           (33, 16, "CNAB2", 1), (65, 20, "SBDF2", 3)])
+def test_products_in_one_launch(fg, R, Nm, scheme, B):
+    """A stage's radial products as one launch (two, five or six of them, the
+    last of twice the batch's columns, none a multiple of the tile): the same
+    bound against mode 1 as above, and mode 4 repeats its own bits whichever
+    way it decided."""
+    got, ref = states(fg, 0, R, Nm, scheme, B), states(fg, 1, R, Nm, scheme, B)
+    for g, r in zip(got, ref):
+        assert max(rel(g[f], r[f]) for f in FIELDS) < 4e-12
+    a, b = states(fg, 4, R, Nm, scheme, B), states(fg, 4, R, Nm, scheme, B)
+    for g, h, r in zip(a, b, ref):
+        assert all(np.array_equal(g[f], h[f]) for f in FIELDS)
+        assert max(rel(g[f], r[f]) for f in FIELDS) < 4e-12
+
+
 def test_longest_contraction(fg, orc):
     """K = 257, the most the fixed-point sums hold."""
     prev = fg.set_gemm_mode(0)
