@@ -57,13 +57,16 @@ __device__ __forceinline__ int exponent_of(double a, int w) {
   if (high == 0u && __double2loint(a) == 0) return kNone;
   return (int)max(high >> 20, 1u) - 1022 + w;
 }
+__device__ __forceinline__ int2 signed_split(unsigned long long t) {
+  return make_int2((int)((unsigned)(t >> 32) + ((unsigned)t >> 31)), (int)t);
+}
 // trunc(a 2^w 2^(bits - e)) split into (h, l signed)
 template <int BITS>
 __device__ __forceinline__ int2 split_of(double a, int w, int e) {
   const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
   unsigned long long t = fx_mag_of(bits, e - w + 1022) >> (59 - BITS);
   if ((long long)bits < 0) t = 0ull - t;
-  return make_int2((int)((unsigned)(t >> 32) + ((unsigned)t >> 31)), (int)t);
+  return signed_split(t);
 }
 // The scale of a row or column whose largest exponent is m, and its exponent.
 __device__ __forceinline__ int scale_of(int m) { return m == INT32_MAX ? 100000 : m == kNone ? 0 : m; }
@@ -124,6 +127,11 @@ __device__ __forceinline__ void copy8(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 8 : 0) : "memory");
 }
 
+__device__ __forceinline__ void copy16(void* dst, const void* src, bool valid) {
+  const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 16 : 0) : "memory");
+}
+
 // One thread per (entry, column k): the exponent of its largest element.
 __global__ void fx_weight_kernel(const double* A, long lda, long sA, int rows, int K, int nb, int* wk) {
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
@@ -154,24 +162,28 @@ __global__ void fx_operator_kernel(const double* A, long lda, long sA, int rows,
   for (int k = 0; k < K; ++k) o[(size_t)k * lda] = split_of<kBitsA>(a[(size_t)k * lda], w ? -w[k] : 0, scale_of(m));
 }
 
-// X panel of a block in shared memory, xs[k * ncol + c] (staged as doubles,
-// complete when this is called): column exponents in cex, integers in place.
-// w: the operator's weights (or null); part: blockDim.x words.
-__device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const int* w, int* cex, int* part) {
-  const int tid = threadIdx.x, J = blockDim.x / ncol, c = tid % ncol, j = tid / ncol;
+// X panel of a block in shared memory, xs[k * (ncol + PAD) + c] (staged as
+// doubles, complete when this is called): column exponents in cex, integers in
+// place.  w: the operator's weights (or null); part: blockDim.x words; spare:
+// leading bits left free.
+template <int PAD = 0>
+__device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const int* w, int* cex, int* part,
+                                              int spare = 0) {
+  const int tid = threadIdx.x, J = blockDim.x / ncol, c = tid % ncol, j = tid / ncol, st = ncol + PAD;
   const bool act = j < J;
   int m = kNone;
   if (act) {
-    for (int k = j; k < K; k += J) m = max(m, exponent_of(xs[k * ncol + c], w ? __ldg(w + k) : 0));
+    for (int k = j; k < K; k += J) m = max(m, exponent_of(xs[k * st + c], w ? __ldg(w + k) : 0));
     part[tid] = m;
   }
   __syncthreads();
   if (act) {
     for (int i = 0; i < J; ++i) m = max(m, part[i * ncol + c]);
+    if (m != INT32_MAX && m != kNone) m += spare;
     if (j == 0) cex[c] = mark_of(m);
     for (int k = j; k < K; k += J) {
-      const int2 v = split_of<kBitsX>(xs[k * ncol + c], w ? __ldg(w + k) : 0, scale_of(m));
-      reinterpret_cast<int2*>(xs)[k * ncol + c] = v;
+      const int2 v = split_of<kBitsX>(xs[k * st + c], w ? __ldg(w + k) : 0, scale_of(m));
+      reinterpret_cast<int2*>(xs)[k * st + c] = v;
     }
   }
   __syncthreads();
@@ -369,6 +381,174 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(GemmArgs g) {
   output_row(g, z, row)[warp] = value_of(s, g.fx_ex[(size_t)z * g.lda + row], cex[warp], g.alpha);
 }
 
+// Complex columns x[c][0..n) through real n x n operators whose rows (or
+// columns) i and n - 1 - i agree up to sign and a few bits (the Chebyshev
+// transforms).  With h = ceil(n / 2) pairs p of X (points p, n - 1 - p summed and
+// differenced, or coefficients 2 p, 2 p + 1) and h pairs of outputs j,
+//   S0 = sum_p A0[p][j] X0[p], S1 = sum_p A1[p][j] X1[p]
+// hold half the products of the dense operator.  What the mirrored half
+// differs by (the rounding of its own cosines, 2^-40 of an element) is a
+// third sum of one 32-bit product each, D = sum (26 bits of the difference)
+// (27 bits of x), added at its scale: outputs are those of the dense operator.
+//   FWD: X0, X1 = x_p +- x_{n-1-p};  out_{2j} = S0 + D0, out_{2j+1} = S1 + D1
+//   else X0, X1 = x_{2p}, x_{2p+1};  out_j = S0 + S1, out_{n-1-j} = +-(S0 - S1) + D
+// A block takes NCOL real columns (re and im side by side) of one operator;
+// loads, outputs (through shared memory) and the operator's chunks of 8 p are
+// coalesced.  Bound: the integer multiply-adds (61 % of that pipe's cycles, 16
+// to 20 warps an SM); 65 points, 10944 columns: fwd 56 us, d1 and d2 102 us
+// (one FP64 dot product a thread: 684 us for the three).
+constexpr int kFxPC = 8;  // p per staged operator chunk
+template <int RPT, int NCOL, bool FWD>
+__global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__ FxColumns g) {
+  constexpr int RG = 64 / NCOL, CP = NCOL / 2, ST = NCOL + 2;  // ST: columns' stores hit every bank
+  extern __shared__ __align__(16) double fsm[];
+  const int n = g.n, h = (n + 1) / 2, nthr = blockDim.x, nw = nthr >> 5, hb = nw * RG * RPT;
+  double* xs = fsm;                                                  // [n + 1][ST]
+  int4* as = reinterpret_cast<int4*>(fsm + (size_t)(n + 1) * ST);    // [2][kFxPC][hb]
+  int2* ds = reinterpret_cast<int2*>(as + 2 * kFxPC * hb);           // [2][kFxPC][hb]
+  int* cex = reinterpret_cast<int*>(ds + 2 * kFxPC * hb);            // [NCOL]
+  int* part = cex + NCOL;                                            // [nthr]
+  const FxColumnsOp& op = g.op[blockIdx.y];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = blockIdx.x * CP;
+  const int rg = lane / CP, cp = lane - rg * CP, rw = (warp * RG + rg) * RPT;
+  for (int c = warp; c < CP; c += nw) {
+    const bool ok = c0 + c < g.ncol;
+    const double2* x = g.in + (size_t)(ok ? c0 + c : 0) * n;
+    for (int k = lane; k < n; k += 32) copy16(xs + k * ST + 2 * c, x + k, ok);
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+  auto issue = [&](int p0, int buf) {
+    const int pc = min(kFxPC, h - p0);
+    for (int i = threadIdx.x; i < pc * h; i += nthr) {
+      const int p = i / h, j = i - p * h, o = (buf * kFxPC + p) * hb + j;
+      copy16(as + o, op.A + (size_t)p0 * h + i, true);
+      copy8(ds + o, op.D + (size_t)p0 * h + i, true);
+    }
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  issue(0, 0);
+  asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+  __syncthreads();
+  convert_panel<ST - NCOL>(xs, n, NCOL, op.w, cex, part, FWD ? 1 : 0);
+  if (FWD) {
+    for (int i = threadIdx.x; i < n / 2 * NCOL; i += nthr) {
+      const int p = i / NCOL, c = i - p * NCOL;
+      int2* a = reinterpret_cast<int2*>(xs) + p * ST + c;
+      int2* b = reinterpret_cast<int2*>(xs) + (n - 1 - p) * ST + c;
+      const long long va = (long long)a->x * 4294967296LL + a->y, vb = (long long)b->x * 4294967296LL + b->y;
+      *a = signed_split(va + vb);
+      *b = signed_split(va - vb);
+    }
+    __syncthreads();
+  }
+  Sum s0[RPT][2], s1[RPT][2];
+  long long d0[RPT][2], d1[RPT][2];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i)
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      s0[i][c] = s1[i][c] = Sum{0, 0, 0};
+      d0[i][c] = d1[i][c] = 0;
+    }
+  int cur = 0;
+  for (int p0 = 0; p0 < h; p0 += kFxPC) {
+    const int pc = min(kFxPC, h - p0);
+    if (p0 + kFxPC < h) {
+      issue(p0 + kFxPC, cur ^ 1);
+      asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+    }
+    __syncthreads();
+    const int4* Aw = as + cur * kFxPC * hb + rw;
+    const int2* Dw = ds + cur * kFxPC * hb + rw;
+    const int4* xp = reinterpret_cast<const int4*>(xs) + cp;
+#pragma unroll 2
+    for (int pp = 0; pp < pc; ++pp) {
+      const int p = p0 + pp;
+      const int4 u = xp[(FWD ? p : 2 * p) * (ST / 2)], v = xp[(FWD ? n - 1 - p : 2 * p + 1) * (ST / 2)];
+      const int2 u0 = make_int2(u.x, u.y), u1 = make_int2(u.z, u.w), v0 = make_int2(v.x, v.y), v1 = make_int2(v.z, v.w);
+      const int u012 = u0.y >> 20, u112 = u1.y >> 20, v012 = v0.y >> 20, v112 = v1.y >> 20;
+      const int m0 = FWD ? (u0.x - v0.x) >> 1 : 0, m1 = FWD ? (u1.x - v1.x) >> 1 : 0;  // x_{n-1-p}
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        const int4 a = Aw[pp * hb + i];
+        const int2 d = Dw[pp * hb + i];
+        const int2 a0 = make_int2(a.x, a.y), a1 = make_int2(a.z, a.w);
+        const int a012 = a0.y >> 20, a112 = a1.y >> 20;
+        add_product(s0[i][0], a0, u0, a012, u012);
+        add_product(s0[i][1], a0, u1, a012, u112);
+        add_product(s1[i][0], a1, v0, a112, v012);
+        add_product(s1[i][1], a1, v1, a112, v112);
+        if (FWD) {
+          d0[i][0] = madw1(d.x, m0, d0[i][0]);
+          d0[i][1] = madw1(d.x, m1, d0[i][1]);
+          d1[i][0] = madw1(d.y, m0, d1[i][0]);
+          d1[i][1] = madw1(d.y, m1, d1[i][1]);
+        } else {
+          d0[i][0] = madw1(d.y, v0.x, madw1(d.x, u0.x, d0[i][0]));
+          d0[i][1] = madw1(d.y, v1.x, madw1(d.x, u1.x, d0[i][1]));
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      carry(s0[i][0]); carry(s0[i][1]);
+      carry(s1[i][0]); carry(s1[i][1]);
+    }
+    __syncthreads();  // the buffer is refilled, after the last chunk the panel
+    cur ^= 1;
+  }
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int j = rw + i;
+    if (j >= h) break;
+    const int4 e = __ldg(op.ex + j);
+    double y[2], z[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const Sum a = s0[i][c], b = s1[i][c];
+      Sum f, m;
+      if (FWD) {
+        f = Sum{a.hh, a.mid + (d0[i][c] >> e.z), a.ll};
+        m = Sum{b.hh, b.mid + (d1[i][c] >> e.w), b.ll};
+      } else {
+        f = Sum{a.hh + b.hh, a.mid + b.mid, a.ll + b.ll};
+        m = op.sign > 0 ? Sum{a.hh - b.hh, a.mid - b.mid, a.ll - b.ll} : Sum{b.hh - a.hh, b.mid - a.mid, b.ll - a.ll};
+        m.mid += d0[i][c] >> e.z;
+      }
+      y[c] = value_of(f, e.x, cex[2 * cp + c], 1.0);
+      z[c] = value_of(m, e.y, cex[2 * cp + c], 1.0);
+    }
+    const int r = FWD ? 2 * j : j, q = FWD ? 2 * j + 1 : n - 1 - j;
+    if (q < n && q != r) *reinterpret_cast<double2*>(xs + q * ST + 2 * cp) = make_double2(z[0], z[1]);
+    *reinterpret_cast<double2*>(xs + r * ST + 2 * cp) = make_double2(y[0], y[1]);
+  }
+  __syncthreads();
+  for (int c = warp; c < CP && c0 + c < g.ncol; c += nw) {
+    double2* y = op.out + (size_t)(c0 + c) * n;
+    for (int k = lane; k < n; k += 32) y[k] = *reinterpret_cast<const double2*>(xs + k * ST + 2 * c);
+  }
+}
+
+template <int RPT, int NCOL, bool FWD>
+cudaError_t launch_fx_columns_shape(const FxColumns& g, cudaStream_t s) {
+  const int h = (g.n + 1) / 2, per = 64 / NCOL * RPT, nw = std::max(2, (h + per - 1) / per), hb = nw * per;
+  const size_t smem = (size_t)(g.n + 1) * (NCOL + 2) * 8 + 2 * kFxPC * hb * 24 + (NCOL + 32 * nw) * 4;
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(fx_columns_kernel<RPT, NCOL, FWD>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return e;
+  }
+  const dim3 grid((g.ncol + NCOL / 2 - 1) / (NCOL / 2), g.nop);
+  fx_columns_kernel<RPT, NCOL, FWD><<<grid, 32 * nw, smem, s>>>(g);
+  return cudaGetLastError();
+}
+template <int RPT, int NCOL>
+cudaError_t launch_fx_columns_dir(const FxColumns& g, cudaStream_t s) {
+  return g.fwd ? launch_fx_columns_shape<RPT, NCOL, true>(g, s) : launch_fx_columns_shape<RPT, NCOL, false>(g, s);
+}
+
 long column_blocks(const GemmArgs& g, int ncol) {
   if (!g.njobs) return ((long)g.N + ncol - 1) / ncol;
   long n = 0;
@@ -485,6 +665,27 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (m.t.ncol == 16) return launch_ncol<16>(g, m.t, s);
   if (m.t.ncol == 32) return launch_ncol<32>(g, m.t, s);
   return launch_ncol<64>(g, m.t, s);
+}
+
+// Shape: NCOL real columns a block, RPT output pairs a thread (64 / NCOL x RPT
+// pairs a warp).  Few columns: small blocks and one pair a thread, for more
+// blocks and shorter chains (65 points, us of fwd / d1d2 at <1, 8>, <1, 16>, <3, 16>:
+// 300 columns 11.1/10.8, 12.7/12.5, 16.6/17.2; 1000 columns 14.5/20.5, 12.7/17.3,
+// 16.7/20.8; 10944 columns 67/117, 62/107, 56/102).  Many: one pair a thread
+// up to 32 pairs (33 points, 20000 columns <1, 32> 39/64, <3, 16> 41/72), above
+// that the shape that pads least (97 points, 10000 columns <2, 16> 113/195,
+// <3, 16> 134/243; 129 points, 2000 columns <3, 32> 41/77, <3, 16> 48/89).
+cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s) {
+  if (g.n < 3 || g.n > 257 || g.ncol < 1 || g.ncol > 65535) return cudaErrorInvalidValue;
+  const int h = (g.n + 1) / 2;
+  const long cols = (long)g.ncol * g.nop;
+  if (cols < 4 * 152) return h <= 128 ? launch_fx_columns_dir<1, 8>(g, s) : launch_fx_columns_dir<2, 8>(g, s);
+  if (h <= 32) return launch_fx_columns_dir<1, 32>(g, s);
+  if (h <= 64) {
+    if (cols < 32 * 152) return launch_fx_columns_dir<1, 16>(g, s);
+    return (h + 11) / 12 * 120 <= 11 * h ? launch_fx_columns_dir<3, 16>(g, s) : launch_fx_columns_dir<2, 16>(g, s);
+  }
+  return h <= 96 ? launch_fx_columns_dir<3, 32>(g, s) : launch_fx_columns_dir<3, 16>(g, s);
 }
 
 }  // namespace falcon

@@ -4104,12 +4104,77 @@ double falcon_fp64_mma_peak_gflops(void) { return measure_fp64_mma_peak(); }
 // fwd = t^T diag(c') / ((n-1) C) (C = sqrt(2/(n-1))).
 // ---------------------------------------------------------------------------
 namespace {
+struct ChebOp {
+  double* m = nullptr;  // dense, for sizes past the fixed-point form
+  FxColumnsOp fx{};
+};
 struct ChebMats {
-  int n = 0;
-  double *fwd = nullptr, *inv = nullptr, *d1 = nullptr, *d2 = nullptr;
+  ChebOp op[4];  // fwd, inv, d1, d2
 };
 std::mutex g_cheb_mu;
 std::map<int, ChebMats> g_cheb;
+
+int2 fx_split(double a, int bits, int e) {  // trunc(a 2^(bits - e)) as h 2^32 + l, l signed
+  const unsigned long long t = (unsigned long long)(long long)std::ldexp(a, bits - e);
+  return make_int2((int)((unsigned)(t >> 32) + ((unsigned)t >> 31)), (int)t);
+}
+
+// An operator in the form of fx_columns_kernel (falcon_fxgemm.cu).  Rows i and
+// n - 1 - i of inv, d1 and d2 (columns of fwd) agree up to the sign
+// parity * (-1)^k and a difference that has to be below 2^-32 of its row's
+// largest element (it is below 2^-36 for n <= 257; false otherwise).  The
+// columns of inv, d1 and d2 are scaled by powers of two, X's rows inversely:
+// their elements grow as k^2 and k^4 where a spectrum falls.
+bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::vector<int4>* A, std::vector<int2>* D,
+                std::vector<int4>* ex, std::vector<int>* w) {
+  const int h = (n + 1) / 2;
+  auto exponent = [](double a) { int e = -100000; if (a != 0.0) std::frexp(a, &e); return e; };
+  A->assign((size_t)h * h, int4{0, 0, 0, 0});
+  D->assign((size_t)h * h, int2{0, 0});
+  ex->assign(h, int4{0, 0, 0, 0});
+  w->assign(n, 0);
+  if (!fwd)
+    for (int k = 0; k < n; ++k) {
+      int e = -100000;
+      for (int i = 0; i < n; ++i) e = std::max(e, exponent(m[(size_t)i * n + k]));
+      (*w)[k] = e == -100000 ? 0 : e;
+    }
+  // element and difference of term t of output pair j: fwd (row 2 j + b, point
+  // t), else (row j, coefficient t)
+  for (int j = 0; j < h; ++j)
+    for (int b = 0; b < (fwd ? 2 : 1); ++b) {
+      const int row = fwd ? 2 * j + b : j, terms = fwd ? h : n;
+      if (row >= n) continue;
+      std::vector<double> a(terms), d(terms);
+      int e = -100000, ed = -100000;
+      for (int t = 0; t < terms; ++t) {
+        const int mir = fwd ? n - 1 - t : n - 1 - row;
+        const double sg = ((fwd ? row : t) & 1) ? -parity : parity;
+        const double v = m[(size_t)row * n + t], mv = fwd ? m[(size_t)row * n + mir] : m[(size_t)mir * n + t];
+        const bool mid = fwd ? mir == t : mir == row;
+        a[t] = std::ldexp(v, -(*w)[t]);
+        d[t] = mid ? 0.0 : std::ldexp(mv - sg * v, -(*w)[t]);
+        e = std::max(e, exponent(a[t]));
+        ed = std::max(ed, exponent(d[t]));
+      }
+      if (e == -100000) e = 0;
+      int sh = ed == -100000 ? 0 : e - 32 - ed;
+      if (sh < 0) return false;
+      if (sh > 60) { sh = 0; std::fill(d.begin(), d.end(), 0.0); }
+      for (int t = 0; t < terms; ++t) {
+        const size_t at = (size_t)(fwd ? t : t / 2) * h + j;
+        const bool second = fwd ? b : t & 1;
+        const int2 s = fx_split(a[t], 58, e);
+        const int q = (int)std::ldexp(d[t], 26 - ed);
+        (second ? (*A)[at].z : (*A)[at].x) = s.x;
+        (second ? (*A)[at].w : (*A)[at].y) = s.y;
+        (second ? (*D)[at].y : (*D)[at].x) = q;
+      }
+      if (b) { (*ex)[j].y = e; (*ex)[j].w = sh; } else { (*ex)[j].x = e; (*ex)[j].z = sh; }
+      if (!fwd) (*ex)[j].y = e;
+    }
+  return true;
+}
 
 int cheb_mats(int n, ChebMats** out) {
   std::lock_guard<std::mutex> lk(g_cheb_mu);
@@ -4117,35 +4182,62 @@ int cheb_mats(int n, ChebMats** out) {
   if (it != g_cheb.end()) { *out = &it->second; return 0; }
   Cheb c = make_cheb(n, 0.35);
   const double C = std::sqrt(2.0 / (double)(n - 1));
-  std::vector<double> fwd((size_t)n * n), inv((size_t)n * n), d1((size_t)n * n), d2((size_t)n * n);
+  std::vector<double> m[4];
+  for (auto& v : m) v.resize((size_t)n * n);
   for (int i = 0; i < n; ++i)
     for (int j = 0; j < n; ++j) {
       const double h = (j == 0 || j == n - 1) ? 0.5 : 1.0;
-      inv[(size_t)i * n + j] = C * c.t[i + (size_t)n * j] * h;
-      d1[(size_t)i * n + j] = C * c.D[i + (size_t)n * j] * h;
-      d2[(size_t)i * n + j] = C * c.D2[i + (size_t)n * j] * h;
       const double cp = (j == 0 || j == n - 1) ? 1.0 : 2.0;  // row i = coefficient, column j = point
-      fwd[(size_t)i * n + j] = c.t[j + (size_t)n * i] * cp / ((double)(n - 1) * C);
+      m[0][(size_t)i * n + j] = c.t[j + (size_t)n * i] * cp / ((double)(n - 1) * C);
+      m[1][(size_t)i * n + j] = C * c.t[i + (size_t)n * j] * h;
+      m[2][(size_t)i * n + j] = C * c.D[i + (size_t)n * j] * h;
+      m[3][(size_t)i * n + j] = C * c.D2[i + (size_t)n * j] * h;
     }
-  ChebMats m;
-  m.n = n;
+  ChebMats mats;
   int rc;
-  if ((rc = upload(&m.fwd, fwd, nullptr)) || (rc = upload(&m.inv, inv, nullptr)) ||
-      (rc = upload(&m.d1, d1, nullptr)) || (rc = upload(&m.d2, d2, nullptr)))
-    return rc;
-  auto res = g_cheb.emplace(n, m);
+  for (int q = 0; q < 4; ++q) {
+    std::vector<int4> A, ex;
+    std::vector<int2> D;
+    std::vector<int> w;
+    ChebOp& o = mats.op[q];
+    o.fx.sign = q == 2 ? -1 : 1;
+    if (n > 257 || !cheb_fixed(m[q], n, q == 0, o.fx.sign, &A, &D, &ex, &w)) {
+      if ((rc = upload(&o.m, m[q], nullptr))) return rc;
+      continue;
+    }
+    int4 *a, *e;
+    int2* d;
+    int* wk = nullptr;
+    if ((rc = upload(&a, A, nullptr)) || (rc = upload(&d, D, nullptr)) || (rc = upload(&e, ex, nullptr)) ||
+        (q && (rc = upload(&wk, w, nullptr))))
+      return rc;
+    o.fx.A = a; o.fx.D = d; o.fx.ex = e; o.fx.w = wk;
+  }
+  auto res = g_cheb.emplace(n, mats);
   *out = &res.first->second;
   return 0;
 }
 
-int cheb_apply(int which, int nr, int ncol, const double* in, double* out, void* stream) {
-  if (nr < 3 || ncol < 1 || !in || !out) return fail(FALCON_EINVAL, "invalid Chebyshev transform arguments");
+// Operator `first` to out[0] and, with count 2, `first` + 1 to out[1].
+int cheb_apply(int first, int count, int nr, int ncol, const double* in, double* const* out, void* stream) {
+  if (nr < 3 || ncol < 1 || !in || !out[0]) return fail(FALCON_EINVAL, "invalid Chebyshev transform arguments");
   ChebMats* m = nullptr;
   int rc = cheb_mats(nr, &m);
   if (rc) return rc;
-  const double* A = which == 0 ? m->fwd : which == 1 ? m->inv : which == 2 ? m->d1 : m->d2;
-  CK(launch_apply_cols(nr, ncol, A, reinterpret_cast<const double2*>(in), reinterpret_cast<double2*>(out),
-                       (cudaStream_t)stream));
+  FxColumns g{};
+  g.n = nr; g.ncol = ncol; g.fwd = first == 0;
+  g.in = reinterpret_cast<const double2*>(in);
+  for (int q = 0; q < count; ++q) {
+    const ChebOp& o = m->op[first + q];
+    double2* y = reinterpret_cast<double2*>(out[q]);
+    if (o.m) {
+      CK(launch_apply_cols(nr, ncol, o.m, g.in, y, (cudaStream_t)stream));
+      continue;
+    }
+    g.op[g.nop] = o.fx;
+    g.op[g.nop++].out = y;
+  }
+  if (g.nop) CK(launch_fx_columns(g, (cudaStream_t)stream));
   return 0;
 }
 }  // namespace
@@ -4322,23 +4414,23 @@ int server_admit_group(falcon_server* s, const OpKey& key, ServerGroup& sg) {
 extern "C" {
 
 int falcon_cheb_fwd_dev(int nr, int ncol, const double* in_dev, double* out_dev, void* stream) {
-  return cheb_apply(0, nr, ncol, in_dev, out_dev, stream);
+  return cheb_apply(0, 1, nr, ncol, in_dev, &out_dev, stream);
 }
 int falcon_cheb_inv_dev(int nr, int ncol, const double* in_dev, double* out_dev, void* stream) {
-  return cheb_apply(1, nr, ncol, in_dev, out_dev, stream);
+  return cheb_apply(1, 1, nr, ncol, in_dev, &out_dev, stream);
 }
 int falcon_cheb_d1_dev(int nr, int ncol, const double* in_dev, double* out_dev, void* stream) {
-  return cheb_apply(2, nr, ncol, in_dev, out_dev, stream);
+  return cheb_apply(2, 1, nr, ncol, in_dev, &out_dev, stream);
 }
 int falcon_cheb_d2_dev(int nr, int ncol, const double* in_dev, double* out_dev, void* stream) {
-  return cheb_apply(3, nr, ncol, in_dev, out_dev, stream);
+  return cheb_apply(3, 1, nr, ncol, in_dev, &out_dev, stream);
 }
 
 int falcon_cheb_d1d2_dev(int nr, int ncol, const double* in_dev, double* d1_dev, double* d2_dev, void* stream) {
   if (!d1_dev || !d2_dev || d1_dev == d2_dev || d1_dev == in_dev || d2_dev == in_dev)
     return fail(FALCON_EINVAL, "falcon_cheb_d1d2_dev: outputs must be two arrays apart from the input");
-  const int rc = cheb_apply(2, nr, ncol, in_dev, d1_dev, stream);
-  return rc ? rc : cheb_apply(3, nr, ncol, in_dev, d2_dev, stream);
+  double* const out[2] = {d1_dev, d2_dev};
+  return cheb_apply(2, 2, nr, ncol, in_dev, out, stream);
 }
 
 int falcon_server_create(size_t hbm_budget_bytes, int max_active, falcon_server** out) {

@@ -402,6 +402,22 @@ cudaError_t launch_extract_mode0(int R, int M, int B, const double2* src, double
 cudaError_t launch_getrs_batched(int n, int nsys, int nrhs, const double* lu, const int* ipiv,
                                  double* b, cudaStream_t s);
 // out[c] = A in[c] for ncol complex columns of length n (A real row-major).
+// Chebyshev transforms of complex columns in fixed point (n <= 257): what the
+// kernel reads of an operator (cheb_fixed) and the call.
+struct FxColumnsOp {
+  const int4* A;  // [p][j]: A0, A1 as (h, l) of 58 bits at the row's scale
+  const int2* D;  // [p][j]: 26 bits of the mirrored halves' differences
+  const int4* ex; // [j]: exponents of the rows of S0 and S1, shifts of D0 and D1
+  const int* w;   // weights of X's rows (or null)
+  double2* out;
+  int sign;
+};
+struct FxColumns {
+  int n, ncol, nop, fwd;
+  const double2* in;
+  FxColumnsOp op[2];
+};
+cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s);
 cudaError_t launch_apply_cols(int n, int ncol, const double* A, const double2* in, double2* out, cudaStream_t s);
 // Instance-column remap of a [rows][B] array (ew doubles per element).
 cudaError_t launch_remap_cols(const double* src, double* dst, size_t rows, int bs, int bd, int ew, const int* map,
