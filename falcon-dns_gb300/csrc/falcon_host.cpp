@@ -13,6 +13,7 @@
 #include <deque>
 #include <fstream>
 #include <functional>
+#include <list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -866,18 +867,78 @@ void falcon::fft_tables_host(const FftPlan& plan, int4* tw, unsigned* pos) {
 
 namespace {
 
+// The current CUDA context's id (0: unknown); a device that was reset has a
+// new one.
+unsigned long long context_id() {
+  using GetCurrent = CUresult (*)(CUcontext*);
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const std::pair<void*, void*> fn = [] {
+    void *cur = nullptr, *id = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    if (cudaGetDriverEntryPointByVersion("cuCtxGetCurrent", &cur, 4000, cudaEnableDefault, &st) != cudaSuccess ||
+        st != cudaDriverEntryPointSuccess ||
+        cudaGetDriverEntryPointByVersion("cuCtxGetId", &id, 12000, cudaEnableDefault, &st) != cudaSuccess ||
+        st != cudaDriverEntryPointSuccess)
+      cur = id = nullptr;
+    return std::make_pair(cur, id);
+  }();
+  CUcontext c = nullptr;
+  unsigned long long id = 0;
+  if (!fn.first || reinterpret_cast<GetCurrent>(fn.first)(&c) != CUDA_SUCCESS ||
+      !c || reinterpret_cast<GetId>(fn.second)(c, &id) != CUDA_SUCCESS)
+    return 0;
+  return id;
+}
+
 struct FftTables {
   FftPlan plan{};
   int4* tw = nullptr;
   unsigned* pos = nullptr;
-  ~FftTables() { cudaFree(tw); cudaFree(pos); }
+  int dev = 0;
+  unsigned long long ctx = 0;
+  ~FftTables() {  // the memory of a context that is gone is not ours any more
+    int cur = 0;
+    const bool here = ctx == 0 || context_id() == ctx;
+    if (!here) {
+      cudaGetDevice(&cur);
+      cudaSetDevice(dev);
+    }
+    if (here || context_id() == ctx) {
+      cudaFree(tw);
+      cudaFree(pos);
+    }
+    if (!here) cudaSetDevice(cur);
+  }
 };
 
 // The transform for 3 Nm azimuthal points: with `grid` on exactly these
 // points (the velocity maxima of a variable time step are taken on them),
-// else of the cheapest length (make_line_plan).
-int make_fft(int Nm, bool grid, std::unique_ptr<FftTables>* out) {
-  auto f = std::make_unique<FftTables>();
+// else of the cheapest length (make_line_plan).  The last kFftKept tables stay
+// for the next caller (making them took 220 of the 434 us that a pass over
+// 65 x 171 x 128 cost its caller: two allocations, two copies, two frees that
+// wait for the device); older ones are freed when their last user is done.
+// They are only read once made, so that any stream or thread may use them.
+constexpr size_t kFftKept = 8;  // 100 KB each at most
+
+int make_fft(int Nm, bool grid, std::shared_ptr<FftTables>* out) {
+  static std::mutex mu;
+  static auto* kept = new std::list<std::pair<std::tuple<int, unsigned long long, int, bool>, std::shared_ptr<FftTables>>>;
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  if (context_id() == 0) CK(cudaFree(nullptr));  // a thread's first call
+  const auto key = std::make_tuple(dev, context_id(), Nm, grid);
+  std::shared_ptr<FftTables> old;  // freed after the lock is
+  std::lock_guard<std::mutex> lk(mu);
+  if (std::get<1>(key) != 0)
+    for (auto it = kept->begin(); it != kept->end(); ++it)
+      if (it->first == key) {
+        kept->splice(kept->begin(), *kept, it);
+        *out = it->second;
+        return 0;
+      }
+  auto f = std::make_shared<FftTables>();
+  f->dev = dev;
+  f->ctx = std::get<1>(key);
   if (make_fft_plan(3 * Nm, &f->plan) != 0)
     return fail(FALCON_EINVAL, "azimuthal length 3*Nm has a prime factor above 64 or too many factors");
   if (!grid) make_line_plan(Nm, kMaxPadded, &f->plan);
@@ -888,6 +949,13 @@ int make_fft(int Nm, bool grid, std::unique_ptr<FftTables>* out) {
   int rc;
   if ((rc = upload(&f->tw, tw, nullptr))) return rc;
   if ((rc = upload(&f->pos, pos, nullptr))) return rc;
+  if (f->ctx) {
+    kept->emplace_front(key, f);
+    if (kept->size() > kFftKept) {
+      old = std::move(kept->back().second);
+      kept->pop_back();
+    }
+  }
   *out = std::move(f);
   return 0;
 }
@@ -905,7 +973,7 @@ struct Group {
   // IMEXRK with a stage-dependent implicit diagonal: the operators of each
   // stage whose diagonal differs from that of stage diag_index (null: ops)
   std::shared_ptr<OpSet> stage_ops[kMaxStages];
-  std::unique_ptr<FftTables> fft;
+  std::shared_ptr<FftTables> fft;
   std::vector<int> members;    // batch indices
   std::vector<double> ra_pr_h; // per instance Ra/Pr
   std::vector<double> pr_h;    // per instance Pr
@@ -4052,7 +4120,7 @@ int falcon_nonlin_dev(int nr, int nm, int nb, const double* t_dev, const double*
                       const double* ur_dev, double* uphi_t_dev, double* ur_t_dev, double* uphi_omg_dev,
                       double* ur_omg_dev, void* stream) {
   if (nr < 1 || nm < 1 || nb < 1) return fail(FALCON_EINVAL, "invalid sizes");
-  std::unique_ptr<FftTables> f;
+  std::shared_ptr<FftTables> f;
   int rc = make_fft(nm, false, &f);
   if (rc) return rc;
   NonlinArgs a{};

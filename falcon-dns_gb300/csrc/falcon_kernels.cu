@@ -928,8 +928,7 @@ double measure_fp64_mma_peak() {
 namespace falcon {
 
 constexpr int kNoAllocMaxP = 4096;
-// twiddles (kNoAllocMaxP int4) followed by positions (kNoAllocMaxP int):
-// 80 KiB, held by every GPU that loads the library until the process exits.
+// the plan's P twiddles (int4) followed by its P positions (int): 80 KiB, held by every GPU that loads the library until the process exits.
 constexpr size_t kNoAllocScratchBytes = (size_t)kNoAllocMaxP * (sizeof(int4) + sizeof(int));
 static __device__ __align__(256) unsigned char g_nonlin_scratch[kNoAllocScratchBytes];
 
@@ -944,8 +943,10 @@ static void* g_scratch_addr[64] = {nullptr};
 // pageable host memory has consumed its source when cudaMemcpyAsync returns,
 // so the buffer is free again once the copies are issued.
 static std::mutex g_noalloc_host_mu;
-static int4 g_noalloc_tw_h[kNoAllocMaxP];
-static unsigned g_noalloc_pos_h[kNoAllocMaxP];
+// They stay as the last call's nm left them (nm 0: none), with its plan.
+static unsigned char g_noalloc_h[kNoAllocScratchBytes];
+static int g_noalloc_nm = 0;
+static FftPlan g_noalloc_plan;
 
 }  // namespace falcon
 
@@ -976,17 +977,10 @@ extern "C" int falcon_nonlin_noalloc_dev(int nr, int nm, int nb, const double* t
                                          void* stream) {
   using namespace falcon;
   if (nr < 1 || nm < 1 || nb < 1) { set_error_message("falcon_nonlin_noalloc_dev: invalid sizes"); return -1; }
-  const int P = 3 * nm;
-  if (P > kNoAllocMaxP) {
+  if (nm > kNoAllocMaxP / 3) {
     set_error_message("falcon_nonlin_noalloc_dev: Np_max = 3*Nm_max exceeds the 4096-point scratch limit");
     return -1;
   }
-  FftPlan plan{};
-  if (make_fft_plan(P, &plan) != 0) {
-    set_error_message("falcon_nonlin_noalloc_dev: 3*Nm_max has a prime factor above 64");
-    return -1;
-  }
-  make_line_plan(nm, kNoAllocMaxP, &plan);  // always finds one: 4096 itself
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess || dev < 0 || dev >= 64) { set_error_message("falcon_nonlin_noalloc_dev: no current device"); return -2; }
@@ -999,16 +993,26 @@ extern "C" int falcon_nonlin_noalloc_dev(int nr, int nm, int nb, const double* t
     return -2;
   }
   int4* tw = reinterpret_cast<int4*>(g_scratch_addr[dev]);
-  unsigned* pos = reinterpret_cast<unsigned*>(reinterpret_cast<unsigned char*>(g_scratch_addr[dev]) +
-                                    (size_t)kNoAllocMaxP * sizeof(int4));
   cudaStream_t s = (cudaStream_t)stream;
+  FftPlan plan{};
   {
     std::lock_guard<std::mutex> lk(g_noalloc_host_mu);
-    fft_tables_host(plan, g_noalloc_tw_h, g_noalloc_pos_h);
-    e = cudaMemcpyAsync(tw, g_noalloc_tw_h, sizeof(int4) * (size_t)plan.P, cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(pos, g_noalloc_pos_h, sizeof(unsigned) * (size_t)plan.P, cudaMemcpyHostToDevice, s);
+    if (g_noalloc_nm != nm) {
+      if (make_fft_plan(3 * nm, &plan) != 0) {
+        set_error_message("falcon_nonlin_noalloc_dev: 3*Nm_max has a prime factor above 64");
+        return -1;
+      }
+      make_line_plan(nm, kNoAllocMaxP, &plan);  // always finds one: 4096 itself
+      int4* t = reinterpret_cast<int4*>(g_noalloc_h);
+      g_noalloc_nm = 0;
+      fft_tables_host(plan, t, reinterpret_cast<unsigned*>(t + plan.P));
+      g_noalloc_plan = plan;
+      g_noalloc_nm = nm;
+    }
+    plan = g_noalloc_plan;
+    e = cudaMemcpyAsync(tw, g_noalloc_h, (sizeof(int4) + sizeof(int)) * (size_t)plan.P, cudaMemcpyHostToDevice, s);
   }
+  const unsigned* pos = reinterpret_cast<const unsigned*>(tw + plan.P);
   if (e != cudaSuccess) { set_error_message(cudaGetErrorString(e)); return -2; }
   NonlinArgs a{};
   a.R = nr; a.M = nm + 1; a.B = nb; a.Nm = nm;
