@@ -6,6 +6,9 @@
 // falcon_fft17.cu, falcon_fft31.cu), which compile in parallel; everything
 // here has internal linkage.
 #pragma once
+#include <algorithm>
+#include <mutex>
+
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -683,9 +686,20 @@ static cudaError_t launch_nonlin_s(const NonlinArgs& a, cudaStream_t s) {
   const int PP = a.plan.rad[0] * a.plan.span[0];
   const int smem = (TWID ? P - a.plan.rad[a.plan.nrad - 1] : 0) * 16 + LPB * (2 * PP * 16 + (int)sizeof(FxLine<S>)) +
                    4 * (frag + (P + 3) / 4 * 4);
-  const cudaError_t e = cudaFuncSetAttribute(nonlin_kernel<MAXP, TWID, S, LPB, MINB>,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return e;
+  // the limit only rises: a thread with a shorter line never takes it from one
+  // that is about to launch a longer
+  static std::mutex mu;
+  static int limit[64] = {0};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  {
+    std::lock_guard<std::mutex> lk(mu);
+    int& most = limit[dev >= 0 && dev < 64 ? dev : 0];
+    most = std::max(most, smem);
+    const cudaError_t e = cudaFuncSetAttribute(nonlin_kernel<MAXP, TWID, S, LPB, MINB>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    if (e != cudaSuccess) return e;
+  }
   nonlin_kernel<MAXP, TWID, S, LPB, MINB><<<(a.R * a.B + LPB - 1) / LPB, 64 * S * LPB, smem, s>>>(a);
   return cudaGetLastError();
 }
