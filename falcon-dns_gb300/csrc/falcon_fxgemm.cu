@@ -46,6 +46,7 @@ namespace falcon {
 namespace {
 
 constexpr int kBitsA = 58, kBitsX = 59;  // of a row's and a column's integers
+constexpr int kFollowRows = 6;           // deepest tiles that do what follows a product (deeper ones would spill)
 constexpr int kFxKC = 16;                // k per staged operator chunk
 constexpr int kBad = INT32_MIN;          // exponent of a row or column with an Inf or NaN
 constexpr int kNone = -100000;           // exponent of a zero
@@ -120,6 +121,20 @@ __device__ __forceinline__ double* output_row(const GemmArgs& g, int z, int row)
   int o = 0;
   while (o + 1 < g.nout && row >= g.rend[o]) ++o;
   return g.Yo[o] + (size_t)z * g.sY + (size_t)(row - (o ? g.rend[o - 1] : 0)) * g.ldy;
+}
+
+// After output row `row` of entry z, columns n (even), n + 1.
+__device__ __forceinline__ void follow_row(const FxFollow& f, int z, int row, int n, double y0, double y1) {
+  const int b = f.b0 + (n >> 1);
+  if (f.kind == kBuoyancy) follow_buoyancy(f, f.m0 + z, row, b, y0, y1);
+  if (f.kind == kVelocity && row >= f.R && row < 2 * f.R) follow_velocity(f, f.m0 + z, row - f.R, b, y0, y1);
+}
+// The grid's share of mode 0.
+__device__ __forceinline__ void follow_modes(const FxFollow& f) {
+  if (f.kind != kVelocity) return;
+  const int nthr = blockDim.x, blk = (blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  const int step = gridDim.x * gridDim.y * gridDim.z * nthr;
+  for (int i = blk * nthr + threadIdx.x; i < f.R * f.B; i += step) follow_mode0(f, i / f.B, i % f.B);
 }
 
 __device__ __forceinline__ void copy8(void* dst, const void* src, bool valid) {
@@ -206,17 +221,19 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   int* part = cex + NCOL;                                             // [nthr]
   const int z = blockIdx.z;
   int N = g.N, nblk = blockIdx.x;
-  long ldx = g.ldx, ldy = g.ldy;
+  long lda = g.lda, ldx = g.ldx, ldy = g.ldy;
   const int2* A = g.fx + (size_t)z * g.sA;
   const int* aex = g.fx_ex + (size_t)z * g.lda;
   const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
   const double* X = g.X + (size_t)z * g.sX;
   double* Y = nullptr;
-  if (g.njobs) {
-    int j = 0;
-    for (int nb; nblk >= (nb = (g.job[j].N + NCOL - 1) / NCOL); ++j) nblk -= nb;
+  if (g.njobs || z >= g.batch) {
+    int j = z >= g.batch ? z - g.batch : 0;
+    if (g.njobs)
+      for (int nb; nblk >= (nb = (g.job[j].N + NCOL - 1) / NCOL); ++j) nblk -= nb;
     const FxJob& q = g.job[j];
     N = q.N;
+    lda = q.lda;
     ldx = q.ldx;
     ldy = q.ldy;
     A = q.fx;
@@ -245,7 +262,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
     for (int kk = warp; kk < kc; kk += nw)
       for (int rr = lane; rr < rows_blk; rr += 32) {
         const bool ok = row0 + rr < g.rows;
-        copy8(buf + kk * rows_blk + rr, ok ? A + (size_t)(k0 + kk) * g.lda + row0 + rr : A, ok);
+        copy8(buf + kk * rows_blk + rr, ok ? A + (size_t)(k0 + kk) * lda + row0 + rr : A, ok);
       }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
@@ -307,78 +324,117 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
           yp[0] = y0;
           yp[1] = y1;
         }
+        if constexpr (RPT <= kFollowRows)
+          if (g.follow.kind && z < g.batch) follow_row(g.follow, z, row, n, y0, y1);
       } else {
         yp[0] = y0;
       }
     }
   }
+  if constexpr (RPT <= kFollowRows)
+    if (g.follow.kind) follow_modes(g.follow);
 }
 
-// Narrow form (N <= 8 columns per batch entry): 32 rows per block, k shared
-// by its eight warps, each of which reads its share of the operator before
-// the X panel is converted (one memory latency, not two) and adds up the
-// columns' partial sums.  Bound by latency, then by the operator's bytes.
+// Narrow form (N <= 8 columns per batch entry): a block takes RB rows and all
+// columns of an entry, thread (row, part) one of KS shares of k; the operator
+// is read once, straight to registers, the next 8 k (and the first ones, before
+// the X panel is converted) in flight while these are multiplied; the shares'
+// sums meet in shared memory, where the threads of a row take its column pairs.
+// Bound by latency for one small run, then by issue.  With 32 rows and eight
+// shares in every block two thirds of the instructions were for converting X
+// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 57 us, 291 x 97 x 6 256 ->
+// 125, 291 x 97 x 2, 341 entries 40 -> 31, 195 x 65 x 8, 170 entries 32 -> 24.
 struct alignas(16) Part {
   long long hh;
   unsigned mid;
   int ll;
 };
 template <int NC>
-__global__ void __launch_bounds__(256) fx_narrow_kernel(GemmArgs g) {
+__global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ GemmArgs g, int RB, int KS) {
   extern __shared__ __align__(16) double fsm[];
-  Part* parts = reinterpret_cast<Part*>(fsm);                    // [8][NC][32]
-  double* xd = reinterpret_cast<double*>(parts + 8 * NC * 32);   // [K][NC]
+  Part* parts = reinterpret_cast<Part*>(fsm);                       // [KS][NC][RB]
+  double* xd = reinterpret_cast<double*>(parts + KS * NC * RB);     // [K][NC]
   __shared__ int cex[NC];
   __shared__ int part[256];
-  constexpr int U = 16;
-  const int z = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int row = blockIdx.x * 32 + lane, kq = (g.K + 7) / 8, kb = min(warp * kq, g.K), ke = min(kb + kq, g.K);
-  const int2* A = g.fx + (size_t)z * g.sA + min(row, g.rows - 1);
+  constexpr int U = 8;
+  const int z = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x;
+  const int kp = tid / RB, rl = tid - kp * RB, row = blockIdx.x * RB + rl;
+  const int kq = (g.K + KS - 1) / KS, kb = min(kp * kq, g.K), ke = min(kb + kq, g.K);
+  long lda = g.lda, ldx = g.ldx;
+  const int2* A = g.fx + (size_t)z * g.sA;
+  const int* aex = g.fx_ex + (size_t)z * g.lda;
+  const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
+  const double* X = g.X + (size_t)z * g.sX;
+  double* Y = nullptr;
+  if (z >= g.batch) {
+    const FxJob& q = g.job[z - g.batch];
+    lda = q.lda;
+    ldx = q.ldx;
+    A = q.fx;
+    aex = q.fx_ex;
+    w = q.fx_w;
+    X = q.X;
+    Y = q.Y + (size_t)row * q.ldy;
+  }
+  A += min(row, g.rows - 1);
   int2 av[U];
 #pragma unroll
-  for (int u = 0; u < U; ++u) av[u] = kb + u < ke ? __ldg(A + (size_t)(kb + u) * g.lda) : make_int2(0, 0);
-  const double* X = g.X + (size_t)z * g.sX;
-  for (int i = tid; i < g.K * NC; i += 256) {
+  for (int u = 0; u < U; ++u) av[u] = kb + u < ke ? __ldg(A + (size_t)(kb + u) * lda) : make_int2(0, 0);
+  for (int i = tid; i < g.K * NC; i += nthr) {
     const int k = i / NC, c = i - k * NC;
-    xd[i] = c < g.N ? X[(size_t)k * g.ldx + c] : 0.0;
+    xd[i] = c < g.N ? X[(size_t)k * ldx + c] : 0.0;
   }
   __syncthreads();
-  convert_panel(xd, g.K, NC, g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr, cex, part);
+  convert_panel(xd, g.K, NC, w, cex, part);
   const int2* xs = reinterpret_cast<const int2*>(xd);
   Sum acc[NC];
 #pragma unroll
   for (int c = 0; c < NC; ++c) acc[c] = Sum{0, 0, 0};
   for (int k0 = kb; k0 < ke; k0 += U) {
-    if (k0 > kb) {
+    int2 nv[U];
 #pragma unroll
-      for (int u = 0; u < U; ++u) av[u] = k0 + u < ke ? __ldg(A + (size_t)(k0 + u) * g.lda) : make_int2(0, 0);
-    }
+    for (int u = 0; u < U; ++u) nv[u] = k0 + U + u < ke ? __ldg(A + (size_t)(k0 + U + u) * lda) : make_int2(0, 0);
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (k0 + u >= ke) break;
       const int a12 = av[u].y >> 20;
+      const int4* xp = reinterpret_cast<const int4*>(xs + (k0 + u) * NC);
 #pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        const int2 x = xs[(k0 + u) * NC + c];
-        add_product(acc[c], av[u], x, a12, x.y >> 20);
+      for (int c = 0; c < NC; c += 2) {
+        const int4 x = xp[c / 2];
+        add_product(acc[c], av[u], make_int2(x.x, x.y), a12, x.y >> 20);
+        add_product(acc[c + 1], av[u], make_int2(x.z, x.w), a12, x.w >> 20);
       }
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) carry(acc[c]);
+#pragma unroll
+    for (int u = 0; u < U; ++u) av[u] = nv[u];
   }
 #pragma unroll
-  for (int c = 0; c < NC; ++c) parts[(warp * NC + c) * 32 + lane] = Part{acc[c].hh, (unsigned)acc[c].mid, acc[c].ll};
+  for (int c = 0; c < NC; ++c) parts[(kp * NC + c) * RB + rl] = Part{acc[c].hh, (unsigned)acc[c].mid, acc[c].ll};
+  if (g.follow.kind) follow_modes(g.follow);
   __syncthreads();
-  if (warp >= min(NC, g.N) || row >= g.rows) return;
-  Sum s{0, 0, 0};  // column `warp`
-#pragma unroll
-  for (int w = 0; w < 8; ++w) {
-    const Part p = parts[(w * NC + warp) * 32 + lane];
-    s.hh += p.hh;
-    s.mid += p.mid;
-    s.ll += p.ll;
+  if (row >= g.rows) return;
+  auto column = [&](int c) {
+    Sum s{0, 0, 0};
+    for (int q = 0; q < KS; ++q) {
+      const Part p = parts[(q * NC + c) * RB + rl];
+      s.hh += p.hh;
+      s.mid += p.mid;
+      s.ll += p.ll;
+    }
+    return value_of(s, aex[row], cex[c], g.alpha);
+  };
+  double* y = Y ? Y : output_row(g, z, row);
+  for (int c = 2 * kp; c < g.N; c += 2 * KS) {
+    const double y0 = column(c);
+    y[c] = y0;
+    if (c + 1 >= g.N) break;
+    const double y1 = column(c + 1);
+    y[c + 1] = y1;
+    if (g.follow.kind && z < g.batch) follow_row(g.follow, z, row, c, y0, y1);
   }
-  output_row(g, z, row)[warp] = value_of(s, g.fx_ex[(size_t)z * g.lda + row], cex[warp], g.alpha);
 }
 
 // Complex columns x[c][0..n) through real n x n operators whose rows (or
@@ -569,7 +625,7 @@ cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream
   }
   const int rows_blk = nw * (64 / NCOL) * RPT;
   const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw) * 4;
-  const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, g.batch);
+  const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, g.batch + g.nextra);
   fx_tile_kernel<RPT, NCOL><<<grid, 32 * nw, smem, s>>>(g);
   return cudaGetLastError();
 }
@@ -586,7 +642,7 @@ TileShape pick_shape(const GemmArgs& g, int nsm) {
   for (int ncol = 16; ncol <= 64; ncol *= 2) {
     if (g.fma_ncol && ncol != g.fma_ncol) continue;
     const int rg = 64 / ncol;
-    const long cb = column_blocks(g, ncol) * g.batch;
+    const long cb = column_blocks(g, ncol) * (g.batch + g.nextra);
     for (int rb = 1; rb <= 16; ++rb)
       for (int nw = 4; nw <= 16; ++nw)
         for (int rpt = 1; rpt <= 8; ++rpt) {
@@ -623,7 +679,33 @@ cudaError_t launch_ncol(const GemmArgs& g, const TileShape& t, cudaStream_t s) {
   }
 }
 
+TileShape tile_shape(const GemmArgs& g) {
+  int dev = 0, nsm = 152;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  // shapes are memoised per problem size: the search runs on the host once
+  struct Memo { int rows, K, N, total, batch, nsm, ncol; TileShape t; };
+  thread_local std::unordered_map<unsigned long long, Memo> memo;
+  unsigned long long key = 1469598103934665603ull;
+  const int total = (int)column_blocks(g, 1);  // columns of all jobs
+  const int batch = g.batch + g.nextra;
+  for (int v : {g.rows, g.K, g.N, total, batch, nsm, g.fma_ncol}) key = (key ^ (unsigned)v) * 1099511628211ull;
+  Memo& m = memo[key];
+  if (m.rows != g.rows || m.K != g.K || m.N != g.N || m.total != total || m.batch != batch || m.nsm != nsm ||
+      m.ncol != g.fma_ncol)
+    m = Memo{g.rows, g.K, g.N, total, batch, nsm, g.fma_ncol, pick_shape(g, nsm)};
+  return m.t;
+}
+
 }  // namespace
+
+// Whether launch_fx_gemm can do what follows g: every narrow form, and tiles of
+// up to kFollowRows rows a thread (a batch of 12 of 33 x 86: a step 63 -> 56 us,
+// 59 with 3 rows at most; with the code in tiles of 7, which spill, 129 x 129 x
+// 2752 columns go from 131 to 134 us).
+bool fx_follows(const GemmArgs& g) {
+  return g.N <= 8 || tile_shape(g).rpt <= kFollowRows;
+}
 
 cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int K, int nb, int* wk, int2* out,
                                int* ex, cudaStream_t s) {
@@ -638,33 +720,34 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.rows <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
   if (g.K > 257 || !g.fx) return cudaErrorInvalidValue;
   if (g.N <= 8 && !g.njobs) {
-    const dim3 grid((g.rows + 31) / 32, g.batch);
-    auto smem = [&](int nc) { return (size_t)nc * (8 * 32 * sizeof(Part) + g.K * sizeof(double)); };
-    if (g.N > 4 && g.K > 170) {  // over 48 KB with the static part
-      const cudaError_t e = cudaFuncSetAttribute(fx_narrow_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-      if (e != cudaSuccess) return e;
-    }
-    if (g.N <= 2) fx_narrow_kernel<2><<<grid, 256, smem(2), s>>>(g);
-    else if (g.N <= 4) fx_narrow_kernel<4><<<grid, 256, smem(4), s>>>(g);
-    else fx_narrow_kernel<8><<<grid, 256, smem(8), s>>>(g);
-    return cudaGetLastError();
+    // k shares until there are 448 threads an SM (one share above that), rows
+    // in even blocks of at most 256 threads, of fewer while SMs are without two
+    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.9, 7.9, 7.8; 65 x 65 x 8,
+    // 171 entries 22.5, 18.1, 16.0, 18.0; 291 x 97 x 2, 341 entries 31.0, 32.4, 36.5, 46.8)
+    const int nz = g.batch + g.nextra;
+    const int KS = (int)std::min(8L, std::max(1L, 152L * 448 / ((long)g.rows * nz)));
+    int nb = (g.rows + 256 / KS - 1) / (256 / KS);
+    while ((long)nb * nz < 2 * 152 && (g.rows + nb - 1) / nb > 16) ++nb;
+    const int RB = (g.rows + nb - 1) / nb;
+    const dim3 grid((g.rows + RB - 1) / RB, nz);
+    auto run = [&](auto kernel, int nc) {
+      const size_t smem = (size_t)nc * ((size_t)KS * RB * sizeof(Part) + g.K * sizeof(double));
+      if (smem > 46 * 1024) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
+        if (e != cudaSuccess) return e;
+      }
+      kernel<<<grid, RB * KS, smem, s>>>(g, RB, KS);
+      return cudaGetLastError();
+    };
+    if (g.N <= 2) return run(fx_narrow_kernel<2>, 2);
+    if (g.N <= 4) return run(fx_narrow_kernel<4>, 4);
+    return g.N <= 6 ? run(fx_narrow_kernel<6>, 6) : run(fx_narrow_kernel<8>, 8);
   }
-  int dev = 0, nsm = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  // shapes are memoised per problem size: the search runs on the host once
-  struct Memo { int rows, K, N, total, batch, nsm, ncol; TileShape t; };
-  thread_local std::unordered_map<unsigned long long, Memo> memo;
-  unsigned long long key = 1469598103934665603ull;
-  const int total = (int)column_blocks(g, 1);  // columns of all jobs
-  for (int v : {g.rows, g.K, g.N, total, g.batch, nsm, g.fma_ncol}) key = (key ^ (unsigned)v) * 1099511628211ull;
-  Memo& m = memo[key];
-  if (m.rows != g.rows || m.K != g.K || m.N != g.N || m.total != total || m.batch != g.batch || m.nsm != nsm ||
-      m.ncol != g.fma_ncol)
-    m = Memo{g.rows, g.K, g.N, total, g.batch, nsm, g.fma_ncol, pick_shape(g, nsm)};
-  if (m.t.ncol == 16) return launch_ncol<16>(g, m.t, s);
-  if (m.t.ncol == 32) return launch_ncol<32>(g, m.t, s);
-  return launch_ncol<64>(g, m.t, s);
+  const TileShape t = tile_shape(g);
+  if (g.follow.kind && t.rpt > kFollowRows) return cudaErrorInvalidValue;  // see fx_follows
+  if (t.ncol == 16) return launch_ncol<16>(g, t, s);
+  if (t.ncol == 32) return launch_ncol<32>(g, t, s);
+  return launch_ncol<64>(g, t, s);
 }
 
 // Shape: NCOL real columns a block, RPT output pairs a thread (64 / NCOL x RPT

@@ -1439,6 +1439,7 @@ TcArgs tc_args(const GemmArgs& q) {
 // width (the same bits as PATH_FMA, whose shape a cost model picks).
 enum { PATH_FMA = 0, PATH_MMA = 1, PATH_TC = 2, PATH_FMA16 = 3, PATH_FMA32 = 4, PATH_FMA64 = 5, PATH_COUNT = 6 };
 inline bool is_fma_path(int p) { return p == PATH_FMA || p >= PATH_FMA16; }
+inline int path_columns(int p) { return p == PATH_FMA16 ? 16 : p == PATH_FMA32 ? 32 : p == PATH_FMA64 ? 64 : 0; }
 
 // Slice planes of q.X for the mma.sync kernel when it does not slice X
 // itself (made unless `reuse` finds them already made for the same X).
@@ -1495,7 +1496,7 @@ int run_path_once(Group* g, int cls, GemmArgs q, int path, bool reuse) {
   if (is_fma_path(path)) {
     q.oz_s = nullptr;
     q.oz_xs = nullptr;
-    q.fma_ncol = path == PATH_FMA16 ? 16 : path == PATH_FMA32 ? 32 : path == PATH_FMA64 ? 64 : 0;
+    q.fma_ncol = path_columns(path);
     if (q.fx) return launch(g, cls, gemm_flops(q), [&]() { return launch_fx_gemm(q, g->stream); });
   }
   return launch(g, cls, gemm_flops(q), [&]() { return launch_gemm(q, g->stream); });
@@ -1745,8 +1746,9 @@ int gemm(Group* g, int cls, const GemmArgs& q0, bool reuse = false) {
 
 // The row blocks v one after another, or, where their path is the
 // fixed-point tiles, as one launch over the merged view `all` (X converted
-// once, one launch instead of up to four).
-int run_blocks(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArgs* all) {
+// once, one launch instead of up to four) and, if given, what follows them.
+int run_blocks(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArgs* all,
+               const FxFollow* follow = nullptr, bool* followed = nullptr) {
   size_t first = 0;
   if (all && all->fx) {
     GemmArgs q = v[0];
@@ -1761,6 +1763,8 @@ int run_blocks(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArgs
         m.rend[o] = r += v[o].rows;
         m.Yo[o] = v[o].Y;
       }
+      m.fma_ncol = path_columns(path);
+      if (follow && (*followed = fx_follows(m))) m.follow = *follow;
       return run_path(g, cls, m, path, false);
     }
     if ((rc = run_path(g, cls, q, path, false))) return rc;
@@ -1813,7 +1817,7 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
       all.oz_s = nullptr;
       all.oz_xs = nullptr;
     }
-    all.job[i] = FxJob{q.fx, q.fx_ex, q.fx_w, q.X, q.Y, q.ldx, q.ldy, q.N};
+    all.job[i] = FxJob{q.fx, q.fx_ex, q.fx_w, q.X, q.Y, q.ldx, q.ldy, q.N, q.lda};
     cols += q.N;
   }
   all.njobs = tiles ? (int)v.size() : 0;
@@ -1919,7 +1923,8 @@ int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArg
 // (fixed-point tiles, tcgen05: fewer, fuller tiles, X converted once), unless
 // an output overlaps X (then a later block reads what an earlier one wrote,
 // and the blocks run one after another).
-int gemm_blocks(Group* g, int cls, std::initializer_list<GemmArgs> blocks) {
+int gemm_blocks(Group* g, int cls, std::initializer_list<GemmArgs> blocks, const FxFollow* follow = nullptr,
+                bool* followed = nullptr) {
   const std::vector<GemmArgs> v(blocks);
   const int mode = g_gemm_mode.load();
   const GemmArgs& f = v[0];
@@ -1948,7 +1953,7 @@ int gemm_blocks(Group* g, int cls, std::initializer_list<GemmArgs> blocks) {
     }
     if (use) return run_merged_tc(g, cls, v, all);
   }
-  return run_blocks(g, cls, v, &all);
+  return run_blocks(g, cls, v, &all, follow, followed);
 }
 
 int elementwise(Group* g, double flops_per_el, std::function<cudaError_t()> f) {
@@ -1976,38 +1981,71 @@ int run_nonlin(Group* g) {
 // st: the IMEXRK stage whose own implicit diagonal the operators take (-1:
 // the scheme's diagonal).  The temperature solve runs once per sub (its Pr),
 // the rest once for all instances.
+//
+// Where the products run as fixed-point integers, the buoyancy follows the
+// temperature product and u_r and mode 0 the (omega, psi, u_phi) product in
+// the same kernels, and the uphi_bar product rides with the temperature's as
+// two more entries: two launches instead of five (a step of one 33 x 43 run: 41 -> 37
+// us; the same bits).
 int solve_all(Group* g, double2* t_out, double2* w_out, double buo_scale, double2* buo_store,
               double* ubar_store, int st = -1) {
   const int R = g->R, M = g->M, B = g->B;
   const OpSet* o = sub_ops(g, 0, st);
   cudaStream_t s = g->stream;
   int rc;
-  for (size_t k = 0; k < g->subs.size(); ++k) {
-    const Group::Sub& u = g->subs[k];
-    GemmArgs q = per_mode(sub_ops(g, (int)k, st)->ST, R, (long)R * R, g->rhs_t + u.b0, t_out + u.b0, R, M, B, 0, M, R);
-    q.N = 2 * (u.b1 - u.b0);
-    if ((rc = gemm(g, KC_GEMM_MODE, q))) return rc;
-  }
-  if ((rc = elementwise(g, 6.0, [&]() {
-         return launch_add_buoyancy(R, M, B, o->inv_r, g->ra_pr, buo_scale, t_out, g->rhs_w, buo_store, s);
-       })))
-    return rc;
-  if (M > 1) {
-    const long sG = 3L * R * R;
-    if ((rc = gemm_blocks(g, KC_GEMM_MODE, {per_mode(o->G, 3 * R, sG, g->rhs_w, w_out, R, M, B, 1, M - 1, R),
-                                            per_mode(o->G + R, 3 * R, sG, g->rhs_w, g->psi, R, M, B, 1, M - 1, R),
-                                            per_mode(o->G + 2 * R, 3 * R, sG, g->rhs_w, g->up, R, M, B, 1, M - 1, R)})))
-      return rc;
-  }
+  FxFollow f{};
+  f.R = R; f.M = M; f.B = B; f.inv_r = o->inv_r; f.ra_pr = g->ra_pr;
+  f.scale = buo_scale; f.rhs_w = g->rhs_w; f.buo = buo_store;
+  f.ub = g->ub; f.ur = g->ur; f.up = g->up; f.w = w_out; f.ubar_new = ubar_store;
   GemmArgs gu{};
   gu.A = o->U; gu.lda = 2 * R;
   gu.X = reinterpret_cast<const double*>(g->rhs_w); gu.ldx = 2L * M * B;
   gu.Y = g->ub; gu.ldy = 2L * B;
   gu.K = R; gu.rows = 2 * R; gu.N = 2 * B; gu.batch = 1; gu.alpha = 1.0;
-  if ((rc = gemm(g, KC_GEMM_MODE, gu))) return rc;
-  return elementwise(g, 3.0, [&]() {
-    return launch_post_w(R, M, B, o->inv_r, g->psi, g->ur, g->up, w_out, g->ub, ubar_store, s);
-  });
+  bool ubar = false;  // uphi_bar is made
+  GemmArgs ride = gu;
+  int pu = PATH_MMA;
+  if (g->subs.size() == 1 && (rc = choose_path(g, KC_GEMM_MODE, &ride, false, &pu))) return rc;
+  for (size_t k = 0; k < g->subs.size(); ++k) {
+    const Group::Sub& u = g->subs[k];
+    GemmArgs q = per_mode(sub_ops(g, (int)k, st)->ST, R, (long)R * R, g->rhs_t + u.b0, t_out + u.b0, R, M, B, 0, M, R);
+    q.N = 2 * (u.b1 - u.b0);
+    int path = PATH_FMA;
+    if ((rc = choose_path(g, KC_GEMM_MODE, &q, false, &path))) return rc;
+    bool follows = false;
+    if (is_fma_path(path) && q.fx) {
+      if (is_fma_path(pu) && ride.fx) {
+        for (int h = 0; h < 2; ++h)
+          q.job[h] = FxJob{ride.fx + h * R, ride.fx_ex + h * R, ride.fx_w, ride.X, ride.Y + h * R * ride.ldy,
+                           ride.ldx, ride.ldy, ride.N, ride.lda};
+        q.nextra = 2;
+        ubar = true;
+      }
+      q.fma_ncol = path_columns(path);
+      if ((follows = fx_follows(q))) {
+        q.follow = f;
+        q.follow.kind = kBuoyancy;
+        q.follow.b0 = u.b0;
+      }
+    }
+    if ((rc = run_path(g, KC_GEMM_MODE, q, path, false))) return rc;
+    if (!follows && (rc = elementwise(g, 6.0, [&]() { return launch_add_buoyancy(f, u.b0, u.b1, t_out, s); }))) return rc;
+  }
+  if (!ubar && (rc = gemm(g, KC_GEMM_MODE, gu))) return rc;
+  bool followed = false;
+  if (M > 1) {
+    const long sG = 3L * R * R;
+    FxFollow v = f;
+    v.kind = kVelocity;
+    v.m0 = 1;
+    if ((rc = gemm_blocks(g, KC_GEMM_MODE, {per_mode(o->G, 3 * R, sG, g->rhs_w, w_out, R, M, B, 1, M - 1, R),
+                                            per_mode(o->G + R, 3 * R, sG, g->rhs_w, g->psi, R, M, B, 1, M - 1, R),
+                                            per_mode(o->G + 2 * R, 3 * R, sG, g->rhs_w, g->up, R, M, B, 1, M - 1, R)},
+                          &v, &followed)))
+      return rc;
+  }
+  if (followed) return 0;
+  return elementwise(g, 3.0, [&]() { return launch_post_w(f, g->psi, s); });
 }
 
 // compute_new_dt from the get_dtvals time scales (src/nonlin.F90:93-106) of

@@ -200,7 +200,7 @@ struct NonlinArgs {
 };
 
 // One product of a launch of several (launch_fx_gemm): as the fields of
-// GemmArgs, with its rows, K, lda and alpha.
+// GemmArgs, with its rows, K and alpha (and lda, but as an extra entry).
 struct FxJob {
   const int2* fx;
   const int *fx_ex, *fx_w;
@@ -208,8 +208,57 @@ struct FxJob {
   double* Y;
   long ldx, ldy;
   int N;
+  long lda;
 };
 constexpr int kFxJobs = 6;
+
+// What a fixed-point per-mode product does with its outputs beyond storing
+// them (batch entry z = mode m0 + z, columns = instances from b0 on).
+// kBuoyancy: the outputs are the new temperature, whose buoyancy goes to buo (or
+// null) and, times scale, into rhs_w.  kVelocity: output rows R..2R-1 are psi,
+// which gives u_r; and mode 0 from uphi_bar and its derivative (ub).
+enum { kNoFollow = 0, kBuoyancy = 1, kVelocity = 2 };
+struct FxFollow {
+  int kind;
+  int R, M, B, m0, b0;
+  const double *inv_r, *ra_pr;
+  double scale;
+  double2 *rhs_w, *buo;
+  const double* ub;
+  double2 *ur, *up, *w;
+  double* ubar_new;
+};
+#ifdef __CUDACC__
+// Buoyancy term -(Ra/Pr) i m r^-1 T, stored and added to the vorticity's
+// right-hand side at interior points.
+__device__ __forceinline__ void follow_buoyancy(const FxFollow& f, int m, int r, int b, double tx, double ty) {
+  if (m == 0) return;
+  const size_t at = ((size_t)r * f.M + m) * f.B + b;
+  const double q = __dmul_rn(f.ra_pr[b], __dmul_rn((double)m, f.inv_r[r]));
+  const double2 bu = make_double2(__dmul_rn(q, ty), __dmul_rn(-q, tx));
+  if (f.buo) f.buo[at] = bu;
+  if (f.rhs_w && r > 0 && r < f.R - 1) {
+    double2 v = f.rhs_w[at];
+    v.x = __fma_rn(f.scale, bu.x, v.x);
+    v.y = __fma_rn(f.scale, bu.y, v.y);
+    f.rhs_w[at] = v;
+  }
+}
+// u_r = i m r^-1 psi (m >= 1)
+__device__ __forceinline__ void follow_velocity(const FxFollow& f, int m, int r, int b, double px, double py) {
+  const double q = __dmul_rn((double)m, f.inv_r[r]);
+  f.ur[((size_t)r * f.M + m) * f.B + b] = make_double2(__dmul_rn(-q, py), __dmul_rn(q, px));
+}
+// mode 0: u_phi = uphi_bar, omega = uphi_bar/r + d uphi_bar/dr, u_r = 0
+__device__ __forceinline__ void follow_mode0(const FxFollow& f, int r, int b) {
+  const size_t at = (size_t)r * f.M * f.B + b;
+  const double u = f.ub[(size_t)r * 2 * f.B + 2 * b], du = f.ub[(size_t)(f.R + r) * 2 * f.B + 2 * b];
+  f.up[at] = make_double2(u, 0.0);
+  f.ur[at] = make_double2(0.0, 0.0);
+  f.w[at] = make_double2(__fma_rn(u, f.inv_r[r], du), 0.0);
+  if (f.ubar_new) f.ubar_new[(size_t)r * f.B + b] = u;
+}
+#endif
 
 // Y[row][n] = alpha * sum_k A[k*lda + row] * X[k*ldx + n] for
 // row < rows, n < N, with a batch index z applying the strides sA, sX, sY.
@@ -251,6 +300,10 @@ struct GemmArgs {
   // fixed-point path: several products of one shape (batch 1) in one launch
   int njobs;
   FxJob job[kFxJobs];
+  // fixed-point paths: entries z >= batch are job[z - batch] (N columns, no
+  // njobs), and what follows the products of the others
+  int nextra;
+  FxFollow follow;
   // fixed-point tiles: 0 = the tile shape of the cost model, 16 / 32 / 64 = the
   // cost model's best shape of that column width (the same bits)
   int fma_ncol;
@@ -371,19 +424,16 @@ cudaError_t launch_nonlin(const NonlinArgs& a, cudaStream_t s);
 cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s);
 // Y = alpha A X in fixed point (g.fx set, K <= 257), and the operator's column
 // weights (wk null: none), integers and row exponents.
+bool fx_follows(const GemmArgs& g);  // host
 cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s);
 cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int K, int nb, int* wk, int2* out,
                                int* ex, cudaStream_t s);
 cudaError_t launch_imex_rhs(const RhsArgs& a, cudaStream_t s);
 // rhs_w(m>=1) += coef_b * (i m / r) * t_new, coef_b = scale * ra_pr[b]
-cudaError_t launch_add_buoyancy(int R, int M, int B, const double* inv_r, const double* ra_pr,
-                                double scale, const double2* t_new, double2* rhs_w,
-                                double2* buo_out, cudaStream_t s);
-// u_r = i m psi / r for m >= 1; m = 0 from the uphi_bar solve output
-// ub (rows 0..R-1: uphi_bar, rows R..2R-1: d uphi_bar/dr, columns 2*b+{0,1}).
-cudaError_t launch_post_w(int R, int M, int B, const double* inv_r, const double2* psi,
-                          double2* ur, double2* up, double2* w, const double* ub,
-                          double* ubar_new, cudaStream_t s);
+// f's buoyancy of t_new for the instance columns [b0, b1); f's velocity and mode 0
+// from psi: the same values as where a product is followed by them.
+cudaError_t launch_add_buoyancy(const FxFollow& f, int b0, int b1, const double2* t_new, cudaStream_t s);
+cudaError_t launch_post_w(const FxFollow& f, const double2* psi, cudaStream_t s);
 cudaError_t launch_stage_rhs(const StageArgs& a, cudaStream_t s);
 cudaError_t launch_stage_deriv(const StageArgs& a, cudaStream_t s);
 // Fortran (M,R) complex of instance b <-> device [r][m][b]

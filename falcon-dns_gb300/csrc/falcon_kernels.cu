@@ -448,66 +448,44 @@ cudaError_t launch_imex_rhs(const RhsArgs& a, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-__global__ void add_buoyancy_kernel(int R, int M, int B, const double* inv_r, const double* ra_pr,
-                                    double scale, const double2* t_new, double2* rhs_w, double2* buo_out) {
-  const size_t total = (size_t)R * M * B;
+// After a temperature solve or a (omega, psi, u_phi) solve that did not do it
+// itself (FxFollow).
+__global__ void add_buoyancy_kernel(FxFollow f, int b0, int nb, const double2* t_new) {
+  const size_t total = (size_t)f.R * f.M * nb;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
        e += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(e % B);
-    const size_t rm = e / B;
-    const int m = (int)(rm % M);
-    const int r = (int)(rm / M);
+    const size_t rm = e / nb;
+    const int b = b0 + (int)(e - rm * nb), r = (int)(rm / f.M), m = (int)(rm - (size_t)r * f.M);
     if (m == 0) continue;
-    const double2 T = t_new[e];
-    const double f = (double)m * inv_r[r];
-    // buoyancy term -(Ra/Pr) i m r^-1 T
-    const double2 bu = make_double2(ra_pr[b] * f * T.y, -ra_pr[b] * f * T.x);
-    if (buo_out) buo_out[e] = bu;
-    if (rhs_w && r > 0 && r < R - 1) {
-      double2 v = rhs_w[e];
-      v.x += scale * bu.x; v.y += scale * bu.y;
-      rhs_w[e] = v;
-    }
+    const double2 T = t_new[rm * f.B + b];
+    follow_buoyancy(f, m, r, b, T.x, T.y);
   }
 }
 
-cudaError_t launch_add_buoyancy(int R, int M, int B, const double* inv_r, const double* ra_pr,
-                                double scale, const double2* t_new, double2* rhs_w, double2* buo_out,
-                                cudaStream_t s) {
-  add_buoyancy_kernel<<<ew_grid((size_t)R * M * B), 256, 0, s>>>(R, M, B, inv_r, ra_pr, scale, t_new,
-                                                                  rhs_w, buo_out);
+cudaError_t launch_add_buoyancy(const FxFollow& f, int b0, int b1, const double2* t_new, cudaStream_t s) {
+  add_buoyancy_kernel<<<ew_grid((size_t)f.R * f.M * (b1 - b0)), 256, 0, s>>>(f, b0, b1 - b0, t_new);
   return cudaGetLastError();
 }
 
 // u_r = i m r^-1 psi (m >= 1); mode 0: u_phi = uphi_bar, omega = uphi_bar/r +
 // d uphi_bar/dr, u_r = 0 (src/fourierloop.F90:267-315).
-__global__ void post_w_kernel(int R, int M, int B, const double* inv_r, const double2* psi, double2* ur,
-                              double2* up, double2* w, const double* ub, double* ubar_new) {
-  const size_t total = (size_t)R * M * B;
+__global__ void post_w_kernel(FxFollow f, const double2* psi) {
+  const size_t total = (size_t)f.R * f.M * f.B;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
        e += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(e % B);
-    const size_t rm = e / B;
-    const int m = (int)(rm % M);
-    const int r = (int)(rm / M);
+    const size_t rm = e / f.B;
+    const int b = (int)(e - rm * f.B), r = (int)(rm / f.M), m = (int)(rm - (size_t)r * f.M);
     if (m > 0) {
       const double2 ps = psi[e];
-      const double f = (double)m * inv_r[r];
-      ur[e] = make_double2(-f * ps.y, f * ps.x);
+      follow_velocity(f, m, r, b, ps.x, ps.y);
     } else {
-      const double u = ub[(size_t)r * 2 * B + 2 * b];
-      const double du = ub[(size_t)(R + r) * 2 * B + 2 * b];
-      up[e] = make_double2(u, 0.0);
-      ur[e] = make_double2(0.0, 0.0);
-      w[e] = make_double2(u * inv_r[r] + du, 0.0);
-      if (ubar_new) ubar_new[(size_t)r * B + b] = u;
+      follow_mode0(f, r, b);
     }
   }
 }
 
-cudaError_t launch_post_w(int R, int M, int B, const double* inv_r, const double2* psi, double2* ur,
-                          double2* up, double2* w, const double* ub, double* ubar_new, cudaStream_t s) {
-  post_w_kernel<<<ew_grid((size_t)R * M * B), 256, 0, s>>>(R, M, B, inv_r, psi, ur, up, w, ub, ubar_new);
+cudaError_t launch_post_w(const FxFollow& f, const double2* psi, cudaStream_t s) {
+  post_w_kernel<<<ew_grid((size_t)f.R * f.M * f.B), 256, 0, s>>>(f, psi);
   return cudaGetLastError();
 }
 

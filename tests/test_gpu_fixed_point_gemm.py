@@ -71,6 +71,18 @@ def test_products_in_one_launch(fg, R, Nm, scheme, B):
         assert max(rel(g[f], r[f]) for f in FIELDS) < 4e-12
 
 
+@pytest.mark.parametrize("R,Nm,scheme,B", [(97, 341, "CNAB2", 1), (65, 170, "SBDF2", 4), (65, 170, "CNAB2", 3),
+                                           (49, 85, "BPR353", 2), (128, 64, "SBDF3", 3), (17, 512, "CNAB2", 2),
+                                           (9, 3, "CNAB2", 1), (129, 85, "ARS222", 4)])
+def test_narrow_shares_and_what_follows(fg, R, Nm, scheme, B):
+    """Narrow products of one to eight k shares and one to many row blocks, with
+    the buoyancy, u_r and mode 0 in the same launches: the same bound against
+    mode 1, which does these in kernels of their own."""
+    got, ref = states(fg, 0, R, Nm, scheme, B), states(fg, 1, R, Nm, scheme, B)
+    for g, r in zip(got, ref):
+        assert max(rel(g[f], r[f]) for f in FIELDS) < 4e-12
+
+
 def test_longest_contraction(fg, orc):
     """K = 257, the most the fixed-point sums hold."""
     prev = fg.set_gemm_mode(0)
