@@ -123,9 +123,9 @@ __device__ __forceinline__ double* output_row(const GemmArgs& g, int z, int row)
   return g.Yo[o] + (size_t)z * g.sY + (size_t)(row - (o ? g.rend[o - 1] : 0)) * g.ldy;
 }
 
-// After output row `row` of entry z, columns n (even), n + 1.
-__device__ __forceinline__ void follow_row(const FxFollow& f, int z, int row, int n, double y0, double y1) {
-  const int b = f.b0 + (n >> 1);
+// After output row `row` of entry z of a product, columns n (even), n + 1.
+__device__ __forceinline__ void follow_row(const FxFollow& f, int b0, int z, int row, int n, double y0, double y1) {
+  const int b = b0 + (n >> 1);
   if (f.kind == kBuoyancy) follow_buoyancy(f, f.m0 + z, row, b, y0, y1);
   if (f.kind == kVelocity && row >= f.R && row < 2 * f.R) follow_velocity(f, f.m0 + z, row - f.R, b, y0, y1);
 }
@@ -220,27 +220,37 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   int* cex = reinterpret_cast<int*>(as + 2 * kFxKC * rows_blk);       // [NCOL]
   int* part = cex + NCOL;                                             // [nthr]
   const int z = blockIdx.z;
-  int N = g.N, nblk = blockIdx.x;
+  int N = g.N, nblk = blockIdx.x, e = z, b0 = g.follow.b0;
+  const int nz = g.nsub ? g.nsub * g.batch : g.batch;
   long lda = g.lda, ldx = g.ldx, ldy = g.ldy;
   const int2* A = g.fx + (size_t)z * g.sA;
   const int* aex = g.fx_ex + (size_t)z * g.lda;
   const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
   const double* X = g.X + (size_t)z * g.sX;
   double* Y = nullptr;
-  if (g.njobs || z >= g.batch) {
-    int j = z >= g.batch ? z - g.batch : 0;
-    if (g.njobs)
+  if (g.njobs || g.nsub || z >= nz) {
+    int j = 0;
+    e = 0;
+    if (g.njobs) {
       for (int nb; nblk >= (nb = (g.job[j].N + NCOL - 1) / NCOL); ++j) nblk -= nb;
+    } else if (z < nz) {
+      j = z / g.batch;
+      e = z - j * g.batch;
+    } else {
+      j = g.nsub + z - nz;
+    }
     const FxJob& q = g.job[j];
     N = q.N;
     lda = q.lda;
     ldx = q.ldx;
     ldy = q.ldy;
-    A = q.fx;
-    aex = q.fx_ex;
-    w = q.fx_w;
-    X = q.X;
-    Y = q.Y;
+    A = q.fx + (size_t)e * g.sA;
+    aex = q.fx_ex + (size_t)e * lda;
+    w = q.fx_w ? q.fx_w + (size_t)e * g.K : nullptr;
+    X = q.X + (size_t)e * g.sX;
+    Y = q.Y + (size_t)e * g.sY;
+    b0 = q.b0;
+    if (nblk * NCOL >= N) return;  // a narrower product than the launch's
   }
   const int n0 = nblk * NCOL, row0 = blockIdx.y * rows_blk;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -325,7 +335,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
           yp[1] = y1;
         }
         if constexpr (RPT <= kFollowRows)
-          if (g.follow.kind && z < g.batch) follow_row(g.follow, z, row, n, y0, y1);
+          if (g.follow.kind && z < nz) follow_row(g.follow, b0, e, row, n, y0, y1);
       } else {
         yp[0] = y0;
       }
@@ -360,21 +370,27 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
   const int z = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x;
   const int kp = tid / RB, rl = tid - kp * RB, row = blockIdx.x * RB + rl;
   const int kq = (g.K + KS - 1) / KS, kb = min(kp * kq, g.K), ke = min(kb + kq, g.K);
+  int N = g.N, e = z, b0 = g.follow.b0;
+  const int nz = g.nsub ? g.nsub * g.batch : g.batch;
   long lda = g.lda, ldx = g.ldx;
   const int2* A = g.fx + (size_t)z * g.sA;
   const int* aex = g.fx_ex + (size_t)z * g.lda;
   const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
   const double* X = g.X + (size_t)z * g.sX;
   double* Y = nullptr;
-  if (z >= g.batch) {
-    const FxJob& q = g.job[z - g.batch];
+  if (g.nsub || z >= nz) {
+    const int j = z < nz ? z / g.batch : g.nsub + z - nz;
+    e = z < nz ? z - j * g.batch : 0;
+    const FxJob& q = g.job[j];
+    N = q.N;
     lda = q.lda;
     ldx = q.ldx;
-    A = q.fx;
-    aex = q.fx_ex;
-    w = q.fx_w;
-    X = q.X;
-    Y = q.Y + (size_t)row * q.ldy;
+    A = q.fx + (size_t)e * g.sA;
+    aex = q.fx_ex + (size_t)e * lda;
+    w = q.fx_w ? q.fx_w + (size_t)e * g.K : nullptr;
+    X = q.X + (size_t)e * g.sX;
+    Y = q.Y + (size_t)e * g.sY + (size_t)row * q.ldy;
+    b0 = q.b0;
   }
   A += min(row, g.rows - 1);
   int2 av[U];
@@ -382,7 +398,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
   for (int u = 0; u < U; ++u) av[u] = kb + u < ke ? __ldg(A + (size_t)(kb + u) * lda) : make_int2(0, 0);
   for (int i = tid; i < g.K * NC; i += nthr) {
     const int k = i / NC, c = i - k * NC;
-    xd[i] = c < g.N ? X[(size_t)k * ldx + c] : 0.0;
+    xd[i] = c < N ? X[(size_t)k * ldx + c] : 0.0;
   }
   __syncthreads();
   convert_panel(xd, g.K, NC, w, cex, part);
@@ -427,13 +443,13 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     return value_of(s, aex[row], cex[c], g.alpha);
   };
   double* y = Y ? Y : output_row(g, z, row);
-  for (int c = 2 * kp; c < g.N; c += 2 * KS) {
+  for (int c = 2 * kp; c < N; c += 2 * KS) {
     const double y0 = column(c);
     y[c] = y0;
-    if (c + 1 >= g.N) break;
+    if (c + 1 >= N) break;
     const double y1 = column(c + 1);
     y[c + 1] = y1;
-    if (g.follow.kind && z < g.batch) follow_row(g.follow, z, row, c, y0, y1);
+    if (g.follow.kind && z < nz) follow_row(g.follow, b0, e, row, c, y0, y1);
   }
 }
 
@@ -605,6 +621,10 @@ cudaError_t launch_fx_columns_dir(const FxColumns& g, cudaStream_t s) {
   return g.fwd ? launch_fx_columns_shape<RPT, NCOL, true>(g, s) : launch_fx_columns_shape<RPT, NCOL, false>(g, s);
 }
 
+// Batch entries of a launch: those of the product, or of each of its
+// sub-products, and the extra ones.
+int entries(const GemmArgs& g) { return g.batch * std::max(1, g.nsub) + g.nextra; }
+
 long column_blocks(const GemmArgs& g, int ncol) {
   if (!g.njobs) return ((long)g.N + ncol - 1) / ncol;
   long n = 0;
@@ -625,7 +645,7 @@ cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream
   }
   const int rows_blk = nw * (64 / NCOL) * RPT;
   const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw) * 4;
-  const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, g.batch + g.nextra);
+  const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, entries(g));
   fx_tile_kernel<RPT, NCOL><<<grid, 32 * nw, smem, s>>>(g);
   return cudaGetLastError();
 }
@@ -642,7 +662,7 @@ TileShape pick_shape(const GemmArgs& g, int nsm) {
   for (int ncol = 16; ncol <= 64; ncol *= 2) {
     if (g.fma_ncol && ncol != g.fma_ncol) continue;
     const int rg = 64 / ncol;
-    const long cb = column_blocks(g, ncol) * (g.batch + g.nextra);
+    const long cb = column_blocks(g, ncol) * entries(g);
     for (int rb = 1; rb <= 16; ++rb)
       for (int nw = 4; nw <= 16; ++nw)
         for (int rpt = 1; rpt <= 8; ++rpt) {
@@ -688,7 +708,7 @@ TileShape tile_shape(const GemmArgs& g) {
   thread_local std::unordered_map<unsigned long long, Memo> memo;
   unsigned long long key = 1469598103934665603ull;
   const int total = (int)column_blocks(g, 1);  // columns of all jobs
-  const int batch = g.batch + g.nextra;
+  const int batch = entries(g);
   for (int v : {g.rows, g.K, g.N, total, batch, nsm, g.fma_ncol}) key = (key ^ (unsigned)v) * 1099511628211ull;
   Memo& m = memo[key];
   if (m.rows != g.rows || m.K != g.K || m.N != g.N || m.total != total || m.batch != batch || m.nsm != nsm ||
@@ -724,7 +744,7 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
     // in even blocks of at most 256 threads, of fewer while SMs are without two
     // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.9, 7.9, 7.8; 65 x 65 x 8,
     // 171 entries 22.5, 18.1, 16.0, 18.0; 291 x 97 x 2, 341 entries 31.0, 32.4, 36.5, 46.8)
-    const int nz = g.batch + g.nextra;
+    const int nz = entries(g);
     const int KS = (int)std::min(8L, std::max(1L, 152L * 448 / ((long)g.rows * nz)));
     int nb = (g.rows + 256 / KS - 1) / (256 / KS);
     while ((long)nb * nz < 2 * 152 && (g.rows + nb - 1) / nb > 16) ++nb;

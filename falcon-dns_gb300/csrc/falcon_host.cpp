@@ -1817,7 +1817,7 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
       all.oz_s = nullptr;
       all.oz_xs = nullptr;
     }
-    all.job[i] = FxJob{q.fx, q.fx_ex, q.fx_w, q.X, q.Y, q.ldx, q.ldy, q.N, q.lda};
+    all.job[i] = FxJob{q.fx, q.fx_ex, q.fx_w, q.X, q.Y, q.ldx, q.ldy, q.N, q.lda, 0};
     cols += q.N;
   }
   all.njobs = tiles ? (int)v.size() : 0;
@@ -1984,8 +1984,9 @@ int run_nonlin(Group* g) {
 //
 // Where the products run as fixed-point integers, the buoyancy follows the
 // temperature product and u_r and mode 0 the (omega, psi, u_phi) product in
-// the same kernels, and the uphi_bar product rides with the temperature's as
-// two more entries: two launches instead of five (a step of one 33 x 43 run: 41 -> 37
+// the same kernels, the temperature products of several Pr are one launch (48
+// mixed instances, three Pr a group: ten steps 14.0 -> 13.0 ms), and the uphi_bar
+// product rides with the temperature's as more entries: two launches instead of five (a step of one 33 x 43 run: 41 -> 37
 // us; the same bits).
 int solve_all(Group* g, double2* t_out, double2* w_out, double buo_scale, double2* buo_store,
               double* ubar_store, int st = -1) {
@@ -2004,29 +2005,71 @@ int solve_all(Group* g, double2* t_out, double2* w_out, double buo_scale, double
   gu.K = R; gu.rows = 2 * R; gu.N = 2 * B; gu.batch = 1; gu.alpha = 1.0;
   bool ubar = false;  // uphi_bar is made
   GemmArgs ride = gu;
-  int pu = PATH_MMA;
-  if (g->subs.size() == 1 && (rc = choose_path(g, KC_GEMM_MODE, &ride, false, &pu))) return rc;
-  for (size_t k = 0; k < g->subs.size(); ++k) {
+  int pu = PATH_FMA;
+  if ((rc = choose_path(g, KC_GEMM_MODE, &ride, false, &pu))) return rc;
+  // uphi_bar's two row halves as extra entries of q, no wider than it is
+  auto take_ride = [&](GemmArgs* q) {
+    const int pieces = (ride.N + q->N - 1) / q->N;
+    if (!is_fma_path(pu) || !ride.fx || q->nsub + 2 * pieces > kFxJobs) return;
+    for (int h = 0; h < 2; ++h)
+      for (int n = 0; n < ride.N; n += q->N)
+        q->job[q->nsub + q->nextra++] =
+            FxJob{ride.fx + h * R, ride.fx_ex + h * R, ride.fx_w, ride.X + n, ride.Y + h * R * ride.ldy + n,
+                  ride.ldx, ride.ldy, std::min(ride.N - n, q->N), ride.lda, 0};
+    ubar = true;
+  };
+  auto follow_it = [&](GemmArgs* q, int b0) {
+    if (!fx_follows(*q)) return false;
+    q->follow = f;
+    q->follow.kind = kBuoyancy;
+    q->follow.b0 = b0;
+    return true;
+  };
+  auto temperature = [&](size_t k) {
     const Group::Sub& u = g->subs[k];
     GemmArgs q = per_mode(sub_ops(g, (int)k, st)->ST, R, (long)R * R, g->rhs_t + u.b0, t_out + u.b0, R, M, B, 0, M, R);
     q.N = 2 * (u.b1 - u.b0);
+    return q;
+  };
+  // several Pr: their temperature products as one launch where all are tiles
+  size_t from = 0;
+  if (g->subs.size() > 1 && (int)g->subs.size() <= kFxJobs) {
+    GemmArgs all{};
+    bool fx = true;
+    int path = PATH_FMA;
+    for (size_t k = 0; k < g->subs.size() && fx; ++k) {
+      GemmArgs q = temperature(k);
+      int p = PATH_FMA;
+      if ((rc = choose_path(g, KC_GEMM_MODE, &q, false, &p))) return rc;
+      if (!(fx = is_fma_path(p) && q.fx)) break;
+      if (q.N > all.N) {
+        const GemmArgs before = all;
+        all = q;
+        for (size_t j = 0; j < k; ++j) all.job[j] = before.job[j];
+        path = p;
+      }
+      all.job[k] = FxJob{q.fx, q.fx_ex, q.fx_w, q.X, q.Y, q.ldx, q.ldy, q.N, q.lda, g->subs[k].b0};
+    }
+    if (fx) {
+      all.nsub = (int)g->subs.size();
+      all.fma_ncol = path_columns(path);
+      take_ride(&all);
+      const bool follows = follow_it(&all, 0);
+      if ((rc = run_path(g, KC_GEMM_MODE, all, path, false))) return rc;
+      if (!follows && (rc = elementwise(g, 6.0, [&]() { return launch_add_buoyancy(f, 0, B, t_out, s); }))) return rc;
+      from = g->subs.size();
+    }
+  }
+  for (size_t k = from; k < g->subs.size(); ++k) {
+    const Group::Sub& u = g->subs[k];
+    GemmArgs q = temperature(k);
     int path = PATH_FMA;
     if ((rc = choose_path(g, KC_GEMM_MODE, &q, false, &path))) return rc;
     bool follows = false;
     if (is_fma_path(path) && q.fx) {
-      if (is_fma_path(pu) && ride.fx) {
-        for (int h = 0; h < 2; ++h)
-          q.job[h] = FxJob{ride.fx + h * R, ride.fx_ex + h * R, ride.fx_w, ride.X, ride.Y + h * R * ride.ldy,
-                           ride.ldx, ride.ldy, ride.N, ride.lda};
-        q.nextra = 2;
-        ubar = true;
-      }
       q.fma_ncol = path_columns(path);
-      if ((follows = fx_follows(q))) {
-        q.follow = f;
-        q.follow.kind = kBuoyancy;
-        q.follow.b0 = u.b0;
-      }
+      if (!ubar) take_ride(&q);
+      follows = follow_it(&q, u.b0);
     }
     if ((rc = run_path(g, KC_GEMM_MODE, q, path, false))) return rc;
     if (!follows && (rc = elementwise(g, 6.0, [&]() { return launch_add_buoyancy(f, u.b0, u.b1, t_out, s); }))) return rc;

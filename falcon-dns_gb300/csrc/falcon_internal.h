@@ -209,8 +209,9 @@ struct FxJob {
   long ldx, ldy;
   int N;
   long lda;
+  int b0;  // first instance column (FxFollow)
 };
-constexpr int kFxJobs = 6;
+constexpr int kFxJobs = 10;
 
 // What a fixed-point per-mode product does with its outputs beyond storing
 // them (batch entry z = mode m0 + z, columns = instances from b0 on).
@@ -300,9 +301,11 @@ struct GemmArgs {
   // fixed-point path: several products of one shape (batch 1) in one launch
   int njobs;
   FxJob job[kFxJobs];
-  // fixed-point paths: entries z >= batch are job[z - batch] (N columns, no
-  // njobs), and what follows the products of the others
-  int nextra;
+  // fixed-point paths (no njobs): nsub products of `batch` entries each, product
+  // s from job[s] on with the strides sA, sX, sY, in place of this one; then
+  // nextra single entries, job[nsub] on; N is the most columns of any.  What
+  // follows the products, but for the extra entries.
+  int nsub, nextra;
   FxFollow follow;
   // fixed-point tiles: 0 = the tile shape of the cost model, 16 / 32 / 64 = the
   // cost model's best shape of that column width (the same bits)

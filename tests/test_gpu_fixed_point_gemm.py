@@ -83,6 +83,36 @@ def test_narrow_shares_and_what_follows(fg, R, Nm, scheme, B):
         assert max(rel(g[f], r[f]) for f in FIELDS) < 4e-12
 
 
+@pytest.mark.parametrize("R,Nm,scheme,counts", [(33, 42, "CNAB2", (2, 1, 1)), (33, 10, "SBDF3", (1, 5)),
+                                                (65, 85, "BPR353", (1, 2, 1)), (17, 20, "CNAB2", (1,) * 10),
+                                                (17, 20, "CNAB2", (1,) * 11), (48, 16, "SBDF2", (9, 2, 6))])
+def test_products_of_several_prandtl_numbers(fg, R, Nm, scheme, counts):
+    """The temperature products of a group's Prandtl numbers in one launch (uneven
+    widths, up to the ten it takes, and one more): the bits of each instance
+    alone, and the bound above against mode 1."""
+    prs = [0.3 * 1.7 ** k for k, c in enumerate(counts) for _ in range(c)]
+
+    def run(mode, which):
+        prev = fg.set_gemm_mode(mode)
+        try:
+            b = fg.Batch([fg.make_params(R, Nm, scheme, ra=1e5 * (1 + k), pr=prs[k], dt=1e-6) for k in which])
+            b.init_noise([70 + k for k in which])
+            b.step(3)
+            out = [b.get_state(i) for i in range(len(which))]
+            b.close()
+            return out
+        finally:
+            fg.set_gemm_mode(prev)
+
+    every = range(len(prs))
+    got, ref = run(0, every), run(1, every)
+    for k in every:
+        assert max(rel(got[k][f], ref[k][f]) for f in FIELDS) < 4e-12
+    for k in (0, len(prs) - 1):
+        alone = run(0, [k])[0]
+        assert all(np.array_equal(alone[f], got[k][f]) for f in FIELDS)
+
+
 def test_longest_contraction(fg, orc):
     """K = 257, the most the fixed-point sums hold."""
     prev = fg.set_gemm_mode(0)
