@@ -2285,6 +2285,14 @@ int step_imexrk(Group* g) {
   a.rhs_t = g->rhs_t; a.rhs_w = g->rhs_w;
   a.ntp = g->ntp; a.ntr = g->ntr; a.dntr = g->dntr; a.nwp = g->nwp; a.nwr = g->nwr; a.dnwr = g->dnwr;
   a.lt = g->lt; a.lw = g->lw; a.lu0 = g->lu0; a.t = g->T(); a.w = g->W(); a.up = g->up;
+  // stages with a nonlinear pass; the temperature of the step's last one is kept
+  auto passes = [&](int st) {
+    double colsum = 0.0;
+    for (int i = 0; i < ns; ++i) colsum += sc.aA[i][st];
+    return (nstep > 1 || st > 0) && (colsum + sc.bA[st] != 0.0);
+  };
+  int last_pass = ns - 1;
+  while (last_pass >= 0 && !passes(last_pass)) --last_pass;
   for (int st = 0; st < ns; ++st) {
     a.st = st;
     for (int i = 0; i < kMaxStages; ++i) { a.aD[i] = sc.aD[st][i]; a.aA[i] = sc.aA[st][i]; }
@@ -2294,11 +2302,9 @@ int step_imexrk(Group* g) {
       const double scale = g->p.buo_imp ? g->cur_dt() * sc.aD[st][st] : 0.0;
       if ((rc = solve_all(g, g->T(), g->W(), scale, g->buo[st], nullptr, st))) return rc;
     }
-    double colsum = 0.0;
-    for (int i = 0; i < ns; ++i) colsum += sc.aA[i][st];
-    if ((nstep > 1 || st > 0) && (colsum + sc.bA[st] != 0.0)) {
+    if (passes(st)) {
       if ((rc = run_nonlin(g))) return rc;
-      CK(cudaMemcpyAsync(g->t_grid, g->T(), sizeof(double2) * n, cudaMemcpyDeviceToDevice, s));
+      if (st == last_pass) CK(cudaMemcpyAsync(g->t_grid, g->T(), sizeof(double2) * n, cudaMemcpyDeviceToDevice, s));
     } else if (nstep == 1 && st == 0) {
       CK(cudaMemsetAsync(g->ntp, 0, sizeof(double2) * n, s));
       CK(cudaMemsetAsync(g->ntr, 0, sizeof(double2) * n, s));

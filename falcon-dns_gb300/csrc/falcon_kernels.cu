@@ -341,99 +341,148 @@ cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s) {
 // IMEX right-hand sides (rhs_construct_temp / _vort / _uphi_bar,
 // src/rhs_create.F90:24-385), one thread per (r, m, b).
 // ---------------------------------------------------------------------------
-// The FP64 pipe bounds this kernel (~35 FP64 instructions per element
-// against ~20 bytes of HBM traffic per instruction's worth of time), so the
-// weights are folded once per thread (c_exp = dt w_exp) and every sum is a
-// chain of FMAs.
-__global__ void imex_rhs_kernel(RhsArgs a) {
-  const unsigned B = (unsigned)a.B, M = (unsigned)a.M;
-  const size_t total = (size_t)a.R * M * B;
-  const double dt = a.dt;
-  double c_exp[4];
+// One thread per element, the grid's rows the radial points: one 32-bit
+// division (by B) an element, where a flat index took two of 64 bits.  All of
+// a field's loads precede its first store and, for the schemes in use (NI and NE
+// history levels, 0: any), are unrolled, so that ten are in flight.  Bound by
+// HBM (20 x 16 bytes an element of SBDF3) and the FP64 pipe (34 instructions of
+// 64 cycles a warp) together: the weights are folded once per thread (c_exp =
+// dt w_exp) and every sum is a chain of FMAs.  65 x 171 x 256, SBDF3: 238 -> 200 us.
+struct Cell {
+  int r, m, b;
+  size_t e;
+};
+__device__ __forceinline__ bool cell_of(int M, int B, Cell* c) {
+  const unsigned j = blockIdx.x * blockDim.x + threadIdx.x, row = (unsigned)M * (unsigned)B;
+  if (j >= row) return false;
+  c->r = blockIdx.y;
+  c->m = (int)(j / (unsigned)B);
+  c->b = (int)(j - (unsigned)c->m * (unsigned)B);
+  c->e = (size_t)blockIdx.y * row + j;
+  return true;
+}
+// Blocks of 128, of 64 while those leave SMs idle (the FP64 pipe is per
+// sub-partition: a small run's warps have to spread).
+struct CellGrid {
+  dim3 grid;
+  int block;
+};
+static CellGrid cell_grid(int R, int M, int B) {
+  const long row = (long)M * B;
+  const int block = (long)R * ((row + 127) / 128) < 2 * 152 ? 64 : 128;
+  return {dim3((unsigned)((row + block - 1) / block), R), block};
+}
+
+template <int NI, int NE, bool CN>
+__global__ void imex_rhs_kernel(const __grid_constant__ RhsArgs a) {
+  Cell c;
+  if (!cell_of(a.M, a.B, &c)) return;
+  const int r = c.r, m = c.m, b = c.b;
+  const size_t e = c.e;
+  const int ni = NI ? NI : a.n_imp, ne = NE ? NE : a.n_exp;
+  constexpr int MI = NI ? NI : 4, ME = NE ? NE : 4;
+  const double dt = a.dt, c_cn = (1.0 - a.w_imp[0]) * dt;
+  double c_exp[ME];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) c_exp[i] = dt * a.w_exp[i];
-  const double c_cn = (1.0 - a.w_imp[0]) * dt;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
-    const size_t rm = e / B;
-    const unsigned b = (unsigned)(e - rm * B);
-    const unsigned r = (unsigned)(rm / M), m = (unsigned)(rm - (size_t)r * M);
-    const double ir = a.inv_r[r];
-    const double dm = (double)(int)m, dmir = dm * ir;
-    // upFR_prev = upFR after the nonlinear pass (src/steptime.F90:212), for
-    // the u_phi balance of the diagnostics
-    if (m == 0 && a.up0_prev) a.up0_prev[(size_t)r * B + b] = a.up[e].x;
-    // explicit (advective) term of T: i m r^-1 (uphi T) + d(ur T)/dr + r^-1 (ur T)
-    {
-      const double2 p = a.ntp[e], q = a.ntr[e], dq = a.dntr[e];
-      const double2 nt = make_double2(fma(-dmir, p.y, fma(ir, q.x, dq.x)), fma(dmir, p.x, fma(ir, q.y, dq.y)));
-      a.nt_new[e] = nt;
-      double2 rhs;
-      if (a.scheme_cn) {
-        const double2 T = a.th[0][e], L = a.lt[e];
-        const double c = c_cn * a.inv_pr[b], k2 = dm * dm * a.inv_r2[r];
-        rhs = make_double2(fma(c, fma(-k2, T.x, L.x), T.x), fma(c, fma(-k2, T.y, L.y), T.y));
-      } else {
-        const double2 h0 = a.th[0][e];
-        rhs = make_double2(a.w_imp[0] * h0.x, a.w_imp[0] * h0.y);
-        for (int i = 1; i < a.n_imp; ++i) {
-          const double2 h = a.th[i][e];
-          rhs.x = fma(a.w_imp[i], h.x, rhs.x); rhs.y = fma(a.w_imp[i], h.y, rhs.y);
-        }
-      }
-      rhs.x = fma(-c_exp[0], nt.x, rhs.x); rhs.y = fma(-c_exp[0], nt.y, rhs.y);
-      for (int i = 1; i < a.n_exp; ++i) {
-        const double2 h = a.nth[i][e];
-        rhs.x = fma(-c_exp[i], h.x, rhs.x); rhs.y = fma(-c_exp[i], h.y, rhs.y);
-      }
-      if (r == 0) rhs = make_double2(m == 0 ? 1.0 : 0.0, 0.0);
-      if (r == (unsigned)a.R - 1) rhs = make_double2(0.0, 0.0);
-      a.rhs_t[e] = rhs;
-    }
-    if (m > 0) {
-      const double2 p = a.nwp[e], q = a.nwr[e], dq = a.dnwr[e];
-      const double2 nw = make_double2(fma(-dmir, p.y, fma(ir, q.x, dq.x)), fma(dmir, p.x, fma(ir, q.y, dq.y)));
-      a.nw_new[e] = nw;
-      double2 rhs;
-      if (a.scheme_cn) {
-        const double2 W = a.wh[0][e], L = a.lw[e], To = a.th[0][e];
-        const double k2 = dm * dm * a.inv_r2[r];
-        const double bc = a.ra_pr[b] * dt * 0.5 * dmir;  // old-T half of the CN buoyancy
-        rhs = make_double2(fma(bc, To.y, fma(c_cn, fma(-k2, W.x, L.x), W.x)),
-                           fma(-bc, To.x, fma(c_cn, fma(-k2, W.y, L.y), W.y)));
-      } else {
-        const double2 h0 = a.wh[0][e];
-        rhs = make_double2(a.w_imp[0] * h0.x, a.w_imp[0] * h0.y);
-        for (int i = 1; i < a.n_imp; ++i) {
-          const double2 h = a.wh[i][e];
-          rhs.x = fma(a.w_imp[i], h.x, rhs.x); rhs.y = fma(a.w_imp[i], h.y, rhs.y);
-        }
-      }
-      rhs.x = fma(-c_exp[0], nw.x, rhs.x); rhs.y = fma(-c_exp[0], nw.y, rhs.y);
-      for (int i = 1; i < a.n_exp; ++i) {
-        const double2 h = a.nwh[i][e];
-        rhs.x = fma(-c_exp[i], h.x, rhs.x); rhs.y = fma(-c_exp[i], h.y, rhs.y);
-      }
-      if (r == 0 || r == (unsigned)a.R - 1) rhs = make_double2(0.0, 0.0);
-      a.rhs_w[e] = rhs;
+  for (int i = 0; i < ME; ++i) c_exp[i] = dt * a.w_exp[i];
+  const double ir = a.inv_r[r];
+  const double dm = (double)m, dmir = dm * ir;
+  // upFR_prev = upFR after the nonlinear pass (src/steptime.F90:212), for
+  // the u_phi balance of the diagnostics
+  if (m == 0 && a.up0_prev) a.up0_prev[(size_t)r * a.B + b] = a.up[e].x;
+  // explicit (advective) term of a field: i m r^-1 (uphi f) + d(ur f)/dr + r^-1 (ur f)
+  auto advective = [&](const double2& p, const double2& q, const double2& dq) {
+    return make_double2(fma(-dmir, p.y, fma(ir, q.x, dq.x)), fma(dmir, p.x, fma(ir, q.y, dq.y)));
+  };
+  {
+    const double2 p = a.ntp[e], q = a.ntr[e], dq = a.dntr[e];
+    double2 h[MI], x[ME], L = make_double2(0.0, 0.0);
+    h[0] = a.th[0][e];
+    if (CN) {
+      L = a.lt[e];
     } else {
-      // mean azimuthal flow: rhs_construct_uphi_bar
-      const size_t rb = (size_t)r * B + b;
-      const double urom = a.nwr[e].x;  // mode-0 coefficient of ur*omg = its azimuthal mean
-      a.urom_new[rb] = urom;
-      double rhs;
-      if (a.scheme_cn) {
-        const double u = a.ubh[0][rb];
-        const double lu = a.lu0[rb].x;
-        rhs = fma(c_cn, fma(-a.inv_r2[r], u, lu), u);
-      } else {
-        rhs = a.w_imp[0] * a.ubh[0][rb];
-        for (int i = 1; i < a.n_imp; ++i) rhs = fma(a.w_imp[i], a.ubh[i][rb], rhs);
-      }
-      rhs = fma(-c_exp[0], urom, rhs);
-      for (int i = 1; i < a.n_exp; ++i) rhs = fma(-c_exp[i], a.uromh[i][rb], rhs);
-      if (r == 0 || r == (unsigned)a.R - 1) rhs = 0.0;
-      a.rhs_w[e] = make_double2(rhs, 0.0);
+#pragma unroll
+      for (int i = 1; i < MI; ++i)
+        if (i < ni) h[i] = a.th[i][e];
     }
+#pragma unroll
+    for (int i = 1; i < ME; ++i)
+      if (i < ne) x[i] = a.nth[i][e];
+    const double2 nt = advective(p, q, dq);
+    a.nt_new[e] = nt;
+    double2 rhs;
+    if (CN) {
+      const double k = c_cn * a.inv_pr[b], k2 = dm * dm * a.inv_r2[r];
+      rhs = make_double2(fma(k, fma(-k2, h[0].x, L.x), h[0].x), fma(k, fma(-k2, h[0].y, L.y), h[0].y));
+    } else {
+      rhs = make_double2(a.w_imp[0] * h[0].x, a.w_imp[0] * h[0].y);
+#pragma unroll
+      for (int i = 1; i < MI; ++i)
+        if (i < ni) { rhs.x = fma(a.w_imp[i], h[i].x, rhs.x); rhs.y = fma(a.w_imp[i], h[i].y, rhs.y); }
+    }
+    rhs.x = fma(-c_exp[0], nt.x, rhs.x); rhs.y = fma(-c_exp[0], nt.y, rhs.y);
+#pragma unroll
+    for (int i = 1; i < ME; ++i)
+      if (i < ne) { rhs.x = fma(-c_exp[i], x[i].x, rhs.x); rhs.y = fma(-c_exp[i], x[i].y, rhs.y); }
+    if (r == 0) rhs = make_double2(m == 0 ? 1.0 : 0.0, 0.0);
+    if (r == a.R - 1) rhs = make_double2(0.0, 0.0);
+    a.rhs_t[e] = rhs;
+  }
+  if (m > 0) {
+    const double2 p = a.nwp[e], q = a.nwr[e], dq = a.dnwr[e];
+    double2 h[MI], x[ME], L = make_double2(0.0, 0.0), To = L;
+    h[0] = a.wh[0][e];
+    if (CN) {
+      L = a.lw[e];
+      To = a.th[0][e];
+    } else {
+#pragma unroll
+      for (int i = 1; i < MI; ++i)
+        if (i < ni) h[i] = a.wh[i][e];
+    }
+#pragma unroll
+    for (int i = 1; i < ME; ++i)
+      if (i < ne) x[i] = a.nwh[i][e];
+    const double2 nw = advective(p, q, dq);
+    a.nw_new[e] = nw;
+    double2 rhs;
+    if (CN) {
+      const double k2 = dm * dm * a.inv_r2[r];
+      const double bc = a.ra_pr[b] * dt * 0.5 * dmir;  // old-T half of the CN buoyancy
+      rhs = make_double2(fma(bc, To.y, fma(c_cn, fma(-k2, h[0].x, L.x), h[0].x)),
+                         fma(-bc, To.x, fma(c_cn, fma(-k2, h[0].y, L.y), h[0].y)));
+    } else {
+      rhs = make_double2(a.w_imp[0] * h[0].x, a.w_imp[0] * h[0].y);
+#pragma unroll
+      for (int i = 1; i < MI; ++i)
+        if (i < ni) { rhs.x = fma(a.w_imp[i], h[i].x, rhs.x); rhs.y = fma(a.w_imp[i], h[i].y, rhs.y); }
+    }
+    rhs.x = fma(-c_exp[0], nw.x, rhs.x); rhs.y = fma(-c_exp[0], nw.y, rhs.y);
+#pragma unroll
+    for (int i = 1; i < ME; ++i)
+      if (i < ne) { rhs.x = fma(-c_exp[i], x[i].x, rhs.x); rhs.y = fma(-c_exp[i], x[i].y, rhs.y); }
+    if (r == 0 || r == a.R - 1) rhs = make_double2(0.0, 0.0);
+    a.rhs_w[e] = rhs;
+  } else {
+    // mean azimuthal flow: rhs_construct_uphi_bar
+    const size_t rb = (size_t)r * a.B + b;
+    const double urom = a.nwr[e].x;  // mode-0 coefficient of ur*omg = its azimuthal mean
+    a.urom_new[rb] = urom;
+    double rhs;
+    if (CN) {
+      const double u = a.ubh[0][rb];
+      const double lu = a.lu0[rb].x;
+      rhs = fma(c_cn, fma(-a.inv_r2[r], u, lu), u);
+    } else {
+      rhs = a.w_imp[0] * a.ubh[0][rb];
+      for (int i = 1; i < ni; ++i) rhs = fma(a.w_imp[i], a.ubh[i][rb], rhs);
+    }
+    rhs = fma(-c_exp[0], urom, rhs);
+#pragma unroll
+    for (int i = 1; i < ME; ++i)
+      if (i < ne) rhs = fma(-c_exp[i], a.uromh[i][rb], rhs);
+    if (r == 0 || r == a.R - 1) rhs = 0.0;
+    a.rhs_w[e] = make_double2(rhs, 0.0);
   }
 }
 
@@ -444,48 +493,47 @@ static int ew_grid(size_t n) {
 }
 
 cudaError_t launch_imex_rhs(const RhsArgs& a, cudaStream_t s) {
-  imex_rhs_kernel<<<ew_grid((size_t)a.R * a.M * a.B), 256, 0, s>>>(a);
+  const CellGrid c = cell_grid(a.R, a.M, a.B);
+  if (a.scheme_cn && a.n_exp == 2) imex_rhs_kernel<1, 2, true><<<c.grid, c.block, 0, s>>>(a);
+  else if (a.scheme_cn) imex_rhs_kernel<1, 0, true><<<c.grid, c.block, 0, s>>>(a);
+  else if (a.n_imp == 2 && a.n_exp == 2) imex_rhs_kernel<2, 2, false><<<c.grid, c.block, 0, s>>>(a);
+  else if (a.n_imp == 3 && a.n_exp == 3) imex_rhs_kernel<3, 3, false><<<c.grid, c.block, 0, s>>>(a);
+  else imex_rhs_kernel<0, 0, false><<<c.grid, c.block, 0, s>>>(a);
   return cudaGetLastError();
 }
 
 // After a temperature solve or a (omega, psi, u_phi) solve that did not do it
 // itself (FxFollow).
 __global__ void add_buoyancy_kernel(FxFollow f, int b0, int nb, const double2* t_new) {
-  const size_t total = (size_t)f.R * f.M * nb;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t rm = e / nb;
-    const int b = b0 + (int)(e - rm * nb), r = (int)(rm / f.M), m = (int)(rm - (size_t)r * f.M);
-    if (m == 0) continue;
-    const double2 T = t_new[rm * f.B + b];
-    follow_buoyancy(f, m, r, b, T.x, T.y);
-  }
+  Cell c;
+  if (!cell_of(f.M, nb, &c) || c.m == 0) return;
+  const int b = b0 + c.b;
+  const double2 T = t_new[((size_t)c.r * f.M + c.m) * f.B + b];
+  follow_buoyancy(f, c.m, c.r, b, T.x, T.y);
 }
 
 cudaError_t launch_add_buoyancy(const FxFollow& f, int b0, int b1, const double2* t_new, cudaStream_t s) {
-  add_buoyancy_kernel<<<ew_grid((size_t)f.R * f.M * (b1 - b0)), 256, 0, s>>>(f, b0, b1 - b0, t_new);
+  const CellGrid c = cell_grid(f.R, f.M, b1 - b0);
+  add_buoyancy_kernel<<<c.grid, c.block, 0, s>>>(f, b0, b1 - b0, t_new);
   return cudaGetLastError();
 }
 
 // u_r = i m r^-1 psi (m >= 1); mode 0: u_phi = uphi_bar, omega = uphi_bar/r +
 // d uphi_bar/dr, u_r = 0 (src/fourierloop.F90:267-315).
 __global__ void post_w_kernel(FxFollow f, const double2* psi) {
-  const size_t total = (size_t)f.R * f.M * f.B;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const size_t rm = e / f.B;
-    const int b = (int)(e - rm * f.B), r = (int)(rm / f.M), m = (int)(rm - (size_t)r * f.M);
-    if (m > 0) {
-      const double2 ps = psi[e];
-      follow_velocity(f, m, r, b, ps.x, ps.y);
-    } else {
-      follow_mode0(f, r, b);
-    }
+  Cell c;
+  if (!cell_of(f.M, f.B, &c)) return;
+  if (c.m > 0) {
+    const double2 ps = psi[c.e];
+    follow_velocity(f, c.m, c.r, c.b, ps.x, ps.y);
+  } else {
+    follow_mode0(f, c.r, c.b);
   }
 }
 
 cudaError_t launch_post_w(const FxFollow& f, const double2* psi, cudaStream_t s) {
-  post_w_kernel<<<ew_grid((size_t)f.R * f.M * f.B), 256, 0, s>>>(f, psi);
+  const CellGrid c = cell_grid(f.R, f.M, f.B);
+  post_w_kernel<<<c.grid, c.block, 0, s>>>(f, psi);
   return cudaGetLastError();
 }
 
@@ -494,105 +542,93 @@ cudaError_t launch_post_w(const FxFollow& f, const double2* psi, cudaStream_t s)
 // 214-354): Y0 + dt * (sum_i aD(s,i) F_d(i) + aA(s,i) F_a(i)) [+ buoyancy].
 // The buoyancy of the current stage is added after the temperature solve.
 // ---------------------------------------------------------------------------
-__global__ void stage_rhs_kernel(StageArgs a) {
-  const size_t total = (size_t)a.R * a.M * a.B;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(e % a.B);
-    const size_t rm = e / a.B;
-    const int m = (int)(rm % a.M);
-    const int r = (int)(rm / a.M);
-    const double dt = a.dt;
-    {
-      double2 fd = make_double2(0, 0), fa = make_double2(0, 0);
-      for (int i = 0; i < a.st; ++i) {
-        const double2 q = a.fdt[i][e];
-        fd.x += a.aD[i] * q.x; fd.y += a.aD[i] * q.y;
-      }
-      for (int i = 0; i < a.st; ++i) {
-        const double2 q = a.fat[i][e];
-        fa.x += a.aA[i] * q.x; fa.y += a.aA[i] * q.y;
-      }
-      const double2 y0 = a.t0[e];
-      double2 rhs = make_double2(y0.x + dt * (fd.x + fa.x), y0.y + dt * (fd.y + fa.y));
-      if (r == 0) rhs = make_double2(m == 0 ? 1.0 : 0.0, 0.0);
-      if (r == a.R - 1) rhs = make_double2(0.0, 0.0);
-      a.rhs_t[e] = rhs;
+// ST: the stage, whose 5 ST loads of derivatives are unrolled (0: any).
+template <int ST>
+__global__ void stage_rhs_kernel(const __grid_constant__ StageArgs a) {
+  Cell c;
+  if (!cell_of(a.M, a.B, &c)) return;
+  const int r = c.r, m = c.m, st = ST ? ST : a.st;
+  const size_t e = c.e;
+  const double dt = a.dt;
+  auto sum = [&](const double2* const* f, const double* w) {
+    double2 y = make_double2(0, 0);
+#pragma unroll
+    for (int i = 0; i < st; ++i) {
+      const double2 q = f[i][e];
+      y.x += w[i] * q.x; y.y += w[i] * q.y;
     }
-    double2 fd = make_double2(0, 0), fa = make_double2(0, 0), fb = make_double2(0, 0);
-    for (int i = 0; i < a.st; ++i) {
-      const double2 q = a.fdw[i][e];
-      fd.x += a.aD[i] * q.x; fd.y += a.aD[i] * q.y;
-    }
-    for (int i = 0; i < a.st; ++i) {
-      const double2 q = a.faw[i][e];
-      fa.x += a.aA[i] * q.x; fa.y += a.aA[i] * q.y;
-    }
-    if (m == 0) {
-      const double y0 = a.u0[(size_t)r * a.B + b];
-      double rhs = y0 + dt * (fd.x + fa.x);
-      if (r == 0 || r == a.R - 1) rhs = 0.0;
-      a.rhs_w[e] = make_double2(rhs, 0.0);
-    } else {
-      for (int i = 0; i < a.st; ++i) {
-        const double2 q = a.buo[i][e];
-        const double c = a.buo_imp ? a.aD[i] : a.aA[i];
-        fb.x += c * q.x; fb.y += c * q.y;
-      }
-      const double2 y0 = a.w0[e];
-      double2 rhs = make_double2(y0.x + dt * (fd.x + fa.x + fb.x), y0.y + dt * (fd.y + fa.y + fb.y));
-      if (r == 0 || r == a.R - 1) rhs = make_double2(0.0, 0.0);
-      a.rhs_w[e] = rhs;
-    }
+    return y;
+  };
+  {
+    const double2 y0 = a.t0[e], fd = sum(a.fdt, a.aD), fa = sum(a.fat, a.aA);
+    double2 rhs = make_double2(y0.x + dt * (fd.x + fa.x), y0.y + dt * (fd.y + fa.y));
+    if (r == 0) rhs = make_double2(m == 0 ? 1.0 : 0.0, 0.0);
+    if (r == a.R - 1) rhs = make_double2(0.0, 0.0);
+    a.rhs_t[e] = rhs;
+  }
+  const double2 fd = sum(a.fdw, a.aD), fa = sum(a.faw, a.aA);
+  if (m == 0) {
+    const double y0 = a.u0[(size_t)r * a.B + c.b];
+    double rhs = y0 + dt * (fd.x + fa.x);
+    if (r == 0 || r == a.R - 1) rhs = 0.0;
+    a.rhs_w[e] = make_double2(rhs, 0.0);
+  } else {
+    const double2 fb = sum(a.buo, a.buo_imp ? a.aD : a.aA);
+    const double2 y0 = a.w0[e];
+    double2 rhs = make_double2(y0.x + dt * (fd.x + fa.x + fb.x), y0.y + dt * (fd.y + fa.y + fb.y));
+    if (r == 0 || r == a.R - 1) rhs = make_double2(0.0, 0.0);
+    a.rhs_w[e] = rhs;
   }
 }
 
 cudaError_t launch_stage_rhs(const StageArgs& a, cudaStream_t s) {
-  stage_rhs_kernel<<<ew_grid((size_t)a.R * a.M * a.B), 256, 0, s>>>(a);
+  const CellGrid c = cell_grid(a.R, a.M, a.B);
+  switch (a.st) {
+    case 1: stage_rhs_kernel<1><<<c.grid, c.block, 0, s>>>(a); break;
+    case 2: stage_rhs_kernel<2><<<c.grid, c.block, 0, s>>>(a); break;
+    case 3: stage_rhs_kernel<3><<<c.grid, c.block, 0, s>>>(a); break;
+    case 4: stage_rhs_kernel<4><<<c.grid, c.block, 0, s>>>(a); break;
+    default: stage_rhs_kernel<0><<<c.grid, c.block, 0, s>>>(a); break;
+  }
   return cudaGetLastError();
 }
 
 // Stage derivatives (RHS_construct_stage, src/fourierloop_imexrk.F90:403-497
 // with src/rhs_create_imexrk.F90): advective -N, diffusive L f, and the
 // stage-1 buoyancy.
-__global__ void stage_deriv_kernel(StageArgs a) {
-  const size_t total = (size_t)a.R * a.M * a.B;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total;
-       e += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(e % a.B);
-    const size_t rm = e / a.B;
-    const int m = (int)(rm % a.M);
-    const int r = (int)(rm / a.M);
-    const double ir = a.inv_r[r], ir2 = a.inv_r2[r];
-    const double dm = (double)m, mm = dm * dm;
-    {
-      const double2 p = a.ntp[e], q = a.ntr[e], dq = a.dntr[e];
-      a.fat_out[e] = make_double2(-(-dm * ir * p.y + dq.x + ir * q.x), -(dm * ir * p.x + dq.y + ir * q.y));
-      const double2 T = a.t[e], L = a.lt[e];
-      const double ip = a.inv_pr[b];
-      a.fdt_out[e] = make_double2(ip * (L.x - mm * ir2 * T.x), ip * (L.y - mm * ir2 * T.y));
-    }
-    if (m == 0) {
-      const size_t rb = (size_t)r * a.B + b;
-      a.faw_out[e] = make_double2(-a.nwr[e].x, 0.0);
-      const double u = a.up[e].x;
-      a.fdw_out[e] = make_double2(a.lu0[rb].x - ir2 * u, 0.0);
-    } else {
-      const double2 p = a.nwp[e], q = a.nwr[e], dq = a.dnwr[e];
-      a.faw_out[e] = make_double2(-(-dm * ir * p.y + dq.x + ir * q.x), -(dm * ir * p.x + dq.y + ir * q.y));
-      const double2 W = a.w[e], L = a.lw[e];
-      a.fdw_out[e] = make_double2(L.x - mm * ir2 * W.x, L.y - mm * ir2 * W.y);
-      if (a.buo_out) {
-        const double2 T = a.t[e];
-        const double f = dm * ir;
-        a.buo_out[e] = make_double2(a.ra_pr[b] * f * T.y, -a.ra_pr[b] * f * T.x);
-      }
+__global__ void stage_deriv_kernel(const __grid_constant__ StageArgs a) {
+  Cell c;
+  if (!cell_of(a.M, a.B, &c)) return;
+  const int r = c.r, m = c.m, b = c.b;
+  const size_t e = c.e;
+  const double ir = a.inv_r[r], ir2 = a.inv_r2[r];
+  const double dm = (double)m, mm = dm * dm;
+  const double2 T = a.t[e];
+  {
+    const double2 p = a.ntp[e], q = a.ntr[e], dq = a.dntr[e], L = a.lt[e];
+    a.fat_out[e] = make_double2(-(-dm * ir * p.y + dq.x + ir * q.x), -(dm * ir * p.x + dq.y + ir * q.y));
+    const double ip = a.inv_pr[b];
+    a.fdt_out[e] = make_double2(ip * (L.x - mm * ir2 * T.x), ip * (L.y - mm * ir2 * T.y));
+  }
+  if (m == 0) {
+    const size_t rb = (size_t)r * a.B + b;
+    a.faw_out[e] = make_double2(-a.nwr[e].x, 0.0);
+    const double u = a.up[e].x;
+    a.fdw_out[e] = make_double2(a.lu0[rb].x - ir2 * u, 0.0);
+  } else {
+    const double2 p = a.nwp[e], q = a.nwr[e], dq = a.dnwr[e], W = a.w[e], L = a.lw[e];
+    a.faw_out[e] = make_double2(-(-dm * ir * p.y + dq.x + ir * q.x), -(dm * ir * p.x + dq.y + ir * q.y));
+    a.fdw_out[e] = make_double2(L.x - mm * ir2 * W.x, L.y - mm * ir2 * W.y);
+    if (a.buo_out) {
+      const double f = dm * ir;
+      a.buo_out[e] = make_double2(a.ra_pr[b] * f * T.y, -a.ra_pr[b] * f * T.x);
     }
   }
 }
 
 cudaError_t launch_stage_deriv(const StageArgs& a, cudaStream_t s) {
-  stage_deriv_kernel<<<ew_grid((size_t)a.R * a.M * a.B), 256, 0, s>>>(a);
+  const CellGrid c = cell_grid(a.R, a.M, a.B);
+  stage_deriv_kernel<<<c.grid, c.block, 0, s>>>(a);
   return cudaGetLastError();
 }
 
