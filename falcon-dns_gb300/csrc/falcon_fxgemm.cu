@@ -3,19 +3,19 @@
 //
 // GB300's FP64 pipe takes 64 cycles per warp instruction and sub-partition,
 // its 32 x 32 + 64-bit multiply-add 5, so a product of two such numbers in
-// three of those (and one of 32 bits) is 4 times cheaper than an FMA.  An
-// operator row and an X column are taken as integers at the scale of their
-// largest element (|a| < 2^e: trunc(a 2^(bits - e)), 58 bits for A, 59 for X,
-// exact for elements within 2^5 of it), split as h 2^32 + l with l signed.
-// Per product
-//   ha hx 2^64 + (ha lx + la hx) 2^32 + (la >> 20)(lx >> 20) 2^40
-// is summed in three integers (64, 64 and 32 bits; |ha| <= 2^26, |hx| <= 2^27
-// and K <= 257 keep them exact: the middle one is carried into the first every
-// 16 k).  The low x low term's bits below 2^40 are left out: 2^-64 of the
-// largest product.  The sum is rounded once to FP64.  Sums of integers do not
-// depend on their order, so results depend neither on the tile nor on the
-// launch: the tile and the narrow kernel give the same bits.  A column (or
-// row) with an Inf or NaN gives NaN.
+// three of those is 4 times cheaper than an FMA.  An operator row and an X
+// column are taken as integers at the scale of their largest element (|a| <
+// 2^e: trunc(a 2^(bits - e)), 58 bits for A, 59 for X, exact for elements
+// within 2^5 of it), split as h 2^31 + l with l signed.  Per product
+//   ha hx 2^62 + (ha lx + la hx) 2^31
+// is summed in two 64-bit integers (|ha| <= 2^27, |hx| <= 2^28, half that past
+// K = 255, and K <= 257 keep them exact: the second is carried into the first
+// every 16 k).  la lx is left out: 2^-57 of the largest product at most, about
+// what the operands' truncation leaves out (a fourth multiply-add for its upper
+// bits took 129 x 129 x 11040 columns from 119 to 129 us).  The sum is rounded
+// once to FP64.  Sums of integers do not depend on their order, so results
+// depend neither on the tile nor on the launch: the tile and the narrow kernel
+// give the same bits.  A column (or row) with an Inf or NaN gives NaN.
 //
 // The solve operators weigh a right-hand side's rows very differently (near
 // the walls by the square of the grid spacing), and the right-hand sides are
@@ -24,11 +24,10 @@
 // neither operand's large elements push the other's out of the 58 bits.
 //
 // Bound: latency for the narrow forms (the radial and per-mode products of a
-// few instances), the integer pipes for the tiles (13 or so instructions per
-// product, issue 55 %).  Against FP64 FMA, us with L2 cold: 97 x 97, 342 modes,
-// 2 columns 44 -> 22; 33 x 33, 43 modes, 2 columns 14 -> 8; 65 x 65, 688
-// columns 22 -> 11; 65 x 65, 43776 columns 316 -> 119 (85 on tcgen05, which
-// the autotuner takes there).
+// few instances), the integer multiply-add pipe for the tiles.  Against FP64
+// FMA, us with L2 cold: 97 x 97, 342 modes, 2 columns 44 -> 17; 33 x 33, 43
+// modes, 2 columns 14 -> 8; 65 x 65, 688 columns 22 -> 11; 65 x 65, 43776 columns
+// 316 -> 111 (84 on tcgen05, which the autotuner takes there).
 //
 // The operators' integers are made once per operator set
 // (launch_fx_operator); X is converted by each block for its own columns.
@@ -59,7 +58,7 @@ __device__ __forceinline__ int exponent_of(double a, int w) {
   return (int)max(high >> 20, 1u) - 1022 + w;
 }
 __device__ __forceinline__ int2 signed_split(unsigned long long t) {
-  return make_int2((int)((unsigned)(t >> 32) + ((unsigned)t >> 31)), (int)t);
+  return make_int2((int)((long long)t >> 31) + (int)((unsigned)t >> 30 & 1), (int)((unsigned)t << 1) >> 1);
 }
 // trunc(a 2^w 2^(bits - e)) split into (h, l signed)
 template <int BITS>
@@ -75,11 +74,10 @@ __device__ __forceinline__ int mark_of(int m) { return m == INT32_MAX ? kBad : s
 
 struct Sum {
   long long hh, mid;
-  int ll;
 };
 // a b + c as one instruction (a product and a 64-bit add on two pipes, as the
-// compiler makes of mad.wide, takes 10 % longer here: 131 against 119 us for
-// 65 x 65 x 43776)
+// compiler makes of mad.wide, took 131 us for 65 x 65 x 43776 where this took
+// 119, with a fourth multiply-add per product)
 __device__ __forceinline__ long long madw1(int a, int b, long long c) {
   long long r;
   asm("{\n\t.reg .u32 lo, hi;\n\tmov.b64 {lo, hi}, %3;\n\tmad.lo.cc.s32 lo, %1, %2, lo;\n\t"
@@ -88,26 +86,24 @@ __device__ __forceinline__ long long madw1(int a, int b, long long c) {
       : "r"(a), "r"(b), "l"(c));
   return r;
 }
-__device__ __forceinline__ void add_product(Sum& s, int2 a, int2 x, int a12, int x12) {
+__device__ __forceinline__ void add_product(Sum& s, int2 a, int2 x) {
   s.hh = madw1(a.x, x.x, s.hh);
   s.mid = madw1(a.x, x.y, s.mid);
   s.mid = madw1(a.y, x.x, s.mid);
-  s.ll += a12 * x12;
 }
 __device__ __forceinline__ void carry(Sum& s) {
-  s.hh += s.mid >> 32;
-  s.mid = (long long)(unsigned)s.mid;
+  s.hh += s.mid >> 31;
+  s.mid &= 0x7fffffff;
 }
-// RN of the sum times 2^(ea + ex): (hh 2^32 + mid + ll 2^8) 2^32 in units of
+// RN of the sum times 2^(ea + ex): (hh 2^31 + mid) 2^31 in units of
 // 2^(ea + ex - kBitsA - kBitsX)
 __device__ __forceinline__ double value_of(Sum s, int ea, int ex, double alpha) {
   if (ea == kBad || ex == kBad) return __longlong_as_double(0x7ff8000000000000LL);
-  s.mid += (long long)s.ll * 256;
   carry(s);
   // the leading 64 bits
-  const int sh = min(__clzll(s.hh ^ (s.hh >> 63)) - 1, 32);
-  const long long v = (s.hh << sh) + (long long)(((unsigned long long)s.mid << sh) >> 32);
-  const int e = ea + ex - kBitsA - kBitsX + 64 - sh;
+  const int sh = min(__clzll(s.hh ^ (s.hh >> 63)) - 1, 31);
+  const long long v = (s.hh << sh) + (long long)((unsigned long long)(s.mid << sh) >> 31);
+  const int e = ea + ex - kBitsA - kBitsX + 62 - sh;
   double y = (double)v;
   if (v) {
     const int top = ((__double2hiint(y) >> 20) & 0x7ff) + e;
@@ -279,10 +275,10 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   issue(0, as);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  convert_panel(xs, g.K, NCOL, w, cex, part);
+  convert_panel(xs, g.K, NCOL, w, cex, part, g.K > 255);
   Sum acc[RPT][2];
 #pragma unroll
-  for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = Sum{0, 0, 0};
+  for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = Sum{0, 0};
   int cur = 0;
   for (int k0 = 0; k0 < g.K; k0 += kFxKC) {
     const int kc = min(kFxKC, g.K - k0);
@@ -298,13 +294,11 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
     auto one = [&](int kk) {
       const int4 xv = Xw[kk * (NCOL / 2)];
       const int2 x0 = make_int2(xv.x, xv.y), x1 = make_int2(xv.z, xv.w);
-      const int x012 = x0.y >> 20, x112 = x1.y >> 20;
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         const int2 av = Aw[kk * rows_blk + i];
-        const int a12 = av.y >> 20;
-        add_product(acc[i][0], av, x0, a12, x012);
-        add_product(acc[i][1], av, x1, a12, x112);
+        add_product(acc[i][0], av, x0);
+        add_product(acc[i][1], av, x1);
       }
     };
     if (kc == kFxKC) {
@@ -352,12 +346,10 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
 // sums meet in shared memory, where the threads of a row take its column pairs.
 // Bound by latency for one small run, then by issue.  With 32 rows and eight
 // shares in every block two thirds of the instructions were for converting X
-// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 57 us, 291 x 97 x 6 256 ->
-// 125, 291 x 97 x 2, 341 entries 40 -> 31, 195 x 65 x 8, 170 entries 32 -> 24.
+// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 52 us, 291 x 97 x 6 256 ->
+// 113, 291 x 97 x 2, 341 entries 40 -> 30, 195 x 65 x 8, 170 entries 32 -> 22.
 struct alignas(16) Part {
-  long long hh;
-  unsigned mid;
-  int ll;
+  long long hh, mid;
 };
 template <int NC>
 __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ GemmArgs g, int RB, int KS) {
@@ -401,11 +393,11 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     xd[i] = c < N ? X[(size_t)k * ldx + c] : 0.0;
   }
   __syncthreads();
-  convert_panel(xd, g.K, NC, w, cex, part);
+  convert_panel(xd, g.K, NC, w, cex, part, g.K > 255);
   const int2* xs = reinterpret_cast<const int2*>(xd);
   Sum acc[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = Sum{0, 0, 0};
+  for (int c = 0; c < NC; ++c) acc[c] = Sum{0, 0};
   for (int k0 = kb; k0 < ke; k0 += U) {
     int2 nv[U];
 #pragma unroll
@@ -413,13 +405,12 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       if (k0 + u >= ke) break;
-      const int a12 = av[u].y >> 20;
       const int4* xp = reinterpret_cast<const int4*>(xs + (k0 + u) * NC);
 #pragma unroll
       for (int c = 0; c < NC; c += 2) {
         const int4 x = xp[c / 2];
-        add_product(acc[c], av[u], make_int2(x.x, x.y), a12, x.y >> 20);
-        add_product(acc[c + 1], av[u], make_int2(x.z, x.w), a12, x.w >> 20);
+        add_product(acc[c], av[u], make_int2(x.x, x.y));
+        add_product(acc[c + 1], av[u], make_int2(x.z, x.w));
       }
     }
 #pragma unroll
@@ -428,17 +419,16 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     for (int u = 0; u < U; ++u) av[u] = nv[u];
   }
 #pragma unroll
-  for (int c = 0; c < NC; ++c) parts[(kp * NC + c) * RB + rl] = Part{acc[c].hh, (unsigned)acc[c].mid, acc[c].ll};
+  for (int c = 0; c < NC; ++c) parts[(kp * NC + c) * RB + rl] = Part{acc[c].hh, acc[c].mid};
   if (g.follow.kind) follow_modes(g.follow);
   __syncthreads();
   if (row >= g.rows) return;
   auto column = [&](int c) {
-    Sum s{0, 0, 0};
+    Sum s{0, 0};
     for (int q = 0; q < KS; ++q) {
       const Part p = parts[(q * NC + c) * RB + rl];
       s.hh += p.hh;
       s.mid += p.mid;
-      s.ll += p.ll;
     }
     return value_of(s, aex[row], cex[c], g.alpha);
   };
@@ -461,13 +451,13 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
 // hold half the products of the dense operator.  What the mirrored half
 // differs by (the rounding of its own cosines, 2^-40 of an element) is a
 // third sum of one 32-bit product each, D = sum (26 bits of the difference)
-// (27 bits of x), added at its scale: outputs are those of the dense operator.
+// (28 bits of x), added at its scale: outputs are those of the dense operator.
 //   FWD: X0, X1 = x_p +- x_{n-1-p};  out_{2j} = S0 + D0, out_{2j+1} = S1 + D1
 //   else X0, X1 = x_{2p}, x_{2p+1};  out_j = S0 + S1, out_{n-1-j} = +-(S0 - S1) + D
 // A block takes NCOL real columns (re and im side by side) of one operator;
 // loads, outputs (through shared memory) and the operator's chunks of 8 p are
 // coalesced.  Bound: the integer multiply-adds (61 % of that pipe's cycles, 16
-// to 20 warps an SM); 65 points, 10944 columns: fwd 56 us, d1 and d2 102 us
+// to 20 warps an SM); 65 points, 10944 columns: fwd 56 us, d1 and d2 93 us
 // (one FP64 dot product a thread: 684 us for the three).
 constexpr int kFxPC = 8;  // p per staged operator chunk
 template <int RPT, int NCOL, bool FWD>
@@ -501,13 +491,13 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   issue(0, 0);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  convert_panel<ST - NCOL>(xs, n, NCOL, op.w, cex, part, FWD ? 1 : 0);
+  convert_panel<ST - NCOL>(xs, n, NCOL, op.w, cex, part, FWD || n > 255);
   if (FWD) {
     for (int i = threadIdx.x; i < n / 2 * NCOL; i += nthr) {
       const int p = i / NCOL, c = i - p * NCOL;
       int2* a = reinterpret_cast<int2*>(xs) + p * ST + c;
       int2* b = reinterpret_cast<int2*>(xs) + (n - 1 - p) * ST + c;
-      const long long va = (long long)a->x * 4294967296LL + a->y, vb = (long long)b->x * 4294967296LL + b->y;
+      const long long va = (long long)a->x * 2147483648LL + a->y, vb = (long long)b->x * 2147483648LL + b->y;
       *a = signed_split(va + vb);
       *b = signed_split(va - vb);
     }
@@ -519,7 +509,7 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   for (int i = 0; i < RPT; ++i)
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      s0[i][c] = s1[i][c] = Sum{0, 0, 0};
+      s0[i][c] = s1[i][c] = Sum{0, 0};
       d0[i][c] = d1[i][c] = 0;
     }
   int cur = 0;
@@ -540,18 +530,16 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
       const int p = p0 + pp;
       const int4 u = xp[(FWD ? p : 2 * p) * (ST / 2)], v = xp[(FWD ? n - 1 - p : 2 * p + 1) * (ST / 2)];
       const int2 u0 = make_int2(u.x, u.y), u1 = make_int2(u.z, u.w), v0 = make_int2(v.x, v.y), v1 = make_int2(v.z, v.w);
-      const int u012 = u0.y >> 20, u112 = u1.y >> 20, v012 = v0.y >> 20, v112 = v1.y >> 20;
       const int m0 = FWD ? (u0.x - v0.x) >> 1 : 0, m1 = FWD ? (u1.x - v1.x) >> 1 : 0;  // x_{n-1-p}
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         const int4 a = Aw[pp * hb + i];
         const int2 d = Dw[pp * hb + i];
         const int2 a0 = make_int2(a.x, a.y), a1 = make_int2(a.z, a.w);
-        const int a012 = a0.y >> 20, a112 = a1.y >> 20;
-        add_product(s0[i][0], a0, u0, a012, u012);
-        add_product(s0[i][1], a0, u1, a012, u112);
-        add_product(s1[i][0], a1, v0, a112, v012);
-        add_product(s1[i][1], a1, v1, a112, v112);
+        add_product(s0[i][0], a0, u0);
+        add_product(s0[i][1], a0, u1);
+        add_product(s1[i][0], a1, v0);
+        add_product(s1[i][1], a1, v1);
         if (FWD) {
           d0[i][0] = madw1(d.x, m0, d0[i][0]);
           d0[i][1] = madw1(d.x, m1, d0[i][1]);
@@ -582,11 +570,11 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
       const Sum a = s0[i][c], b = s1[i][c];
       Sum f, m;
       if (FWD) {
-        f = Sum{a.hh, a.mid + (d0[i][c] >> e.z), a.ll};
-        m = Sum{b.hh, b.mid + (d1[i][c] >> e.w), b.ll};
+        f = Sum{a.hh, a.mid + (d0[i][c] >> e.z)};
+        m = Sum{b.hh, b.mid + (d1[i][c] >> e.w)};
       } else {
-        f = Sum{a.hh + b.hh, a.mid + b.mid, a.ll + b.ll};
-        m = op.sign > 0 ? Sum{a.hh - b.hh, a.mid - b.mid, a.ll - b.ll} : Sum{b.hh - a.hh, b.mid - a.mid, b.ll - a.ll};
+        f = Sum{a.hh + b.hh, a.mid + b.mid};
+        m = op.sign > 0 ? Sum{a.hh - b.hh, a.mid - b.mid} : Sum{b.hh - a.hh, b.mid - a.mid};
         m.mid += d0[i][c] >> e.z;
       }
       y[c] = value_of(f, e.x, cex[2 * cp + c], 1.0);
@@ -665,7 +653,7 @@ TileShape pick_shape(const GemmArgs& g, int nsm) {
     const long cb = column_blocks(g, ncol) * entries(g);
     for (int rb = 1; rb <= 16; ++rb)
       for (int nw = 4; nw <= 16; ++nw)
-        for (int rpt = 1; rpt <= 8; ++rpt) {
+        for (int rpt = 1; rpt <= 7; ++rpt) {
           const int rows_blk = nw * rg * rpt;
           if ((long)rb * rows_blk < g.rows || (long)(rb - 1) * rows_blk >= g.rows || rows_blk > 256) continue;
           const long smem = ((long)g.K * ncol + 2 * kFxKC * rows_blk) * 8 + (ncol + 32 * nw) * 4;
@@ -694,8 +682,7 @@ cudaError_t launch_ncol(const GemmArgs& g, const TileShape& t, cudaStream_t s) {
     case 4: return launch_fx_tile<4, NCOL>(g, t.nw, t.rb, s);
     case 5: return launch_fx_tile<5, NCOL>(g, t.nw, t.rb, s);
     case 6: return launch_fx_tile<6, NCOL>(g, t.nw, t.rb, s);
-    case 7: return launch_fx_tile<7, NCOL>(g, t.nw, t.rb, s);
-    default: return launch_fx_tile<8, NCOL>(g, t.nw, t.rb, s);
+    default: return launch_fx_tile<7, NCOL>(g, t.nw, t.rb, s);
   }
 }
 
@@ -742,8 +729,8 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.N <= 8 && !g.njobs) {
     // k shares until there are 448 threads an SM (one share above that), rows
     // in even blocks of at most 256 threads, of fewer while SMs are without two
-    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.9, 7.9, 7.8; 65 x 65 x 8,
-    // 171 entries 22.5, 18.1, 16.0, 18.0; 291 x 97 x 2, 341 entries 31.0, 32.4, 36.5, 46.8)
+    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.0, 7.8, 7.8; 65 x 65 x 8,
+    // 171 entries 21.2, 17.0, 14.0, 18.1; 291 x 97 x 2, 341 entries 30.3, 32.4, 34.4, 44.7)
     const int nz = entries(g);
     const int KS = (int)std::min(8L, std::max(1L, 152L * 448 / ((long)g.rows * nz)));
     int nb = (g.rows + 256 / KS - 1) / (256 / KS);
@@ -773,11 +760,11 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
 // Shape: NCOL real columns a block, RPT output pairs a thread (64 / NCOL x RPT
 // pairs a warp).  Few columns: small blocks and one pair a thread, for more
 // blocks and shorter chains (65 points, us of fwd / d1d2 at <1, 8>, <1, 16>, <3, 16>:
-// 300 columns 11.1/10.8, 12.7/12.5, 16.6/17.2; 1000 columns 14.5/20.5, 12.7/17.3,
-// 16.7/20.8; 10944 columns 67/117, 62/107, 56/102).  Many: one pair a thread
-// up to 32 pairs (33 points, 20000 columns <1, 32> 39/64, <3, 16> 41/72), above
-// that the shape that pads least (97 points, 10000 columns <2, 16> 113/195,
-// <3, 16> 134/243; 129 points, 2000 columns <3, 32> 41/77, <3, 16> 48/89).
+// 300 columns 10.9/11.1, 12.5/11.6, 16.6/16.6; 1000 columns 12.9/19.3, 12.5/17.1,
+// 16.6/19.2; 10944 columns 64/113, 60/103, 56/93).  Many: one pair a thread
+// up to 32 pairs (17 points, 20000 columns <1, 32> 17/27, <3, 16> 29/48), above
+// that the shape that pads least (97 points, 10000 columns <2, 16> 109/183,
+// <3, 16> 133/215; 129 points, 2000 columns <3, 32> 40/71, <3, 16> 48/80).
 cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s) {
   if (g.n < 3 || g.n > 257 || g.ncol < 1 || g.ncol > 65535) return cudaErrorInvalidValue;
   const int h = (g.n + 1) / 2;

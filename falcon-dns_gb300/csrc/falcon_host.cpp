@@ -4269,9 +4269,9 @@ struct ChebMats {
 std::mutex g_cheb_mu;
 std::map<int, ChebMats> g_cheb;
 
-int2 fx_split(double a, int bits, int e) {  // trunc(a 2^(bits - e)) as h 2^32 + l, l signed
+int2 fx_split(double a, int bits, int e) {  // trunc(a 2^(bits - e)) as h 2^31 + l, l signed
   const unsigned long long t = (unsigned long long)(long long)std::ldexp(a, bits - e);
-  return make_int2((int)((unsigned)(t >> 32) + ((unsigned)t >> 31)), (int)t);
+  return make_int2((int)((long long)t >> 31) + (int)((unsigned)t >> 30 & 1), (int)((unsigned)t << 1) >> 1);
 }
 
 // An operator in the form of fx_columns_kernel (falcon_fxgemm.cu).  Rows i and

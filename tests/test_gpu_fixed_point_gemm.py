@@ -5,8 +5,8 @@ batch sizes around their column tiles.
 
 - an instance's bits do not depend on the batch it steps in (the narrow
   kernel alone, tiles of every width in batches: sums of integers);
-- against the exact bf16 slices on mma.sync (mode 1).  Both keep 58 or more
-  bits of an operand relative to the largest of its row or column, so a
+- against the exact bf16 slices on mma.sync (mode 1).  Both keep 57 or more
+  bits of a product relative to the largest of its row or column, so a
   contraction's outputs differ by at most sqrt(2 K) 2^-57 max|A| max|X|, the
   rounding of an FP64 product sum (K = 131: 2^-53); steps amplify a rounding
   by the operators' condition, 1e-12 over 20 steps at Nr = 65 for FP64 tiles,
