@@ -727,12 +727,12 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.rows <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
   if (g.K > 257 || !g.fx) return cudaErrorInvalidValue;
   if (g.N <= 8 && !g.njobs) {
-    // k shares until there are 448 threads an SM (one share above that), rows
+    // k shares until there are 448 threads an SM (above that one, a warp at least), rows
     // in even blocks of at most 256 threads, of fewer while SMs are without two
     // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.0, 7.8, 7.8; 65 x 65 x 8,
     // 171 entries 21.2, 17.0, 14.0, 18.1; 291 x 97 x 2, 341 entries 30.3, 32.4, 34.4, 44.7)
     const int nz = entries(g);
-    const int KS = (int)std::min(8L, std::max(1L, 152L * 448 / ((long)g.rows * nz)));
+    const int KS = (int)std::min(8L, std::max((31L + g.rows) / g.rows, 152L * 448 / ((long)g.rows * nz)));
     int nb = (g.rows + 256 / KS - 1) / (256 / KS);
     while ((long)nb * nz < 2 * 152 && (g.rows + nb - 1) / nb > 16) ++nb;
     const int RB = (g.rows + nb - 1) / nb;
