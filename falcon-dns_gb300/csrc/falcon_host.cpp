@@ -1052,12 +1052,16 @@ struct Group {
   // the autotuner, which measures only outside capture): set when the
   // captured steps are dropped.
   bool direct_next = false;
+  bool dropped = false;        // after a step: this group changes
+  std::vector<int> visited;    // phases run directly once since then
   void drop_graphs() {
     // a step launched from one of these graphs may still run on the stream
     if (stream && !graphs.empty()) cudaStreamSynchronize(stream);
     for (auto& sg : graphs) cudaGraphExecDestroy(sg.exec);
     graphs.clear();
+    visited.clear();
     direct_next = true;
+    dropped = dropped || n_step > 0;
   }
   ~Group() {
     // work queued on the stream may still read or write the arrays
@@ -2485,8 +2489,12 @@ void group_advance(Group* g) {
 
 // One time step.  From the second step on, the launch sequence of a step is
 // fixed up to the ring-buffer phase, so each phase is captured once into a
-// CUDA graph and replayed: one launch instead of 11 (IMEX) to ~60 (IMEXRK)
-// kernel launches, which lets many small groups keep the GPU busy.
+// CUDA graph and replayed: one launch instead of 5 (IMEX) to ~60 (IMEXRK)
+// kernel launches, which lets many small groups keep the GPU busy.  In a group
+// whose graphs were dropped once (its columns change) a phase is captured when it
+// comes round again: making a graph takes as long as some ten direct steps, and
+// a served group whose members leave every two or three steps captured graphs
+// that it never replayed (a burst of 16 requests 15.6 -> 14.7 ms).
 int group_step(Group* g) {
   // upFR_prev = upFR at the start of a run (src/init.F90:253); the IMEX
   // loop renews it every step after the nonlinear pass (in imex_rhs_kernel),
@@ -2505,6 +2513,10 @@ int group_step(Group* g) {
       group_advance(g);
       return 0;
     }
+  if (g->dropped && std::find(g->visited.begin(), g->visited.end(), phase) == g->visited.end()) {
+    g->visited.push_back(phase);
+    return group_step_direct(g);
+  }
   const long long before = g_launches.load();
   CK(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
   const int rc = group_step_direct(g);  // advances the host state once
