@@ -1,27 +1,35 @@
-// Operator contractions Y = alpha A X in 59-bit fixed point on integer
+// Operator contractions Y = alpha A X in 60-bit fixed point on integer
 // multiply-adds.
 //
 // GB300's FP64 pipe takes 64 cycles per warp instruction and sub-partition,
 // its 32 x 32 + 64-bit multiply-add 5, so a product of two such numbers in
 // three of those is 4 times cheaper than an FMA.  An operator row and an X
 // column are taken as integers at the scale of their largest element (|a| <
-// 2^e: trunc(a 2^(bits - e)), 58 bits for A, 59 for X, exact for elements
-// within 2^5 of it), split as h 2^31 + l with l signed.  Per product
-//   ha hx 2^62 + (ha lx + la hx) 2^31
-// is summed in two 64-bit integers (|ha| <= 2^27, |hx| <= 2^28, half that past
-// K = 255, and K <= 257 keep them exact: the second is carried into the first
-// every 16 k).  la lx is left out: 2^-57 of the largest product at most, about
-// what the operands' truncation leaves out (a fourth multiply-add for its upper
-// bits took 129 x 129 x 11040 columns from 119 to 129 us).  The sum is rounded
-// once to FP64.  Sums of integers do not depend on their order, so results
-// depend neither on the tile nor on the launch: the tile and the narrow kernel
-// give the same bits.  A column (or row) with an Inf or NaN gives NaN.
+// 2^e: a 2^(60 - e) rounded, exact for elements within 2^7 of it), split as h
+// 2^30 + l with l signed.  Per product
+//   ha hx 2^60 + (ha lx + la hx) 2^30
+// is summed in two 64-bit integers and a word for the first one's carries
+// (|h| <= 2^30 and |l| <= 2^29: exact for 4 products between carries).  la lx is
+// left out: 2^-62 of the largest product at most, what the operands' rounding
+// leaves out.  The sum is rounded once to FP64.  Sums of integers do not depend
+// on their order, so results depend neither on the tile nor on the launch: the
+// tile and the narrow kernel give the same bits.  A column (or row) with an Inf
+// or NaN gives NaN.
 //
-// The solve operators weigh a right-hand side's rows very differently (near
-// the walls by the square of the grid spacing), and the right-hand sides are
-// large where the weights are small: their columns are divided by powers of
-// two 2^w_k (the largest element's exponent), X's rows multiplied, so that
-// neither operand's large elements push the other's out of the 58 bits.
+// Operators weigh the rows of X very differently: the radial derivatives and
+// their products with a field are largest at the walls (by n^2 for d/dr, n^4
+// for the Laplacian), the solve operators smallest, where their right-hand sides
+// are largest.  With one scale for a row the small elements, which meet the
+// large values of fields that vanish at the walls, lose their digits; with
+// columns divided by their largest element and X's rows multiplied, X's values
+// away from the walls lose theirs.  So columns are divided by 2^w_k, w_k half the
+// largest element's exponent, and the spread is shared.
+//
+// Errors over the norm of a column's output against 64 bits (FP64 sums, this
+// form; a form of 58 x 59 bits, truncated, with weights of 0 for the derivatives
+// and 1 for the solves): d/dr of (1 - x^2)^2 f(x), 129 points, 1.2e-15, 1.4e-16
+// (3e-14); the Laplacian of f(x) 2e-11, 1e-12 (3e-11), of (1 - x^2)^2 f(x) 8e-14,
+// 6e-14 (3e-11); the vorticity solve of a run 5.7e-16, 1.3e-16 (2.7e-16).
 //
 // Bound: latency for the narrow forms (the radial and per-mode products of a
 // few instances), the integer multiply-add pipe for the tiles.  Against FP64
@@ -44,7 +52,8 @@
 namespace falcon {
 namespace {
 
-constexpr int kBitsA = 58, kBitsX = 59;  // of a row's and a column's integers
+constexpr int kBits = 60, kLow = 30;      // of a row's and a column's integers, of their low halves
+constexpr int kCarry = 4;                 // products between carries
 constexpr int kFollowRows = 6;           // deepest tiles that do what follows a product (deeper ones would spill)
 constexpr int kFxKC = 16;                // k per staged operator chunk
 constexpr int kBad = INT32_MIN;          // exponent of a row or column with an Inf or NaN
@@ -58,13 +67,16 @@ __device__ __forceinline__ int exponent_of(double a, int w) {
   return (int)max(high >> 20, 1u) - 1022 + w;
 }
 __device__ __forceinline__ int2 signed_split(unsigned long long t) {
-  return make_int2((int)((long long)t >> 31) + (int)((unsigned)t >> 30 & 1), (int)((unsigned)t << 1) >> 1);
+  return make_int2((int)((long long)t >> kLow) + (int)((unsigned)t >> (kLow - 1) & 1),
+                   (int)((unsigned)t << (32 - kLow)) >> (32 - kLow));
 }
-// trunc(a 2^w 2^(bits - e)) split into (h, l signed)
-template <int BITS>
+// a 2^w 2^(kBits - e) rounded, split into (h, l signed)
 __device__ __forceinline__ int2 split_of(double a, int w, int e) {
   const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
-  unsigned long long t = fx_mag_of(bits, e - w + 1022) >> (59 - BITS);
+  const int eb = (int)(bits >> 52) & 0x7ff;
+  const unsigned long long m = ((bits & 0xfffffffffffffULL) | (eb ? 1ULL << 52 : 0ULL)) << (kBits - 53);
+  const unsigned sh = min((unsigned)(e - w + 1022 - max(eb, 1)), kBits + 1u);  // (negative only for a zero)
+  unsigned long long t = (m + (1ULL << sh >> 1)) >> sh;
   if ((long long)bits < 0) t = 0ull - t;
   return signed_split(t);
 }
@@ -73,6 +85,7 @@ __device__ __forceinline__ int scale_of(int m) { return m == INT32_MAX ? 100000 
 __device__ __forceinline__ int mark_of(int m) { return m == INT32_MAX ? kBad : scale_of(m); }
 
 struct Sum {
+  int top;  // top 2^40 + hh
   long long hh, mid;
 };
 // a b + c as one instruction (a product and a 64-bit add on two pipes, as the
@@ -92,18 +105,39 @@ __device__ __forceinline__ void add_product(Sum& s, int2 a, int2 x) {
   s.mid = madw1(a.y, x.x, s.mid);
 }
 __device__ __forceinline__ void carry(Sum& s) {
-  s.hh += s.mid >> 31;
-  s.mid &= 0x7fffffff;
+  s.hh += s.mid >> kLow;
+  s.mid &= (1 << kLow) - 1;
+  s.top += (int)(s.hh >> 40);
+  s.hh &= (1LL << 40) - 1;
 }
-// RN of the sum times 2^(ea + ex): (hh 2^31 + mid) 2^31 in units of
-// 2^(ea + ex - kBitsA - kBitsX)
-__device__ __forceinline__ double value_of(Sum s, int ea, int ex, double alpha) {
-  if (ea == kBad || ex == kBad) return __longlong_as_double(0x7ff8000000000000LL);
+// A sum as hi 2^64 + lo, in units of 2^(kLow - 2 kBits) of the scales.
+struct alignas(16) Wide {
+  long long hi;
+  unsigned long long lo;
+};
+__device__ __forceinline__ Wide wide_of(Sum s) {
   carry(s);
-  // the leading 64 bits
-  const int sh = min(__clzll(s.hh ^ (s.hh >> 63)) - 1, 31);
-  const long long v = (s.hh << sh) + (long long)((unsigned long long)(s.mid << sh) >> 31);
-  const int e = ea + ex - kBitsA - kBitsX + 62 - sh;
+  return {((long long)s.top << (40 + kLow - 64)) + (s.hh >> (64 - kLow)),
+          ((unsigned long long)s.hh << kLow) | (unsigned long long)s.mid};
+}
+__device__ __forceinline__ Wide add(Wide a, Wide b) {
+  const unsigned long long lo = a.lo + b.lo;
+  return {a.hi + b.hi + (lo < b.lo), lo};
+}
+__device__ __forceinline__ Wide sub(Wide a, Wide b) {
+  return {a.hi - b.hi - (a.lo < b.lo), a.lo - b.lo};
+}
+__device__ __forceinline__ Wide add(Wide a, long long b) { return add(a, Wide{b >> 63, (unsigned long long)b}); }
+// RN of the sum times 2^(ea + ex)
+__device__ __forceinline__ double value_of(Wide s, int ea, int ex, double alpha) {
+  if (ea == kBad || ex == kBad) return __longlong_as_double(0x7ff8000000000000LL);
+  long long v = (long long)s.lo;
+  int e = ea + ex + kLow - 2 * kBits;
+  if (s.hi != v >> 63) {  // the leading 64 bits, and whether others are set
+    const int up = __clzll(s.hi ^ (s.hi >> 63)) - 1;
+    v = (s.hi << up) | (long long)(s.lo >> (64 - up)) | (long long)((s.lo << up) != 0);
+    e += 64 - up;
+  }
   double y = (double)v;
   if (v) {
     const int top = ((__double2hiint(y) >> 20) & 0x7ff) + e;
@@ -143,7 +177,7 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-// One thread per (entry, column k): the exponent of its largest element.
+// One thread per (entry, column k): half the exponent of its largest element.
 __global__ void fx_weight_kernel(const double* A, long lda, long sA, int rows, int K, int nb, int* wk) {
   const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
   if (t >= (long)nb * K) return;
@@ -154,7 +188,7 @@ __global__ void fx_weight_kernel(const double* A, long lda, long sA, int rows, i
     const int e = exponent_of(a[r], 0);
     if (e != INT32_MAX) m = max(m, e);
   }
-  wk[t] = m == kNone ? 0 : m;
+  wk[t] = m == kNone ? 0 : m >> 1;
 }
 
 // One thread per (entry, row): the row's exponent, then its integers, in the
@@ -165,17 +199,17 @@ __global__ void fx_operator_kernel(const double* A, long lda, long sA, int rows,
   if (t >= (long)nb * rows) return;
   const int z = (int)(t / rows), r = (int)(t - (long)z * rows);
   const double* a = A + (size_t)z * sA + r;
-  const int* w = wk ? wk + (size_t)z * K : nullptr;
+  const int* w = wk + (size_t)z * K;
   int m = kNone;
-  for (int k = 0; k < K; ++k) m = max(m, exponent_of(a[(size_t)k * lda], w ? -w[k] : 0));
+  for (int k = 0; k < K; ++k) m = max(m, exponent_of(a[(size_t)k * lda], -w[k]));
   ex[(size_t)z * lda + r] = mark_of(m);
   int2* o = out + (size_t)z * sA + r;
-  for (int k = 0; k < K; ++k) o[(size_t)k * lda] = split_of<kBitsA>(a[(size_t)k * lda], w ? -w[k] : 0, scale_of(m));
+  for (int k = 0; k < K; ++k) o[(size_t)k * lda] = split_of(a[(size_t)k * lda], -w[k], scale_of(m));
 }
 
 // X panel of a block in shared memory, xs[k * (ncol + PAD) + c] (staged as
 // doubles, complete when this is called): column exponents in cex, integers in
-// place.  w: the operator's weights (or null); part: blockDim.x words; spare:
+// place.  w: the operator's weights (or null: fwd); part: blockDim.x words; spare:
 // leading bits left free.
 template <int PAD = 0>
 __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const int* w, int* cex, int* part,
@@ -193,7 +227,7 @@ __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const
     if (m != INT32_MAX && m != kNone) m += spare;
     if (j == 0) cex[c] = mark_of(m);
     for (int k = j; k < K; k += J) {
-      const int2 v = split_of<kBitsX>(xs[k * st + c], w ? __ldg(w + k) : 0, scale_of(m));
+      const int2 v = split_of(xs[k * st + c], w ? __ldg(w + k) : 0, scale_of(m));
       reinterpret_cast<int2*>(xs)[k * st + c] = v;
     }
   }
@@ -221,7 +255,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   long lda = g.lda, ldx = g.ldx, ldy = g.ldy;
   const int2* A = g.fx + (size_t)z * g.sA;
   const int* aex = g.fx_ex + (size_t)z * g.lda;
-  const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
+  const int* w = g.fx_w + (size_t)z * g.K;
   const double* X = g.X + (size_t)z * g.sX;
   double* Y = nullptr;
   if (g.njobs || g.nsub || z >= nz) {
@@ -242,7 +276,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
     ldy = q.ldy;
     A = q.fx + (size_t)e * g.sA;
     aex = q.fx_ex + (size_t)e * lda;
-    w = q.fx_w ? q.fx_w + (size_t)e * g.K : nullptr;
+    w = q.fx_w + (size_t)e * g.K;
     X = q.X + (size_t)e * g.sX;
     Y = q.Y + (size_t)e * g.sY;
     b0 = q.b0;
@@ -275,10 +309,10 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   issue(0, as);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  convert_panel(xs, g.K, NCOL, w, cex, part, g.K > 255);
+  convert_panel(xs, g.K, NCOL, w, cex, part);
   Sum acc[RPT][2];
 #pragma unroll
-  for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = Sum{0, 0};
+  for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = Sum{0, 0, 0};
   int cur = 0;
   for (int k0 = 0; k0 < g.K; k0 += kFxKC) {
     const int kc = min(kFxKC, g.K - k0);
@@ -301,14 +335,16 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
         add_product(acc[i][1], av, x1);
       }
     };
-    if (kc == kFxKC) {
-#pragma unroll 4
-      for (int kk = 0; kk < kFxKC; ++kk) one(kk);
-    } else {
-      for (int kk = 0; kk < kc; ++kk) one(kk);
-    }
+    for (int k4 = 0; k4 < kc; k4 += kCarry) {
+      if (kc - k4 >= kCarry) {
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) { carry(acc[i][0]); carry(acc[i][1]); }
+        for (int kk = 0; kk < kCarry; ++kk) one(k4 + kk);
+      } else {
+        for (int kk = k4; kk < kc; ++kk) one(kk);
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) { carry(acc[i][0]); carry(acc[i][1]); }
+    }
     __syncthreads();  // every thread is done with this buffer before it is refilled
     cur ^= 1;
   }
@@ -319,9 +355,9 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
     if (row < g.rows && n < N) {
       const int ea = aex[row];
       double* yp = (Y ? Y + (size_t)row * ldy : output_row(g, z, row)) + n;
-      const double y0 = value_of(acc[i][0], ea, e0, g.alpha);
+      const double y0 = value_of(wide_of(acc[i][0]), ea, e0, g.alpha);
       if (n + 1 < N) {
-        const double y1 = value_of(acc[i][1], ea, e1, g.alpha);
+        const double y1 = value_of(wide_of(acc[i][1]), ea, e1, g.alpha);
         if ((reinterpret_cast<uintptr_t>(yp) & 15) == 0) {
           *reinterpret_cast<double2*>(yp) = make_double2(y0, y1);
         } else {  // odd leading dimension or offset
@@ -348,13 +384,10 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
 // shares in every block two thirds of the instructions were for converting X
 // and adding shares: 97 x 97 x 6, 1026 entries 114 -> 52 us, 291 x 97 x 6 256 ->
 // 113, 291 x 97 x 2, 341 entries 40 -> 30, 195 x 65 x 8, 170 entries 32 -> 22.
-struct alignas(16) Part {
-  long long hh, mid;
-};
 template <int NC>
 __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ GemmArgs g, int RB, int KS) {
   extern __shared__ __align__(16) double fsm[];
-  Part* parts = reinterpret_cast<Part*>(fsm);                       // [KS][NC][RB]
+  Wide* parts = reinterpret_cast<Wide*>(fsm);                       // [KS][NC][RB]
   double* xd = reinterpret_cast<double*>(parts + KS * NC * RB);     // [K][NC]
   __shared__ int cex[NC];
   __shared__ int part[256];
@@ -367,7 +400,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
   long lda = g.lda, ldx = g.ldx;
   const int2* A = g.fx + (size_t)z * g.sA;
   const int* aex = g.fx_ex + (size_t)z * g.lda;
-  const int* w = g.fx_w ? g.fx_w + (size_t)z * g.K : nullptr;
+  const int* w = g.fx_w + (size_t)z * g.K;
   const double* X = g.X + (size_t)z * g.sX;
   double* Y = nullptr;
   if (g.nsub || z >= nz) {
@@ -379,7 +412,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     ldx = q.ldx;
     A = q.fx + (size_t)e * g.sA;
     aex = q.fx_ex + (size_t)e * lda;
-    w = q.fx_w ? q.fx_w + (size_t)e * g.K : nullptr;
+    w = q.fx_w + (size_t)e * g.K;
     X = q.X + (size_t)e * g.sX;
     Y = q.Y + (size_t)e * g.sY + (size_t)row * q.ldy;
     b0 = q.b0;
@@ -393,11 +426,11 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     xd[i] = c < N ? X[(size_t)k * ldx + c] : 0.0;
   }
   __syncthreads();
-  convert_panel(xd, g.K, NC, w, cex, part, g.K > 255);
+  convert_panel(xd, g.K, NC, w, cex, part);
   const int2* xs = reinterpret_cast<const int2*>(xd);
   Sum acc[NC];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) acc[c] = Sum{0, 0};
+  for (int c = 0; c < NC; ++c) acc[c] = Sum{0, 0, 0};
   for (int k0 = kb; k0 < ke; k0 += U) {
     int2 nv[U];
 #pragma unroll
@@ -412,6 +445,10 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
         add_product(acc[c], av[u], make_int2(x.x, x.y));
         add_product(acc[c + 1], av[u], make_int2(x.z, x.w));
       }
+      if (u % kCarry == kCarry - 1 && u < U - 1) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) carry(acc[c]);
+      }
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) carry(acc[c]);
@@ -419,17 +456,13 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     for (int u = 0; u < U; ++u) av[u] = nv[u];
   }
 #pragma unroll
-  for (int c = 0; c < NC; ++c) parts[(kp * NC + c) * RB + rl] = Part{acc[c].hh, acc[c].mid};
+  for (int c = 0; c < NC; ++c) parts[(kp * NC + c) * RB + rl] = wide_of(acc[c]);
   if (g.follow.kind) follow_modes(g.follow);
   __syncthreads();
   if (row >= g.rows) return;
   auto column = [&](int c) {
-    Sum s{0, 0};
-    for (int q = 0; q < KS; ++q) {
-      const Part p = parts[(q * NC + c) * RB + rl];
-      s.hh += p.hh;
-      s.mid += p.mid;
-    }
+    Wide s{0, 0};
+    for (int q = 0; q < KS; ++q) s = add(s, parts[(q * NC + c) * RB + rl]);
     return value_of(s, aex[row], cex[c], g.alpha);
   };
   double* y = Y ? Y : output_row(g, z, row);
@@ -450,8 +483,8 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
 //   S0 = sum_p A0[p][j] X0[p], S1 = sum_p A1[p][j] X1[p]
 // hold half the products of the dense operator.  What the mirrored half
 // differs by (the rounding of its own cosines, 2^-40 of an element) is a
-// third sum of one 32-bit product each, D = sum (26 bits of the difference)
-// (28 bits of x), added at its scale: outputs are those of the dense operator.
+// third sum of one 32-bit product each, D = sum (24 bits of the difference)
+// (30 bits of x), added at its scale: outputs are those of the dense operator.
 //   FWD: X0, X1 = x_p +- x_{n-1-p};  out_{2j} = S0 + D0, out_{2j+1} = S1 + D1
 //   else X0, X1 = x_{2p}, x_{2p+1};  out_j = S0 + S1, out_{n-1-j} = +-(S0 - S1) + D
 // A block takes NCOL real columns (re and im side by side) of one operator;
@@ -491,13 +524,13 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   issue(0, 0);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  convert_panel<ST - NCOL>(xs, n, NCOL, op.w, cex, part, FWD || n > 255);
+  convert_panel<ST - NCOL>(xs, n, NCOL, op.w, cex, part, FWD);
   if (FWD) {
     for (int i = threadIdx.x; i < n / 2 * NCOL; i += nthr) {
       const int p = i / NCOL, c = i - p * NCOL;
       int2* a = reinterpret_cast<int2*>(xs) + p * ST + c;
       int2* b = reinterpret_cast<int2*>(xs) + (n - 1 - p) * ST + c;
-      const long long va = (long long)a->x * 2147483648LL + a->y, vb = (long long)b->x * 2147483648LL + b->y;
+      const long long va = ((long long)a->x << kLow) + a->y, vb = ((long long)b->x << kLow) + b->y;
       *a = signed_split(va + vb);
       *b = signed_split(va - vb);
     }
@@ -509,7 +542,7 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   for (int i = 0; i < RPT; ++i)
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      s0[i][c] = s1[i][c] = Sum{0, 0};
+      s0[i][c] = s1[i][c] = Sum{0, 0, 0};
       d0[i][c] = d1[i][c] = 0;
     }
   int cur = 0;
@@ -525,8 +558,7 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
     const int4* Aw = as + cur * kFxPC * hb + rw;
     const int2* Dw = ds + cur * kFxPC * hb + rw;
     const int4* xp = reinterpret_cast<const int4*>(xs) + cp;
-#pragma unroll 2
-    for (int pp = 0; pp < pc; ++pp) {
+    auto one = [&](int pp) {
       const int p = p0 + pp;
       const int4 u = xp[(FWD ? p : 2 * p) * (ST / 2)], v = xp[(FWD ? n - 1 - p : 2 * p + 1) * (ST / 2)];
       const int2 u0 = make_int2(u.x, u.y), u1 = make_int2(u.z, u.w), v0 = make_int2(v.x, v.y), v1 = make_int2(v.z, v.w);
@@ -550,11 +582,16 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
           d0[i][1] = madw1(d.y, v1.x, madw1(d.x, u1.x, d0[i][1]));
         }
       }
-    }
+    };
+    for (int p4 = 0; p4 < pc; p4 += kCarry) {
+      const int pe = min(p4 + kCarry, pc);
+#pragma unroll 2
+      for (int pp = p4; pp < pe; ++pp) one(pp);
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) {
-      carry(s0[i][0]); carry(s0[i][1]);
-      carry(s1[i][0]); carry(s1[i][1]);
+      for (int i = 0; i < RPT; ++i) {
+        carry(s0[i][0]); carry(s0[i][1]);
+        carry(s1[i][0]); carry(s1[i][1]);
+      }
     }
     __syncthreads();  // the buffer is refilled, after the last chunk the panel
     cur ^= 1;
@@ -567,15 +604,14 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
     double y[2], z[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-      const Sum a = s0[i][c], b = s1[i][c];
-      Sum f, m;
+      const Wide a = wide_of(s0[i][c]), b = wide_of(s1[i][c]);
+      Wide f, m;
       if (FWD) {
-        f = Sum{a.hh, a.mid + (d0[i][c] >> e.z)};
-        m = Sum{b.hh, b.mid + (d1[i][c] >> e.w)};
+        f = add(a, d0[i][c] >> e.z);
+        m = add(b, d1[i][c] >> e.w);
       } else {
-        f = Sum{a.hh + b.hh, a.mid + b.mid};
-        m = op.sign > 0 ? Sum{a.hh - b.hh, a.mid - b.mid} : Sum{b.hh - a.hh, b.mid - a.mid};
-        m.mid += d0[i][c] >> e.z;
+        f = add(a, b);
+        m = add(op.sign > 0 ? sub(a, b) : sub(b, a), d0[i][c] >> e.z);
       }
       y[c] = value_of(f, e.x, cex[2 * cp + c], 1.0);
       z[c] = value_of(m, e.y, cex[2 * cp + c], 1.0);
@@ -718,7 +754,7 @@ cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int
                                int* ex, cudaStream_t s) {
   const long n = (long)nb * rows, m = (long)nb * K;
   if (n <= 0) return cudaSuccess;
-  if (wk) fx_weight_kernel<<<(unsigned)((m + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk);
+  fx_weight_kernel<<<(unsigned)((m + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk);
   fx_operator_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk, out, ex);
   return cudaGetLastError();
 }
@@ -738,7 +774,7 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
     const int RB = (g.rows + nb - 1) / nb;
     const dim3 grid((g.rows + RB - 1) / RB, nz);
     auto run = [&](auto kernel, int nc) {
-      const size_t smem = (size_t)nc * ((size_t)KS * RB * sizeof(Part) + g.K * sizeof(double));
+      const size_t smem = (size_t)nc * ((size_t)KS * RB * sizeof(Wide) + g.K * sizeof(double));
       if (smem > 46 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
         if (e != cudaSuccess) return e;

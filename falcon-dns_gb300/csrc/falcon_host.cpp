@@ -221,7 +221,7 @@ struct OpSet {
     int* ex = nullptr;
     int2* fx = nullptr;       // fixed-point integers and row exponents (launch_fx_operator)
     int* fx_ex = nullptr;
-    int* fx_w = nullptr;      // column weights of solve operators
+    int* fx_w = nullptr;      // column weights
     CUtensorMap tmap{};     // the slices for the tcgen05 kernel's copies
     bool tmap_ok = false;
   };
@@ -245,9 +245,8 @@ struct OpSet {
 std::atomic<int> g_gemm_mode{4};
 
 // Slices and fixed-point integers of one column-major operator array (rows x
-// K, lda = rows, nb entries of stride sA) for the contraction kernels; the
-// integers of a solve operator with weighted columns.
-int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA, bool solve = false) {
+// K, lda = rows, nb entries of stride sA) for the contraction kernels.
+int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA) {
   if (!base || K > 257) return 0;
   OpSet::Oz o;
   o.base = base; o.lda = rows; o.sA = sA; o.rows = rows; o.K = K; o.nb = nb;
@@ -265,10 +264,10 @@ int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA, boo
   const size_t nf = (size_t)(nb - 1) * sA + (size_t)rows * K;
   CK(cudaMalloc(&o.fx, nf * sizeof(int2)));
   CK(cudaMalloc(&o.fx_ex, (size_t)nb * rows * sizeof(int)));
-  if (solve) CK(cudaMalloc(&o.fx_w, (size_t)nb * K * sizeof(int)));
+  CK(cudaMalloc(&o.fx_w, (size_t)nb * K * sizeof(int)));
   CK(launch_fx_operator(base, rows, sA, rows, K, nb, o.fx_w, o.fx, o.fx_ex, 0));
   ops->bytes += ns * sizeof(uint16_t) + ne * sizeof(int) + nf * sizeof(int2) + (size_t)nb * rows * sizeof(int) +
-                (solve ? (size_t)nb * K * sizeof(int) : 0);
+                (size_t)nb * K * sizeof(int);
   ops->oz.push_back(o);
   return 0;
 }
@@ -671,9 +670,9 @@ int build_opset(const OpKey& k, std::shared_ptr<OpSet>* out, const HostFactors* 
   {
     const long RR = (long)R * R;
     if ((rc = add_oz(ops.get(), ops->D1p, R, R, 1, RR)) || (rc = add_oz(ops.get(), ops->Lp, R, R, 1, RR)) ||
-        (rc = add_oz(ops.get(), ops->ST, R, R, M, RR, true)) || (rc = add_oz(ops.get(), ops->G, 3 * R, R, M, 3 * RR, true)) ||
-        (rc = add_oz(ops.get(), ops->U, 2 * R, R, 1, 2 * RR, true)) ||
-        (rc = add_oz(ops.get(), ops->LAP, 2 * R + 2, R, M, (long)(2 * R + 2) * R, true)) ||
+        (rc = add_oz(ops.get(), ops->ST, R, R, M, RR)) || (rc = add_oz(ops.get(), ops->G, 3 * R, R, M, 3 * RR)) ||
+        (rc = add_oz(ops.get(), ops->U, 2 * R, R, 1, 2 * RR)) ||
+        (rc = add_oz(ops.get(), ops->LAP, 2 * R + 2, R, M, (long)(2 * R + 2) * R)) ||
         (rc = add_oz(ops.get(), ops->D1c, R, R, 1, RR)) || (rc = add_oz(ops.get(), ops->Lc, R, R, 1, RR)))
       return rc;
     CK(cudaDeviceSynchronize());
@@ -1382,7 +1381,7 @@ bool attach_oz(const OpSet* o, GemmArgs* q) {
     q->oz_z0 = (int)z0;
     q->fx = z.fx + delta;
     q->fx_ex = z.fx_ex + z0 * z.rows + row0;
-    q->fx_w = z.fx_w ? z.fx_w + z0 * z.K : nullptr;
+    q->fx_w = z.fx_w + z0 * z.K;
     return true;
   }
   return false;
@@ -1433,7 +1432,7 @@ TcArgs tc_args(const GemmArgs& q) {
 
 // ---------------------------------------------------------------------------
 // Contraction paths and their autotuner.  A contraction with an attached
-// view can run as tiles of 58-bit integers (PATH_FMA, falcon_fxgemm.cu; FP64
+// view can run as tiles of 60-bit integers (PATH_FMA, falcon_fxgemm.cu; FP64
 // FMA tiles without a view), on the mma.sync slice kernel (PATH_MMA; X sliced
 // in the kernel, or into slice planes first) or on the tcgen05 kernel
 // (PATH_TC).  PATH_MMA and PATH_TC give the same bits; PATH_FMA differs from
@@ -4281,17 +4280,19 @@ struct ChebMats {
 std::mutex g_cheb_mu;
 std::map<int, ChebMats> g_cheb;
 
-int2 fx_split(double a, int bits, int e) {  // trunc(a 2^(bits - e)) as h 2^31 + l, l signed
-  const unsigned long long t = (unsigned long long)(long long)std::ldexp(a, bits - e);
-  return make_int2((int)((long long)t >> 31) + (int)((unsigned)t >> 30 & 1), (int)((unsigned)t << 1) >> 1);
+int2 fx_split(double a, int e) {  // a 2^(60 - e) rounded, as h 2^30 + l, l signed
+  const long long t = std::llrint(std::ldexp(a, 60 - e)), h = (t + (1LL << 29)) >> 30;
+  return make_int2((int)h, (int)(t - h * (1LL << 30)));
 }
 
 // An operator in the form of fx_columns_kernel (falcon_fxgemm.cu).  Rows i and
 // n - 1 - i of inv, d1 and d2 (columns of fwd) agree up to the sign
-// parity * (-1)^k and a difference that has to be below 2^-32 of its row's
-// largest element (it is below 2^-36 for n <= 257; false otherwise).  The
-// columns of inv, d1 and d2 are scaled by powers of two, X's rows inversely:
-// their elements grow as k^2 and k^4 where a spectrum falls.
+// parity * (-1)^k and a difference that has to be below 2^-36 of its row's
+// largest element (it is for n <= 257; false otherwise).  The columns of inv, d1
+// and d2 are divided by powers of two, X's rows multiplied: half the exponent of
+// a column's largest element (falcon_fxgemm.cu), which grows as k^2 and k^4 at
+// the walls, in the middle as k and k^2.  With all of it d2 lost up to 2^11 of
+// FP64's accuracy in the middle rows.
 bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::vector<int4>* A, std::vector<int2>* D,
                 std::vector<int4>* ex, std::vector<int>* w) {
   const int h = (n + 1) / 2;
@@ -4304,7 +4305,7 @@ bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::
     for (int k = 0; k < n; ++k) {
       int e = -100000;
       for (int i = 0; i < n; ++i) e = std::max(e, exponent(m[(size_t)i * n + k]));
-      (*w)[k] = e == -100000 ? 0 : e;
+      (*w)[k] = e == -100000 ? 0 : (e >= 0 ? e / 2 : -((1 - e) / 2));
     }
   // element and difference of term t of output pair j: fwd (row 2 j + b, point
   // t), else (row j, coefficient t)
@@ -4325,14 +4326,14 @@ bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::
         ed = std::max(ed, exponent(d[t]));
       }
       if (e == -100000) e = 0;
-      int sh = ed == -100000 ? 0 : e - 32 - ed;
+      int sh = ed == -100000 ? 0 : e - 36 - ed;
       if (sh < 0) return false;
       if (sh > 60) { sh = 0; std::fill(d.begin(), d.end(), 0.0); }
       for (int t = 0; t < terms; ++t) {
         const size_t at = (size_t)(fwd ? t : t / 2) * h + j;
         const bool second = fwd ? b : t & 1;
-        const int2 s = fx_split(a[t], 58, e);
-        const int q = (int)std::ldexp(d[t], 26 - ed);
+        const int2 s = fx_split(a[t], e);
+        const int q = (int)std::lrint(std::ldexp(d[t], 24 - ed));
         (second ? (*A)[at].z : (*A)[at].x) = s.x;
         (second ? (*A)[at].w : (*A)[at].y) = s.y;
         (second ? (*D)[at].y : (*D)[at].x) = q;

@@ -458,8 +458,8 @@ cudaError_t launch_getrs_batched(int n, int nsys, int nrhs, const double* lu, co
 // Chebyshev transforms of complex columns in fixed point (n <= 257): what the
 // kernel reads of an operator (cheb_fixed) and the call.
 struct FxColumnsOp {
-  const int4* A;  // [p][j]: A0, A1 as (h, l) of 58 bits at the row's scale
-  const int2* D;  // [p][j]: 26 bits of the mirrored halves' differences
+  const int4* A;  // [p][j]: A0, A1 as (h, l) of 60 bits at the row's scale
+  const int2* D;  // [p][j]: 24 bits of the mirrored halves' differences
   const int4* ex; // [j]: exponents of the rows of S0 and S1, shifts of D0 and D1
   const int* w;   // weights of X's rows (or null)
   double2* out;

@@ -365,7 +365,7 @@ long long falcon_launch_count(void);
  * No reference counterpart (launch mechanics of the GPU step). */
 int falcon_set_step_graphs(int enable);
 /* Operator contractions (the radial derivative / Laplacian and per-mode
- * solve products) run on one of three paths: tiles of 58-bit fixed-point
+ * solve products) run on one of three paths: tiles of 60-bit fixed-point
  * integers; the bf16 tensor cores by exact
  * integer slicing of the FP64 operands on warp-level mma.sync; the same
  * slices on the 5th-generation tcgen05 MMA with accumulators in tensor

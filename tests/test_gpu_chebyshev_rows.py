@@ -1,0 +1,41 @@
+"""Chebyshev transforms row by row: the rows away from the walls, whose elements
+are smaller by k (d1) and k^2 (d2) than the largest of their columns, are as
+accurate as the others.
+
+With w_k = floor(e_k / 2) (falcon-dns_gb300/csrc/falcon_fxgemm.cu; 0 for fwd),
+an operator row and a column of X are rounded to 60 bits (59 for fwd, whose
+points are added in pairs) at the power of two above their largest weighted
+element, and the low halves' product is left out: for A_i and X the largest
+weighted elements, 2^-59 A_i |x_k| 2^w_k + 2^-59 X |A_ik| 2^-w_k + 2^-59 A_i X
+a term at most; the mirrored rows' differences (below 2^-36 A_i) in 24 bits of
+30 bits of X: 2^-59 A_i X a term; the sum is rounded once, and so were the
+operator's elements, read back as columns of the identity (2^-53 each, of
+sum_k |A_ik x_k|).  So |error| <= 2^-52 sum_k |A_ik x_k| + 4 n 2^-59 A_i X."""
+import numpy as np
+import pytest
+
+from test_gpu_fixed_point_chebyshev import NAMES, call
+
+pytestmark = pytest.mark.gpu
+
+
+def operator(fg, n, fn):
+    return call(fg, fn, n, np.eye(n) + 0j).real.T
+
+
+@pytest.mark.parametrize("n", [17, 64, 65, 129, 257])
+def test_every_row(fg, n):
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((60, n)) + 0j
+    x[::3] *= np.exp2(-0.25 * np.arange(n))
+    x[1::3] *= np.arange(n) + 1.0
+    for q, fn in enumerate(NAMES):
+        A = operator(fg, n, fn)
+        top = np.abs(A).max(0)
+        w = np.floor_divide(np.frexp(top)[1], 2) if q else np.zeros(n, int)
+        amax = np.abs(A * np.exp2(-w.astype(float))).max(1)
+        A, xp = A.astype(np.longdouble), x.real.astype(np.longdouble)
+        xmax = np.abs(xp * np.exp2(w.astype(float))).max(1)
+        tol = 2.0 ** -52 * (np.abs(xp) @ np.abs(A).T) + 4 * n * 2.0 ** -59 * np.outer(xmax, amax)
+        err = np.abs(call(fg, fn, n, x).real - xp @ A.T)
+        assert (err <= tol).all(), (fn, float((err / tol).max()))
