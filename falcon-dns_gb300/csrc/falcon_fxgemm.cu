@@ -23,7 +23,8 @@
 // large values of fields that vanish at the walls, lose their digits; with
 // columns divided by their largest element and X's rows multiplied, X's values
 // away from the walls lose theirs.  So columns are divided by 2^w_k, w_k half the
-// largest element's exponent, and the spread is shared.
+// largest element's exponent, and the spread is shared.  A column of zeros
+// weighs nothing, whatever X has there.
 //
 // Errors over the norm of a column's output against 64 bits (FP64 sums, this
 // form; a form of 58 x 59 bits, truncated, with weights of 0 for the derivatives
@@ -58,6 +59,7 @@ constexpr int kFollowRows = 6;           // deepest tiles that do what follows a
 constexpr int kFxKC = 16;                // k per staged operator chunk
 constexpr int kBad = INT32_MIN;          // exponent of a row or column with an Inf or NaN
 constexpr int kNone = -100000;           // exponent of a zero
+constexpr int kNoWeight = -30000;        // of a column of zeros: below every other
 
 // e with |a 2^w| < 2^e (kNone for a zero, INT32_MAX for Inf and NaN)
 __device__ __forceinline__ int exponent_of(double a, int w) {
@@ -188,7 +190,7 @@ __global__ void fx_weight_kernel(const double* A, long lda, long sA, int rows, i
     const int e = exponent_of(a[r], 0);
     if (e != INT32_MAX) m = max(m, e);
   }
-  wk[t] = m == kNone ? 0 : m >> 1;
+  wk[t] = m == kNone ? kNoWeight : m >> 1;
 }
 
 // One thread per (entry, row): the row's exponent, then its integers, in the

@@ -4292,7 +4292,7 @@ int2 fx_split(double a, int e) {  // a 2^(60 - e) rounded, as h 2^30 + l, l sign
 // and d2 are divided by powers of two, X's rows multiplied: half the exponent of
 // a column's largest element (falcon_fxgemm.cu), which grows as k^2 and k^4 at
 // the walls, in the middle as k and k^2.  With all of it d2 lost up to 2^11 of
-// FP64's accuracy in the middle rows.
+// FP64's accuracy in the middle rows; a column of zeros weighs nothing.
 bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::vector<int4>* A, std::vector<int2>* D,
                 std::vector<int4>* ex, std::vector<int>* w) {
   const int h = (n + 1) / 2;
@@ -4305,7 +4305,7 @@ bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::
     for (int k = 0; k < n; ++k) {
       int e = -100000;
       for (int i = 0; i < n; ++i) e = std::max(e, exponent(m[(size_t)i * n + k]));
-      (*w)[k] = e == -100000 ? 0 : (e >= 0 ? e / 2 : -((1 - e) / 2));
+      (*w)[k] = e == -100000 ? -30000 : (e >= 0 ? e / 2 : -((1 - e) / 2));
     }
   // element and difference of term t of output pair j: fwd (row 2 j + b, point
   // t), else (row j, coefficient t)

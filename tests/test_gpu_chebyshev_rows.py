@@ -32,10 +32,26 @@ def test_every_row(fg, n):
     for q, fn in enumerate(NAMES):
         A = operator(fg, n, fn)
         top = np.abs(A).max(0)
-        w = np.floor_divide(np.frexp(top)[1], 2) if q else np.zeros(n, int)
-        amax = np.abs(A * np.exp2(-w.astype(float))).max(1)
+        w = np.where(top > 0, np.floor_divide(np.frexp(top)[1], 2), -1000) if q else np.zeros(n, int)
+        amax = np.abs(A * np.exp2(-np.maximum(w, -999).astype(float))).max(1)
         A, xp = A.astype(np.longdouble), x.real.astype(np.longdouble)
         xmax = np.abs(xp * np.exp2(w.astype(float))).max(1)
         tol = 2.0 ** -52 * (np.abs(xp) @ np.abs(A).T) + 4 * n * 2.0 ** -59 * np.outer(xmax, amax)
         err = np.abs(call(fg, fn, n, x).real - xp @ A.T)
         assert (err <= tol).all(), (fn, float((err / tol).max()))
+
+
+@pytest.mark.parametrize("n", [17, 65, 128])
+def test_a_constant_has_no_derivative(fg, n):
+    """Coefficient 0 (and 1 in d2) meets a column of zeros: whatever it is, the
+    others keep their digits; a NaN in it is one in the result."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((8, n)) + 1j * rng.standard_normal((8, n))
+    for fn, count in ((NAMES[2], 1), (NAMES[3], 2)):
+        x[:, :count] = 0.0
+        want = call(fg, fn, n, x)
+        x[:, :count] = 1e30
+        assert np.array_equal(call(fg, fn, n, x), want), fn
+        x[3, 0] = np.nan
+        got = call(fg, fn, n, x)
+        assert np.isnan(got[3].real).all() and np.array_equal(got[4], want[4])
