@@ -383,7 +383,7 @@ def gpu_warmup(args):
 # groups take the tcgen05 kernel in gemm mode 2, the mma.sync one in mode 1)
 def kernel_of_class(c, gemm_mode):
     if c in ("gemm_radial", "gemm_mode_solve"):
-        return "tc_gemm_kernel" if gemm_mode >= 2 else "oz_mma_kernel"
+        return {0: "gemm_tile_kernel", 1: "oz_mma_kernel", 5: "fx_tile_kernel"}.get(gemm_mode, "tc_gemm_kernel")
     return {"nonlin_fft": "nonlin_kernel", "elementwise": "elementwise kernels"}.get(c, c)
 
 
@@ -618,7 +618,7 @@ def run_gpu(args):
                          "tcgen05 slices (tensor memory accumulators), measured at the first warm-up step",
                       3: "tcgen05 for every sliced contraction",
                       2: "fixed rules: tcgen05 for contractions that fill the GPU, mma.sync below, FMA under 16 columns",
-                      1: "mma.sync", 0: "fixed-point tiles"}[args.gemm_mode],
+                      1: "mma.sync", 0: "FP64 FMA", 5: "fixed-point tiles"}[args.gemm_mode],
         "tuned_shapes": fg.tune_entries()[0],
         "state_finite": bool(finite),
         # last, so that a reader of the line's tail sees the target ratio
@@ -647,9 +647,9 @@ def main():
                     help="the uniform batch alone (profiling captures): no e2e, one-at-a-time, plain, single, mixed")
     ap.add_argument("--single-steps", dest="single_steps", type=int, default=200)
     ap.add_argument("--plain-steps", dest="plain_steps", type=int, default=500)
-    ap.add_argument("--gemm-mode", dest="gemm_mode", type=int, default=4, choices=[0, 1, 2, 3, 4],
-                    help="operator contractions: 4 autotuned per shape (FMA / mma.sync / tcgen05), 3 tcgen05, "
-                         "2 fixed rules, 1 mma.sync slices, 0 fixed-point tiles")
+    ap.add_argument("--gemm-mode", dest="gemm_mode", type=int, default=4, choices=[0, 1, 2, 3, 4, 5],
+                    help="operator contractions: 4 autotuned per shape (fixed point / mma.sync / tcgen05), "
+                         "3 tcgen05, 2 fixed rules, 1 mma.sync slices, 0 FP64, 5 fixed-point tiles")
     ap.add_argument("--uneven-instances", dest="uneven_instances", type=int, default=512)
     ap.add_argument("--uneven-steps", dest="uneven_steps", type=int, default=500)
     ap.add_argument("--serve-rate", dest="serve_rate", type=float, default=50.0)

@@ -240,8 +240,9 @@ struct OpSet {
 
 // Contraction paths (the modes of gemm() below): 4 (default) measured per
 // shape by the autotuner; 3 tcgen05 wherever possible; 2 tcgen05 where a
-// contraction fills the GPU, mma.sync otherwise; 1 mma.sync only; 0 tiles.
-// The two sliced kernels give the same bits; all paths are FP64-accurate.
+// contraction fills the GPU, mma.sync otherwise; 1 mma.sync only; 0 FP64 FMA;
+// 5 fixed-point tiles wherever possible.  The two sliced kernels give the same
+// bits.
 std::atomic<int> g_gemm_mode{4};
 
 // Slices and fixed-point integers of one column-major operator array (rows x
@@ -1388,8 +1389,9 @@ bool attach_oz(const OpSet* o, GemmArgs* q) {
 }
 
 // The slice view of q.A in any operator set of the group (its subs' and
-// their stages' included).
-bool attach_group(const Group* g, GemmArgs* q) {
+// their stages' included), and its fixed-point integers under the modes that
+// use them.
+bool attach_any(const Group* g, GemmArgs* q) {
   for (size_t k = 0; k < std::max<size_t>(g->subs.size(), 1); ++k) {
     if (k > 0 && attach_oz(g->subs[k].ops.get(), q)) return true;
     if (k == 0 && attach_oz(g->ops.get(), q)) return true;
@@ -1399,6 +1401,11 @@ bool attach_group(const Group* g, GemmArgs* q) {
     }
   }
   return false;
+}
+bool attach_group(const Group* g, GemmArgs* q) {
+  if (!attach_any(g, q)) return false;
+  if (g_gemm_mode.load() < 4) q->fx = nullptr;
+  return true;
 }
 
 // Contractions that take the tcgen05 kernel: at least two of its
@@ -1433,10 +1440,9 @@ TcArgs tc_args(const GemmArgs& q) {
 // ---------------------------------------------------------------------------
 // Contraction paths and their autotuner.  A contraction with an attached
 // view can run as tiles of 60-bit integers (PATH_FMA, falcon_fxgemm.cu; FP64
-// FMA tiles without a view), on the mma.sync slice kernel (PATH_MMA; X sliced
-// in the kernel, or into slice planes first) or on the tcgen05 kernel
-// (PATH_TC).  PATH_MMA and PATH_TC give the same bits; PATH_FMA differs from
-// them by rounding (all are FP64-accurate).
+// FMA tiles without a view and under modes 0 to 3), on the mma.sync slice kernel
+// (PATH_MMA; X sliced in the kernel, or into slice planes first) or on the
+// tcgen05 kernel (PATH_TC).  PATH_MMA and PATH_TC give the same bits.
 // ---------------------------------------------------------------------------
 // PATH_FMA16/32/64: the tiles with the best tile shape of that column
 // width (the same bits as PATH_FMA, whose shape a cost model picks).
@@ -1705,13 +1711,14 @@ int tuned_path(Group* g, int cls, const GemmArgs& q, bool reuse, bool tc_ok, int
 // since (the blocks of one operator applied to one right-hand side); its
 // slice planes are reused when they match.
 //
-// Modes: 0 tiles; 1 mma.sync for every contraction with a slice view; 2
+// Modes: 0 FP64 FMA; 1 mma.sync for every contraction with a slice view; 2
 // fixed rules: tcgen05 for contractions that fill the GPU (at least two 128 x
 // 24 tiles per SM), mma.sync for the other ones of at least 16 columns per
-// batch entry, tiles for narrower ones (the per-mode solves of groups of up
+// batch entry, FP64 FMA for narrower ones (the per-mode solves of groups of up
 // to 7 instances); 3 tcgen05 for every contraction with a slice view (the
-// same bits as 1); 4 (default) the measured fastest of tiles, mma.sync and
-// tcgen05 per shape.
+// same bits as 1); 4 (default) the measured fastest of fixed-point tiles,
+// mma.sync and tcgen05 per shape; 5 fixed-point tiles for every contraction with
+// a view.
 // The path of q (which receives its operator's views).
 int choose_path(Group* g, int cls, GemmArgs* q, bool reuse, int* path) {
   q->oz_s = nullptr;
@@ -1724,7 +1731,7 @@ int choose_path(Group* g, int cls, GemmArgs* q, bool reuse, int* path) {
   const int mode = g_gemm_mode.load();
   const bool view = attach_group(g, q);
   *path = PATH_FMA;
-  if (!(view && mode && g->oz_xs && (q->N >= 16 || mode != 2))) return 0;
+  if (!(view && mode && mode != 5 && g->oz_xs && (q->N >= 16 || mode != 2))) return 0;
   const bool tc_ok = mode >= 2 && q->oz_tmap != nullptr;
   *path = PATH_MMA;
   if (mode == 3 && tc_ok) *path = PATH_TC;
@@ -1808,7 +1815,7 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
   std::vector<GemmArgs> v(products);
   const int mode = g_gemm_mode.load();
   GemmArgs all{};
-  bool tiles = (mode == 0 || mode == 4) && v.size() > 1 && v.size() <= (size_t)kFxJobs;
+  bool tiles = mode >= 4 && v.size() > 1 && v.size() <= (size_t)kFxJobs;
   long cols = 0;
   for (size_t i = 0; i < v.size() && tiles; ++i) {
     GemmArgs q = v[i];
@@ -1835,7 +1842,7 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
   for (const GemmArgs& q : v) flops += gemm_flops(q);
   auto together = [&]() { return launch(g, cls, flops, [&]() { return launch_fx_gemm(all, g->stream); }); };
   if (!tiles) return apart();
-  if (mode == 0) return together();
+  if (mode == 5) return together();
   TuneKey k{device_tag(), v[0].rows, v[0].K, (int)cols, 1, all.oz_w, 16 + (int)v.size(), 0};
   int known = -1;
   {
@@ -1947,7 +1954,7 @@ int gemm_blocks(Group* g, int cls, std::initializer_list<GemmArgs> blocks, const
   all.oz_s = nullptr;
   all.oz_xs = nullptr;
   if (!merge || !attach_group(g, &all)) return run_blocks(g, cls, v, nullptr);
-  if (mode >= 2 && g->oz_xs && (f.N >= 16 || mode >= 3) && all.oz_tmap && (mode == 3 || tc_worth_it(all))) {
+  if (mode >= 2 && mode != 5 && g->oz_xs && (f.N >= 16 || mode >= 3) && all.oz_tmap && (mode == 3 || tc_worth_it(all))) {
     bool use = true;
     if (mode == 4) {
       g->oz_key.valid = false;  // the blocks' own X slicing starts afresh
@@ -4793,7 +4800,7 @@ extern "C" {
 long long falcon_launch_count(void) { return g_launches.load(); }
 
 int falcon_set_step_graphs(int enable) { return g_graphs.exchange(enable ? 1 : 0); }
-int falcon_set_gemm_mode(int mode) { return g_gemm_mode.exchange(mode < 0 || mode > 4 ? 4 : mode); }
+int falcon_set_gemm_mode(int mode) { return g_gemm_mode.exchange(mode < 0 || mode > 5 ? 4 : mode); }
 
 int falcon_set_tune_cache(const char* path) {
   std::lock_guard<std::mutex> lk(g_tune_mu);

@@ -512,10 +512,9 @@ def set_gemm_mode(mode):
     """Operator contraction paths: 4 (default) the fastest measured per shape
     (autotuned, see set_tune_cache); 3 tcgen05 for every sliced contraction;
     2 fixed rules (tcgen05 where a contraction fills the GPU, mma.sync for
-    other ones of >= 16 columns, tiles below); 1 mma.sync for every sliced
-    contraction (the same bits as 3); 0 tiles (60-bit fixed point; FP64 FMA for
-    Nr > 257).  Returns the
-    previous mode."""
+    other ones of >= 16 columns, FP64 below); 1 mma.sync for every sliced
+    contraction (the same bits as 3); 0 FP64; 5 tiles of 60-bit fixed-point
+    integers.  Returns the previous mode."""
     return lib().falcon_set_gemm_mode(int(mode))
 
 

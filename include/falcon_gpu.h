@@ -365,12 +365,14 @@ long long falcon_launch_count(void);
  * No reference counterpart (launch mechanics of the GPU step). */
 int falcon_set_step_graphs(int enable);
 /* Operator contractions (the radial derivative / Laplacian and per-mode
- * solve products) run on one of three paths: tiles of 60-bit fixed-point
- * integers; the bf16 tensor cores by exact
- * integer slicing of the FP64 operands on warp-level mma.sync; the same
- * slices on the 5th-generation tcgen05 MMA with accumulators in tensor
- * memory.  The two sliced paths give the same bits; all give FP64-accurate
- * results (error of the order of K 2^-56 max|A_row| max|X_col|), several
+ * solve products) run on one of four paths: FP64 multiply-adds; tiles of
+ * 60-bit fixed-point integers; the bf16 tensor cores by exact integer slicing
+ * of the FP64 operands on warp-level mma.sync; the same slices on the
+ * 5th-generation tcgen05 MMA with accumulators in tensor memory.  The two
+ * sliced paths give the same bits.  Errors are bounded relative to the largest
+ * element of a row and of a column: about K 2^-56 max|A_row| max|X_col| for the
+ * slices, K 2^-60 of the same with evened-out columns for the tiles (in norm
+ * below FP64's on the operators and fields of the annulus); both are several
  * times faster than GB300's FP64 pipe.  Modes:
  *   4 (default) autotuned: the first time a contraction shape runs outside
  *     graph capture, every available path is timed on it (the device
@@ -383,9 +385,10 @@ int falcon_set_step_graphs(int enable);
  *     (mma.sync where that view has no tensor map): the same bits as 1;
  *   2 fixed rules: tcgen05 for contractions of at least two 128 x 24 tiles
  *     per SM, mma.sync for the other ones of at least 16 columns per batch
- *     entry, tiles for narrower ones;
+ *     entry, FP64 for narrower ones;
  *   1 mma.sync for every contraction with a slice view;
- *   0 tiles only.
+ *   0 FP64 only;
+ *   5 tiles for every contraction with a slice view.
  * Applies to launches after the call (step graphs already captured keep
  * their paths).  Returns the previous mode; an unknown mode selects 4.
  * No counterpart in the reference, which uses LAPACK dgetrs

@@ -139,8 +139,7 @@ def test_uneven_products(product, n, ncol):
 
 @pytest.mark.parametrize("ncol", [2, 40])
 def test_fp64_products(product, ncol):
-    """launch_gemm, which operators of more than 257 columns (and mode 0) take:
-    |error| <= (K + 1) 2^-53 sum |a x|."""
+    """launch_gemm, which modes 0 and 2 and operators without integers take: |error| <= (K + 1) 2^-53 sum |a x|."""
     rng = np.random.default_rng(3)
     for n in (33, 258, 300):
         A, X = rng.standard_normal((2, n + 1, n)), rng.standard_normal((2, n, ncol))
