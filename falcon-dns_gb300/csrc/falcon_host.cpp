@@ -3620,7 +3620,9 @@ static int batch_create(const falcon_params* ps, int n, falcon_batch** out) {
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
     return fail(FALCON_ECUDA, "no CUDA device: the GB300 library has no CPU fallback");
-  tc_error_read_and_clear();  // the error word exists before any step is captured
+  // (the word exists before any step is captured; what another batch's steps
+  // left in it is theirs to report)
+  if (!tc_error_word()) return fail(FALCON_ENOMEM, "no page-locked memory for the kernels' error word");
   std::unique_ptr<falcon_batch> b(new falcon_batch());
   b->params.assign(ps, ps + n);
   CK(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
@@ -4613,7 +4615,9 @@ int falcon_server_create(size_t hbm_budget_bytes, int max_active, falcon_server*
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0)
     return fail(FALCON_ECUDA, "no CUDA device: the GB300 library has no CPU fallback");
-  tc_error_read_and_clear();  // the error word exists before any step is captured
+  // (the word exists before any step is captured; what another batch's steps
+  // left in it is theirs to report)
+  if (!tc_error_word()) return fail(FALCON_ENOMEM, "no page-locked memory for the kernels' error word");
   auto* s = new falcon_server();
   s->budget = hbm_budget_bytes;
   s->max_active = max_active > 0 ? max_active : (1 << 30);

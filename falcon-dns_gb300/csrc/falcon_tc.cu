@@ -606,10 +606,14 @@ cudaError_t launch_tc_gemm(const TcArgs& a, const CUtensorMap& map, cudaStream_t
   return a.w == 7 ? launch_tc_w<7>(a, map, s) : launch_tc_w<6>(a, map, s);
 }
 
-int tc_error_read_and_clear() {
+int* tc_error_word() {
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-  volatile int* p = tc_err_ptr(dev);
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  return tc_err_ptr(dev);
+}
+
+int tc_error_read_and_clear() {
+  volatile int* p = tc_error_word();
   if (!p) return 0;  // no such kernel has run
   const int v = *p;
   if (v) *p = 0;

@@ -80,7 +80,10 @@ int tc_make_operator_map(CUtensorMap* map, const uint16_t* slices, int nb, int S
 // every accumulator inside the allocated tensor memory (0, or < 0).  Host.
 int tc_stage_layout_check(int w, int KP);
 cudaError_t launch_tc_gemm(const TcArgs& a, const CUtensorMap& map, cudaStream_t s);
-// The kernels' error word (a wait that timed out: 1-8), read and cleared.
+// The host address of the kernels' error word (a wait that timed out: 1-8) on
+// the current device, made by the first call; null without page-locked memory.
+int* tc_error_word();
+// The word, read and cleared: only where its value is reported.
 int tc_error_read_and_clear();
 
 }  // namespace falcon
