@@ -660,15 +660,9 @@ long column_blocks(const GemmArgs& g, int ncol) {
 
 template <int RPT, int NCOL>
 cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream_t s) {
-  static std::atomic<bool> opted[64];  // opted in to large shared memory, per device
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(dev >= 0 && dev < 64 && opted[dev].load())) {
-    const cudaError_t e = cudaFuncSetAttribute(fx_tile_kernel<RPT, NCOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               227 * 1024);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) opted[dev].store(true);
-  }
+  static std::atomic<unsigned long long> opted[64];
+  const cudaError_t e = allow_shared((const void*)fx_tile_kernel<RPT, NCOL>, 227 * 1024, opted);
+  if (e != cudaSuccess) return e;
   const int rows_blk = nw * (64 / NCOL) * RPT;
   const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw) * 4;
   const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, entries(g));

@@ -865,11 +865,7 @@ void falcon::fft_tables_host(const FftPlan& plan, int4* tw, unsigned* pos) {
   }
 }
 
-namespace {
-
-// The current CUDA context's id (0: unknown); a device that was reset has a
-// new one.
-unsigned long long context_id() {
+unsigned long long falcon::context_id() {
   using GetCurrent = CUresult (*)(CUcontext*);
   using GetId = CUresult (*)(CUcontext, unsigned long long*);
   static const std::pair<void*, void*> fn = [] {
@@ -889,6 +885,8 @@ unsigned long long context_id() {
     return 0;
   return id;
 }
+
+namespace {
 
 struct FftTables {
   FftPlan plan{};
@@ -1604,16 +1602,16 @@ long operand_span(long ld, long sz, int K, int N, int batch) {
 // A device buffer larger than L2 (129 MB on GB300), written before each
 // timed run of the tuner: in a step the operators and operands of a
 // contraction come from HBM (the step's working set is larger than L2), so
-// the candidates are timed with a cold L2 too.  One per device, kept for
-// the process.
+// the candidates are timed with a cold L2 too.  One per device and context, kept
+// for its life.
 constexpr size_t kTuneFlushBytes = (size_t)256 << 20;
 void* tune_flush_buffer() {
   static std::mutex mu;
-  static std::map<int, void*> bufs;
+  static std::map<std::pair<int, unsigned long long>, void*> bufs;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> lk(mu);
-  void*& b = bufs[dev];
+  void*& b = bufs[{dev, context_id()}];
   if (!b && cudaMalloc(&b, kTuneFlushBytes) != cudaSuccess) b = nullptr;
   return b;
 }

@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #include "falcon_fixed.h"
 
 namespace falcon {
@@ -421,6 +423,23 @@ struct AsmArgs {
   double2 *t0, *w0, *rhs_w;
   double* u0;
 };
+
+// The current CUDA context's id (0: unknown); a device that was reset has a new
+// one, and what was kept for the old one went with it (falcon_host.cpp).
+unsigned long long context_id();
+// A kernel's limit of dynamic shared memory, set once per context; done: 64
+// entries of the caller's.
+inline cudaError_t allow_shared(const void* kernel, int bytes, std::atomic<unsigned long long>* done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long id = context_id();
+  const bool slot = id && dev >= 0 && dev < 64;
+  if (slot && done[dev].load() == id) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && slot) done[dev].store(id);
+  return e;
+}
 
 // ---- launchers (falcon_kernels.cu; the nonlinear pass dispatches to falcon_fft*.cu) ----
 cudaError_t launch_nonlin(const NonlinArgs& a, cudaStream_t s);

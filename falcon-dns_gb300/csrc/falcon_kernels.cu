@@ -210,16 +210,10 @@ __global__ void __launch_bounds__(32) dfma_gemv_kernel(GemmArgs g) {
 
 template <int RPT, int NCOL>
 static cudaError_t launch_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream_t s) {
-  // two K-chunk buffers; above 48 KB the kernel is opted in once per device
-  static std::atomic<bool> opted[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (!(dev >= 0 && dev < 64 && opted[dev].load())) {
-    const cudaError_t e = cudaFuncSetAttribute(gemm_tile_kernel<RPT, NCOL>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-    if (e != cudaSuccess) return e;
-    if (dev >= 0 && dev < 64) opted[dev].store(true);
-  }
+  // two K-chunk buffers
+  static std::atomic<unsigned long long> opted[64];
+  const cudaError_t e = allow_shared((const void*)gemm_tile_kernel<RPT, NCOL>, 96 * 1024, opted);
+  if (e != cudaSuccess) return e;
   dim3 grid((g.N + NCOL - 1) / NCOL, row_blocks, g.batch);
   const size_t smem = (size_t)2 * kKC * (nw * (64 / NCOL) * RPT + NCOL) * sizeof(double);
   gemm_tile_kernel<RPT, NCOL><<<grid, 32 * nw, smem, s>>>(g);

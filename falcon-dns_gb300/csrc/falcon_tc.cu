@@ -44,7 +44,9 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <map>
 #include <mutex>
+#include <utility>
 
 #include "falcon_internal.h"
 #include "falcon_slices.cuh"
@@ -492,39 +494,19 @@ __global__ void __launch_bounds__(448, 1) tc_gemm_kernel(const __grid_constant__
   }
 }
 
-// The error word, in page-locked host memory that the kernels write directly:
-// the host reads it after a synchronisation without a copy.
-std::once_flag g_tc_err_once[64];
-int* g_tc_err_addr[64];
-
-int* tc_err_ptr(int dev) {
-  std::call_once(g_tc_err_once[dev], [dev] {
-    void* p = nullptr;
-    if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
-      *static_cast<int*>(p) = 0;
-      g_tc_err_addr[dev] = static_cast<int*>(p);
-    }
-  });
-  return g_tc_err_addr[dev];
-}
-
 template <int W>
 cudaError_t launch_tc_w(const TcArgs& a, const CUtensorMap& map, cudaStream_t s) {
   using C = TcCfg<W>;
-  static std::atomic<bool> opted[64];
+  static std::atomic<unsigned long long> opted[64];
   int dev = 0, nsm = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
-  if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
-  if (!opted[dev].load()) {
-    e = cudaFuncSetAttribute(tc_gemm_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) return e;
-    opted[dev].store(true);
-  }
+  e = allow_shared((const void*)tc_gemm_kernel<W>, C::SMEM, opted);
+  if (e != cudaSuccess) return e;
   e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   if (e != cudaSuccess) return e;
   TcArgs q = a;
-  int* err = tc_err_ptr(dev);
+  int* err = tc_error_word();
   if (!err) return cudaErrorMemoryAllocation;
   void* err_dev = nullptr;
   e = cudaHostGetDevicePointer(&err_dev, err, 0);
@@ -606,10 +588,23 @@ cudaError_t launch_tc_gemm(const TcArgs& a, const CUtensorMap& map, cudaStream_t
   return a.w == 7 ? launch_tc_w<7>(a, map, s) : launch_tc_w<6>(a, map, s);
 }
 
+// In page-locked host memory that the kernels write directly: the host reads it
+// after a synchronisation without a copy.  One per device and context: a word
+// goes with its context.
 int* tc_error_word() {
+  static std::mutex mu;
+  static auto* words = new std::map<std::pair<int, unsigned long long>, int*>;
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
-  return tc_err_ptr(dev);
+  if (cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+  if (context_id() == 0 && cudaFree(nullptr) != cudaSuccess) return nullptr;  // a thread's first call
+  std::lock_guard<std::mutex> lk(mu);
+  int*& w = (*words)[{dev, context_id()}];
+  void* p = nullptr;
+  if (!w && cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) == cudaSuccess) {
+    w = static_cast<int*>(p);
+    *w = 0;
+  }
+  return w;
 }
 
 int tc_error_read_and_clear() {

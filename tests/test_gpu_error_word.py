@@ -1,8 +1,9 @@
 """The error word of the tcgen05 contraction's bounded waits: set here from the
-host, in place of a kernel whose wait ran out."""
+host, in place of a kernel whose wait ran out; and what else is kept per context."""
 import ctypes
 import os
 import subprocess
+import sys
 
 import pytest
 
@@ -48,3 +49,34 @@ def test_a_new_batch_or_server_leaves_it(fg, set_word):
     a.close()
     b.close()
     del s
+
+
+RESET = """
+import ctypes
+import numpy as np
+import falcon_gpu as fg
+
+def run(mode, nm=42):
+    fg.set_gemm_mode(mode)
+    b = fg.Batch([fg.make_params(65, nm, "SBDF3", ra=1e5 * (k + 1), dt=1e-6) for k in range(12)])
+    b.init_noise(range(12))
+    b.step(3)
+    out = b.get_state(11)["omg"]
+    b.close()
+    return out
+
+first = [run(m) for m in (0, 1, 3, 4, 5)]
+assert ctypes.CDLL("libcudart.so.13").cudaDeviceReset() == 0
+for m, x in zip((0, 1, 3, 4, 5), first):
+    assert np.array_equal(run(m), x), m
+run(4, 20)  # shapes that are measured anew
+print("ok")
+"""
+
+
+def test_after_a_device_reset(fg):
+    """The error word, the kernels' shared-memory limits and the autotuner's buffer
+    go with their context: a device that was reset steps on, with the same bits."""
+    r = subprocess.run([sys.executable, "-c", RESET], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, PYTHONPATH=PKG))
+    assert r.returncode == 0 and r.stdout.split()[-1] == "ok", (r.returncode, r.stdout, r.stderr[-2000:])
