@@ -4285,7 +4285,7 @@ struct ChebMats {
   ChebOp op[4];  // fwd, inv, d1, d2
 };
 std::mutex g_cheb_mu;
-std::map<int, ChebMats> g_cheb;
+std::map<std::tuple<int, unsigned long long, int>, ChebMats> g_cheb;  // by device, context id and size
 
 int2 fx_split(double a, int e) {  // a 2^(60 - e) rounded, as h 2^30 + l, l signed
   const long long t = std::llrint(std::ldexp(a, 60 - e)), h = (t + (1LL << 29)) >> 30;
@@ -4352,8 +4352,12 @@ bool cheb_fixed(const std::vector<double>& m, int n, bool fwd, int parity, std::
 }
 
 int cheb_mats(int n, ChebMats** out) {
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  if (context_id() == 0) CK(cudaFree(nullptr));  // a thread's first call
+  const auto key = std::make_tuple(dev, context_id(), n);
   std::lock_guard<std::mutex> lk(g_cheb_mu);
-  auto it = g_cheb.find(n);
+  auto it = g_cheb.find(key);
   if (it != g_cheb.end()) { *out = &it->second; return 0; }
   Cheb c = make_cheb(n, 0.35);
   const double C = std::sqrt(2.0 / (double)(n - 1));
@@ -4388,7 +4392,7 @@ int cheb_mats(int n, ChebMats** out) {
       return rc;
     o.fx.A = a; o.fx.D = d; o.fx.ex = e; o.fx.w = wk;
   }
-  auto res = g_cheb.emplace(n, mats);
+  auto res = g_cheb.emplace(key, mats);
   *out = &res.first->second;
   return 0;
 }

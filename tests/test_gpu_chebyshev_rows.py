@@ -11,9 +11,14 @@ a term at most; the mirrored rows' differences (below 2^-36 A_i) in 24 bits of
 30 bits of X: 2^-59 A_i X a term; the sum is rounded once, and so were the
 operator's elements, read back as columns of the identity (2^-53 each, of
 sum_k |A_ik x_k|).  So |error| <= 2^-52 sum_k |A_ik x_k| + 4 n 2^-59 A_i X."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
+from conftest import PKG
 from test_gpu_fixed_point_chebyshev import NAMES, call
 
 pytestmark = pytest.mark.gpu
@@ -55,3 +60,38 @@ def test_a_constant_has_no_derivative(fg, n):
         x[3, 0] = np.nan
         got = call(fg, fn, n, x)
         assert np.isnan(got[3].real).all() and np.array_equal(got[4], want[4])
+
+
+RESET = """
+import ctypes
+import numpy as np
+import falcon_gpu as fg
+
+rt = ctypes.CDLL("libcudart.so.13")
+x = np.random.default_rng(2).standard_normal((40, 33, 2))
+
+def run():
+    a, b = ctypes.c_void_p(), ctypes.c_void_p()
+    y = np.empty_like(x)
+    for p in (a, b):
+        assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(x.nbytes)) == 0
+    assert rt.cudaMemcpy(a, x.ctypes.data_as(ctypes.c_void_p), ctypes.c_size_t(x.nbytes), 1) == 0
+    fg.check(fg.lib().falcon_cheb_d1_dev(33, 40, a, b, None))
+    assert rt.cudaMemcpy(y.ctypes.data_as(ctypes.c_void_p), b, ctypes.c_size_t(x.nbytes), 2) == 0
+    return y
+
+first = run()
+assert rt.cudaDeviceReset() == 0
+spare = ctypes.c_void_p()
+assert rt.cudaMalloc(ctypes.byref(spare), ctypes.c_size_t(1 << 20)) == 0
+assert np.array_equal(run(), first)
+print("ok")
+"""
+
+
+def test_after_a_device_reset(fg):
+    """The operators go with their context: those of a size used before are made
+    again in a new one."""
+    r = subprocess.run([sys.executable, "-c", RESET], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, PYTHONPATH=PKG))
+    assert r.returncode == 0 and r.stdout.split()[-1] == "ok", (r.returncode, r.stdout, r.stderr[-2000:])
