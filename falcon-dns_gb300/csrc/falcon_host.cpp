@@ -4497,9 +4497,22 @@ size_t instance_bytes(const falcon_params& p) {
   return n;
 }
 
+// Device bytes of a request's operator set as admission counts them: the FP64
+// operators of an implicit scheme and every operator's fixed-point integers
+// (add_oz), not the slices.
 size_t opset_bytes(const falcon_params& p) {
   const size_t R = p.nr_max, M = p.nm_max + 1;
-  return 8 * (2 * R * R + M * R * R + M * 3 * R * R + 2 * R * R + 2 * R);
+  Scheme s;
+  scheme_weights(p.scheme_type, p.scheme_imp, p.scheme_exp, &s);
+  const OpKey k = key_of(p, s);
+  size_t n = 8 * (2 * R * R + M * R * R + M * 3 * R * R + 2 * R * R + 2 * R);
+  auto integers = [&](size_t rows, size_t nb) { n += nb * (rows * R * sizeof(int2) + (rows + R) * sizeof(int)); };
+  integers(R, 2);
+  integers(2 * R, 1);
+  if (k.type == FALCON_RK) integers(R, 2);
+  else integers(R, M), integers(3 * R, M);
+  if (k.needs_lap) integers(2 * R + 2, M);
+  return n;
 }
 
 // Request r's initial state into slot j of its group: the caller's fields,
