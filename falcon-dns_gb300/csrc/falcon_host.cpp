@@ -1518,8 +1518,9 @@ int run_path_once(Group* g, int cls, GemmArgs q, int path, bool reuse) {
 // device = the CUDA device name with blanks as '_' and "_sm<SM count>";
 // per_mode = 1 when the batch entries have their own X (sX != 0), 2 + n for n
 // merged row blocks, 16 + n for n products of one launch; reuse = 1
-// when X's slice planes were made by the contraction before; w = the slice
-// format (6 or 7); path 0 tiles (cost-model shape), 1 mma.sync, 2 tcgen05,
+// when X's slice planes were made by the contraction before; w = 60 + the slice
+// format (66 or 67; 6 or 7 where paths 0 and 3-5 were FP64 or other tiles: read,
+// and never met); path 0 tiles (cost-model shape), 1 mma.sync, 2 tcgen05,
 // 3/4/5 tiles of 16/32/64 columns; us_p = the measured
 // microseconds per contraction on path p (-1: not measured).
 struct TuneKey {
@@ -1537,6 +1538,7 @@ std::string g_tune_path;          // cache file ("" none)
 bool g_tune_env_checked = false;
 std::atomic<long long> g_tune_measured(0);
 constexpr const char* kTuneHeader = "falcon-contraction-tuning 2";
+constexpr int kTuneTiles = 60;  // bits of the tiles' integers: entries measured with other tiles don't match
 
 int tune_load_locked(const std::string& path) {
   std::ifstream f(path);
@@ -1647,7 +1649,7 @@ int time_fastest(Group* g, void* flush, cudaEvent_t a, cudaEvent_t b, const std:
 // X, are not measured: they take the fixed rule of mode 2.
 int tuned_path(Group* g, int cls, const GemmArgs& q, bool reuse, bool tc_ok, int fixed, int* path) {
   *path = fixed;
-  TuneKey k{device_tag(), q.rows, q.K, q.N, q.batch, q.oz_w, q.sX != 0 ? 1 : 0, reuse ? 1 : 0};
+  TuneKey k{device_tag(), q.rows, q.K, q.N, q.batch, kTuneTiles + q.oz_w, q.sX != 0 ? 1 : 0, reuse ? 1 : 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     if (!g_tune_env_checked) {
@@ -1841,7 +1843,7 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
   auto together = [&]() { return launch(g, cls, flops, [&]() { return launch_fx_gemm(all, g->stream); }); };
   if (!tiles) return apart();
   if (mode == 5) return together();
-  TuneKey k{device_tag(), v[0].rows, v[0].K, (int)cols, 1, all.oz_w, 16 + (int)v.size(), 0};
+  TuneKey k{device_tag(), v[0].rows, v[0].K, (int)cols, 1, kTuneTiles + all.oz_w, 16 + (int)v.size(), 0};
   int known = -1;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
@@ -1887,7 +1889,7 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
 // timed together.
 int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArgs& all, bool* merged) {
   *merged = all.N >= 16;
-  TuneKey k{device_tag(), all.rows, all.K, all.N, all.batch, all.oz_w, 2 + (int)v.size(), 0};
+  TuneKey k{device_tag(), all.rows, all.K, all.N, all.batch, kTuneTiles + all.oz_w, 2 + (int)v.size(), 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
     auto it = g_tune.find(k);

@@ -401,7 +401,9 @@ int falcon_set_gemm_mode(int mode);
  *   <device> <rows> <K> <N> <batch> <w> <per_mode> <reuse> <path> <us_0> <us_1> <us_2> <us_3> <us_4> <us_5>
  * device = CUDA device name with blanks as '_' plus "_sm<SM count>"
  * (falcon_device_tag); rows, K, N, batch = the contraction's shape (rows x K
- * operator, N columns per batch entry); w = slice format in bits (6 or 7);
+ * operator, N columns per batch entry); w = 60 + the slice format in bits (66 or 67;
+ * entries of 6 or 7 are of earlier libraries, whose paths 0 and 3-5 were other
+ * kernels: they are read and match nothing);
  * per_mode = 1 when every batch entry has its own columns (2 + n: n row
  * blocks of one operator, merged into one tcgen05 launch, path 2, or run on
  * the blocks' own path, path 0; 16 + n: n products of one launch of tiles,
