@@ -2631,20 +2631,35 @@ int group_set_columns(Group* g, const std::vector<HostRun>& runs) {
   return 0;
 }
 
-// The device's address of a host array of nb bytes when all of it is
-// page-locked and 16-byte aligned, else null.
+// The device's address of a host array of nb bytes when all of it lies in one
+// page-locked allocation and is 16-byte aligned, else null.  (Registered memory
+// is staged: the device may only be allowed to read it, and an array can begin
+// and end in two registrations with a gap in between.)
 double2* mapped_address(void* p, size_t nb) {
-  if (reinterpret_cast<uintptr_t>(p) & 15) return nullptr;
-  cudaPointerAttributes a{}, e{};
-  if (cudaPointerGetAttributes(&a, p) != cudaSuccess ||
-      cudaPointerGetAttributes(&e, static_cast<char*>(p) + nb - 1) != cudaSuccess) {
+  using GetAttribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+  static const GetAttribute get = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult st;
+    return cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 4000, cudaEnableDefault, &st) == cudaSuccess &&
+                   st == cudaDriverEntryPointSuccess
+               ? reinterpret_cast<GetAttribute>(f)
+               : nullptr;
+  }();
+  if (!get || (reinterpret_cast<uintptr_t>(p) & 15)) return nullptr;
+  unsigned flags = 0;
+  if (cudaHostGetFlags(&flags, p) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
-  if (a.type != cudaMemoryTypeHost || e.type != cudaMemoryTypeHost || !a.devicePointer || !e.devicePointer ||
-      static_cast<char*>(e.devicePointer) - static_cast<char*>(a.devicePointer) != (ptrdiff_t)(nb - 1))
+  const CUdeviceptr at = reinterpret_cast<CUdeviceptr>(p);
+  CUdeviceptr dev = 0, start = 0;
+  size_t size = 0;
+  if (get(&dev, CU_POINTER_ATTRIBUTE_DEVICE_POINTER, at) != CUDA_SUCCESS || !dev ||
+      get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, at) != CUDA_SUCCESS ||
+      get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, at) != CUDA_SUCCESS || dev < start || size < nb ||
+      dev - start > size - nb)
     return nullptr;
-  return static_cast<double2*>(a.devicePointer);
+  return reinterpret_cast<double2*>(dev);
 }
 
 // One instance's fields to the host: one kernel writes them all into the
