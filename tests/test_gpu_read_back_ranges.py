@@ -46,3 +46,24 @@ def test_partly_registered_arrays(fg):
         for at in registered:
             assert rt.cudaHostUnregister(ctypes.c_void_p(at)) == 0
         b.close()
+
+
+def test_overlapping_arrays(fg):
+    """Two fields into one page-locked array: the later one's values, as with a copy per field."""
+    import torch
+    R, Nm = 65, 170
+    n = 2 * R * (Nm + 1)
+    b = fg.Batch([fg.make_params(R, Nm, "CNAB2", ra=1e5, dt=1e-6)])
+    b.init_noise([1])
+    b.step(2)
+    want = {k: v.view(np.float64).ravel() for k, v in b.get_state(0).items()}
+    ptr = ctypes.POINTER(ctypes.c_double)
+    a = torch.zeros(n + n // 2, dtype=torch.float64, pin_memory=True).numpy()
+    at = lambda v: v.ctypes.data_as(ptr)  # noqa: E731
+    for _ in range(20):
+        a[:] = np.nan
+        fg.check(fg.lib().falcon_batch_get_state(b.h, 0, at(a), at(a), None, None, at(a)))
+        assert np.array_equal(a[:n], want["psi"]) and np.isnan(a[n:]).all()
+        fg.check(fg.lib().falcon_batch_get_state(b.h, 0, at(a[n // 2:]), None, at(a), None, None))
+        assert np.array_equal(a[:n], want["up"]) and np.array_equal(a[n:], want["T"][n // 2:])
+    b.close()
