@@ -758,6 +758,9 @@ cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int
 cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.rows <= 0 || g.N <= 0 || g.batch <= 0) return cudaSuccess;
   if (g.K > 257 || !g.fx) return cudaErrorInvalidValue;
+  // mode 0 is shared out over the whole grid, of which blocks past a narrower
+  // product's columns leave early
+  if (g.follow.kind == kVelocity && (g.njobs || g.nsub || g.nextra)) return cudaErrorInvalidValue;
   if (g.N <= 8 && !g.njobs) {
     // k shares until there are 448 threads an SM (above that one, a warp at least), rows
     // in even blocks of at most 256 threads, of fewer while SMs are without two
