@@ -13,10 +13,7 @@ namespace falcon {
 // points 157 / 132 / 134; 129 x 8 of 1536 points 200 / 165 / 144.
 cudaError_t launch_nonlin_8(const NonlinArgs& a, cudaStream_t s) {
   if (a.plan.pfa) return launch_nonlin_s<8, false, 4, 1, 1>(a, s);
-  int dev = 0, nsm = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  if ((long)a.R * a.B <= 2 * nsm || a.plan.P > 1152) return launch_nonlin_s<8, true, 4, 1, 2>(a, s);
+  if ((long)a.R * a.B <= 2 * sm_count() || a.plan.P > 1152) return launch_nonlin_s<8, true, 4, 1, 2>(a, s);
   if (a.plan.P > 640) return launch_nonlin_s<8, true, 2, 1, 4>(a, s);
   return launch_nonlin_s<8, true, 1, 2, 4>(a, s);
 }

@@ -719,9 +719,7 @@ cudaError_t launch_ncol(const GemmArgs& g, const TileShape& t, cudaStream_t s) {
 }
 
 TileShape tile_shape(const GemmArgs& g) {
-  int dev = 0, nsm = 152;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const int nsm = sm_count();
   // shapes are memoised per problem size: the search runs on the host once
   struct Memo { int rows, K, N, total, batch, nsm, ncol; TileShape t; };
   thread_local std::unordered_map<unsigned long long, Memo> memo;
@@ -766,10 +764,10 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
     // in even blocks of at most 256 threads, of fewer while SMs are without two
     // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.0, 7.8, 7.8; 65 x 65 x 8,
     // 171 entries 21.2, 17.0, 14.0, 18.1; 291 x 97 x 2, 341 entries 30.3, 32.4, 34.4, 44.7)
-    const int nz = entries(g);
-    const int KS = (int)std::min(8L, std::max((31L + g.rows) / g.rows, 152L * 448 / ((long)g.rows * nz)));
+    const int nz = entries(g), nsm = sm_count();
+    const int KS = (int)std::min(8L, std::max((31L + g.rows) / g.rows, nsm * 448L / ((long)g.rows * nz)));
     int nb = (g.rows + 256 / KS - 1) / (256 / KS);
-    while ((long)nb * nz < 2 * 152 && (g.rows + nb - 1) / nb > 16) ++nb;
+    while ((long)nb * nz < 2 * nsm && (g.rows + nb - 1) / nb > 16) ++nb;
     const int RB = (g.rows + nb - 1) / nb;
     const dim3 grid((g.rows + RB - 1) / RB, nz);
     auto run = [&](auto kernel, int nc) {
@@ -803,11 +801,11 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
 cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s) {
   if (g.n < 3 || g.n > 257 || g.ncol < 1 || g.ncol > 65535) return cudaErrorInvalidValue;
   const int h = (g.n + 1) / 2;
-  const long cols = (long)g.ncol * g.nop;
-  if (cols < 4 * 152) return h <= 128 ? launch_fx_columns_dir<1, 8>(g, s) : launch_fx_columns_dir<2, 8>(g, s);
+  const long cols = (long)g.ncol * g.nop, nsm = sm_count();
+  if (cols < 4 * nsm) return h <= 128 ? launch_fx_columns_dir<1, 8>(g, s) : launch_fx_columns_dir<2, 8>(g, s);
   if (h <= 32) return launch_fx_columns_dir<1, 32>(g, s);
   if (h <= 64) {
-    if (cols < 32 * 152) return launch_fx_columns_dir<1, 16>(g, s);
+    if (cols < 32 * nsm) return launch_fx_columns_dir<1, 16>(g, s);
     return (h + 11) / 12 * 120 <= 11 * h ? launch_fx_columns_dir<3, 16>(g, s) : launch_fx_columns_dir<2, 16>(g, s);
   }
   return h <= 96 ? launch_fx_columns_dir<3, 32>(g, s) : launch_fx_columns_dir<3, 16>(g, s);

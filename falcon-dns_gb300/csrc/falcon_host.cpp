@@ -1411,16 +1411,8 @@ bool attach_group(const Group* g, GemmArgs* q) {
 // faster on the mma.sync kernel that slices its own X columns, whose
 // per-launch cost is lower; both give the same bits.
 bool tc_worth_it(const GemmArgs& q) {
-  static std::atomic<int> nsm{0};
-  int n = nsm.load();
-  if (n == 0) {
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-      n = 152;
-    nsm.store(n);
-  }
   const long tiles = (long)q.batch * ((q.rows + kTcBM - 1) / kTcBM) * ((q.N + kTcBN - 1) / kTcBN);
-  return tiles >= 2L * n;
+  return tiles >= 2L * sm_count();
 }
 
 // The tcgen05 contraction of one GEMM with an attached slice view.

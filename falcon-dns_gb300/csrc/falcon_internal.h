@@ -427,6 +427,7 @@ struct AsmArgs {
 // The current CUDA context's id (0: unknown); a device that was reset has a new
 // one, and what was kept for the old one went with it (falcon_host.cpp).
 unsigned long long context_id();
+int sm_count();  // of the current device (falcon_kernels.cu)
 // A kernel's limit of dynamic shared memory, set once per context; done: 64
 // entries of the caller's.
 inline cudaError_t allow_shared(const void* kernel, int bytes, std::atomic<unsigned long long>* done) {

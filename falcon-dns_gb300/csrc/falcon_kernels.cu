@@ -27,6 +27,17 @@ cudaError_t launch_nonlin_8(const NonlinArgs& a, cudaStream_t s);
 cudaError_t launch_nonlin_17(const NonlinArgs& a, cudaStream_t s);
 cudaError_t launch_nonlin_31(const NonlinArgs& a, cudaStream_t s);
 
+int sm_count() {
+  static std::atomic<int> known[64];
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  const bool slot = dev >= 0 && dev < 64;
+  if (slot && (n = known[dev].load()) > 0) return n;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 152;
+  if (slot) known[dev].store(n);
+  return n;
+}
+
 cudaError_t launch_nonlin(const NonlinArgs& a, cudaStream_t s) {
   int maxp = 0;
   for (int i = 0; i < a.plan.nrad; ++i) maxp = a.plan.rad[i] > maxp ? a.plan.rad[i] : maxp;
@@ -298,15 +309,7 @@ cudaError_t launch_gemm(const GemmArgs& g, cudaStream_t s) {
     else dfma_gemv_kernel<8><<<grid, 32, sm, s>>>(g);
     return cudaGetLastError();
   }
-  static int nsm_dev[64] = {0};
-  int dev = 0;
-  cudaGetDevice(&dev);
-  int nsm = (dev >= 0 && dev < 64) ? nsm_dev[dev] : 0;
-  if (nsm == 0) {
-    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-    if (nsm <= 0) nsm = 152;
-    if (dev >= 0 && dev < 64) nsm_dev[dev] = nsm;
-  }
+  const int nsm = sm_count();
   // shapes are memoised per (rows, N, batch, SM count, column width asked
   // for): the search runs on the host once per problem size
   struct Memo { int rows, N, batch, nsm, ncol; TileShape t; };
@@ -363,7 +366,7 @@ struct CellGrid {
 };
 static CellGrid cell_grid(int R, int M, int B) {
   const long row = (long)M * B;
-  const int block = (long)R * ((row + 127) / 128) < 2 * 152 ? 64 : 128;
+  const int block = (long)R * ((row + 127) / 128) < 2 * sm_count() ? 64 : 128;
   return {dim3((unsigned)((row + block - 1) / block), R), block};
 }
 
