@@ -179,34 +179,42 @@ __device__ __forceinline__ void copy16(void* dst, const void* src, bool valid) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 16 : 0) : "memory");
 }
 
-// One thread per (entry, column k): half the exponent of its largest element.
+// One warp per (entry, column k): half the exponent of its largest element.
 __global__ void fx_weight_kernel(const double* A, long lda, long sA, int rows, int K, int nb, int* wk) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
+  const long t = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   if (t >= (long)nb * K) return;
   const int z = (int)(t / K), k = (int)(t - (long)z * K);
   const double* a = A + (size_t)z * sA + (size_t)k * lda;
   int m = kNone;
-  for (int r = 0; r < rows; ++r) {
+  for (int r = threadIdx.x & 31; r < rows; r += 32) {
     const int e = exponent_of(a[r], 0);
     if (e != INT32_MAX) m = max(m, e);
   }
-  wk[t] = m == kNone ? kNoWeight : m >> 1;
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0) wk[t] = m == kNone ? kNoWeight : m >> 1;
 }
 
-// One thread per (entry, row): the row's exponent, then its integers, in the
-// operator's own layout.
-__global__ void fx_operator_kernel(const double* A, long lda, long sA, int rows, int K, int nb, const int* wk,
-                                   int2* out, int* ex) {
-  const long t = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (t >= (long)nb * rows) return;
-  const int z = (int)(t / rows), r = (int)(t - (long)z * rows);
+// Eight threads per (entry, row): the row's exponent, then its integers, in the
+// operator's own layout.  (One thread a row waited for 2 K loads one after
+// another: 40 us an operator of 65 points.)
+__global__ void __launch_bounds__(256) fx_operator_kernel(const double* A, long lda, long sA, int rows, int K, int nb,
+                                                          const int* wk, int2* out, int* ex) {
+  __shared__ int part[8][32];
+  const long t = blockIdx.x * 32L + threadIdx.x;
+  const bool act = t < (long)nb * rows;
+  const int z = act ? (int)(t / rows) : 0, r = act ? (int)(t - (long)z * rows) : 0;
   const double* a = A + (size_t)z * sA + r;
   const int* w = wk + (size_t)z * K;
   int m = kNone;
-  for (int k = 0; k < K; ++k) m = max(m, exponent_of(a[(size_t)k * lda], -w[k]));
-  ex[(size_t)z * lda + r] = mark_of(m);
+  if (act)
+    for (int k = threadIdx.y; k < K; k += 8) m = max(m, exponent_of(a[(size_t)k * lda], -w[k]));
+  part[threadIdx.y][threadIdx.x] = m;
+  __syncthreads();
+  if (!act) return;
+  for (int i = 0; i < 8; ++i) m = max(m, part[i][threadIdx.x]);
+  if (threadIdx.y == 0) ex[(size_t)z * lda + r] = mark_of(m);
   int2* o = out + (size_t)z * sA + r;
-  for (int k = 0; k < K; ++k) o[(size_t)k * lda] = split_of(a[(size_t)k * lda], -w[k], scale_of(m));
+  for (int k = threadIdx.y; k < K; k += 8) o[(size_t)k * lda] = split_of(a[(size_t)k * lda], -w[k], scale_of(m));
 }
 
 // X panel of a block in shared memory, xs[k * (ncol + PAD) + c] (staged as
@@ -748,8 +756,8 @@ cudaError_t launch_fx_operator(const double* A, long lda, long sA, int rows, int
                                int* ex, cudaStream_t s) {
   const long n = (long)nb * rows, m = (long)nb * K;
   if (n <= 0) return cudaSuccess;
-  fx_weight_kernel<<<(unsigned)((m + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk);
-  fx_operator_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk, out, ex);
+  fx_weight_kernel<<<(unsigned)((m + 3) / 4), 128, 0, s>>>(A, lda, sA, rows, K, nb, wk);
+  fx_operator_kernel<<<(unsigned)((n + 31) / 32), dim3(32, 8), 0, s>>>(A, lda, sA, rows, K, nb, wk, out, ex);
   return cudaGetLastError();
 }
 

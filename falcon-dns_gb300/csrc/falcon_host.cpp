@@ -226,6 +226,7 @@ struct OpSet {
     bool tmap_ok = false;
   };
   std::vector<Oz> oz;
+  char* views = nullptr;  // their arrays
   size_t bytes = 0;
   ~OpSet() {
     // the last group holding the set is gone, but a kernel of any group's
@@ -234,7 +235,7 @@ struct OpSet {
     cudaFree(D1p); cudaFree(Lp); cudaFree(ST); cudaFree(G); cudaFree(U); cudaFree(LAP);
     cudaFree(inv_r); cudaFree(inv_r2); cudaFree(wq); cudaFree(d1_0); cudaFree(d1_R);
     cudaFree(D1c); cudaFree(Lc);
-    for (auto& o : oz) { cudaFree(o.s); cudaFree(o.ex); cudaFree(o.fx); cudaFree(o.fx_ex); cudaFree(o.fx_w); }
+    cudaFree(views);
   }
 };
 
@@ -245,31 +246,61 @@ struct OpSet {
 // bits.
 std::atomic<int> g_gemm_mode{4};
 
-// Slices and fixed-point integers of one column-major operator array (rows x
-// K, lda = rows, nb entries of stride sA) for the contraction kernels.
-int add_oz(OpSet* ops, const double* base, int rows, int K, int nb, long sA) {
-  if (!base || K > 257) return 0;
-  OpSet::Oz o;
-  o.base = base; o.lda = rows; o.sA = sA; o.rows = rows; o.K = K; o.nb = nb;
-  o.rowsP = oz_rows_padded(rows);
-  o.KP = ((K + 15) / 16) * 16;
-  o.w = oz_width_for(o.KP);
-  const size_t ns = (size_t)nb * oz_slices(o.w) * o.rowsP * o.KP, ne = (size_t)nb * o.rowsP;
-  CK(cudaMalloc(&o.s, ns * sizeof(uint16_t)));
-  CK(cudaMalloc(&o.ex, ne * sizeof(int)));
-  CK(cudaMemset(o.s, 0, ns * sizeof(uint16_t)));
-  CK(cudaMemset(o.ex, 0, ne * sizeof(int)));
-  CK(launch_oz_slice_rows(base, rows, sA, rows, K, nb, o.s, o.ex, o.rowsP, o.KP, o.w, 0));
-  o.tmap_ok = tc_stage_layout_check(o.w, o.KP) == 0 &&
-              tc_make_operator_map(&o.tmap, o.s, nb, oz_slices(o.w), o.KP, o.rowsP) == 0;
-  const size_t nf = (size_t)(nb - 1) * sA + (size_t)rows * K;
-  CK(cudaMalloc(&o.fx, nf * sizeof(int2)));
-  CK(cudaMalloc(&o.fx_ex, (size_t)nb * rows * sizeof(int)));
-  CK(cudaMalloc(&o.fx_w, (size_t)nb * K * sizeof(int)));
-  CK(launch_fx_operator(base, rows, sA, rows, K, nb, o.fx_w, o.fx, o.fx_ex, 0));
-  ops->bytes += ns * sizeof(uint16_t) + ne * sizeof(int) + nf * sizeof(int2) + (size_t)nb * rows * sizeof(int) +
-                (size_t)nb * K * sizeof(int);
-  ops->oz.push_back(o);
+// Slices and fixed-point integers of column-major operator arrays (rows x K, lda
+// = rows, nb entries of stride sA) for the contraction kernels, all in one
+// allocation: a variable time step makes the operators anew whenever it changes.
+// A step that does, CNAB2: 33 x 43 2.05 ms with the slices alone, an allocation an
+// array; 2.19 with the integers too; 1.98 with one allocation; 65 x 86 5.63, 5.76
+// and 5.64; 65 x 171 8.18, 8.31 and 8.10.
+struct OpView {
+  const double* base;
+  int rows, K, nb;
+  long sA;
+};
+int add_views(OpSet* ops, std::initializer_list<OpView> views) {
+  size_t zeroed = 0, rest = 0;  // bytes that start as zeros, others
+  auto take = [](size_t* at, size_t n) {
+    const size_t a = *at;
+    *at += (n + 255) / 256 * 256;
+    return a;
+  };
+  struct Place { size_t s, ex, fx, fx_ex, fx_w; };
+  std::vector<Place> at;
+  const size_t first = ops->oz.size();
+  for (const OpView& v : views) {
+    if (!v.base || v.K > 257) continue;
+    OpSet::Oz o;
+    o.base = v.base; o.lda = v.rows; o.sA = v.sA; o.rows = v.rows; o.K = v.K; o.nb = v.nb;
+    o.rowsP = oz_rows_padded(v.rows);
+    o.KP = ((v.K + 15) / 16) * 16;
+    o.w = oz_width_for(o.KP);
+    const size_t nb = v.nb;
+    Place q;
+    q.s = take(&zeroed, nb * oz_slices(o.w) * o.rowsP * o.KP * sizeof(uint16_t));
+    q.ex = take(&zeroed, nb * o.rowsP * sizeof(int));
+    q.fx = take(&rest, ((nb - 1) * v.sA + (size_t)v.rows * v.K) * sizeof(int2));
+    q.fx_ex = take(&rest, nb * v.rows * sizeof(int));
+    q.fx_w = take(&rest, nb * v.K * sizeof(int));
+    at.push_back(q);
+    ops->oz.push_back(o);
+  }
+  if (at.empty()) return 0;
+  CK(cudaMalloc(&ops->views, zeroed + rest));
+  ops->bytes += zeroed + rest;
+  CK(cudaMemset(ops->views, 0, zeroed));
+  for (size_t i = 0; i < at.size(); ++i) {
+    OpSet::Oz& o = ops->oz[first + i];
+    char *z = ops->views, *r = z + zeroed;
+    o.s = reinterpret_cast<uint16_t*>(z + at[i].s);
+    o.ex = reinterpret_cast<int*>(z + at[i].ex);
+    o.fx = reinterpret_cast<int2*>(r + at[i].fx);
+    o.fx_ex = reinterpret_cast<int*>(r + at[i].fx_ex);
+    o.fx_w = reinterpret_cast<int*>(r + at[i].fx_w);
+    CK(launch_oz_slice_rows(o.base, o.rows, o.sA, o.rows, o.K, o.nb, o.s, o.ex, o.rowsP, o.KP, o.w, 0));
+    o.tmap_ok = tc_stage_layout_check(o.w, o.KP) == 0 &&
+                tc_make_operator_map(&o.tmap, o.s, o.nb, oz_slices(o.w), o.KP, o.rowsP) == 0;
+    CK(launch_fx_operator(o.base, o.rows, o.sA, o.rows, o.K, o.nb, o.fx_w, o.fx, o.fx_ex, 0));
+  }
   return 0;
 }
 
@@ -670,11 +701,10 @@ int build_opset(const OpKey& k, std::shared_ptr<OpSet>* out, const HostFactors* 
   }
   {
     const long RR = (long)R * R;
-    if ((rc = add_oz(ops.get(), ops->D1p, R, R, 1, RR)) || (rc = add_oz(ops.get(), ops->Lp, R, R, 1, RR)) ||
-        (rc = add_oz(ops.get(), ops->ST, R, R, M, RR)) || (rc = add_oz(ops.get(), ops->G, 3 * R, R, M, 3 * RR)) ||
-        (rc = add_oz(ops.get(), ops->U, 2 * R, R, 1, 2 * RR)) ||
-        (rc = add_oz(ops.get(), ops->LAP, 2 * R + 2, R, M, (long)(2 * R + 2) * R)) ||
-        (rc = add_oz(ops.get(), ops->D1c, R, R, 1, RR)) || (rc = add_oz(ops.get(), ops->Lc, R, R, 1, RR)))
+    if ((rc = add_views(ops.get(), {{ops->D1p, R, R, 1, RR}, {ops->Lp, R, R, 1, RR}, {ops->ST, R, R, M, RR},
+                                    {ops->G, 3 * R, R, M, 3 * RR}, {ops->U, 2 * R, R, 1, 2 * RR},
+                                    {ops->LAP, 2 * R + 2, R, M, (long)(2 * R + 2) * R}, {ops->D1c, R, R, 1, RR},
+                                    {ops->Lc, R, R, 1, RR}})))
       return rc;
     CK(cudaDeviceSynchronize());
   }
@@ -4513,7 +4543,7 @@ size_t instance_bytes(const falcon_params& p) {
 
 // Device bytes of a request's operator set as admission counts them: the FP64
 // operators of an implicit scheme and every operator's fixed-point integers
-// (add_oz), not the slices.
+// (add_views), not the slices.
 size_t opset_bytes(const falcon_params& p) {
   const size_t R = p.nr_max, M = p.nm_max + 1;
   Scheme s;
