@@ -169,6 +169,10 @@ __device__ __forceinline__ void follow_modes(const FxFollow& f) {
   for (int i = blk * nthr + threadIdx.x; i < f.R * f.B; i += step) follow_mode0(f, i / f.B, i % f.B);
 }
 
+__device__ __forceinline__ void copy4(void* dst, const void* src) {
+  const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(saddr), "l"(src) : "memory");
+}
 __device__ __forceinline__ void copy8(void* dst, const void* src, bool valid) {
   const unsigned saddr = (unsigned)__cvta_generic_to_shared(dst);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(saddr), "l"(src), "r"(valid ? 8 : 0) : "memory");
@@ -219,8 +223,8 @@ __global__ void __launch_bounds__(256) fx_operator_kernel(const double* A, long 
 
 // X panel of a block in shared memory, xs[k * (ncol + PAD) + c] (staged as
 // doubles, complete when this is called): column exponents in cex, integers in
-// place.  w: the operator's weights (or null: fwd); part: blockDim.x words; spare:
-// leading bits left free.
+// place.  w: the operator's weights, staged with it (or null: fwd); part:
+// blockDim.x words; spare: leading bits left free.
 template <int PAD = 0>
 __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const int* w, int* cex, int* part,
                                               int spare = 0) {
@@ -228,7 +232,7 @@ __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const
   const bool act = j < J;
   int m = kNone;
   if (act) {
-    for (int k = j; k < K; k += J) m = max(m, exponent_of(xs[k * st + c], w ? __ldg(w + k) : 0));
+    for (int k = j; k < K; k += J) m = max(m, exponent_of(xs[k * st + c], w ? w[k] : 0));
     part[tid] = m;
   }
   __syncthreads();
@@ -237,7 +241,7 @@ __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const
     if (m != INT32_MAX && m != kNone) m += spare;
     if (j == 0) cex[c] = mark_of(m);
     for (int k = j; k < K; k += J) {
-      const int2 v = split_of(xs[k * st + c], w ? __ldg(w + k) : 0, scale_of(m));
+      const int2 v = split_of(xs[k * st + c], w ? w[k] : 0, scale_of(m));
       reinterpret_cast<int2*>(xs)[k * st + c] = v;
     }
   }
@@ -259,6 +263,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   int2* as = reinterpret_cast<int2*>(fsm + (size_t)g.K * NCOL);       // [2][kFxKC][rows_blk]
   int* cex = reinterpret_cast<int*>(as + 2 * kFxKC * rows_blk);       // [NCOL]
   int* part = cex + NCOL;                                             // [nthr]
+  int* ws = part + nthr;                                              // [K]
   const int z = blockIdx.z;
   int N = g.N, nblk = blockIdx.x, e = z, b0 = g.follow.b0;
   const int nz = g.nsub ? g.nsub * g.batch : g.batch;
@@ -296,6 +301,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rg = lane / CP, cp = lane - rg * CP;
   const int rw = (warp * RG + rg) * RPT;
+  for (int k = threadIdx.x; k < g.K; k += nthr) copy4(ws + k, w + k);
   {
     constexpr int KW = NCOL >= 32 ? 1 : 32 / NCOL, HW = NCOL >= 32 ? NCOL / 32 : 1;  // k, column halves per warp
     for (int i = warp; i < (g.K + KW - 1) / KW * HW; i += nw) {
@@ -319,7 +325,7 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
   issue(0, as);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  convert_panel(xs, g.K, NCOL, w, cex, part);
+  convert_panel(xs, g.K, NCOL, ws, cex, part);
   Sum acc[RPT][2];
 #pragma unroll
   for (int i = 0; i < RPT; ++i) acc[i][0] = acc[i][1] = Sum{0, 0, 0};
@@ -400,7 +406,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
   Wide* parts = reinterpret_cast<Wide*>(fsm);                       // [KS][NC][RB]
   double* xd = reinterpret_cast<double*>(parts + KS * NC * RB);     // [K][NC]
   __shared__ int cex[NC];
-  __shared__ int part[256];
+  __shared__ int part[256], ws[257];
   constexpr int U = 8;
   const int z = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x;
   const int kp = tid / RB, rl = tid - kp * RB, row = blockIdx.x * RB + rl;
@@ -435,8 +441,10 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
     const int k = i / NC, c = i - k * NC;
     xd[i] = c < N ? X[(size_t)k * ldx + c] : 0.0;
   }
+  for (int k = tid; k < g.K; k += nthr) ws[k] = __ldg(w + k);
+  const int ea = row < g.rows ? __ldg(aex + row) : 0;
   __syncthreads();
-  convert_panel(xd, g.K, NC, w, cex, part);
+  convert_panel(xd, g.K, NC, ws, cex, part);
   const int2* xs = reinterpret_cast<const int2*>(xd);
   Sum acc[NC];
 #pragma unroll
@@ -473,7 +481,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
   auto column = [&](int c) {
     Wide s{0, 0};
     for (int q = 0; q < KS; ++q) s = add(s, parts[(q * NC + c) * RB + rl]);
-    return value_of(s, aex[row], cex[c], g.alpha);
+    return value_of(s, ea, cex[c], g.alpha);
   };
   double* y = Y ? Y : output_row(g, z, row);
   for (int c = 2 * kp; c < N; c += 2 * KS) {
@@ -497,25 +505,31 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
 // (30 bits of x), added at its scale: outputs are those of the dense operator.
 //   FWD: X0, X1 = x_p +- x_{n-1-p};  out_{2j} = S0 + D0, out_{2j+1} = S1 + D1
 //   else X0, X1 = x_{2p}, x_{2p+1};  out_j = S0 + S1, out_{n-1-j} = +-(S0 - S1) + D
-// A block takes NCOL real columns (re and im side by side) of one operator;
-// loads, outputs (through shared memory) and the operator's chunks of 8 p are
+// A block takes NCOL real columns (re and im side by side) of one operator, and
+// all its output pairs or, with few columns, a share of them (grid z: not in
+// place); loads, outputs (through shared memory) and the operator's chunks of 8 p are
 // coalesced.  Bound: the integer multiply-adds (61 % of that pipe's cycles, 16
-// to 20 warps an SM); 65 points, 10944 columns: fwd 56 us, d1 and d2 93 us
+// to 20 warps an SM); 65 points, 10944 columns: fwd 62 us, d1 and d2 103 us
 // (one FP64 dot product a thread: 684 us for the three).
-constexpr int kFxPC = 8;  // p per staged operator chunk
+constexpr int kFxPC = 8;  // p per staged operator chunk (g.pc: this, or all of them in one)
 template <int RPT, int NCOL, bool FWD>
 __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__ FxColumns g) {
   constexpr int RG = 64 / NCOL, CP = NCOL / 2, ST = NCOL + 2;  // ST: columns' stores hit every bank
   extern __shared__ __align__(16) double fsm[];
-  const int n = g.n, h = (n + 1) / 2, nthr = blockDim.x, nw = nthr >> 5, hb = nw * RG * RPT;
+  const int n = g.n, h = (n + 1) / 2, nthr = blockDim.x, nw = nthr >> 5, hb = nw * RG * RPT, PC = g.pc;
   double* xs = fsm;                                                  // [n + 1][ST]
-  int4* as = reinterpret_cast<int4*>(fsm + (size_t)(n + 1) * ST);    // [2][kFxPC][hb]
-  int2* ds = reinterpret_cast<int2*>(as + 2 * kFxPC * hb);           // [2][kFxPC][hb]
-  int* cex = reinterpret_cast<int*>(ds + 2 * kFxPC * hb);            // [NCOL]
+  int4* as = reinterpret_cast<int4*>(fsm + (size_t)(n + 1) * ST);    // [1 or 2][PC][hb]
+  const int nbuf = PC < h ? 2 : 1;
+  int2* ds = reinterpret_cast<int2*>(as + nbuf * PC * hb);           // the same
+  int* cex = reinterpret_cast<int*>(ds + nbuf * PC * hb);            // [NCOL]
   int* part = cex + NCOL;                                            // [nthr]
+  int* ws = part + nthr;                                             // [n]
   const FxColumnsOp& op = g.op[blockIdx.y];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, c0 = blockIdx.x * CP;
   const int rg = lane / CP, cp = lane - rg * CP, rw = (warp * RG + rg) * RPT;
+  const int j0 = blockIdx.z * hb, hv = min(hb, h - j0);  // the block's output pairs
+  if (!FWD)
+    for (int k = threadIdx.x; k < n; k += nthr) copy4(ws + k, op.w + k);
   for (int c = warp; c < CP; c += nw) {
     const bool ok = c0 + c < g.ncol;
     const double2* x = g.in + (size_t)(ok ? c0 + c : 0) * n;
@@ -523,18 +537,20 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
   auto issue = [&](int p0, int buf) {
-    const int pc = min(kFxPC, h - p0);
-    for (int i = threadIdx.x; i < pc * h; i += nthr) {
-      const int p = i / h, j = i - p * h, o = (buf * kFxPC + p) * hb + j;
-      copy16(as + o, op.A + (size_t)p0 * h + i, true);
-      copy8(ds + o, op.D + (size_t)p0 * h + i, true);
+    const int pc = min(PC, h - p0);
+    for (int i = threadIdx.x; i < pc * hv; i += nthr) {
+      const int p = i / hv, j = i - p * hv, o = (buf * PC + p) * hb + j;
+      const size_t at = (size_t)(p0 + p) * h + j0 + j;
+      copy16(as + o, op.A + at, true);
+      copy8(ds + o, op.D + at, true);
     }
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   issue(0, 0);
+  const int4 ex = __ldg(op.ex + min(j0 + rw, h - 1));
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
-  convert_panel<ST - NCOL>(xs, n, NCOL, op.w, cex, part, FWD);
+  convert_panel<ST - NCOL>(xs, n, NCOL, FWD ? nullptr : ws, cex, part, FWD);
   if (FWD) {
     for (int i = threadIdx.x; i < n / 2 * NCOL; i += nthr) {
       const int p = i / NCOL, c = i - p * NCOL;
@@ -556,17 +572,17 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
       d0[i][c] = d1[i][c] = 0;
     }
   int cur = 0;
-  for (int p0 = 0; p0 < h; p0 += kFxPC) {
-    const int pc = min(kFxPC, h - p0);
-    if (p0 + kFxPC < h) {
-      issue(p0 + kFxPC, cur ^ 1);
+  for (int p0 = 0; p0 < h; p0 += PC) {
+    const int pc = min(PC, h - p0);
+    if (p0 + PC < h) {
+      issue(p0 + PC, cur ^ 1);
       asm volatile("cp.async.wait_group 1;\n" ::: "memory");
     } else {
       asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     }
     __syncthreads();
-    const int4* Aw = as + cur * kFxPC * hb + rw;
-    const int2* Dw = ds + cur * kFxPC * hb + rw;
+    const int4* Aw = as + cur * PC * hb + rw;
+    const int2* Dw = ds + cur * PC * hb + rw;
     const int4* xp = reinterpret_cast<const int4*>(xs) + cp;
     auto one = [&](int pp) {
       const int p = p0 + pp;
@@ -608,9 +624,9 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   }
 #pragma unroll
   for (int i = 0; i < RPT; ++i) {
-    const int j = rw + i;
-    if (j >= h) break;
-    const int4 e = __ldg(op.ex + j);
+    const int j = j0 + rw + i;
+    if (rw + i >= hv) break;
+    const int4 e = i == 0 ? ex : __ldg(op.ex + j);
     double y[2], z[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -633,26 +649,39 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   __syncthreads();
   for (int c = warp; c < CP && c0 + c < g.ncol; c += nw) {
     double2* y = op.out + (size_t)(c0 + c) * n;
-    for (int k = lane; k < n; k += 32) y[k] = *reinterpret_cast<const double2*>(xs + k * ST + 2 * c);
+    auto store = [&](int k) { y[k] = *reinterpret_cast<const double2*>(xs + k * ST + 2 * c); };
+    if (gridDim.z == 1) {
+      for (int k = lane; k < n; k += 32) store(k);
+    } else if (FWD) {
+      for (int k = 2 * j0 + lane; k < min(2 * (j0 + hv), n); k += 32) store(k);
+    } else {
+      for (int j = j0 + lane; j < j0 + hv; j += 32) {
+        store(j);
+        store(n - 1 - j);
+      }
+    }
   }
 }
 
 template <int RPT, int NCOL, bool FWD>
-cudaError_t launch_fx_columns_shape(const FxColumns& g, cudaStream_t s) {
-  const int h = (g.n + 1) / 2, per = 64 / NCOL * RPT, nw = std::max(2, (h + per - 1) / per), hb = nw * per;
-  const size_t smem = (size_t)(g.n + 1) * (NCOL + 2) * 8 + 2 * kFxPC * hb * 24 + (NCOL + 32 * nw) * 4;
+cudaError_t launch_fx_columns_shape(FxColumns g, int most, cudaStream_t s) {
+  const int h = (g.n + 1) / 2, per = 64 / NCOL * RPT, nw = std::min(most, std::max(2, (h + per - 1) / per)), hb = nw * per;
+  // the operator in one chunk where it is small: no barriers between chunks
+  g.pc = (h <= 32 || NCOL == 8) && h * hb * 24 <= 64 * 1024 ? h : kFxPC;
+  const size_t smem = (size_t)(g.n + 1) * (NCOL + 2) * 8 + (g.pc < h ? 2 : 1) * g.pc * hb * 24 + (NCOL + 32 * nw + g.n) * 4;
   if (smem > 48 * 1024) {
     const cudaError_t e = cudaFuncSetAttribute(fx_columns_kernel<RPT, NCOL, FWD>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return e;
   }
-  const dim3 grid((g.ncol + NCOL / 2 - 1) / (NCOL / 2), g.nop);
+  const dim3 grid((g.ncol + NCOL / 2 - 1) / (NCOL / 2), g.nop, (h + hb - 1) / hb);
   fx_columns_kernel<RPT, NCOL, FWD><<<grid, 32 * nw, smem, s>>>(g);
   return cudaGetLastError();
 }
 template <int RPT, int NCOL>
-cudaError_t launch_fx_columns_dir(const FxColumns& g, cudaStream_t s) {
-  return g.fwd ? launch_fx_columns_shape<RPT, NCOL, true>(g, s) : launch_fx_columns_shape<RPT, NCOL, false>(g, s);
+cudaError_t launch_fx_columns_dir(const FxColumns& g, cudaStream_t s, int most = 16) {
+  return g.fwd ? launch_fx_columns_shape<RPT, NCOL, true>(g, most, s)
+               : launch_fx_columns_shape<RPT, NCOL, false>(g, most, s);
 }
 
 // Batch entries of a launch: those of the product, or of each of its
@@ -672,7 +701,7 @@ cudaError_t launch_fx_tile(const GemmArgs& g, int nw, int row_blocks, cudaStream
   const cudaError_t e = allow_shared((const void*)fx_tile_kernel<RPT, NCOL>, 227 * 1024, opted);
   if (e != cudaSuccess) return e;
   const int rows_blk = nw * (64 / NCOL) * RPT;
-  const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw) * 4;
+  const size_t smem = ((size_t)g.K * NCOL + 2 * kFxKC * rows_blk) * 8 + (size_t)(NCOL + 32 * nw + g.K) * 4;
   const dim3 grid((unsigned)column_blocks(g, NCOL), row_blocks, entries(g));
   fx_tile_kernel<RPT, NCOL><<<grid, 32 * nw, smem, s>>>(g);
   return cudaGetLastError();
@@ -696,7 +725,7 @@ TileShape pick_shape(const GemmArgs& g, int nsm) {
         for (int rpt = 1; rpt <= 7; ++rpt) {
           const int rows_blk = nw * rg * rpt;
           if ((long)rb * rows_blk < g.rows || (long)(rb - 1) * rows_blk >= g.rows || rows_blk > 256) continue;
-          const long smem = ((long)g.K * ncol + 2 * kFxKC * rows_blk) * 8 + (ncol + 32 * nw) * 4;
+          const long smem = ((long)g.K * ncol + 2 * kFxKC * rows_blk) * 8 + (ncol + 32 * nw + g.K) * 4;
           if (smem > 227 * 1024) continue;
           const long blocks = cb * rb;
           const long fit = std::max(1L, std::min({220L * 1024 / smem, 64L / nw, 65536L / (32L * nw * (40 + 12 * rpt))}));
@@ -801,19 +830,27 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
 // Shape: NCOL real columns a block, RPT output pairs a thread (64 / NCOL x RPT
 // pairs a warp).  Few columns: small blocks and one pair a thread, for more
 // blocks and shorter chains (65 points, us of fwd / d1d2 at <1, 8>, <1, 16>, <3, 16>:
-// 300 columns 10.9/11.1, 12.5/11.6, 16.6/16.6; 1000 columns 12.9/19.3, 12.5/17.1,
-// 16.6/19.2; 10944 columns 64/113, 60/103, 56/93).  Many: one pair a thread
-// up to 32 pairs (17 points, 20000 columns <1, 32> 17/27, <3, 16> 29/48), above
-// that the shape that pads least (97 points, 10000 columns <2, 16> 109/183,
-// <3, 16> 133/215; 129 points, 2000 columns <3, 32> 40/71, <3, 16> 48/80).
+// 300 columns 10.4/10.5, 12.6/12.5, 18.6/16.6; 1000 columns 12.5/18.6, 12.7/18.6,
+// 18.7/20.6; 10944 columns 66/115, 74/119, 62/103; 17 points, 700 columns, fwd 6.3,
+// 6.4 and, at <1, 32>, 8.3), and while SMs are idle the pairs of a column on several
+// of them (fwd of 257 points, 4 columns 52 -> 23, 129 points 21 -> 14.5).  Many: one
+// pair a thread up to 32 pairs (17 points, 20000 columns <1, 16> 21/35, <1, 32>
+// 21/31, <3, 16> 35/53), above that the shape that pads least (97 points, 10000
+// columns <2, 16> 122/216, <3, 16> 142/225; 129 points, 2000 columns <3, 32> 45/76,
+// <3, 16> 52/86; 193 points, 3000 columns <3, 32> 215/315, <3, 16> 176/254).
 cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s) {
   if (g.n < 3 || g.n > 257 || g.ncol < 1 || g.ncol > 65535) return cudaErrorInvalidValue;
   const int h = (g.n + 1) / 2;
   const long cols = (long)g.ncol * g.nop, nsm = sm_count();
-  if (cols < 4 * nsm) return h <= 128 ? launch_fx_columns_dir<1, 8>(g, s) : launch_fx_columns_dir<2, 8>(g, s);
+  if (cols < 4 * nsm) {
+    // pairs shared out over blocks of at least two warps while SMs are idle
+    const long blocks = (g.ncol + 3) / 4 * (long)g.nop, share = std::max(1L, nsm / blocks), warps = (h + 7) / 8;
+    if (g.apart && share > 1) return launch_fx_columns_dir<1, 8>(g, s, (int)std::min(16L, std::max(2L, (warps + share - 1) / share)));
+    return h <= 128 ? launch_fx_columns_dir<1, 8>(g, s) : launch_fx_columns_dir<2, 8>(g, s);
+  }
+  if (h <= 64 && cols < 32 * nsm) return launch_fx_columns_dir<1, 16>(g, s);
   if (h <= 32) return launch_fx_columns_dir<1, 32>(g, s);
   if (h <= 64) {
-    if (cols < 32 * nsm) return launch_fx_columns_dir<1, 16>(g, s);
     return (h + 11) / 12 * 120 <= 11 * h ? launch_fx_columns_dir<3, 16>(g, s) : launch_fx_columns_dir<2, 16>(g, s);
   }
   return h <= 96 ? launch_fx_columns_dir<3, 32>(g, s) : launch_fx_columns_dir<3, 16>(g, s);

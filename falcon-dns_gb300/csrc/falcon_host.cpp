@@ -4321,12 +4321,10 @@ double falcon_fp64_mma_peak_gflops(void) { return measure_fp64_mma_peak(); }
 // fwd = t^T diag(c') / ((n-1) C) (C = sqrt(2/(n-1))).
 // ---------------------------------------------------------------------------
 namespace {
-struct ChebOp {
-  double* m = nullptr;  // dense, for sizes past the fixed-point form
-  FxColumnsOp fx{};
-};
-struct ChebMats {
-  ChebOp op[4];  // fwd, inv, d1, d2
+struct ChebMats {  // fwd, inv, d1, d2
+  const double* dense[4];
+  FxColumnsOp fx[4];
+  bool fixed;  // fx is made
 };
 std::mutex g_cheb_mu;
 std::map<std::tuple<int, unsigned long long, int>, ChebMats> g_cheb;  // by device, context id and size
@@ -4416,25 +4414,42 @@ int cheb_mats(int n, ChebMats** out) {
       m[2][(size_t)i * n + j] = C * c.D[i + (size_t)n * j] * h;
       m[3][(size_t)i * n + j] = C * c.D2[i + (size_t)n * j] * h;
     }
-  ChebMats mats;
-  int rc;
+  ChebMats mats{};
+  std::vector<int4> A[4], ex[4];
+  std::vector<int2> D[4];
+  std::vector<int> w[4];
+  mats.fixed = n <= 257;
+  for (int q = 0; q < 4 && mats.fixed; ++q) {
+    mats.fx[q].sign = q == 2 ? -1 : 1;
+    mats.fixed = cheb_fixed(m[q], n, q == 0, mats.fx[q].sign, &A[q], &D[q], &ex[q], &w[q]);
+  }
+  // one allocation and one copy (16-byte steps)
+  std::vector<int4> all;
+  auto put = [&](const void* v, size_t bytes) {
+    const size_t at = all.size();
+    all.resize(at + (bytes + 15) / 16);
+    std::memcpy(&all[at], v, bytes);
+    return at;
+  };
+  size_t at[4][5] = {};
   for (int q = 0; q < 4; ++q) {
-    std::vector<int4> A, ex;
-    std::vector<int2> D;
-    std::vector<int> w;
-    ChebOp& o = mats.op[q];
-    o.fx.sign = q == 2 ? -1 : 1;
-    if (n > 257 || !cheb_fixed(m[q], n, q == 0, o.fx.sign, &A, &D, &ex, &w)) {
-      if ((rc = upload(&o.m, m[q], nullptr))) return rc;
-      continue;
-    }
-    int4 *a, *e;
-    int2* d;
-    int* wk = nullptr;
-    if ((rc = upload(&a, A, nullptr)) || (rc = upload(&d, D, nullptr)) || (rc = upload(&e, ex, nullptr)) ||
-        (q && (rc = upload(&wk, w, nullptr))))
-      return rc;
-    o.fx.A = a; o.fx.D = d; o.fx.ex = e; o.fx.w = wk;
+    at[q][0] = put(m[q].data(), sizeof(double) * m[q].size());
+    if (!mats.fixed) continue;
+    at[q][1] = put(A[q].data(), sizeof(int4) * A[q].size());
+    at[q][2] = put(D[q].data(), sizeof(int2) * D[q].size());
+    at[q][3] = put(ex[q].data(), sizeof(int4) * ex[q].size());
+    at[q][4] = put(w[q].data(), sizeof(int) * w[q].size());
+  }
+  int4* base = nullptr;
+  const int rc = upload(&base, all, nullptr);
+  if (rc) return rc;
+  for (int q = 0; q < 4; ++q) {
+    mats.dense[q] = reinterpret_cast<const double*>(base + at[q][0]);
+    FxColumnsOp& o = mats.fx[q];
+    o.A = base + at[q][1];
+    o.D = reinterpret_cast<const int2*>(base + at[q][2]);
+    o.ex = base + at[q][3];
+    o.w = q ? reinterpret_cast<const int*>(base + at[q][4]) : nullptr;
   }
   auto res = g_cheb.emplace(key, mats);
   *out = &res.first->second;
@@ -4442,25 +4457,34 @@ int cheb_mats(int n, ChebMats** out) {
 }
 
 // Operator `first` to out[0] and, with count 2, `first` + 1 to out[1].
+// Dense FP64 products for the smallest sizes, where a thread's few multiply-adds
+// end before the fixed-point form's conversions and barriers do (us, FP64 / fixed
+// point: 3 points, 16 columns 4.0 / 5.2, 5000 columns 6.2 / 6.4; 9 points, 43
+// columns 4.3 / 6.2, 1500 columns 6.2 / 6.4, 2500 8.4 / 6.4; 13 points, 64 columns
+// 4.3 / 6.2, 1500 6.3 / 6.4; 17 points, 16 columns 6.2 / 6.2).  In place only the
+// fixed-point form is safe.
 int cheb_apply(int first, int count, int nr, int ncol, const double* in, double* const* out, void* stream) {
   if (nr < 3 || ncol < 1 || !in || !out[0]) return fail(FALCON_EINVAL, "invalid Chebyshev transform arguments");
   ChebMats* m = nullptr;
   int rc = cheb_mats(nr, &m);
   if (rc) return rc;
-  FxColumns g{};
-  g.n = nr; g.ncol = ncol; g.fwd = first == 0;
-  g.in = reinterpret_cast<const double2*>(in);
-  for (int q = 0; q < count; ++q) {
-    const ChebOp& o = m->op[first + q];
-    double2* y = reinterpret_cast<double2*>(out[q]);
-    if (o.m) {
-      CK(launch_apply_cols(nr, ncol, o.m, g.in, y, (cudaStream_t)stream));
-      continue;
-    }
-    g.op[g.nop] = o.fx;
-    g.op[g.nop++].out = y;
+  const double2* x = reinterpret_cast<const double2*>(in);
+  double2* y[2] = {reinterpret_cast<double2*>(out[0]), reinterpret_cast<double2*>(out[count - 1])};
+  const long span = 2L * nr * ncol;
+  const bool few = nr <= 13 && (long)nr * ncol <= 20000;
+  const bool apart = !spans_overlap(in, span, out[0], span) && !spans_overlap(in, span, out[count - 1], span);
+  if (!m->fixed || (few && apart)) {
+    CK(launch_apply_cols(nr, ncol, count, m->dense[first], m->dense[first + count - 1], x, y[0], y[1],
+                         (cudaStream_t)stream));
+    return 0;
   }
-  if (g.nop) CK(launch_fx_columns(g, (cudaStream_t)stream));
+  FxColumns g{};
+  g.n = nr; g.ncol = ncol; g.nop = count; g.fwd = first == 0; g.apart = apart; g.in = x;
+  for (int q = 0; q < count; ++q) {
+    g.op[q] = m->fx[first + q];
+    g.op[q].out = y[q];
+  }
+  CK(launch_fx_columns(g, (cudaStream_t)stream));
   return 0;
 }
 }  // namespace

@@ -474,7 +474,6 @@ cudaError_t launch_gather_instance(int R, int M, int B, int b, const double2* sr
 cudaError_t launch_extract_mode0(int R, int M, int B, const double2* src, double* dst, cudaStream_t s);
 cudaError_t launch_getrs_batched(int n, int nsys, int nrhs, const double* lu, const int* ipiv,
                                  double* b, cudaStream_t s);
-// out[c] = A in[c] for ncol complex columns of length n (A real row-major).
 // Chebyshev transforms of complex columns in fixed point (n <= 257): what the
 // kernel reads of an operator (cheb_fixed) and the call.
 struct FxColumnsOp {
@@ -486,12 +485,15 @@ struct FxColumnsOp {
   int sign;
 };
 struct FxColumns {
-  int n, ncol, nop, fwd;
+  int n, ncol, nop, fwd, apart, pc;  // apart: no output overlaps the input; pc: the launcher's
   const double2* in;
   FxColumnsOp op[2];
 };
 cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s);
-cudaError_t launch_apply_cols(int n, int ncol, const double* A, const double2* in, double2* out, cudaStream_t s);
+// out[c] = A in[c] in FP64 for ncol complex columns of length n, one or two (nop)
+// real row-major operators.
+cudaError_t launch_apply_cols(int n, int ncol, int nop, const double* A0, const double* A1, const double2* in,
+                              double2* out0, double2* out1, cudaStream_t s);
 // Instance-column remap of a [rows][B] array (ew doubles per element).
 cudaError_t launch_remap_cols(const double* src, double* dst, size_t rows, int bs, int bd, int ew, const int* map,
                               cudaStream_t s);

@@ -796,9 +796,13 @@ double measure_fp64_peak() {
 namespace falcon {
 
 // out[c][i] = sum_k A[i*n + k] * in[c][k] for complex columns (A real,
-// row-major n x n): the Chebyshev transforms as dense operators.
-__global__ void apply_cols_kernel(int n, int ncol, const double* A, const double2* in, double2* out) {
+// row-major n x n): the Chebyshev transforms as dense operators, A1 and out1 for
+// the second row of the grid.
+__global__ void apply_cols_kernel(int n, int ncol, const double* A0, const double* A1, const double2* in,
+                                  double2* out0, double2* out1) {
   const int c = blockIdx.y;
+  const double* A = blockIdx.z ? A1 : A0;
+  double2* out = blockIdx.z ? out1 : out0;
   const double2* x = in + (size_t)c * n;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double sr = 0.0, si = 0.0;
@@ -812,9 +816,10 @@ __global__ void apply_cols_kernel(int n, int ncol, const double* A, const double
   }
 }
 
-cudaError_t launch_apply_cols(int n, int ncol, const double* A, const double2* in, double2* out, cudaStream_t s) {
-  dim3 grid((n + 127) / 128, ncol);
-  apply_cols_kernel<<<grid, 128, 0, s>>>(n, ncol, A, in, out);
+cudaError_t launch_apply_cols(int n, int ncol, int nop, const double* A0, const double* A1, const double2* in,
+                              double2* out0, double2* out1, cudaStream_t s) {
+  dim3 grid((n + 127) / 128, ncol, nop);
+  apply_cols_kernel<<<grid, 128, 0, s>>>(n, ncol, A0, A1, in, out0, out1);
   return cudaGetLastError();
 }
 

@@ -62,6 +62,40 @@ def test_a_constant_has_no_derivative(fg, n):
         assert np.isnan(got[3].real).all() and np.array_equal(got[4], want[4])
 
 
+@pytest.mark.parametrize("n,few", [(3, 6666), (9, 2222), (13, 1538), (14, 40), (33, 20), (129, 43), (257, 128)])
+def test_few_columns(fg, n, few):
+    """Both sides of the rule that gives calls of up to 13 points to FP64 products,
+    pairs shared out over blocks, and in place, which does neither:
+    within the bound above, or (n + 1) 2^-53 sum_k |A_ik x_k| of an FP64 sum on
+    top of it, of the same operator times the columns; d1 and d2 together as apart."""
+    rng = np.random.default_rng(n)
+    x = rng.standard_normal((few + 1, n)) + 1j * rng.standard_normal((few + 1, n))
+    some = np.unique(np.r_[0:4, few - 4:few])
+    for q, fn in enumerate(NAMES):
+        A = operator(fg, n, fn)
+        top = np.abs(A).max(0)
+        w = np.where(top > 0, np.floor_divide(np.frexp(top)[1], 2), -1000) if q else np.zeros(n, int)
+        amax = np.abs(A * np.exp2(-np.maximum(w, -999).astype(float))).max(1)
+        xp = x[some]
+        size = np.abs(xp.real) + np.abs(xp.imag)
+        tol = (n + 4) * 2.0 ** -53 * (size @ np.abs(A).T) + 4 * n * 2.0 ** -59 * np.outer(
+            (size * np.exp2(w.astype(float))).max(1), amax)
+        want = xp.astype(np.clongdouble) @ A.astype(np.clongdouble).T
+        for y in (call(fg, fn, n, x[:few]), call(fg, fn, n, x), in_place(fg, fn, n, x[:few])):
+            assert (np.abs(y[some].real - want.real) <= tol).all() and (np.abs(y[some].imag - want.imag) <= tol).all(), fn
+    for c in (few, few + 1):
+        d1, d2 = call(fg, "falcon_cheb_d1d2_dev", n, x[:c], 2)
+        assert np.array_equal(d1, call(fg, NAMES[2], n, x[:c])) and np.array_equal(d2, call(fg, NAMES[3], n, x[:c]))
+
+
+def in_place(fg, fn, n, x):
+    import torch
+    y = torch.from_numpy(np.ascontiguousarray(x).view(np.float64)).cuda()
+    fg.check(getattr(fg.lib(), fn)(n, x.shape[0], y.data_ptr(), y.data_ptr(), None))
+    torch.cuda.synchronize()
+    return y.cpu().numpy().view(np.complex128)
+
+
 RESET = """
 import ctypes
 import numpy as np
