@@ -1,10 +1,10 @@
 // Fixed-point arithmetic of the azimuthal transforms: complex values as two
 // 64-bit integers at a power of two shared by a radial line's transform and
 // renewed before every stage (block floating point), |V| < 2^61 in modulus,
-// multiplied by Q62 constants (round(c 2^62)) with 32-bit multiply-adds.  GB300 issues an FP64 instruction every 64 cycles per sub-partition
-// and a 32-bit integer one every 2, so a 64-bit integer add (2 instructions)
-// and a product with a constant (7) cost a fraction of their FP64 forms,
-// and 61 bits against one scale leave the transform's rounding below that of
+// multiplied by Q62 constants (round(c 2^62)) with 32-bit multiply-adds.  GB300
+// issues an FP64 instruction every 64 cycles per sub-partition and a 32-bit
+// integer one every 2, so a 64-bit integer add (2 instructions) and a product
+// with a constant (7) cost a fraction of their FP64 forms, and 61 bits against one scale leave the transform's rounding below that of
 // FP64 butterflies.  Host and device: the CPU tests run these butterflies.
 #pragma once
 #include <stdint.h>
@@ -247,7 +247,7 @@ template <> struct FxDft<31> {
       -4558505550962299988LL, -4324618396573163188LL, -3913680856907234956LL, -3342516763121549146LL,
       -2634509640324623222LL, -1818645383311068024LL, -928325570622998360LL};
 };
-constexpr long long kFxSqrtHalf = 3260954456333195554LL, kFxCos16 = 4260642322793532498LL, kFxSin16 = 1764815834521887442LL;  // sqrt(1/2), cos and sin(pi/8)
+constexpr long long kFxSqrtHalf = 3260954456333195554LL;  // sqrt(1/2)
 constexpr long long kFxSqrt5Q = 2578010857022246788LL;  // sqrt(5)/4
 
 // Forward DFT of length p in registers, v_j <- sum_q v_q exp(-2 pi i j q/p),
@@ -270,7 +270,7 @@ FALCON_HD void fx_dft3(longlong2& v0, longlong2& v1, longlong2& v2) {
 }
 template <int p>
 FALCON_HD void fx_dft(longlong2 (&v)[p]) {
-  static_assert((p >= 2 && p <= 8) || p == 16, "register butterflies");
+  static_assert(p >= 2 && p <= 8, "register butterflies");
   if constexpr (p == 2) {
     const longlong2 a = v[0], b = v[1];
     v[0] = fx_add(a, b);
@@ -310,9 +310,9 @@ FALCON_HD void fx_dft(longlong2 (&v)[p]) {
     v[1] = fx_sub(w1, z1);
     v[2] = fx_add(w2, z2);
     v[5] = fx_sub(w2, z2);
-  } else if constexpr (p == 8 || p == 16) {
+  } else if constexpr (p == 8) {
     // one decimation-in-frequency split: even outputs from the sums, odd
-    // ones from the differences turned by exp(-2 pi i j/p)
+    // ones from the differences turned by exp(-2 pi i j/8)
     constexpr int h = p / 2;
     constexpr FxC r = fx_const(kFxSqrtHalf);
     longlong2 t[h], u[h];
@@ -325,29 +325,9 @@ FALCON_HD void fx_dft(longlong2 (&v)[p]) {
       return fx_make(fx_mul(fx_prep(z.x + z.y), r), fx_mul(fx_prep(z.y - z.x), r));
     };
     auto turn2 = [&](longlong2 z) { return fx_make(z.y, -z.x); };  // -i
-    if constexpr (p == 8) {
-      u[1] = turn1(u[1]);
-      u[2] = turn2(u[2]);
-      u[3] = turn2(turn1(u[3]));
-    } else {
-      constexpr FxC c = fx_const(kFxCos16), sn = fx_const(kFxSin16), ns = fx_const(-kFxSin16);
-      auto turnc = [&](longlong2 z) {  // exp(-i pi/8)
-        const FxMul x = fx_prep(z.x), y = fx_prep(z.y);
-        return fx_make(fx_mul2(x, c, y, sn), fx_mul2(y, c, x, ns));
-      };
-      auto turns = [&](longlong2 z) {  // exp(-3 i pi/8)
-        const FxMul x = fx_prep(z.x), y = fx_prep(z.y);
-        constexpr FxC nc = fx_const(-kFxCos16);
-        return fx_make(fx_mul2(x, sn, y, c), fx_mul2(y, sn, x, nc));
-      };
-      u[1] = turnc(u[1]);
-      u[2] = turn1(u[2]);
-      u[3] = turns(u[3]);
-      u[4] = turn2(u[4]);
-      u[5] = turn2(turnc(u[5]));
-      u[6] = turn2(turn1(u[6]));
-      u[7] = turn2(turns(u[7]));
-    }
+    u[1] = turn1(u[1]);
+    u[2] = turn2(u[2]);
+    u[3] = turn2(turn1(u[3]));
     fx_dft<h>(t);
     fx_dft<h>(u);
 #pragma unroll
