@@ -31,8 +31,9 @@ namespace {
 // sums stay below 0.9 2^22 (p = 31: sum over pairs and products of |digit
 // of c| 256), so the sums are exact and the accumulator's bits are
 // 0x4b400000 + sum, an integer with no conversion instruction.  The dropped
-// pairs weigh 3 units a product at most, 0.4 rms (tests/test_balanced_digits.py);
-// a line's largest value has 2^56 units or more in every stage.
+// pairs weigh 3 units a product at most, 0.4 rms (tests/test_balanced_digits.py),
+// of values whose largest is 2^54 (radix 23 to 31) or 2^55 units going in: grids
+// of 345 and 1023 points 5e-16 of a result's norm, of 255 and 429 2e-16.
 // ---------------------------------------------------------------------------
 constexpr int kFxS = 7;
 constexpr int kFxMagic = 0x4b400000;  // bits of 1.5 2^23
