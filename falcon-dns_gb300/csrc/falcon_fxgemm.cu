@@ -9,7 +9,7 @@
 // 2^30 + l with l signed.  Per product
 //   ha hx 2^60 + (ha lx + la hx) 2^30
 // is summed in two 64-bit integers and a word for the first one's carries
-// (|h| <= 2^30 and |l| <= 2^29: exact for 4 products between carries).  la lx is
+// (|h| <= 2^30 and |l| <= 2^29: exact for 7 products between carries).  la lx is
 // left out: 2^-62 of the largest product at most, what the operands' rounding
 // leaves out.  The sum is rounded once to FP64.  Sums of integers do not depend
 // on their order, so results depend neither on the tile nor on the launch: the
@@ -33,10 +33,12 @@
 // 6e-14 (3e-11); the vorticity solve of a run 5.7e-16, 1.3e-16 (2.7e-16).
 //
 // Bound: latency for the narrow forms (the radial and per-mode products of a
-// few instances), the integer multiply-add pipe for the tiles.  Against FP64
-// FMA, us with L2 cold: 97 x 97, 342 modes, 2 columns 44 -> 17; 33 x 33, 43
-// modes, 2 columns 14 -> 8; 65 x 65, 688 columns 22 -> 11; 65 x 65, 43776 columns
-// 316 -> 111 (84 on tcgen05, which the autotuner takes there).
+// few instances), the integer multiply-add pipe for the tiles.  FP64 FMA -> this, us
+// with L2 cold: 97 x 97, 342 modes, 2 columns 22 -> 18, 1026 modes, 6 columns 180 ->
+// 57; 33 x 33, 43 modes, 2 columns 10.6 -> 8.5; 65 x 65, 688 columns 14 -> 12, 43776
+// columns 317 -> 122 (84 on tcgen05, which the autotuner takes there); 129 x 129,
+// 11040 columns 324 -> 127.  (With 58 and 59 bits and carries every 16 k the large
+// ones took 114 and 120; with carries every 4 k 126 and 129.)
 //
 // The operators' integers are made once per operator set
 // (launch_fx_operator); X is converted by each block for its own columns.
@@ -54,9 +56,9 @@ namespace falcon {
 namespace {
 
 constexpr int kBits = 60, kLow = 30;      // of a row's and a column's integers, of their low halves
-constexpr int kCarry = 4;                 // products between carries
+constexpr int kCarry = 7;                 // products between carries, at most
 constexpr int kFollowRows = 6;           // deepest tiles that do what follows a product (deeper ones would spill)
-constexpr int kFxKC = 16;                // k per staged operator chunk
+constexpr int kFxKC = 2 * kCarry;         // k per staged operator chunk
 constexpr int kBad = INT32_MIN;          // exponent of a row or column with an Inf or NaN
 constexpr int kNone = -100000;           // exponent of a zero
 constexpr int kNoWeight = -30000;        // of a column of zeros: below every other
@@ -250,7 +252,7 @@ __device__ __forceinline__ void convert_panel(double* xs, int K, int ncol, const
 
 // Tile: a block covers NCOL columns and nw * RG * RPT rows, RG = 64 / NCOL;
 // lane = (row group rg, column pair cp).  The X panel (all of K) stays in
-// shared memory, the operator is staged in double-buffered chunks of 16 k.
+// shared memory, the operator is staged in double-buffered chunks of 14 k.
 // With g.njobs, several products of one shape (rows, K) in one launch: the
 // grid's column blocks run through the jobs.
 template <int RPT, int NCOL>
@@ -398,8 +400,8 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
 // sums meet in shared memory, where the threads of a row take its column pairs.
 // Bound by latency for one small run, then by issue.  With 32 rows and eight
 // shares in every block two thirds of the instructions were for converting X
-// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 52 us, 291 x 97 x 6 256 ->
-// 113, 291 x 97 x 2, 341 entries 40 -> 30, 195 x 65 x 8, 170 entries 32 -> 22.
+// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 57 us, 291 x 97 x 6 256 ->
+// 123, 291 x 97 x 2, 341 entries 40 -> 30, 195 x 65 x 8, 170 entries 32 -> 29.
 template <int NC>
 __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ GemmArgs g, int RB, int KS) {
   extern __shared__ __align__(16) double fsm[];
@@ -463,7 +465,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
         add_product(acc[c], av[u], make_int2(x.x, x.y));
         add_product(acc[c + 1], av[u], make_int2(x.z, x.w));
       }
-      if (u % kCarry == kCarry - 1 && u < U - 1) {
+      if (u == 3) {
 #pragma unroll
         for (int c = 0; c < NC; ++c) carry(acc[c]);
       }
@@ -547,7 +549,8 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
     asm volatile("cp.async.commit_group;\n" ::: "memory");
   };
   issue(0, 0);
-  const int4 ex = __ldg(op.ex + min(j0 + rw, h - 1));
+  // (few columns: ahead of the products; the wider shapes lack the registers)
+  const int4 ex = NCOL == 8 ? __ldg(op.ex + min(j0 + rw, h - 1)) : make_int4(0, 0, 0, 0);
   asm volatile("cp.async.wait_group 1;\n" ::: "memory");
   __syncthreads();
   convert_panel<ST - NCOL>(xs, n, NCOL, FWD ? nullptr : ws, cex, part, FWD);
@@ -609,8 +612,8 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
         }
       }
     };
-    for (int p4 = 0; p4 < pc; p4 += kCarry) {
-      const int pe = min(p4 + kCarry, pc);
+    for (int p4 = 0; p4 < pc; p4 += 4) {
+      const int pe = min(p4 + 4, pc);
 #pragma unroll 2
       for (int pp = p4; pp < pe; ++pp) one(pp);
 #pragma unroll
@@ -626,7 +629,7 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
   for (int i = 0; i < RPT; ++i) {
     const int j = j0 + rw + i;
     if (rw + i >= hv) break;
-    const int4 e = i == 0 ? ex : __ldg(op.ex + j);
+    const int4 e = NCOL == 8 && i == 0 ? ex : __ldg(op.ex + j);
     double y[2], z[2];
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
@@ -775,8 +778,7 @@ TileShape tile_shape(const GemmArgs& g) {
 
 // Whether launch_fx_gemm can do what follows g: every narrow form, and tiles of
 // up to kFollowRows rows a thread (a batch of 12 of 33 x 86: a step 63 -> 56 us,
-// 59 with 3 rows at most; with the code in tiles of 7, which spill, 129 x 129 x
-// 2752 columns go from 131 to 134 us).
+// 59 with 3 rows at most; tiles of 7 would spill).
 bool fx_follows(const GemmArgs& g) {
   return g.N <= 8 || tile_shape(g).rpt <= kFollowRows;
 }
@@ -799,8 +801,8 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.N <= 8 && !g.njobs) {
     // k shares until there are 448 threads an SM (above that one, a warp at least), rows
     // in even blocks of at most 256 threads, of fewer while SMs are without two
-    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 11.9, 9.0, 7.8, 7.8; 65 x 65 x 8,
-    // 171 entries 21.2, 17.0, 14.0, 18.1; 291 x 97 x 2, 341 entries 30.3, 32.4, 34.4, 44.7)
+    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 12.0, 10.9, 8.9, 7.9; 65 x 65 x 8,
+    // 171 entries 26.3, 20.1, 16.0, 20.1; 291 x 97 x 2, 341 entries 30.3, 32.4, 37.5, 47.4)
     const int nz = entries(g), nsm = sm_count();
     const int KS = (int)std::min(8L, std::max((31L + g.rows) / g.rows, nsm * 448L / ((long)g.rows * nz)));
     int nb = (g.rows + 256 / KS - 1) / (256 / KS);
