@@ -137,6 +137,24 @@ def test_uneven_products(product, n, ncol):
                 assert np.linalg.norm(err.astype(float)) <= np.linalg.norm(ref.astype(float)), (op, kind)
 
 
+@pytest.mark.parametrize("ncol", [2, 7, 40])
+@pytest.mark.parametrize("n", [3, 7, 8, 14, 15, 64, 129, 256, 257])
+def test_largest_sums(product, n, ncol):
+    """Every element the largest its scale holds, of one sign (columns 0), alternating
+    (1) and with opposite low halves (the others): sums at the limit of the carries,
+    within the element bound."""
+    a = np.full((1, 33, n), 1.0 - 2.0 ** -53)
+    x = np.full((1, n, ncol), -(1.0 - 2.0 ** -53))
+    x[0, :, 1] *= np.where(np.arange(n) % 2, 1.0, -1.0)
+    x[0, :, 2:] -= 2.0 ** -30 + 2.0 ** -31
+    a[0, 1::2] -= 2.0 ** -31
+    exact = a[0].astype(np.longdouble) @ x[0].astype(np.longdouble)
+    err = np.abs(product(1, a, x)[0] - exact)
+    w = np.floor_divide(np.frexp(np.abs(a[0]).max(0))[1], 2)
+    assert (w == 0).all()
+    assert (err <= 3 * n * 2.0 ** -60 * 1.01 + 2.0 ** -52 * np.abs(exact)).all()
+
+
 @pytest.mark.parametrize("ncol", [2, 40])
 def test_fp64_products(product, ncol):
     """launch_gemm, which modes 0 and 2 and operators without integers take: |error| <= (K + 1) 2^-53 sum |a x|."""
