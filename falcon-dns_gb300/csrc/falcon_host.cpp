@@ -1584,6 +1584,23 @@ int tune_load_locked(const std::string& path) {
   return 0;
 }
 
+// The decision held for a shape, or null; the first lookup of a process reads the
+// environment's file.
+int tune_find_locked(const TuneKey& k, const TuneEntry** e) {
+  if (!g_tune_env_checked) {
+    g_tune_env_checked = true;
+    const char* env = std::getenv("FALCON_TUNE_CACHE");
+    if (g_tune_path.empty() && env && *env) {
+      g_tune_path = env;
+      const int rc = tune_load_locked(g_tune_path);
+      if (rc) return rc;
+    }
+  }
+  const auto it = g_tune.find(k);
+  *e = it == g_tune.end() ? nullptr : &it->second;
+  return 0;
+}
+
 void tune_store_locked(const TuneKey& k, const TuneEntry& e) {
   if (g_tune_path.empty()) return;
   std::FILE* f = std::fopen(g_tune_path.c_str(), "a+");
@@ -1674,18 +1691,11 @@ int tuned_path(Group* g, int cls, const GemmArgs& q, bool reuse, bool tc_ok, int
   TuneKey k{device_tag(), q.rows, q.K, q.N, q.batch, kTuneTiles + q.oz_w, q.sX != 0 ? 1 : 0, reuse ? 1 : 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    if (!g_tune_env_checked) {
-      g_tune_env_checked = true;
-      const char* env = std::getenv("FALCON_TUNE_CACHE");
-      if (g_tune_path.empty() && env && *env) {
-        g_tune_path = env;
-        int rc = tune_load_locked(g_tune_path);
-        if (rc) return rc;
-      }
-    }
-    auto it = g_tune.find(k);
-    if (it != g_tune.end()) {
-      *path = it->second.path;
+    const TuneEntry* known = nullptr;
+    const int rc = tune_find_locked(k, &known);
+    if (rc) return rc;
+    if (known) {
+      *path = known->path;
       if (*path == PATH_TC && !tc_ok) *path = PATH_MMA;
       return 0;
     }
@@ -1866,16 +1876,16 @@ int gemm_set(Group* g, int cls, std::initializer_list<GemmArgs> products) {
   if (!tiles) return apart();
   if (mode == 5) return together();
   TuneKey k{device_tag(), v[0].rows, v[0].K, (int)cols, 1, kTuneTiles + all.oz_w, 16 + (int)v.size(), 0};
-  int known = -1;
+  int known = -1, rc = 0;
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune.find(k);
-    if (it != g_tune.end()) known = it->second.path;
+    const TuneEntry* e = nullptr;
+    if ((rc = tune_find_locked(k, &e))) return rc;
+    if (e) known = e->path;
   }
   if (known >= 0) return known == PATH_FMA ? together() : apart();
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   CK(cudaStreamIsCapturing(g->stream, &cs));
-  int rc = 0;
   if (cs != cudaStreamCaptureStatusNone || g->prof) return apart();
   void* flush = tune_flush_buffer();
   if (!flush) return fail(FALCON_ENOMEM, "contraction tuning: no device memory for the L2 flush buffer");
@@ -1914,9 +1924,11 @@ int tuned_merge(Group* g, int cls, const std::vector<GemmArgs>& v, const GemmArg
   TuneKey k{device_tag(), all.rows, all.K, all.N, all.batch, kTuneTiles + all.oz_w, 2 + (int)v.size(), 0};
   {
     std::lock_guard<std::mutex> lk(g_tune_mu);
-    auto it = g_tune.find(k);
-    if (it != g_tune.end()) {
-      *merged = it->second.path == PATH_TC;
+    const TuneEntry* e = nullptr;
+    const int rc = tune_find_locked(k, &e);
+    if (rc) return rc;
+    if (e) {
+      *merged = e->path == PATH_TC;
       return 0;
     }
   }
