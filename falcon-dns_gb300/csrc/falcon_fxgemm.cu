@@ -811,7 +811,7 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
     const dim3 grid((g.rows + RB - 1) / RB, nz);
     auto run = [&](auto kernel, int nc) {
       const size_t smem = (size_t)nc * ((size_t)KS * RB * sizeof(Wide) + g.K * sizeof(double));
-      if (smem > 46 * 1024) {
+      if (smem > 45 * 1024) {  // (2.1 KB of static arrays beside it)
         const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
         if (e != cudaSuccess) return e;
       }
