@@ -35,8 +35,8 @@
 // Bound: latency for the narrow forms (the radial and per-mode products of a
 // few instances), the integer multiply-add pipe for the tiles.  FP64 FMA -> this, us
 // with L2 cold: 97 x 97, 342 modes, 2 columns 22 -> 18, 1026 modes, 6 columns 180 ->
-// 57; 33 x 33, 43 modes, 2 columns 10.6 -> 8.5; 65 x 65, 688 columns 14 -> 12, 43776
-// columns 317 -> 122 (84 on tcgen05, which the autotuner takes there); 129 x 129,
+// 53; 33 x 33, 43 modes, 2 columns 12 -> 8; 65 x 65, 688 columns 15 -> 12, 43776
+// columns 317 -> 123 (84 on tcgen05, which the autotuner takes there); 129 x 129,
 // 11040 columns 324 -> 127.  (With 58 and 59 bits and carries every 16 k the large
 // ones took 114 and 120; with carries every 4 k 126 and 129.)
 //
@@ -395,13 +395,14 @@ __global__ void __launch_bounds__(512) fx_tile_kernel(const __grid_constant__ Ge
 
 // Narrow form (N <= 8 columns per batch entry): a block takes RB rows and all
 // columns of an entry, thread (row, part) one of KS shares of k; the operator
-// is read once, straight to registers, the next 8 k (and the first ones, before
+// is read once, straight to registers, the next 7 k (and the first ones, before
 // the X panel is converted) in flight while these are multiplied; the shares'
 // sums meet in shared memory, where the threads of a row take its column pairs.
 // Bound by latency for one small run, then by issue.  With 32 rows and eight
 // shares in every block two thirds of the instructions were for converting X
-// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 57 us, 291 x 97 x 6 256 ->
-// 123, 291 x 97 x 2, 341 entries 40 -> 30, 195 x 65 x 8, 170 entries 32 -> 29.
+// and adding shares: 97 x 97 x 6, 1026 entries 114 -> 53 us, 291 x 97 x 6 256 ->
+// 117, 291 x 97 x 2, 341 entries 40 -> 30, 195 x 65 x 8, 170 entries 32 -> 28.  (With
+// 8 k in flight, carried every 4: 57, 124, 31 and 30.)
 template <int NC>
 __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ GemmArgs g, int RB, int KS) {
   extern __shared__ __align__(16) double fsm[];
@@ -409,7 +410,7 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
   double* xd = reinterpret_cast<double*>(parts + KS * NC * RB);     // [K][NC]
   __shared__ int cex[NC];
   __shared__ int part[256], ws[257];
-  constexpr int U = 8;
+  constexpr int U = kCarry;
   const int z = blockIdx.y, tid = threadIdx.x, nthr = blockDim.x;
   const int kp = tid / RB, rl = tid - kp * RB, row = blockIdx.x * RB + rl;
   const int kq = (g.K + KS - 1) / KS, kb = min(kp * kq, g.K), ke = min(kb + kq, g.K);
@@ -465,10 +466,6 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
         add_product(acc[c], av[u], make_int2(x.x, x.y));
         add_product(acc[c + 1], av[u], make_int2(x.z, x.w));
       }
-      if (u == 3) {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) carry(acc[c]);
-      }
     }
 #pragma unroll
     for (int c = 0; c < NC; ++c) carry(acc[c]);
@@ -509,11 +506,12 @@ __global__ void __launch_bounds__(256) fx_narrow_kernel(const __grid_constant__ 
 //   else X0, X1 = x_{2p}, x_{2p+1};  out_j = S0 + S1, out_{n-1-j} = +-(S0 - S1) + D
 // A block takes NCOL real columns (re and im side by side) of one operator, and
 // all its output pairs or, with few columns, a share of them (grid z: not in
-// place); loads, outputs (through shared memory) and the operator's chunks of 8 p are
+// place); loads, outputs (through shared memory) and the operator's chunks of 7 p are
 // coalesced.  Bound: the integer multiply-adds (61 % of that pipe's cycles, 16
-// to 20 warps an SM); 65 points, 10944 columns: fwd 62 us, d1 and d2 103 us
-// (one FP64 dot product a thread: 684 us for the three).
-constexpr int kFxPC = 8;  // p per staged operator chunk (g.pc: this, or all of them in one)
+// to 20 warps an SM); 65 points, 10944 columns: fwd 56 us, d1 and d2 102 us
+// (one FP64 dot product a thread: 684 us for the three; chunks of 8, carried every
+// 4: 62 and 103).
+constexpr int kFxPC = kCarry;  // p per staged operator chunk (g.pc: this, or all of them in one)
 template <int RPT, int NCOL, bool FWD>
 __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__ FxColumns g) {
   constexpr int RG = 64 / NCOL, CP = NCOL / 2, ST = NCOL + 2;  // ST: columns' stores hit every bank
@@ -612,10 +610,10 @@ __global__ void __launch_bounds__(512) fx_columns_kernel(const __grid_constant__
         }
       }
     };
-    for (int p4 = 0; p4 < pc; p4 += 4) {
-      const int pe = min(p4 + 4, pc);
+    for (int p7 = 0; p7 < pc; p7 += kCarry) {
+      const int pe = min(p7 + kCarry, pc);
 #pragma unroll 2
-      for (int pp = p4; pp < pe; ++pp) one(pp);
+      for (int pp = p7; pp < pe; ++pp) one(pp);
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         carry(s0[i][0]); carry(s0[i][1]);
@@ -801,8 +799,8 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
   if (g.N <= 8 && !g.njobs) {
     // k shares until there are 448 threads an SM (above that one, a warp at least), rows
     // in even blocks of at most 256 threads, of fewer while SMs are without two
-    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 12.0, 10.9, 8.9, 7.9; 65 x 65 x 8,
-    // 171 entries 26.3, 20.1, 16.0, 20.1; 291 x 97 x 2, 341 entries 30.3, 32.4, 37.5, 47.4)
+    // (us at 1, 2, 4, 8 shares: 33 x 33 x 2, 43 entries 13.0, 11.9, 9.9, 8.5; 65 x 65 x 8,
+    // 171 entries 26.3, 20.8, 16.0, 21.1; 291 x 97 x 2, 341 entries 30.4, 33.1, 38.5, 47.7)
     const int nz = entries(g), nsm = sm_count();
     const int KS = (int)std::min(8L, std::max((31L + g.rows) / g.rows, nsm * 448L / ((long)g.rows * nz)));
     int nb = (g.rows + 256 / KS - 1) / (256 / KS);
@@ -832,14 +830,14 @@ cudaError_t launch_fx_gemm(const GemmArgs& g, cudaStream_t s) {
 // Shape: NCOL real columns a block, RPT output pairs a thread (64 / NCOL x RPT
 // pairs a warp).  Few columns: small blocks and one pair a thread, for more
 // blocks and shorter chains (65 points, us of fwd / d1d2 at <1, 8>, <1, 16>, <3, 16>:
-// 300 columns 10.4/10.5, 12.6/12.5, 18.6/16.6; 1000 columns 12.5/18.6, 12.7/18.6,
-// 18.7/20.6; 10944 columns 66/115, 74/119, 62/103; 17 points, 700 columns, fwd 6.3,
-// 6.4 and, at <1, 32>, 8.3), and while SMs are idle the pairs of a column on several
-// of them (fwd of 257 points, 4 columns 52 -> 23, 129 points 21 -> 14.5).  Many: one
-// pair a thread up to 32 pairs (17 points, 20000 columns <1, 16> 21/35, <1, 32>
-// 21/31, <3, 16> 35/53), above that the shape that pads least (97 points, 10000
-// columns <2, 16> 122/216, <3, 16> 142/225; 129 points, 2000 columns <3, 32> 45/76,
-// <3, 16> 52/86; 193 points, 3000 columns <3, 32> 215/315, <3, 16> 176/254).
+// 300 columns 10.4/10.4, 12.5/12.4, 16.5/16.5; 1000 columns 12.4/18.5, 12.5/18.5,
+// 16.5/20.6; 10944 columns 64/111, 64/113, 57/102; 17 points, 700 columns, fwd 6.3,
+// 6.3 and, at <1, 32>, 8.3), and while SMs are idle the pairs of a column on several
+// of them (fwd of 257 points, 4 columns 53 -> 23, 129 points 20 -> 14.4).  Many: one
+// pair a thread up to 32 pairs (17 points, 20000 columns <1, 16> 21/33, <1, 32>
+// 19/31, <3, 16> 31/52), above that the shape that pads least (97 points, 10000
+// columns <2, 16> 115/197, <3, 16> 133/236; 129 points, 2000 columns <3, 32> 41/78,
+// <3, 16> 49/88; 193 points, 3000 columns <3, 32> 195/320, <3, 16> 161/258).
 cudaError_t launch_fx_columns(const FxColumns& g, cudaStream_t s) {
   if (g.n < 3 || g.n > 257 || g.ncol < 1 || g.ncol > 65535) return cudaErrorInvalidValue;
   const int h = (g.n + 1) / 2;
