@@ -4470,11 +4470,12 @@ int cheb_mats(int n, ChebMats** out) {
 
 // Operator `first` to out[0] and, with count 2, `first` + 1 to out[1].
 // Dense FP64 products for the smallest sizes, where a thread's few multiply-adds
-// end before the fixed-point form's conversions and barriers do (us, FP64 / fixed
-// point: 3 points, 16 columns 4.0 / 5.2, 5000 columns 6.2 / 6.4; 9 points, 43
-// columns 4.3 / 6.2, 1500 columns 6.2 / 6.4, 2500 8.4 / 6.4; 13 points, 64 columns
-// 4.3 / 6.2, 1500 6.3 / 6.4; 17 points, 16 columns 6.2 / 6.2).  In place only the
-// fixed-point form is safe.
+// end before the fixed-point form's conversions and barriers do (us of fwd / d1d2,
+// FP64 and fixed point: 3 points, 1000 columns 4.2/4.2, 6.3/6.3, 6666 7.2/10.4, 8.3/8.3;
+// 5 points, 1500 columns 4.2/6.3, 6.3/6.3, 2000 6.2/8.1, 6.3/6.3; 9 points, 400 columns
+// 4.3/4.2, 6.2/6.3, 1200 5.2/6.3, 6.3/6.3, 1500 6.3/8.3, 6.3/6.3; 13 points, 64 columns
+// 4.2/4.2, 6.3/6.3, 800 5.8/6.3, 6.3/6.3, 1000 6.3/8.1, 6.3/6.3; 17 points, 16 columns
+// 6.2/6.2, 6.3/6.3).  In place only the fixed-point form is safe.
 int cheb_apply(int first, int count, int nr, int ncol, const double* in, double* const* out, void* stream) {
   if (nr < 3 || ncol < 1 || !in || !out[0]) return fail(FALCON_EINVAL, "invalid Chebyshev transform arguments");
   ChebMats* m = nullptr;
@@ -4483,7 +4484,7 @@ int cheb_apply(int first, int count, int nr, int ncol, const double* in, double*
   const double2* x = reinterpret_cast<const double2*>(in);
   double2* y[2] = {reinterpret_cast<double2*>(out[0]), reinterpret_cast<double2*>(out[count - 1])};
   const long span = 2L * nr * ncol;
-  const bool few = nr <= 13 && (long)nr * ncol <= 20000;
+  const bool few = nr <= 13 && ncol <= 1700 && nr * ncol <= 10400;
   const bool apart = !spans_overlap(in, span, out[0], span) && !spans_overlap(in, span, out[count - 1], span);
   if (!m->fixed || (few && apart)) {
     CK(launch_apply_cols(nr, ncol, count, m->dense[first], m->dense[first + count - 1], x, y[0], y[1],

@@ -62,7 +62,8 @@ def test_a_constant_has_no_derivative(fg, n):
         assert np.isnan(got[3].real).all() and np.array_equal(got[4], want[4])
 
 
-@pytest.mark.parametrize("n,few", [(3, 6666), (9, 2222), (13, 1538), (14, 40), (33, 20), (129, 43), (257, 128)])
+@pytest.mark.parametrize("n,few", [(3, 1700), (3, 6666), (7, 1485), (9, 1155), (9, 2222), (13, 800),
+                                   (13, 1538), (14, 40), (33, 20), (129, 43), (257, 128)])
 def test_few_columns(fg, n, few):
     """Both sides of the rule that gives calls of up to 13 points to FP64 products,
     pairs shared out over blocks, and in place, which does neither:
