@@ -392,15 +392,17 @@ struct alignas(16) FxLine {
 // stage by what its growth can take, from the largest value of the stage
 // before.  The grid values are shifted up to 62 bits (by the largest of each
 // field) before they are multiplied.  Every sum is exact; errors are those
-// of the products with constants (half a unit rms each).  All the maxima behind
+// of the truncation going in, the products with constants (half a unit rms each)
+// and the grid products' low x low terms (a quarter unit).  All the maxima behind
 // the scales are integers, so results do not depend on S.  A line with an
 // Inf or NaN input gives NaN.
 //
 // Bound: issue of integer instructions (about half of the cycles) and their
 // latency at the 16 warps an SM that registers and shared memory allow.
 // Against FP64 butterflies on grids of 3 Nm points (radix 11 to 31 on the
-// tensor cores), us for Nr = 65, Nm = 170, 128 instances: 950 -> 200; Nr =
-// 129, Nm = 512, 8: 500 -> 125; one instance of Nr = 97, Nm = 341: 80 -> 30.
+// tensor cores), us of the kernel for Nr = 65, Nm = 170, 128 instances: 1085 -> 222;
+// of a call for Nr = 129, Nm = 512, 8: 751 -> 153; one instance of Nr = 33, Nm = 341:
+// 95 -> 23.
 // The error against 64 bits fell from 7e-16 to 4e-16 (products with omega)
 // and from 7e-14 to 4e-16 (with T, which FP64 packed with a larger omega).
 // ---------------------------------------------------------------------------
